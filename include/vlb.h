@@ -319,7 +319,8 @@ vlb_status vlb_bake_ex(vlb_ctx* ctx, const vlb_scene* scene, const float* probe_
 vlb_status vlb_bake_async(vlb_ctx* ctx, const vlb_scene* scene, const float* probe_xyz, uint32_t nprobes,
                           const vlb_bake_params* params, float* out, void* done_event);
 /* Measurement aid (no reference counterpart; the reference's traversal is
- * inside the driver): one instrumented bake of the same rays, counting
+ * inside the driver): one instrumented bake of the same rays, every walk from
+ * the tree's root (a bake may start its walks further down), counting
  * out[0] primary rays, out[1] shadow rays, out[2] BVH node fetches (one per
  * 32-ray packet visit, or per lane in the lane walks), out[3] triangle
  * fetches (48 B each), out[4] node tests summed over rays, out[5] the bytes

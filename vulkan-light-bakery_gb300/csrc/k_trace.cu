@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace_dyn(const TraceArgs 
   const uint32_t P = (a.nprobes + 31) / 32 * 32;
   const uint32_t R = P * a.S;
   Work w;
-  int stack[kLaneStack];
+  int stack[kLaneStackFront];
   LaneRay L;
   make_ray(L.ray, 0.f, 0.f, 0.f, 1.f, 1.f, 1.f);
   bool exhausted = false;
@@ -283,13 +283,16 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace_dyn(const TraceArgs 
         const uint32_t sl = r / a.S, t = r - sl * a.S;
         if (sl < a.nprobes) lr_start(a, L, a.order[sl], __ldg(a.dir_order + t));
       }
+      if constexpr (!WIDE) {
+        if (a.front) lr_front(a, L, L.has, stack);
+      }
     }
     if (!__any_sync(kFull, L.has)) {
       if (exhausted) break;
       continue;
     }
     // node phase (all lanes take part in the votes)
-    lr_node_phase<COUNT, TraceArgs, WIDE>(a, L, stack, w, kNodeSteps);
+    lr_node_steps<COUNT, TraceArgs, WIDE>(a, L, stack, w, kNodeSteps);
     lr_park(L, stack);
     if (!L.has) continue;
     // leaf phase
@@ -796,11 +799,7 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_trace_batch(const BakeJobD
         if (r0 >= r1) break;
         continue;
       }
-      // one while-while turn, as in k_trace_dyn (the octant-specialised node
-      // phase measured 4 % slower here, also when only jobs of 1024
-      // directions take it: its eight copies cost this kernel more than they
-      // save)
-      lr_node_steps<false, BakeJobDev, false, true, -1>(j, L, stack, w, kNodeSteps);
+      lr_node_steps<false, BakeJobDev>(j, L, stack, w, kNodeSteps);  // one while-while turn, as in k_trace_dyn
       lr_park(L, stack);
       if (!L.has) continue;
       if (L.leaf >= 0) lr_leaf<false>(j, L, w);

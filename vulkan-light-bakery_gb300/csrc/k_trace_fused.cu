@@ -262,8 +262,7 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace_fused(const BakeJ
     if (__any_sync(kFull, L.has)) {
       const BakeJobDev& J = job_of<MULTI>(jobs, one, fw.q[lslot >> 8].job);
       // one while-while turn (as k_trace_dyn): node phase, then leaf phase
-      // (the octant-specialised node phase gained nothing here)
-      lr_node_steps<false, BakeJobDev, false, !MULTI, -1>(J, L, stack, w, node_steps);
+      lr_node_steps<false, BakeJobDev, false, !MULTI>(J, L, stack, w, node_steps);
       lr_park(L, stack);
       if (L.has) {
         if (L.leaf >= 0) lr_leaf<false>(J, L, w);

@@ -512,6 +512,84 @@ __device__ __forceinline__ void lr_start(const A& a, LaneRay& L, uint32_t p, uin
   }
 }
 
+// Entries a lane's stack may hold.
+__device__ __forceinline__ int stack_limit(const TraceArgs& a) { return int(a.stack_lim); }
+__device__ __forceinline__ int stack_limit(const BakeJobDev&) { return kLaneStack; }
+
+// Order-preserving map of a float to an unsigned integer (NaN-free input).
+__device__ __forceinline__ uint32_t ordered_u32(float f) {
+  const uint32_t u = __float_as_uint(f);
+  return u ^ (uint32_t(int32_t(u) >> 31) | 0x80000000u);
+}
+__device__ __forceinline__ float ordered_f32(uint32_t k) {
+  return __uint_as_float(k ^ (uint32_t(int32_t(~k) >> 31) | 0x80000000u));
+}
+
+// Starts the primary walks of the lanes that just took a ray (`mine`) from
+// their probe's frontier (k_front.cu).  The lanes' rays share an origin, so
+// relative to it a plane at x is crossed at x / d.  First each lane tests one
+// entry against the whole group: the entry's crossings under the group's range
+// of 1/d per axis (an axis whose directions change sign does not constrain).
+// Then, farthest first, every lane tests its own ray against the entries left
+// and stacks those it hits; the walk goes on from the nearest.  All 32 lanes
+// take part; a group that straddles two probes goes probe by probe.
+template <class A>
+__device__ __forceinline__ void lr_front(const A& a, LaneRay& L, bool mine, int* stack) {
+  const uint32_t lane = threadIdx.x & 31;
+  unsigned pending = __ballot_sync(kFull, mine);
+  while (pending) {
+    const uint32_t q = __shfl_sync(kFull, L.p, __ffs(pending) - 1);
+    const bool now = mine && L.p == q;
+    const float4* f = a.front + size_t(q) * (2 * a.front_cap);
+    const int n = int(__ldg(a.front_n + q));
+    const float lim = prune_limit(L.tb);
+    float imin[3], imax[3];
+    const float iv[3] = {L.ray.ixy.x, L.ray.ixy.y, L.ray.izz.x};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const uint32_t k = ordered_u32(iv[c]);
+      imin[c] = ordered_f32(__reduce_min_sync(kFull, now ? k : 0xffffffffu));
+      imax[c] = ordered_f32(__reduce_max_sync(kFull, now ? k : 0u));
+    }
+    const float far = __uint_as_float(__reduce_max_sync(kFull, now ? __float_as_uint(lim) : 0u));
+    for (int w = (n - 1) & ~31; w >= 0; w -= 32) {
+      bool in = false;
+      if (w + int(lane) < n) {
+        const float4 x = __ldg(f + 2 * (w + lane)), y = __ldg(f + 2 * (w + lane) + 1);
+        const float lo[3] = {x.x, x.y, y.x}, hi[3] = {x.z, x.w, y.y};
+        float tn = 0.f, tf = far;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const bool neg = imin[c] < 0.f;
+          const float e = neg ? hi[c] : lo[c], g = neg ? lo[c] : hi[c];  // entry and exit planes
+          if (!(neg && imax[c] > 0.f)) {
+            tn = fmaxf(tn, fminf(e * imin[c], e * imax[c]));
+            tf = fminf(tf, fmaxf(g * imin[c], g * imax[c]));
+          }
+        }
+        in = tn <= tf;
+      }
+      unsigned hits = __ballot_sync(kFull, in);
+      while (hits) {
+        const int i = 31 - __clz(hits);
+        hits ^= 1u << i;
+        float lx, ly, hx, hy, lz, hz, rf, d2;
+        asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=f"(lx), "=f"(ly), "=f"(hx), "=f"(hy), "=f"(lz), "=f"(hz), "=f"(rf), "=f"(d2)
+            : "l"(f + 2 * (w + i)));
+        const float2 zero = make_float2(0.f, 0.f);
+        const float2 l = fma_pair(lx, ly, L.ray.ixy, zero), u = fma_pair(hx, hy, L.ray.ixy, zero);
+        const float2 z = fma_pair(lz, hz, L.ray.izz, zero);
+        const float tn = fmax3(fminf(l.x, u.x), fminf(l.y, u.y), fmaxf(fminf(z.x, z.y), a.tmin));
+        const float tf = fmin3(fmaxf(l.x, u.x), fmaxf(l.y, u.y), fminf(fmaxf(z.x, z.y), lim));
+        if (now && tn <= tf) stack[L.sp++] = __float_as_int(rf);
+      }
+    }
+    if (now) L.cur = L.sp ? stack[--L.sp] : kWalkEnd;
+    pending &= ~__ballot_sync(kFull, now);
+  }
+}
+
 // The reference baker's sample encoding: the sRGB curve of
 // shaders/env_map.rchit:27-34 (the same in main.rmiss:9-16), then the 8-bit
 // UNORM store of its R8G8B8A8 env map (round to nearest, clamped to [0, 1]).
@@ -603,10 +681,10 @@ __device__ __forceinline__ bool lr_finish(const A& a, LaneRay& L, Shaded& o, Wor
     const float ndl = nx * a.sun.x + ny * a.sun.y + nz * a.sun.z;
     if (!(ndl > 0.f)) return true;
     if constexpr (COUNT) ++w.shadow;
-    make_ray_inv(L.ray, fmaf(L.tb, L.d.x, L.ox) + a.bias * nx, fmaf(L.tb, L.d.y, L.oy) + a.bias * ny,
-                 fmaf(L.tb, L.d.z, L.oz) + a.bias * nz, a.sun.x, a.sun.y, a.sun.z, a.sun_inv.x, a.sun_inv.y,
-                 a.sun_inv.z);
+    const float hx = fmaf(L.tb, L.d.x, L.ox) + a.bias * nx, hy = fmaf(L.tb, L.d.y, L.oy) + a.bias * ny,
+                hz = fmaf(L.tb, L.d.z, L.oz) + a.bias * nz;
     L.lit = a.sun_scale * ndl;
+    make_ray_inv(L.ray, hx, hy, hz, a.sun.x, a.sun.y, a.sun.z, a.sun_inv.x, a.sun_inv.y, a.sun_inv.z);
     L.shadow = true;
     L.cur = walk_root(a.ntris);
     L.sp = 0;
@@ -719,44 +797,13 @@ __device__ __forceinline__ void lr_node_wide(const A& a, LaneRay& L, int* stack,
   L.cur = next != kWalkEnd ? next : (L.sp ? stack[--L.sp] : kWalkEnd);
 }
 
-// slab_pair_rt for a ray in octant OCT (bit a set: 1/d_a < 0): each axis's
-// entry and exit planes are known, so the per-axis min/max goes.  The same
-// bits as slab_pair_rt: a plane crossing fma(p, inv, -o * inv) is monotone in
-// p, so the entry plane's crossing is the minimum of the two.  (A crossing is
-// NaN only when p * inv and o * inv both overflow -- a direction component
-// below 1e-30, so inv = +-1e30, with coordinates beyond 3.4e8 -- and there
-// the two forms may differ, as the packet walk's compile-time octant may.)
-template <int OCT>
-__device__ __forceinline__ void slab_pair_oct(const RayCtx& r, const float4 q0, const float4 q1, const float4 q2,
-                                              float tmin, float tmax, bool& h0, bool& h1, float& tn0, float& tn1) {
-  constexpr bool fx = OCT & 1, fy = OCT & 2, fz = OCT & 4;
-  const float2 l0 = fma_pair(q0.x, q0.y, r.ixy, r.nxy), u0 = fma_pair(q0.z, q0.w, r.ixy, r.nxy);
-  const float2 l1 = fma_pair(q1.x, q1.y, r.ixy, r.nxy), u1 = fma_pair(q1.z, q1.w, r.ixy, r.nxy);
-  const float2 z0 = fma_pair(q2.x, q2.y, r.izz, r.nzz), z1 = fma_pair(q2.z, q2.w, r.izz, r.nzz);
-  tn0 = fmax3(fx ? u0.x : l0.x, fy ? u0.y : l0.y, fmaxf(fz ? z0.y : z0.x, tmin));
-  tn1 = fmax3(fx ? u1.x : l1.x, fy ? u1.y : l1.y, fmaxf(fz ? z1.y : z1.x, tmin));
-  h0 = tn0 <= fmin3(fx ? l0.x : u0.x, fy ? l0.y : u0.y, fminf(fz ? z0.x : z0.y, tmax));
-  h1 = tn1 <= fmin3(fx ? l1.x : u1.x, fy ? l1.y : u1.y, fminf(fz ? z1.x : z1.y, tmax));
-}
-
-// The octant every lane with a ray shares (-1 if they differ).  A lane's ray
-// changes only between node phases, so one vote serves a whole phase.
-__device__ __forceinline__ int lr_warp_octant(const LaneRay& L) {
-  const int o = (L.ray.ixy.x < 0.f ? 1 : 0) | (L.ray.ixy.y < 0.f ? 2 : 0) | (L.ray.izz.x < 0.f ? 4 : 0);
-  const unsigned has = __ballot_sync(kFull, L.has);
-  if (!has) return -1;
-  const int first = __shfl_sync(kFull, o, __ffs(has) - 1);
-  return __all_sync(kFull, !L.has || o == first) ? first : -1;
-}
-
 // One inner node: nearer hit child next, the farther one on the stack.  WIDE:
 // the node is a node of the 8-wide tree (kernels built for it walk it when
 // the scene has one; the others walk the binary tree, with the same results).
 // PACKED: the box tests' plane crossings by packed FMAs (slab_pair_rt), else
 // by scalar ones (slab_rt; the same bits, for kernels whose registers do not
-// leave room for the pairs).  OCT >= 0: the lane's ray is in that octant
-// (slab_pair_oct).
-template <bool COUNT, class A, bool WIDE = false, bool PACKED = true, int OCT = -1>
+// leave room for the pairs).
+template <bool COUNT, class A, bool WIDE = false, bool PACKED = true>
 __device__ __forceinline__ void lr_node(const A& a, LaneRay& L, int* stack, Work& w) {
   if constexpr (WIDE) {
     lr_node_wide<COUNT>(a, L, stack, w);
@@ -769,9 +816,7 @@ __device__ __forceinline__ void lr_node(const A& a, LaneRay& L, int* stack, Work
   ldg_node(a.nodes + 4 * L.cur, n0, n1, n2, n3);
   float tn0, tn1;
   bool h0, h1;
-  if constexpr (OCT >= 0) {
-    slab_pair_oct<OCT>(L.ray, n0, n1, n2, tlo, prune_limit(L.tb), h0, h1, tn0, tn1);
-  } else if constexpr (PACKED) {
+  if constexpr (PACKED) {
     slab_pair_rt(L.ray, n0, n1, n2, tlo, prune_limit(L.tb), h0, h1, tn0, tn1);
   } else {
     const float lim = prune_limit(L.tb);
@@ -781,7 +826,7 @@ __device__ __forceinline__ void lr_node(const A& a, LaneRay& L, int* stack, Work
   const int c0 = __float_as_int(n3.x), c1 = __float_as_int(n3.y);
   if (h0 && h1) {
     const bool first0 = tn0 <= tn1;
-    if (L.sp < kLaneStack) stack[L.sp++] = first0 ? c1 : c0;
+    if (L.sp < stack_limit(a)) stack[L.sp++] = first0 ? c1 : c0;
     else atomicAdd(a.err + kErrStackOverflow, 1);
     L.cur = first0 ? c0 : c1;
   } else if (h0) {
@@ -812,40 +857,19 @@ __device__ __forceinline__ void lr_leaf(const A& a, LaneRay& L, Work& w) {
 }
 
 // Up to `steps` node steps of the warp's lanes (every lane takes part in the
-// votes); OCT: the octant all the warp's rays share, or -1.
-template <bool COUNT, class A, bool WIDE, bool PACKED, int OCT>
+// votes).  One copy for all rays: eight more, each specialised to an octant
+// the warp's rays share, saved 2.7 % while a ray walked from the root, but
+// with the walks started at the probe frontiers they cost more in
+// instruction-cache misses (3141 x 1000 directions per probe: 57.5 ms with
+// them, 47.0 ms without; 262,144 probes x 1024 directions: no difference).
+template <bool COUNT, class A, bool WIDE = false, bool PACKED = true>
 __device__ __forceinline__ void lr_node_steps(const A& a, LaneRay& L, int* stack, Work& w, uint32_t steps) {
 #pragma unroll 1
   for (uint32_t k = 0; k < steps; ++k) {
     lr_park(L, stack);
     const bool at_node = L.has && L.cur >= 0;
     if (!__any_sync(kFull, at_node && L.leaf < 0)) break;
-    if (at_node) lr_node<COUNT, A, WIDE, PACKED, OCT>(a, L, stack, w);
-  }
-}
-
-// A turn's node phase, specialised to the warp's octant when all its rays
-// share one (the binary tree's packed walk; the others take the generic one).
-// Measured on the single-bake tile walk: 129.3 -> 125.7 ms on the bake of
-// 64^3 probes x 1024 directions in the 4096-box scene; the multi-job walks
-// measured 4 % slower with it (also when only jobs of 1024 directions took
-// it) and keep the generic phase.
-template <bool COUNT, class A, bool WIDE = false, bool PACKED = true>
-__device__ __forceinline__ void lr_node_phase(const A& a, LaneRay& L, int* stack, Work& w, uint32_t steps) {
-  if constexpr (WIDE || !PACKED) {
-    lr_node_steps<COUNT, A, WIDE, PACKED, -1>(a, L, stack, w, steps);
-  } else {
-    switch (lr_warp_octant(L)) {
-      case 0: lr_node_steps<COUNT, A, false, true, 0>(a, L, stack, w, steps); break;
-      case 1: lr_node_steps<COUNT, A, false, true, 1>(a, L, stack, w, steps); break;
-      case 2: lr_node_steps<COUNT, A, false, true, 2>(a, L, stack, w, steps); break;
-      case 3: lr_node_steps<COUNT, A, false, true, 3>(a, L, stack, w, steps); break;
-      case 4: lr_node_steps<COUNT, A, false, true, 4>(a, L, stack, w, steps); break;
-      case 5: lr_node_steps<COUNT, A, false, true, 5>(a, L, stack, w, steps); break;
-      case 6: lr_node_steps<COUNT, A, false, true, 6>(a, L, stack, w, steps); break;
-      case 7: lr_node_steps<COUNT, A, false, true, 7>(a, L, stack, w, steps); break;
-      default: lr_node_steps<COUNT, A, false, true, -1>(a, L, stack, w, steps); break;
-    }
+    if (at_node) lr_node<COUNT, A, WIDE, PACKED>(a, L, stack, w);
   }
 }
 

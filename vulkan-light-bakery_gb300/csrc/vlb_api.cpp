@@ -1026,6 +1026,24 @@ static bool grid_mode(const vlb_scene* scene, uint32_t nprobes, uint32_t S, cons
          p->shading == VLB_SHADE_LAMBERT_SUN;  // the grids hold the sun's parallel shadow rays
 }
 
+// Entries per probe of a bake's probe frontiers (k_front.cu), 0 for walks from
+// the root.  A frontier costs a warp some twenty dependent loads per probe and
+// its rays share it: at 64 rays a probe that is a wash (64 probes: 94 us with
+// and without), at 256 it saves.  Trees deeper than the lane stack keep the
+// root (their walks may overflow the stack, and must say so).  1 GiB of
+// entries at most.
+static uint32_t front_cap(const vlb_scene* scene, uint64_t nprobes, uint32_t S) {
+  if (scene->ntris < 64 || scene->wnodes || scene->depth > uint32_t(vlbk::kLaneStack) || S < 128 || !nprobes) return 0;
+  const uint64_t cap = std::min<uint64_t>(vlbk::kFrontCap, (1ull << 25) / nprobes);
+  return cap < 32 ? 0 : uint32_t(cap);
+}
+
+static float bounds_scale(const vlb_scene* scene) {
+  float m = 0.f;
+  for (float b : scene->bounds) m = std::max(m, std::fabs(b));
+  return m;
+}
+
 // Checks the parameters of one bake; *sun_len gets |sun_dir| (FP64).
 static vlb_status check_params(vlb_ctx* ctx, const vlb_scene* scene, const vlb_bake_params* p, double* sun_len) {
   if (!scene || !p || !p->dirs) return fail(ctx, VLB_ERR_INVALID, "scene, params and params->dirs are required");
@@ -1049,7 +1067,7 @@ static vlb_status check_params(vlb_ctx* ctx, const vlb_scene* scene, const vlb_b
 }
 
 static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const float* probe_xyz, uint32_t nprobes,
-                                const vlb_bake_params* p, vlbk::TraceArgs* out) {
+                                const vlb_bake_params* p, vlbk::TraceArgs* out, bool from_root = false) {
   double sl = 0.0;
   vlb_status st = check_params(ctx, scene, p, &sl);
   if (st) return st;
@@ -1087,7 +1105,23 @@ static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const floa
   a.lane = lane_mode(scene, nprobes, p->flags, p->shading);
   a.shading = p->shading;
   a.light = make_float3(p->light_pos[0], p->light_pos[1], p->light_pos[2]);
-  if (grid_mode(scene, nprobes, a.S, p)) {
+  a.stack_lim = vlbk::kLaneStack;
+  const bool grid = grid_mode(scene, nprobes, a.S, p);
+  const bool tile_walk = a.lane && !grid && p->precision != VLB_PREC_FUSED;
+  const uint32_t cap = tile_walk && !from_root ? front_cap(scene, nprobes, a.S) : 0;
+  void *ent, *cnt;
+  if (cap && scratch(ctx, "front_ent", size_t(nprobes) * cap * 32, &ent) == VLB_OK &&
+      scratch(ctx, "front_cnt", size_t(nprobes) * 4, &cnt) == VLB_OK) {
+    const vlbk::FrontArgs f{scene->nodes, scene->ntris, a.probes, nprobes, bounds_scale(scene), cap,
+                            static_cast<float4*>(ent), static_cast<uint32_t*>(cnt), ctx->d_err};
+    KScope k(ctx, "probe_front");
+    vlbk::launch_probe_front(f, ctx->stream);
+    a.front = f.ent;
+    a.front_n = f.cnt;
+    a.front_cap = cap;
+    a.stack_lim = vlbk::kLaneStackFront;
+  }
+  if (grid) {
     const uint32_t G = grid_cells_per_side(scene->ntris), T = scene->ntris;
     const size_t n = size_t(a.S) + 1;
     void *hdr, *cells, *ent, *box, *dep;
@@ -1284,7 +1318,7 @@ vlb_status vlb_bake_trace_stats(vlb_ctx* ctx, const vlb_scene* scene, const floa
   cudaSetDevice(ctx->device);
   if (!out || nprobes == 0) return fail(ctx, VLB_ERR_INVALID, "no probes or no output");
   vlbk::TraceArgs a;
-  vlb_status st = prepare_trace(ctx, scene, probe_xyz, nprobes, p, &a);
+  vlb_status st = prepare_trace(ctx, scene, probe_xyz, nprobes, p, &a, true);
   if (st) return st;
   void *tile, *cnt;
   if ((st = scratch(ctx, "bake_tile", size_t(nprobes) * a.S * 12, &tile)) ||

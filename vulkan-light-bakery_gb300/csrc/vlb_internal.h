@@ -47,6 +47,9 @@ __device__ __forceinline__ bool inb_checked(long long i, long long n, int* err) 
 // the per-lane stacks of the lane walks (a wide node pushes up to 7 children).
 constexpr int kTraceStack = 64;
 constexpr int kLaneStack = 96;
+// With probe frontiers a walk starts with up to kFrontCap entries on its
+// stack; only trees at most kLaneStack deep use them, so it cannot overflow.
+constexpr int kLaneStackFront = kLaneStack + 128;
 
 // ---- binary traversal node (64 bytes) -------------------------------------------
 // The two children's boxes (lo xyz, hi xyz) grouped by axis, so that one
@@ -185,6 +188,23 @@ size_t probe_order_scratch_bytes(uint32_t n);
 int launch_probe_order(const float* probes, uint32_t n, const float bounds[6], uint32_t* order, void* scratch,
                        uint32_t* zero_word, cudaStream_t s);
 
+// ---- probe frontiers (k_front.cu) ------------------------------------------------
+// Entries per probe: 32 bytes each, [lx ly hx hy] [lz hz ref dist^2], the box
+// relative to the probe, nearest first; cnt[probe] of them.
+constexpr int kFrontCap = 128;
+struct FrontArgs {
+  const float4* nodes;
+  uint32_t ntris;
+  const float* probes;    // device nprobes*3
+  uint32_t nprobes;
+  float scale;            // largest coordinate of the scene's bounds
+  uint32_t cap;           // entries kept per probe, at most kFrontCap
+  float4* ent;            // [nprobes][cap][2]
+  uint32_t* cnt;          // [nprobes]
+  int* err;
+};
+void launch_probe_front(const FrontArgs& a, cudaStream_t s);
+
 // ---- trace + shade --------------------------------------------------------------
 struct TraceArgs {
   const float4* nodes;
@@ -227,6 +247,10 @@ struct TraceArgs {
   uint32_t dirs_per_warp;
   uint32_t chunks;        // direction chunks per packet
   uint32_t lane;          // 1: per-lane traversal, 0: packet traversal
+  const float4* front;    // probe frontiers (FrontArgs.ent) or null: the walks start at the root
+  const uint32_t* front_n;
+  uint32_t front_cap;
+  uint32_t stack_lim;     // entries a lane's stack may hold (kLaneStack, or kLaneStackFront with frontiers)
   uint32_t ray_block;     // tile lane walk: rays a warp takes from the counter at once (set by its launch)
   unsigned long long* counters;  // null, or [warp node fetches, warp triangle fetches, shadow rays, lane node tests]
   int* err;
@@ -461,6 +485,7 @@ struct vlb_scene {
   float4* nodes = nullptr;
   float4* wnodes = nullptr;  // 8-wide quantised traversal tree (wide_bvh.cpp), or null
   uint32_t nwide = 0;
+  uint32_t depth = 0;        // levels of inner nodes in the binary traversal tree
   float4* tris = nullptr;
   float4* albedo = nullptr;
   uint64_t bytes = 0;

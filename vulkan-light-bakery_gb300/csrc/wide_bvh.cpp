@@ -181,11 +181,13 @@ vlb_status vlbh::pair_siblings(vlb_ctx* ctx, vlb_scene* sc) {
   }
   std::vector<float4> out(nslots * 4, make_float4(0.f, 0.f, 0.f, 0.f));
   // (old index, new slot) of nodes whose children still need slots
-  std::vector<std::pair<int32_t, uint32_t>> stack{{0, 0}};
+  struct Todo { int32_t oi; uint32_t ns, level; };
+  std::vector<Todo> stack{{0, 0, 1}};
   uint32_t next = 2;
   while (!stack.empty()) {
-    const auto [oi, ns] = stack.back();
+    const auto [oi, ns, level] = stack.back();
     stack.pop_back();
+    sc->depth = std::max(sc->depth, level);
     float4 q[4];
     for (int k = 0; k < 4; ++k) q[k] = old[4 * size_t(oi) + k];
     int32_t c[2];
@@ -206,7 +208,7 @@ vlb_status vlbh::pair_siblings(vlb_ctx* ctx, vlb_scene* sc) {
       std::memcpy(&q[3].y, &nc[1], 4);
       // push the second child first so the first is laid out (and walked) first
       for (int h = 1; h >= 0; --h)
-        if (c[h] >= 0) stack.push_back({c[h], uint32_t(nc[h])});
+        if (c[h] >= 0) stack.push_back({c[h], uint32_t(nc[h]), level + 1});
     }
     for (int k = 0; k < 4; ++k) out[4 * size_t(ns) + k] = q[k];
   }
