@@ -1,0 +1,167 @@
+// k_lightmap.cu -- sun maps: shadow rays answered without a walk.
+//
+// All shadow rays of a bake run toward the sun, so they are parallel: seen
+// along the sun direction a ray is one point of a plane plus its origin's
+// depth.  This kernel rasterises the scene's triangles onto that plane and
+// keeps two depths (along the direction to the sun) per cell:
+//   cover  the largest depth below which every ray of the cell is occluded:
+//          some triangle covers the whole cell and lies above it everywhere;
+//   top    a depth above which no ray of the cell meets anything.
+// A shadow ray that starts below its cell's cover is occluded, one that
+// starts above top is lit, and only the rest walk the tree.  Both bounds are
+// conservative against the FP32 triangle test the walk would run: cells are
+// widened by `margin` (2^-17 of the scene's coordinate scale), a covering
+// triangle must contain the widened cell with room for the test's rounding
+// (grazing triangles, where that grows, do not cover), and top is raised by
+// the test's depth error, so every ray keeps the answer its walk gives.
+//
+// Thread k of a CTA sets up one triangle; the CTA's triangles' cells are then
+// numbered through and shared by all its threads (a binary search finds a
+// cell's triangle), so slivers and walls cost what their cells cost.  Several
+// CTAs (slices) share a group of triangles row by row: the walls of a room
+// fill the map and would otherwise be drawn by a single CTA.  A cell is read
+// before its atomic maximum: in deep scenes most triangles lie below one
+// already drawn.  Latency bound: 15 us for 778 triangles, 40 us for 164 k small
+// ones, 130 us for the 49 k faces of 4096 boxes.
+#include <algorithm>
+
+#include "vlb_device.cuh"
+#include "vlb_internal.h"
+
+namespace vlbk {
+namespace {
+
+constexpr int kMapThreads = 256;
+// Order-preserving map of a float to an unsigned integer; 0 is below every float.
+__device__ __forceinline__ uint32_t ordered(float f) {
+  const uint32_t u = __float_as_uint(f);
+  return u ^ (uint32_t(int32_t(u) >> 31) | 0x80000000u);
+}
+
+struct MapTri {
+  float ea[3], eb[3], ec[3];  // edge k: ea u + eb v + ec = distance inside it
+  float au, av, ac;           // depth = au u + av v + ac
+  float dmax, slack, pad;     // pad: how far inside its edges a ray must pass to be surely hit
+  int i0, i1, j0, j1, first;  // cells; the slice's first row
+  int covers;
+};
+
+__device__ __forceinline__ float dotm(float x, float y, float z, float3 a) {
+  return fmaf(z, a.z, fmaf(y, a.y, x * a.x));
+}
+
+__device__ __forceinline__ void map_setup(const SunMap& m, const float4 a, const float4 e1, const float4 e2,
+                                          MapTri& T) {
+  const float au = dotm(a.x, a.y, a.z, m.u), av = dotm(a.x, a.y, a.z, m.v), ad = dotm(a.x, a.y, a.z, m.s);
+  const float bu = dotm(e1.x, e1.y, e1.z, m.u), bv = dotm(e1.x, e1.y, e1.z, m.v), bd = dotm(e1.x, e1.y, e1.z, m.s);
+  const float cu = dotm(e2.x, e2.y, e2.z, m.u), cv = dotm(e2.x, e2.y, e2.z, m.v), cd = dotm(e2.x, e2.y, e2.z, m.s);
+  const float det = bu * cv - bv * cu;  // twice the projected area, signed
+  const float l1 = e1.x * e1.x + e1.y * e1.y + e1.z * e1.z, l2 = e2.x * e2.x + e2.y * e2.y + e2.z * e2.z;
+  // the triangle test's rounding grows with |e1| |e2| / |det|
+  const float grow = sqrtf(l1 * l2) / fabsf(det);
+  const bool steep = !(grow < 256.f);
+  T.slack = steep ? INFINITY : m.margin * (1.f + grow);
+  T.pad = T.slack;
+  T.covers = !steep;
+  T.dmax = ad + fmaxf(0.f, fmaxf(bd, cd)) + T.slack;
+  const float inv = steep ? 0.f : 1.f / det;
+  T.au = (bd * cv - cd * bv) * inv;
+  T.av = (cd * bu - bd * cu) * inv;
+  T.ac = ad - T.au * au - T.av * av;
+  const float sg = det < 0.f ? -1.f : 1.f;
+  const float pu[3] = {au, au + bu, au + cu}, pv[3] = {av, av + bv, av + cv};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int n = k == 2 ? 0 : k + 1;
+    const float du = pu[n] - pu[k], dv = pv[n] - pv[k];
+    const float rn = steep ? 0.f : sg * rsqrtf(fmaxf(du * du + dv * dv, 1e-30f));
+    T.ea[k] = -dv * rn;
+    T.eb[k] = du * rn;
+    T.ec[k] = -(T.ea[k] * pu[k] + T.eb[k] * pv[k]);
+  }
+  const float G1 = float(m.G - 1);
+  auto cell = [&](float x, float x0) { return int(fminf(fmaxf((x - x0) * m.inv, 0.f), G1)); };
+  T.i0 = cell(fminf(pu[0], fminf(pu[1], pu[2])) - m.margin, m.u0);
+  T.i1 = cell(fmaxf(pu[0], fmaxf(pu[1], pu[2])) + m.margin, m.u0);
+  T.j0 = cell(fminf(pv[0], fminf(pv[1], pv[2])) - m.margin, m.v0);
+  T.j1 = cell(fmaxf(pv[0], fmaxf(pv[1], pv[2])) + m.margin, m.v0);
+}
+
+__device__ __forceinline__ void map_cell(const SunMap& m, const MapTri& T, int i, int j) {
+  const float half = 0.5f * m.cell + m.margin;
+  const float cu = fmaf(float(i) + 0.5f, m.cell, m.u0), cv = fmaf(float(j) + 0.5f, m.cell, m.v0);
+  bool out = false, in = T.covers != 0;
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    const float d = fmaf(T.ea[e], cu, fmaf(T.eb[e], cv, T.ec[e]));
+    const float r = half * (fabsf(T.ea[e]) + fabsf(T.eb[e]));
+    out = out || d + r < -m.margin;
+    in = in && d - r > T.pad;
+  }
+  if (out) return;
+  const float zc = fmaf(T.au, cu, fmaf(T.av, cv, T.ac)), zr = half * (fabsf(T.au) + fabsf(T.av));
+  const float hi = T.covers ? fminf(T.dmax, zc + zr + T.slack) : T.dmax;
+  uint32_t* at = m.cells + 2 * (size_t(j) * m.G + i);
+  const uint2 now = __ldcg(reinterpret_cast<const uint2*>(at));
+  const uint32_t ht = ordered(hi);
+  if (now.y < ht) atomicMax(at + 1, ht);
+  if (in) {
+    const uint32_t hc = ordered(zc - zr - T.slack);
+    if (now.x < hc) atomicMax(at, hc);
+  }
+}
+
+// Slice y of a group of kMapThreads triangles: the rows of each that are
+// congruent to y modulo the slice count.
+__global__ void __launch_bounds__(kMapThreads) k_sun_map(const SunMap m, const float4* __restrict__ tris,
+                                                         uint32_t ntris) {
+  __shared__ MapTri st[kMapThreads];
+  __shared__ int s_end[kMapThreads];  // cells of triangles 0 .. k
+  __shared__ int s_warp[kMapThreads / 32];
+  const int tid = int(threadIdx.x), lane = tid & 31, warp = tid >> 5;
+  const int slices = int(gridDim.y), slice = int(blockIdx.y);
+  const uint32_t t = blockIdx.x * kMapThreads + threadIdx.x;
+  int n = 0;
+  if (t < ntris) {
+    MapTri& T = st[tid];
+    map_setup(m, __ldg(tris + 3 * size_t(t)), __ldg(tris + 3 * size_t(t) + 1), __ldg(tris + 3 * size_t(t) + 2), T);
+    int off = (slice - T.j0) % slices;
+    off += off < 0 ? slices : 0;
+    T.first = T.j0 + off;
+    n = T.first <= T.j1 ? ((T.j1 - T.first) / slices + 1) * (T.i1 - T.i0 + 1) : 0;
+  }
+  int end = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, end, o);
+    if (lane >= o) end += y;
+  }
+  if (lane == 31) s_warp[warp] = end;
+  __syncthreads();
+  for (int k = 0; k < warp; ++k) end += s_warp[k];
+  s_end[tid] = end;
+  __syncthreads();
+  const int total = s_end[kMapThreads - 1];
+#pragma unroll 2
+  for (int c = tid; c < total; c += kMapThreads) {
+    int k = 0;  // the first triangle whose end exceeds c
+#pragma unroll
+    for (int step = kMapThreads / 2; step > 0; step >>= 1)
+      if (s_end[k + step - 1] <= c) k += step;
+    const MapTri& T = st[k];
+    const int at = c - (k ? s_end[k - 1] : 0), w = T.i1 - T.i0 + 1, r = at / w;
+    map_cell(m, T, T.i0 + at - r * w, T.first + r * slices);
+  }
+}
+
+}  // namespace
+
+void launch_sun_map(const SunMap& m, const float4* tris, uint32_t ntris, cudaStream_t s) {
+  if (!ntris) return;
+  cudaMemsetAsync(m.cells, 0, size_t(m.G) * m.G * 8, s);
+  const uint32_t groups = (ntris + kMapThreads - 1) / kMapThreads;
+  const uint32_t slices = std::min(64u, std::max(2u, 1024u / groups));  // about seven CTAs per SM
+  k_sun_map<<<dim3(groups, slices), kMapThreads, 0, s>>>(m, tris, ntris);
+}
+
+}  // namespace vlbk

@@ -645,6 +645,20 @@ __device__ __forceinline__ bool lr_finish_ref_primary(const A& a, LaneRay& L, Sh
   return false;
 }
 
+// The sun map's answer for a shadow ray from (x, y, z): 0 occluded, 1 lit, 2
+// not known (walk).  A ray occluded at no more than `top` above its origin
+// must meet its occluder before tmax.
+__device__ __forceinline__ int sun_map_query(const SunMap& m, float x, float y, float z, float tmax) {
+  const float fu = (fmaf(z, m.u.z, fmaf(y, m.u.y, x * m.u.x)) - m.u0) * m.inv;
+  const float fv = (fmaf(z, m.v.z, fmaf(y, m.v.y, x * m.v.x)) - m.v0) * m.inv;
+  const float G = float(m.G);
+  if (!(fu >= 0.f && fu < G && fv >= 0.f && fv < G)) return 2;
+  const float d = fmaf(z, m.s.z, fmaf(y, m.s.y, x * m.s.x));
+  const uint2 c = __ldg(reinterpret_cast<const uint2*>(m.cells) + (uint32_t(fv) * m.G + uint32_t(fu)));
+  if (ordered_u32(d - m.margin) > c.y) return 1;
+  return ordered_u32(d + m.margin) < c.x && c.y < ordered_u32(d + 0.99f * tmax) ? 0 : 2;
+}
+
 // After a walk (REF: the reference's shading, vlb_shading
 // VLB_SHADE_REF_PHONG; the kernels are built for one shading or the other).
 // A finished primary walk is shaded: a miss takes the sky, a
@@ -684,6 +698,17 @@ __device__ __forceinline__ bool lr_finish(const A& a, LaneRay& L, Shaded& o, Wor
     const float hx = fmaf(L.tb, L.d.x, L.ox) + a.bias * nx, hy = fmaf(L.tb, L.d.y, L.oy) + a.bias * ny,
                 hz = fmaf(L.tb, L.d.z, L.oz) + a.bias * nz;
     L.lit = a.sun_scale * ndl;
+    if (a.sun_map.cells) {
+      const int known = sun_map_query(a.sun_map, hx, hy, hz, a.tmax);
+      if (known != 2) {
+        o.vis = uint8_t(known);
+        if (known) {
+          const float4 alb = __ldg(a.albedo + VLB_CLAMP(L.id, a.ntris, a.err));
+          o.r = alb.x * L.lit; o.g = alb.y * L.lit; o.b = alb.z * L.lit;
+        }
+        return true;
+      }
+    }
     make_ray_inv(L.ray, hx, hy, hz, a.sun.x, a.sun.y, a.sun.z, a.sun_inv.x, a.sun_inv.y, a.sun_inv.z);
     L.shadow = true;
     L.cur = walk_root(a.ntris);

@@ -1044,6 +1044,52 @@ static float bounds_scale(const vlb_scene* scene) {
   return m;
 }
 
+// Sun maps (k_lightmap.cu) pay when the rays are many (1 M rays in 778
+// triangles: 15 us for the map, the trace 212 -> 162 us; 4096 rays: 13 us for
+// 6 us) and outnumber the triangles to draw (2.4 M rays, 164 k triangles: 40 us
+// for 55 us in the tile walk, nothing gained in the fused walk).  256 cells a
+// side: 512 save 6 % more of that trace and cost 25 us more.
+constexpr uint32_t kMapSide = 256;
+static bool sun_map_pays(uint64_t rays, uint32_t ntris) { return rays >= std::max(1ull << 19, 24ull * ntris); }
+
+// Plane, extent and margins of a scene's sun map (k_lightmap.cu).
+static void sun_map_plan(const vlb_scene* scene, float3 s, float bias, uint32_t G, uint32_t* cells, vlbk::SunMap* m) {
+  const double d[3] = {s.x, s.y, s.z};
+  int least = 0;
+  for (int a = 1; a < 3; ++a)
+    if (std::fabs(d[a]) < std::fabs(d[least])) least = a;
+  double e[3] = {0, 0, 0};
+  e[least] = 1.0;
+  double u[3] = {d[1] * e[2] - d[2] * e[1], d[2] * e[0] - d[0] * e[2], d[0] * e[1] - d[1] * e[0]};
+  const double un = std::sqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+  for (double& x : u) x /= un;
+  const double v[3] = {d[1] * u[2] - d[2] * u[1], d[2] * u[0] - d[0] * u[2], d[0] * u[1] - d[1] * u[0]};
+  const double scale = std::max(std::fabs(bias), bounds_scale(scene));
+  double ext = 0.0, mid[2] = {0, 0};
+  for (int c = 0; c < 2; ++c) {
+    const double* ax = c ? v : u;
+    double lo = 0, hi = 0;
+    for (int a = 0; a < 3; ++a) {
+      lo += std::min(ax[a] * scene->bounds[a], ax[a] * scene->bounds[3 + a]);
+      hi += std::max(ax[a] * scene->bounds[a], ax[a] * scene->bounds[3 + a]);
+    }
+    mid[c] = 0.5 * (lo + hi);
+    ext = std::max(ext, hi - lo);
+  }
+  const double margin = scale * 0x1p-17;
+  ext += 2.0 * (std::fabs(double(bias)) + 4.0 * margin);
+  m->cells = cells;
+  m->u = make_float3(float(u[0]), float(u[1]), float(u[2]));
+  m->v = make_float3(float(v[0]), float(v[1]), float(v[2]));
+  m->s = s;
+  m->u0 = float(mid[0] - 0.5 * ext);
+  m->v0 = float(mid[1] - 0.5 * ext);
+  m->inv = float(G / ext);
+  m->cell = float(ext / G);
+  m->margin = float(margin);
+  m->G = G;
+}
+
 // Checks the parameters of one bake; *sun_len gets |sun_dir| (FP64).
 static vlb_status check_params(vlb_ctx* ctx, const vlb_scene* scene, const vlb_bake_params* p, double* sun_len) {
   if (!scene || !p || !p->dirs) return fail(ctx, VLB_ERR_INVALID, "scene, params and params->dirs are required");
@@ -1105,6 +1151,14 @@ static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const floa
   a.lane = lane_mode(scene, nprobes, p->flags, p->shading);
   a.shading = p->shading;
   a.light = make_float3(p->light_pos[0], p->light_pos[1], p->light_pos[2]);
+  if (a.lane && !from_root && a.ntris && a.shading == VLB_SHADE_LAMBERT_SUN &&
+      sun_map_pays(uint64_t(nprobes) * a.S, scene->ntris)) {
+    void* cells;
+    if ((st = scratch(ctx, "sun_map", size_t(kMapSide) * kMapSide * 8, &cells))) return st;
+    sun_map_plan(scene, a.sun, a.bias, kMapSide, static_cast<uint32_t*>(cells), &a.sun_map);
+    KScope k(ctx, "sun_map");
+    vlbk::launch_sun_map(a.sun_map, scene->tris, scene->ntris, ctx->stream);
+  }
   a.stack_lim = vlbk::kLaneStack;
   const bool grid = grid_mode(scene, nprobes, a.S, p);
   const bool tile_walk = a.lane && !grid && p->precision != VLB_PREC_FUSED;
@@ -1180,7 +1234,7 @@ static void job_from_trace(const vlbk::TraceArgs& a, vlbk::BakeJobDev* j) {
   j->tmin = a.tmin; j->tmax = a.tmax; j->bias = a.bias;
   j->sun = a.sun; j->sun_inv = a.sun_inv; j->sun_scale = a.sun_scale;
   j->sky = a.sky; j->sky_n = a.sky_n; j->err = a.err;
-  j->shading = a.shading; j->light = a.light;
+  j->shading = a.shading; j->light = a.light; j->sun_map = a.sun_map;
   j->probes = a.probes; j->order = const_cast<uint32_t*>(a.order); j->nprobes = a.nprobes;
   j->dirs = a.dirs; j->dinv = a.dinv; j->dir_order = a.dir_order; j->S = a.S;
   j->basis16 = a.basis16;

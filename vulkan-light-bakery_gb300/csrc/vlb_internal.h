@@ -205,6 +205,17 @@ struct FrontArgs {
 };
 void launch_probe_front(const FrontArgs& a, cudaStream_t s);
 
+// ---- sun maps (k_lightmap.cu) ------------------------------------------------------
+struct SunMap {
+  uint32_t* cells;   // [G][G] (cover, top) as ordered integers, or null: every shadow ray walks
+  float3 u, v, s;    // unit: across and along the direction to the sun
+  float u0, v0;      // origin of cell (0, 0)
+  float inv, cell;   // cells per unit, its reciprocal
+  float margin;
+  uint32_t G;
+};
+void launch_sun_map(const SunMap& m, const float4* tris, uint32_t ntris, cudaStream_t s);
+
 // ---- trace + shade --------------------------------------------------------------
 struct TraceArgs {
   const float4* nodes;
@@ -247,6 +258,7 @@ struct TraceArgs {
   uint32_t dirs_per_warp;
   uint32_t chunks;        // direction chunks per packet
   uint32_t lane;          // 1: per-lane traversal, 0: packet traversal
+  SunMap sun_map;
   const float4* front;    // probe frontiers (FrontArgs.ent) or null: the walks start at the root
   const uint32_t* front_n;
   uint32_t front_cap;
@@ -301,6 +313,7 @@ struct BakeJobDev {
   uint32_t shading;       // vlb_shading
   float3 light;           // VLB_SHADE_REF_PHONG point light
   int* err;
+  SunMap sun_map;
   // probes and directions
   const float* probes;    // device nprobes*3
   uint32_t* order;        // device nprobes: packet slot -> probe (written by the batched sort)
