@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace_dyn(const TraceArgs 
   const uint32_t P = (a.nprobes + 31) / 32 * 32;
   const uint32_t R = P * a.S;
   Work w;
-  int stack[kLaneStackFront];
+  int stack[kLaneStackFront + 1];
   LaneRay L;
   make_ray(L.ray, 0.f, 0.f, 0.f, 1.f, 1.f, 1.f);
   bool exhausted = false;
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace_dyn(const TraceArgs 
       const uint32_t r = wb + lane;
       if (r < R) {
         const uint32_t sl = r / a.S, t = r - sl * a.S;
-        if (sl < a.nprobes) lr_start(a, L, a.order[sl], __ldg(a.dir_order + t));
+        if (sl < a.nprobes) lr_start(a, L, a.order[sl], __ldg(a.dir_order + t), stack);
       }
       if constexpr (!WIDE) {
         if (a.front) lr_front(a, L, L.has, stack);
@@ -294,14 +294,19 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace_dyn(const TraceArgs 
     // node phase (all lanes take part in the votes)
     lr_node_steps<COUNT, TraceArgs, WIDE>(a, L, stack, w, kNodeSteps);
     lr_park(L, stack);
-    if (!L.has) continue;
     // leaf phase
-    if (L.leaf >= 0) lr_leaf<COUNT>(a, L, w);
-    if (L.cur != kWalkEnd) continue;
+    if (L.has && L.leaf >= 0) lr_leaf<COUNT>(a, L, w);
+    // The warp shades when all its walks have ended: it refills only when all
+    // its lanes are idle anyway, so a lane that is done early loses nothing, and
+    // the shading runs once per group (twice with shadow walks) instead of once
+    // per turn in which some lane ends (1 M rays in 778 triangles: 160 -> 137 us;
+    // 262,144 probes x 1024 directions in 4096 boxes: 8 % less).
+    if (__any_sync(kFull, L.has && L.cur != kWalkEnd)) continue;
     Shaded o;
-    if (!lr_finish<COUNT, TraceArgs, REF>(a, L, o, w)) continue;
-    L.has = false;
-    emit_tile(a, L, o);
+    if (L.has && lr_finish<COUNT, TraceArgs, REF>(a, L, o, w, stack)) {
+      L.has = false;
+      emit_tile(a, L, o);
+    }
   }
   if constexpr (COUNT) {
     atomicAdd(a.counters + 0, (unsigned long long)w.wnodes);
@@ -644,7 +649,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_grid(const TraceArgs a)
         if (r < R) {
           const uint32_t t = r / P, sl = r - t * P;
           if (sl < a.nprobes) {
-            lr_start(a, L, a.order[sl], __ldg(a.dir_order + t));
+            lr_start(a, L, a.order[sl], __ldg(a.dir_order + t), nullptr);
             grid_begin<COUNT>(a, L, g, w);
           }
         }
@@ -662,7 +667,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_grid(const TraceArgs a)
     }
     if (!L.has || g.e < g.e1) continue;
     Shaded o;
-    if (!lr_finish<COUNT>(a, L, o, w)) {  // a lit hit: its shadow walk
+    if (!lr_finish<COUNT>(a, L, o, w, nullptr)) {  // a lit hit: its shadow walk
       grid_begin<COUNT>(a, L, g, w);
       continue;
     }
@@ -750,7 +755,7 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_trace_batch(const BakeJobD
                                                                uint32_t total, uint32_t chunk, uint32_t* counter) {
   const uint32_t lane = threadIdx.x & 31;
   Work w;
-  int stack[kLaneStack];
+  int stack[kLaneStackFront + 1];
   LaneRay L;
   make_ray(L.ray, 0.f, 0.f, 0.f, 1.f, 1.f, 1.f);
   for (;;) {
@@ -780,14 +785,14 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_trace_batch(const BakeJobD
           const uint32_t sl = r / j.S, t = r - sl * j.S;
           if (sl < j.nprobes) {
             const uint32_t p = j.order[sl];
-            lr_start(j, L, p, __ldg(j.dir_order + t));
+            lr_start(j, L, p, __ldg(j.dir_order + t), stack);
             if (j.hits_in) {  // relight: the kept primary hit, only the shadow walk remains
               const int2 h = __ldg(j.hits_in + size_t(p) * j.S + L.s);
               L.slot = h.x;
               L.tb = __int_as_float(h.y);
               L.id = h.x >= 0 ? __float_as_int(__ldg(j.tris + 3 * VLB_CLAMP(h.x, j.ntris, j.err)).w) : -1;
               Shaded o;
-              if (lr_finish<false, BakeJobDev, REF>(j, L, o, w)) {
+              if (lr_finish<false, BakeJobDev, REF>(j, L, o, w, stack)) {
                 L.has = false;
                 batch_emit(j, L.p, L.s, o);
               }
@@ -801,12 +806,12 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_trace_batch(const BakeJobD
       }
       lr_node_steps<false, BakeJobDev>(j, L, stack, w, kNodeSteps);  // one while-while turn, as in k_trace_dyn
       lr_park(L, stack);
+      if (L.has && L.leaf >= 0) lr_leaf<false>(j, L, w);
+      if (__any_sync(kFull, L.has && L.cur != kWalkEnd)) continue;  // the warp shades together, as in k_trace_dyn
       if (!L.has) continue;
-      if (L.leaf >= 0) lr_leaf<false>(j, L, w);
-      if (L.cur != kWalkEnd) continue;
       if (!L.shadow && j.hits_out) j.hits_out[size_t(L.p) * j.S + L.s] = make_int2(L.slot, __float_as_int(L.tb));
       Shaded o;
-      if (!lr_finish<false, BakeJobDev, REF>(j, L, o, w)) continue;
+      if (!lr_finish<false, BakeJobDev, REF>(j, L, o, w, stack)) continue;
       L.has = false;
       batch_emit(j, L.p, L.s, o);
     }

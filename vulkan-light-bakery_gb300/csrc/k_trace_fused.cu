@@ -84,14 +84,30 @@ __device__ __forceinline__ void retire_head(FusedWarp<3 * K>& fw, const BakeJobD
   const uint32_t e = fw.head;
   const SubBatch q = fw.q[e];
   const BakeJobDev& J = job_of<MULTI>(jobs, one, q.job);
-  const uint32_t* dord = J.dir_order + q.t0;
-  for (int v = int(lane); v < V; v += 32) {
-    const int k = v / 3, ch = v - 3 * k;
-    float s = 0.f;
-#pragma unroll 4
-    for (uint32_t i = 0; i < q.cnt; ++i)
-      s = fmaf(__ldg(J.basis16 + size_t(VLB_CLAMP(__ldg(dord + i), J.S, J.err)) * 16 + k), fw.rad[e][ch][i], s);
-    fw.acc[v] = ((q.flags & kSubFirst) ? 0.0 : fw.acc[v]) + double(s);
+  // lane v sums output v, and v + 32 where V > 32, in ray order; lane i fetches
+  // ray i's direction index once, so the basis loads depend on no other load
+  // and eight rays' are in flight at once
+  const uint32_t sl = lane < q.cnt ? VLB_CLAMP(__ldg(J.dir_order + q.t0 + lane), J.S, J.err) : 0;
+  constexpr int P = (V + 31) / 32;
+  int k[P], ch[P];
+  float s[P];
+#pragma unroll
+  for (int h = 0; h < P; ++h) {
+    const int v = min(int(lane) + 32 * h, V - 1);
+    k[h] = v / 3;
+    ch[h] = v - 3 * k[h];
+    s[h] = 0.f;
+  }
+#pragma unroll 8
+  for (uint32_t i = 0; i < q.cnt; ++i) {
+    const float* row = J.basis16 + size_t(__shfl_sync(kFull, sl, i)) * 16;
+#pragma unroll
+    for (int h = 0; h < P; ++h) s[h] = fmaf(__ldg(row + k[h]), fw.rad[e][ch[h]][i], s[h]);
+  }
+#pragma unroll
+  for (int h = 0; h < P; ++h) {
+    const int v = int(lane) + 32 * h;
+    if (v < V) fw.acc[v] = ((q.flags & kSubFirst) ? 0.0 : fw.acc[v]) + double(s[h]);
   }
   if ((q.flags & kSubLast) && VLB_INB(q.p, J.nprobes, J.err) && VLB_INB(q.c, J.chunks, J.err)) {
     float* dst = J.chunks == 1 ? J.out + size_t(q.p) * V : J.partial + (size_t(q.p) * J.chunks + q.c) * V;
@@ -214,7 +230,7 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace_fused(const BakeJ
   }
   __syncwarp();
   Work w;
-  int stack[kLaneStack];
+  int stack[kLaneStackFront + 1];
   LaneRay L;
   make_ray(L.ray, 0.f, 0.f, 0.f, 1.f, 1.f, 1.f);
   uint32_t lslot = 0;  // the lane's ray: ring slot << 8 | position
@@ -233,19 +249,20 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace_fused(const BakeJ
         if (!avail) continue;
         const uint32_t take = min(avail, uint32_t(__popc(idle)));
         const uint32_t rank = __popc(idle & lane_lt_mask());
-        if (((idle >> lane) & 1u) && rank < take) {
+        const bool took = ((idle >> lane) & 1u) && rank < take;
+        const BakeJobDev& J = job_of<MULTI>(jobs, one, fw.q[e].job);
+        if (took) {
           const uint32_t pos = issued + rank;
-          const BakeJobDev& J = job_of<MULTI>(jobs, one, fw.q[e].job);
           const uint32_t s = __ldg(J.dir_order + fw.q[e].t0 + pos);
           lslot = (e << 8) | pos;
-          lr_start(J, L, fw.q[e].p, s);
+          lr_start(J, L, fw.q[e].p, s, stack);
           if (J.hits_in) {  // relight: the kept primary hit, only the shadow walk remains
             const int2 hk = __ldg(J.hits_in + size_t(L.p) * J.S + s);
             L.slot = hk.x;
             L.tb = __int_as_float(hk.y);
             L.id = hk.x >= 0 ? __float_as_int(__ldg(J.tris + 3 * VLB_CLAMP(hk.x, J.ntris, J.err)).w) : -1;
             Shaded o;
-            if (lr_finish<false, BakeJobDev, REF>(J, L, o, w)) {
+            if (lr_finish<false, BakeJobDev, REF>(J, L, o, w, stack)) {
               L.has = false;
               done_now = true;
               store_ray(fw, J, L, o, lslot);
@@ -253,6 +270,7 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace_fused(const BakeJ
           }
         }
         __syncwarp();
+        if (J.front && !J.hits_in) lr_front(J, L, took, stack);
         if (lane == 0) fw.q[e].issued = issued + take;
         idle = __ballot_sync(kFull, !L.has && !done_now);
         __syncwarp();
@@ -264,13 +282,15 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace_fused(const BakeJ
       // one while-while turn (as k_trace_dyn): node phase, then leaf phase
       lr_node_steps<false, BakeJobDev, false, !MULTI>(J, L, stack, w, node_steps);
       lr_park(L, stack);
-      if (L.has) {
-        if (L.leaf >= 0) lr_leaf<false>(J, L, w);
+      if (L.has && L.leaf >= 0) lr_leaf<false>(J, L, w);
+      // a warp that refills only when all of it is idle shades together too
+      const bool wait = refill_idle >= 32 && __any_sync(kFull, L.has && L.cur != kWalkEnd);
+      if (L.has && !wait) {
         if (L.cur == kWalkEnd) {
           if (!L.shadow && J.hits_out)
             J.hits_out[size_t(L.p) * J.S + L.s] = make_int2(L.slot, __float_as_int(L.tb));
           Shaded o;
-          if (lr_finish<false, BakeJobDev, REF>(J, L, o, w)) {
+          if (lr_finish<false, BakeJobDev, REF>(J, L, o, w, stack)) {
             L.has = false;
             done_now = true;
             store_ray(fw, J, L, o, lslot);

@@ -484,9 +484,22 @@ __device__ __forceinline__ float lr_try(const A& a, const LaneRay& L, int ts, in
   return tri_hit(L.ray, v0, e1, e2);
 }
 
+// Empties a lane's stack.  Its bottom entry is kWalkEnd, so a pop needs no
+// test.  Where walks start at probe frontiers (trees at most kLaneStack deep)
+// the whole array is used and cannot overflow; elsewhere a walk has kLaneStack
+// entries and reports one more as an overflow.  (stack null: a walk that keeps
+// none.)
+template <class A>
+__device__ __forceinline__ void lr_empty(const A& a, LaneRay& L, int* stack) {
+  if (!stack) return;
+  const int base = a.front ? 0 : kLaneStackFront - kLaneStack;
+  stack[base] = kWalkEnd;
+  L.sp = base + 1;
+}
+
 // A: TraceArgs or BakeJobDev (scene, shading, probes and dirs fields).
 template <class A>
-__device__ __forceinline__ void lr_start(const A& a, LaneRay& L, uint32_t p, uint32_t s) {
+__device__ __forceinline__ void lr_start(const A& a, LaneRay& L, uint32_t p, uint32_t s, int* stack) {
   p = VLB_CLAMP(p, a.nprobes, a.err);
   s = VLB_CLAMP(s, a.S, a.err);
   L.p = p;
@@ -500,7 +513,7 @@ __device__ __forceinline__ void lr_start(const A& a, LaneRay& L, uint32_t p, uin
   L.has = true;
   L.shadow = false;
   L.cur = walk_root(a.ntris);
-  L.sp = 0;
+  lr_empty(a, L, stack);
   L.slot = -1;
   L.id = -1;
   L.leaf = -1;
@@ -511,10 +524,6 @@ __device__ __forceinline__ void lr_start(const A& a, LaneRay& L, uint32_t p, uin
     if (t > a.tmin && t < L.tb) { L.tb = t; L.slot = L.hprev; L.id = id; }
   }
 }
-
-// Entries a lane's stack may hold.
-__device__ __forceinline__ int stack_limit(const TraceArgs& a) { return int(a.stack_lim); }
-__device__ __forceinline__ int stack_limit(const BakeJobDev&) { return kLaneStack; }
 
 // Order-preserving map of a float to an unsigned integer (NaN-free input).
 __device__ __forceinline__ uint32_t ordered_u32(float f) {
@@ -585,7 +594,7 @@ __device__ __forceinline__ void lr_front(const A& a, LaneRay& L, bool mine, int*
         if (now && tn <= tf) stack[L.sp++] = __float_as_int(rf);
       }
     }
-    if (now) L.cur = L.sp ? stack[--L.sp] : kWalkEnd;
+    if (now) L.cur = stack[--L.sp];
     pending &= ~__ballot_sync(kFull, now);
   }
 }
@@ -603,7 +612,7 @@ __device__ __forceinline__ float ref_unorm8(float c) { return rintf(fminf(fmaxf(
 // facing the point light starts its shadow walk toward it (returns false;
 // diffuse + specular wait in lit), any other hit is black.
 template <class A>
-__device__ __forceinline__ bool lr_finish_ref_primary(const A& a, LaneRay& L, Shaded& o) {
+__device__ __forceinline__ bool lr_finish_ref_primary(const A& a, LaneRay& L, Shaded& o, int* stack) {
   if (L.slot < 0) {
     if (a.sky) {
       const float* tx =
@@ -634,7 +643,7 @@ __device__ __forceinline__ bool lr_finish_ref_primary(const A& a, LaneRay& L, Sh
   make_ray(L.ray, px + a.bias * nx, py + a.bias * ny, pz + a.bias * nz, lx, ly, lz);
   L.shadow = true;
   L.cur = walk_root(a.ntris);
-  L.sp = 0;
+  lr_empty(a, L, stack);
   L.slot = -1;
   L.tb = len;
   if (L.oprev >= 0 && uint32_t(L.oprev) < a.ntris) {
@@ -667,12 +676,12 @@ __device__ __forceinline__ int sun_map_query(const SunMap& m, float x, float y, 
 // finished shadow walk gives the Lambert term or 0.  Returns true with the
 // sample in `o` when the ray is complete.
 template <bool COUNT, class A, bool REF = false>
-__device__ __forceinline__ bool lr_finish(const A& a, LaneRay& L, Shaded& o, Work& w) {
+__device__ __forceinline__ bool lr_finish(const A& a, LaneRay& L, Shaded& o, Work& w, int* stack) {
   o = Shaded{0.f, 0.f, 0.f, -1, 2};
   if constexpr (REF) {
     if (!L.shadow) {
       L.hprev = L.slot;
-      return lr_finish_ref_primary(a, L, o);
+      return lr_finish_ref_primary(a, L, o, stack);
     }
   }
   if (!L.shadow) {
@@ -712,7 +721,7 @@ __device__ __forceinline__ bool lr_finish(const A& a, LaneRay& L, Shaded& o, Wor
     make_ray_inv(L.ray, hx, hy, hz, a.sun.x, a.sun.y, a.sun.z, a.sun_inv.x, a.sun_inv.y, a.sun_inv.z);
     L.shadow = true;
     L.cur = walk_root(a.ntris);
-    L.sp = 0;
+    lr_empty(a, L, stack);
     L.slot = -1;
     L.tb = a.tmax;
     if (L.oprev >= 0 && uint32_t(L.oprev) < a.ntris) {
@@ -752,7 +761,7 @@ __device__ __forceinline__ bool lr_is_tri(int cur) { return cur < 0 && cur != kW
 __device__ __forceinline__ void lr_park(LaneRay& L, const int* stack) {
   if (L.has && L.leaf < 0 && lr_is_tri(L.cur)) {
     L.leaf = ~L.cur;
-    L.cur = L.sp ? stack[--L.sp] : kWalkEnd;
+    L.cur = stack[--L.sp];
   }
 }
 
@@ -770,7 +779,7 @@ __device__ __forceinline__ float q8(uint32_t word, int c) {
 // when its box is hit, to keep the walk's registers few.
 template <bool COUNT, class A>
 __device__ __forceinline__ void lr_node_wide(const A& a, LaneRay& L, int* stack, Work& w) {
-  if (!VLB_INB(L.cur, a.nwide, a.err)) { L.cur = kWalkEnd; L.sp = 0; return; }
+  if (!VLB_INB(L.cur, a.nwide, a.err)) { L.cur = kWalkEnd; return; }
   if constexpr (COUNT) { ++w.wnodes; ++w.lnodes; }
   const float tlo = L.shadow ? 0.0f : a.tmin;
   const float4* nd = a.wnodes + 6 * size_t(L.cur);
@@ -812,14 +821,14 @@ __device__ __forceinline__ void lr_node_wide(const A& a, LaneRay& L, int* stack,
             tnext = tn;
           }
           if (push != kWalkEnd) {
-            if (L.sp < kLaneStack) stack[L.sp++] = push;
+            if (L.sp <= kLaneStackFront) stack[L.sp++] = push;
             else atomicAdd(a.err + kErrStackOverflow, 1);
           }
         }
       }
     }
   }
-  L.cur = next != kWalkEnd ? next : (L.sp ? stack[--L.sp] : kWalkEnd);
+  L.cur = next != kWalkEnd ? next : stack[--L.sp];
 }
 
 // One inner node: nearer hit child next, the farther one on the stack.  WIDE:
@@ -834,7 +843,7 @@ __device__ __forceinline__ void lr_node(const A& a, LaneRay& L, int* stack, Work
     lr_node_wide<COUNT>(a, L, stack, w);
     return;
   }
-  if (!VLB_INB(L.cur, 2 * a.ntris - 2, a.err)) { L.cur = kWalkEnd; L.sp = 0; return; }
+  if (!VLB_INB(L.cur, 2 * a.ntris - 2, a.err)) { L.cur = kWalkEnd; return; }
   if constexpr (COUNT) { ++w.wnodes; ++w.lnodes; }
   const float tlo = L.shadow ? 0.0f : a.tmin;
   float4 n0, n1, n2, n3;
@@ -851,7 +860,7 @@ __device__ __forceinline__ void lr_node(const A& a, LaneRay& L, int* stack, Work
   const int c0 = __float_as_int(n3.x), c1 = __float_as_int(n3.y);
   if (h0 && h1) {
     const bool first0 = tn0 <= tn1;
-    if (L.sp < stack_limit(a)) stack[L.sp++] = first0 ? c1 : c0;
+    if (L.sp <= kLaneStackFront) stack[L.sp++] = first0 ? c1 : c0;
     else atomicAdd(a.err + kErrStackOverflow, 1);
     L.cur = first0 ? c0 : c1;
   } else if (h0) {
@@ -859,7 +868,7 @@ __device__ __forceinline__ void lr_node(const A& a, LaneRay& L, int* stack, Work
   } else if (h1) {
     L.cur = c1;
   } else {
-    L.cur = L.sp ? stack[--L.sp] : kWalkEnd;
+    L.cur = stack[--L.sp];
   }
 }
 
@@ -874,7 +883,7 @@ __device__ __forceinline__ void lr_leaf(const A& a, LaneRay& L, Work& w) {
   const float t = tri_hit(L.ray, v0, e1, e2);
   if (!(t > tlo)) return;
   if (L.shadow) {
-    if (t < L.tb) { L.slot = ts; L.cur = kWalkEnd; L.sp = 0; }
+    if (t < L.tb) { L.slot = ts; L.cur = kWalkEnd; }
     return;
   }
   const int tid = __float_as_int(v0.w);

@@ -1159,10 +1159,8 @@ static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const floa
     KScope k(ctx, "sun_map");
     vlbk::launch_sun_map(a.sun_map, scene->tris, scene->ntris, ctx->stream);
   }
-  a.stack_lim = vlbk::kLaneStack;
   const bool grid = grid_mode(scene, nprobes, a.S, p);
-  const bool tile_walk = a.lane && !grid && p->precision != VLB_PREC_FUSED;
-  const uint32_t cap = tile_walk && !from_root ? front_cap(scene, nprobes, a.S) : 0;
+  const uint32_t cap = a.lane && !grid && !from_root ? front_cap(scene, nprobes, a.S) : 0;
   void *ent, *cnt;
   if (cap && scratch(ctx, "front_ent", size_t(nprobes) * cap * 32, &ent) == VLB_OK &&
       scratch(ctx, "front_cnt", size_t(nprobes) * 4, &cnt) == VLB_OK) {
@@ -1173,7 +1171,6 @@ static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const floa
     a.front = f.ent;
     a.front_n = f.cnt;
     a.front_cap = cap;
-    a.stack_lim = vlbk::kLaneStackFront;
   }
   if (grid) {
     const uint32_t G = grid_cells_per_side(scene->ntris), T = scene->ntris;
@@ -1235,6 +1232,7 @@ static void job_from_trace(const vlbk::TraceArgs& a, vlbk::BakeJobDev* j) {
   j->sun = a.sun; j->sun_inv = a.sun_inv; j->sun_scale = a.sun_scale;
   j->sky = a.sky; j->sky_n = a.sky_n; j->err = a.err;
   j->shading = a.shading; j->light = a.light; j->sun_map = a.sun_map;
+  j->front = a.front; j->front_n = a.front_n; j->front_cap = a.front_cap;
   j->probes = a.probes; j->order = const_cast<uint32_t*>(a.order); j->nprobes = a.nprobes;
   j->dirs = a.dirs; j->dinv = a.dinv; j->dir_order = a.dir_order; j->S = a.S;
   j->basis16 = a.basis16;

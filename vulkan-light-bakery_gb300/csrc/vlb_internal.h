@@ -262,7 +262,6 @@ struct TraceArgs {
   const float4* front;    // probe frontiers (FrontArgs.ent) or null: the walks start at the root
   const uint32_t* front_n;
   uint32_t front_cap;
-  uint32_t stack_lim;     // entries a lane's stack may hold (kLaneStack, or kLaneStackFront with frontiers)
   uint32_t ray_block;     // tile lane walk: rays a warp takes from the counter at once (set by its launch)
   unsigned long long* counters;  // null, or [warp node fetches, warp triangle fetches, shadow rays, lane node tests]
   int* err;
@@ -314,6 +313,9 @@ struct BakeJobDev {
   float3 light;           // VLB_SHADE_REF_PHONG point light
   int* err;
   SunMap sun_map;
+  const float4* front;    // probe frontiers (FrontArgs.ent) or null
+  const uint32_t* front_n;
+  uint32_t front_cap;
   // probes and directions
   const float* probes;    // device nprobes*3
   uint32_t* order;        // device nprobes: packet slot -> probe (written by the batched sort)
