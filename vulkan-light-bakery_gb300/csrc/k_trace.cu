@@ -240,6 +240,7 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace_dyn(const TraceArgs 
   LaneRay L;
   make_ray(L.ray, 0.f, 0.f, 0.f, 1.f, 1.f, 1.f);
   bool exhausted = false;
+  int fnext = 0;  // next frontier entry of the group's walks, 0: none left
   // A warp takes its rays in blocks of `block` consecutive rays (whole 32-ray
   // groups of one probe's neighbouring directions) and hands a block's groups
   // to its lanes one by one: its next rays then reuse the nodes its last ones
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace_dyn(const TraceArgs 
         if (sl < a.nprobes) lr_start(a, L, a.order[sl], __ldg(a.dir_order + t), stack);
       }
       if constexpr (!WIDE) {
-        if (a.front) lr_front(a, L, L.has, stack);
+        if (a.front) fnext = lr_front_next(a, L, L.has, 0, stack);
       }
     }
     if (!__any_sync(kFull, L.has)) {
@@ -302,6 +303,12 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace_dyn(const TraceArgs 
     // per turn in which some lane ends (1 M rays in 778 triangles: 160 -> 137 us;
     // 262,144 probes x 1024 directions in 4096 boxes: 8 % less).
     if (__any_sync(kFull, L.has && L.cur != kWalkEnd)) continue;
+    if constexpr (!WIDE) {
+      if (fnext) {  // the group's primary walks go on with the rest of their frontier
+        fnext = lr_front_next(a, L, L.has, fnext, stack);
+        if (fnext || __any_sync(kFull, L.has && L.cur != kWalkEnd)) continue;
+      }
+    }
     Shaded o;
     if (L.has && lr_finish<COUNT, TraceArgs, REF>(a, L, o, w, stack)) {
       L.has = false;

@@ -234,6 +234,10 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace_fused(const BakeJ
   LaneRay L;
   make_ray(L.ray, 0.f, 0.f, 0.f, 1.f, 1.f, 1.f);
   uint32_t lslot = 0;  // the lane's ray: ring slot << 8 | position
+  // a warp that refills only when all of it is idle shades together and takes
+  // its frontiers in stages, as the tile lane walk
+  const bool staged = refill_idle >= 32;
+  int fnext = 0;
   for (;;) {
     // Bookkeeping only when enough of the warp is idle, as in the tile lane
     // walk: retire complete sub-batches, refill the ring, hand out rays.
@@ -243,6 +247,7 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace_fused(const BakeJ
       while (fw.n > 0 && fw.q[fw.head].fin == fw.q[fw.head].cnt) retire_head<K, MULTI>(fw, jobs, one, lane);
       fill_ring<MULTI>(fw, jobs, one, njobs, total, counter, lane);
       const uint32_t n = fw.n, head = fw.head;
+      fnext = 0;
       for (uint32_t k = 0; k < n && idle; ++k) {
         const uint32_t e = (head + k) % kSubBufs;
         const uint32_t issued = fw.q[e].issued, avail = fw.q[e].cnt - issued;
@@ -270,7 +275,15 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace_fused(const BakeJ
           }
         }
         __syncwarp();
-        if (J.front && !J.hits_in) lr_front(J, L, took, stack);
+        if (J.front && !J.hits_in) {
+          if (staged) {
+            fnext = max(fnext, lr_front_next(J, L, took, 0, stack));
+          } else {  // all of it, nearest on top
+            for (int f = kFrontCap - kFrontStage; f > 0; f -= kFrontStage) lr_front(J, L, took, f, stack);
+            lr_front(J, L, took, 0, stack);
+            if (took) L.cur = stack[--L.sp];
+          }
+        }
         if (lane == 0) fw.q[e].issued = issued + take;
         idle = __ballot_sync(kFull, !L.has && !done_now);
         __syncwarp();
@@ -283,8 +296,20 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace_fused(const BakeJ
       lr_node_steps<false, BakeJobDev, false, !MULTI>(J, L, stack, w, node_steps);
       lr_park(L, stack);
       if (L.has && L.leaf >= 0) lr_leaf<false>(J, L, w);
-      // a warp that refills only when all of it is idle shades together too
-      const bool wait = refill_idle >= 32 && __any_sync(kFull, L.has && L.cur != kWalkEnd);
+      bool wait = staged && __any_sync(kFull, L.has && L.cur != kWalkEnd);
+      if (fnext && !wait) {
+        int next = 0;
+        unsigned pending = __ballot_sync(kFull, L.has && !L.shadow);
+        while (pending) {
+          const uint32_t e = __shfl_sync(kFull, lslot >> 8, __ffs(pending) - 1);
+          const bool mine = L.has && !L.shadow && (lslot >> 8) == e;
+          const BakeJobDev& Q = job_of<MULTI>(jobs, one, fw.q[e].job);
+          if (Q.front) next = max(next, lr_front_next(Q, L, mine, fnext, stack));
+          pending &= ~__ballot_sync(kFull, mine);
+        }
+        fnext = next;
+        wait = fnext || __any_sync(kFull, L.has && L.cur != kWalkEnd);
+      }
       if (L.has && !wait) {
         if (L.cur == kWalkEnd) {
           if (!L.shadow && J.hits_out)

@@ -534,24 +534,38 @@ __device__ __forceinline__ float ordered_f32(uint32_t k) {
   return __uint_as_float(k ^ (uint32_t(int32_t(~k) >> 31) | 0x80000000u));
 }
 
-// Starts the primary walks of the lanes that just took a ray (`mine`) from
-// their probe's frontier (k_front.cu).  The lanes' rays share an origin, so
-// relative to it a plane at x is crossed at x / d.  First each lane tests one
-// entry against the whole group: the entry's crossings under the group's range
-// of 1/d per axis (an axis whose directions change sign does not constrain).
-// Then, farthest first, every lane tests its own ray against the entries left
-// and stacks those it hits; the walk goes on from the nearest.  All 32 lanes
+// Probe frontiers (k_front.cu).  The lanes `mine` test their primary rays
+// against entries [first, first + 32) of their probe's frontier and stack
+// those they hit, nearest on top; returns whether any of them has entries left.
+// The rays share an origin, so relative to it a plane at x is crossed at x / d.
+// First each lane tests one entry against the whole group -- the entry's
+// crossings under the group's range of 1/d per axis (an axis whose directions
+// change sign does not constrain) up to the farthest limit -- then every lane
+// tests its own ray against the entries left, farthest first.  All 32 lanes
 // take part; a group that straddles two probes goes probe by probe.
+//
+// A walk takes its frontier 32 entries at a time: entries are sorted by
+// distance, and when the whole group has walked the nearest, the rest are
+// culled by the hits found (262,144 probes x 1024 directions in 4096 boxes,
+// lists of 64: all entries at once 8.1, 32 at a time 6.4, 16 at a time 6.2 ms
+// on an eighth of the probes; 3141 x 1000 directions in 64 boxes 39.6 at 32
+// and 43.6 at 16).
+constexpr int kFrontStage = 32;
 template <class A>
-__device__ __forceinline__ void lr_front(const A& a, LaneRay& L, bool mine, int* stack) {
+__device__ __forceinline__ bool lr_front(const A& a, LaneRay& L, bool mine, int first, int* stack) {
   const uint32_t lane = threadIdx.x & 31;
   unsigned pending = __ballot_sync(kFull, mine);
+  bool more = false;
   while (pending) {
     const uint32_t q = __shfl_sync(kFull, L.p, __ffs(pending) - 1);
     const bool now = mine && L.p == q;
-    const float4* f = a.front + size_t(q) * (2 * a.front_cap);
+    pending &= ~__ballot_sync(kFull, now);
     const int n = int(__ldg(a.front_n + q));
+    if (first >= n) continue;
+    more = more || first + kFrontStage < n;
+    const float4* f = a.front + (size_t(q) * a.front_cap + first) * 2;
     const float lim = prune_limit(L.tb);
+    const float far = __uint_as_float(__reduce_max_sync(kFull, now ? __float_as_uint(lim) : 0u));
     float imin[3], imax[3];
     const float iv[3] = {L.ray.ixy.x, L.ray.ixy.y, L.ray.izz.x};
 #pragma unroll
@@ -560,43 +574,49 @@ __device__ __forceinline__ void lr_front(const A& a, LaneRay& L, bool mine, int*
       imin[c] = ordered_f32(__reduce_min_sync(kFull, now ? k : 0xffffffffu));
       imax[c] = ordered_f32(__reduce_max_sync(kFull, now ? k : 0u));
     }
-    const float far = __uint_as_float(__reduce_max_sync(kFull, now ? __float_as_uint(lim) : 0u));
-    for (int w = (n - 1) & ~31; w >= 0; w -= 32) {
-      bool in = false;
-      if (w + int(lane) < n) {
-        const float4 x = __ldg(f + 2 * (w + lane)), y = __ldg(f + 2 * (w + lane) + 1);
-        const float lo[3] = {x.x, x.y, y.x}, hi[3] = {x.z, x.w, y.y};
-        float tn = 0.f, tf = far;
+    bool in = false;
+    if (first + int(lane) < n) {
+      const float4 x = __ldg(f + 2 * lane), y = __ldg(f + 2 * lane + 1);
+      const float lo[3] = {x.x, x.y, y.x}, hi[3] = {x.z, x.w, y.y};
+      float tn = 0.f, tf = far;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const bool neg = imin[c] < 0.f;
-          const float e = neg ? hi[c] : lo[c], g = neg ? lo[c] : hi[c];  // entry and exit planes
-          if (!(neg && imax[c] > 0.f)) {
-            tn = fmaxf(tn, fminf(e * imin[c], e * imax[c]));
-            tf = fminf(tf, fmaxf(g * imin[c], g * imax[c]));
-          }
+      for (int c = 0; c < 3; ++c) {
+        const bool neg = imin[c] < 0.f;
+        const float e = neg ? hi[c] : lo[c], g = neg ? lo[c] : hi[c];  // entry and exit planes
+        if (!(neg && imax[c] > 0.f)) {
+          tn = fmaxf(tn, fminf(e * imin[c], e * imax[c]));
+          tf = fminf(tf, fmaxf(g * imin[c], g * imax[c]));
         }
-        in = tn <= tf;
       }
-      unsigned hits = __ballot_sync(kFull, in);
-      while (hits) {
-        const int i = 31 - __clz(hits);
-        hits ^= 1u << i;
-        float lx, ly, hx, hy, lz, hz, rf, d2;
-        asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-            : "=f"(lx), "=f"(ly), "=f"(hx), "=f"(hy), "=f"(lz), "=f"(hz), "=f"(rf), "=f"(d2)
-            : "l"(f + 2 * (w + i)));
-        const float2 zero = make_float2(0.f, 0.f);
-        const float2 l = fma_pair(lx, ly, L.ray.ixy, zero), u = fma_pair(hx, hy, L.ray.ixy, zero);
-        const float2 z = fma_pair(lz, hz, L.ray.izz, zero);
-        const float tn = fmax3(fminf(l.x, u.x), fminf(l.y, u.y), fmaxf(fminf(z.x, z.y), a.tmin));
-        const float tf = fmin3(fmaxf(l.x, u.x), fmaxf(l.y, u.y), fminf(fmaxf(z.x, z.y), lim));
-        if (now && tn <= tf) stack[L.sp++] = __float_as_int(rf);
-      }
+      in = tn <= tf;
     }
-    if (now) L.cur = stack[--L.sp];
-    pending &= ~__ballot_sync(kFull, now);
+    unsigned hits = __ballot_sync(kFull, in);
+    while (hits) {
+      const int i = 31 - __clz(hits);
+      hits ^= 1u << i;
+      float lx, ly, hx, hy, lz, hz, rf, d2;
+      asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+          : "=f"(lx), "=f"(ly), "=f"(hx), "=f"(hy), "=f"(lz), "=f"(hz), "=f"(rf), "=f"(d2)
+          : "l"(f + 2 * i));
+      const float2 zero = make_float2(0.f, 0.f);
+      const float2 l = fma_pair(lx, ly, L.ray.ixy, zero), u = fma_pair(hx, hy, L.ray.ixy, zero);
+      const float2 z = fma_pair(lz, hz, L.ray.izz, zero);
+      const float tn = fmax3(fminf(l.x, u.x), fminf(l.y, u.y), fmaxf(fminf(z.x, z.y), a.tmin));
+      const float tf = fmin3(fmaxf(l.x, u.x), fmaxf(l.y, u.y), fminf(fmaxf(z.x, z.y), lim));
+      if (now && tn <= tf) stack[L.sp++] = __float_as_int(rf);
+    }
   }
+  return more;
+}
+
+// The next stage of a group whose walks `mine` have all ended: returns the
+// entry to go on from after it, 0 when the frontier is done.
+template <class A>
+__device__ __forceinline__ int lr_front_next(const A& a, LaneRay& L, bool mine, int first, int* stack) {
+  if (first && mine) lr_empty(a, L, stack);
+  const bool more = lr_front(a, L, mine, first, stack);
+  if (mine) L.cur = stack[--L.sp];
+  return more ? first + kFrontStage : 0;
 }
 
 // The reference baker's sample encoding: the sRGB curve of
