@@ -60,25 +60,26 @@ constexpr float kFrontLarge = 10.f;
 constexpr int kFrontLook = 32;
 constexpr int kFrontRounds = 8;
 
-__global__ void __launch_bounds__(kFrontWarps * 32) k_probe_front(const FrontArgs a) {
-  __shared__ FrontBox s_open[2][kFrontWarps][kFrontCap];
-  __shared__ FrontBox s_done[kFrontWarps][kFrontCap];
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t p = blockIdx.x * kFrontWarps + warp;
-  if (p >= a.nprobes) return;
+struct FrontShared {
+  FrontBox open[2][kFrontCap], done[kFrontCap];
+};
+
+// One warp: probe p's frontier.
+__device__ __forceinline__ void front_probe(const FrontArgs& a, uint32_t p, FrontShared& sh) {
+  const uint32_t lane = threadIdx.x & 31;
   const int cap = int(a.cap);
   const float ox = a.probes[3 * size_t(p)], oy = a.probes[3 * size_t(p) + 1], oz = a.probes[3 * size_t(p) + 2];
   const unsigned below = (1u << lane) - 1u;
-  FrontBox* done = s_done[warp];
+  FrontBox* done = sh.done;
   if (lane == 0) {
-    s_open[0][warp][0].a = make_float4(0.f, 0.f, 0.f, 0.f);
-    s_open[0][warp][0].b = make_float4(0.f, 0.f, __int_as_float(0), 0.f);
+    sh.open[0][0].a = make_float4(0.f, 0.f, 0.f, 0.f);
+    sh.open[0][0].b = make_float4(0.f, 0.f, __int_as_float(0), 0.f);
   }
   __syncwarp();
   int n_open = 1, n_done = 0;
   for (int level = 0; n_open > 0; ++level) {
-    const FrontBox* open = s_open[level & 1][warp];
-    FrontBox* next = s_open[(level + 1) & 1][warp];
+    const FrontBox* open = sh.open[level & 1];
+    FrontBox* next = sh.open[(level + 1) & 1];
     int n_next = 0;
     for (int base = 0; base < n_open; base += 32) {
       const bool have = base + int(lane) < n_open;
@@ -157,11 +158,40 @@ __global__ void __launch_bounds__(kFrontWarps * 32) k_probe_front(const FrontArg
   if (lane == 0) a.cnt[p] = uint32_t(n_done);
 }
 
+__global__ void __launch_bounds__(kFrontWarps * 32) k_probe_front(const FrontArgs a) {
+  __shared__ FrontShared sh[kFrontWarps];
+  const uint32_t warp = threadIdx.x >> 5, p = blockIdx.x * kFrontWarps + warp;
+  if (p < a.nprobes) front_probe(a, p, sh[warp]);
+}
+
+__global__ void __launch_bounds__(kFrontWarps * 32)
+    k_probe_front_batch(const BakeJobDev* __restrict__ jobs, uint32_t njobs, uint32_t total) {
+  __shared__ FrontShared sh[kFrontWarps];
+  const uint32_t warp = threadIdx.x >> 5, w = blockIdx.x * kFrontWarps + warp;
+  if (w >= total) return;
+  uint32_t lo = 0, hi = njobs - 1;  // the last job that begins at or before w
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi + 1) >> 1;
+    if (__ldg(&jobs[mid].front_begin) <= w) lo = mid; else hi = mid - 1;
+  }
+  const BakeJobDev& j = jobs[lo];
+  const uint32_t p = w - j.front_begin;
+  if (!j.front || p >= j.nprobes) return;
+  const FrontArgs a{j.nodes, j.ntris, j.probes, j.nprobes, j.front_scale, j.front_cap, const_cast<float4*>(j.front),
+                    const_cast<uint32_t*>(j.front_n), j.err};
+  front_probe(a, p, sh[warp]);
+}
+
 }  // namespace
 
 void launch_probe_front(const FrontArgs& a, cudaStream_t s) {
   if (!a.nprobes) return;
   k_probe_front<<<(a.nprobes + kFrontWarps - 1) / kFrontWarps, kFrontWarps * 32, 0, s>>>(a);
+}
+
+void launch_probe_front_batch(const BakeJobDev* jobs, uint32_t njobs, uint32_t total, cudaStream_t s) {
+  if (!total) return;
+  k_probe_front_batch<<<(total + kFrontWarps - 1) / kFrontWarps, kFrontWarps * 32, 0, s>>>(jobs, njobs, total);
 }
 
 }  // namespace vlbk

@@ -111,19 +111,21 @@ __device__ __forceinline__ void map_cell(const SunMap& m, const MapTri& T, int i
   }
 }
 
-// Slice y of a group of kMapThreads triangles: the rows of each that are
-// congruent to y modulo the slice count.
-__global__ void __launch_bounds__(kMapThreads) k_sun_map(const SunMap m, const float4* __restrict__ tris,
-                                                         uint32_t ntris) {
-  __shared__ MapTri st[kMapThreads];
-  __shared__ int s_end[kMapThreads];  // cells of triangles 0 .. k
-  __shared__ int s_warp[kMapThreads / 32];
+struct MapShared {
+  MapTri st[kMapThreads];
+  int end[kMapThreads];  // cells of triangles 0 .. k
+  int warp[kMapThreads / 32];
+};
+
+// One CTA: slice `slice` of a group of kMapThreads triangles, the rows of each
+// that are congruent to it modulo the slice count.
+__device__ __forceinline__ void map_draw(const SunMap& m, const float4* __restrict__ tris, uint32_t ntris,
+                                         uint32_t group, int slice, int slices, MapShared& sh) {
   const int tid = int(threadIdx.x), lane = tid & 31, warp = tid >> 5;
-  const int slices = int(gridDim.y), slice = int(blockIdx.y);
-  const uint32_t t = blockIdx.x * kMapThreads + threadIdx.x;
+  const uint32_t t = group * kMapThreads + threadIdx.x;
   int n = 0;
   if (t < ntris) {
-    MapTri& T = st[tid];
+    MapTri& T = sh.st[tid];
     map_setup(m, __ldg(tris + 3 * size_t(t)), __ldg(tris + 3 * size_t(t) + 1), __ldg(tris + 3 * size_t(t) + 2), T);
     int off = (slice - T.j0) % slices;
     off += off < 0 ? slices : 0;
@@ -136,32 +138,63 @@ __global__ void __launch_bounds__(kMapThreads) k_sun_map(const SunMap m, const f
     const int y = __shfl_up_sync(0xffffffffu, end, o);
     if (lane >= o) end += y;
   }
-  if (lane == 31) s_warp[warp] = end;
+  if (lane == 31) sh.warp[warp] = end;
   __syncthreads();
-  for (int k = 0; k < warp; ++k) end += s_warp[k];
-  s_end[tid] = end;
+  for (int k = 0; k < warp; ++k) end += sh.warp[k];
+  sh.end[tid] = end;
   __syncthreads();
-  const int total = s_end[kMapThreads - 1];
+  const int total = sh.end[kMapThreads - 1];
 #pragma unroll 2
   for (int c = tid; c < total; c += kMapThreads) {
     int k = 0;  // the first triangle whose end exceeds c
 #pragma unroll
     for (int step = kMapThreads / 2; step > 0; step >>= 1)
-      if (s_end[k + step - 1] <= c) k += step;
-    const MapTri& T = st[k];
-    const int at = c - (k ? s_end[k - 1] : 0), w = T.i1 - T.i0 + 1, r = at / w;
+      if (sh.end[k + step - 1] <= c) k += step;
+    const MapTri& T = sh.st[k];
+    const int at = c - (k ? sh.end[k - 1] : 0), w = T.i1 - T.i0 + 1, r = at / w;
     map_cell(m, T, T.i0 + at - r * w, T.first + r * slices);
   }
 }
 
+__global__ void __launch_bounds__(kMapThreads) k_sun_map(const SunMap m, const float4* __restrict__ tris,
+                                                         uint32_t ntris) {
+  __shared__ MapShared sh;
+  map_draw(m, tris, ntris, blockIdx.x, int(blockIdx.y), int(gridDim.y), sh);
+}
+
+__global__ void __launch_bounds__(kMapThreads) k_sun_map_batch(const BakeJobDev* __restrict__ jobs, uint32_t njobs) {
+  __shared__ MapShared sh;
+  uint32_t lo = 0, hi = njobs - 1;  // the last job that begins at or before this CTA
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi + 1) >> 1;
+    if (__ldg(&jobs[mid].map_begin) <= blockIdx.x) lo = mid; else hi = mid - 1;
+  }
+  const BakeJobDev& j = jobs[lo];
+  const uint32_t c = blockIdx.x - j.map_begin;
+  if (!j.sun_map.cells || c / j.map_slices * kMapThreads >= j.ntris) return;
+  map_draw(j.sun_map, j.tris, j.ntris, c / j.map_slices, int(c % j.map_slices), int(j.map_slices), sh);
+}
+
 }  // namespace
+
+// CTAs per group of triangles: about seven CTAs per SM in all.
+uint32_t sun_map_slices(uint32_t ntris) {
+  const uint32_t groups = (ntris + kMapThreads - 1) / kMapThreads;
+  return std::min(64u, std::max(2u, 1024u / std::max(groups, 1u)));
+}
 
 void launch_sun_map(const SunMap& m, const float4* tris, uint32_t ntris, cudaStream_t s) {
   if (!ntris) return;
   cudaMemsetAsync(m.cells, 0, size_t(m.G) * m.G * 8, s);
-  const uint32_t groups = (ntris + kMapThreads - 1) / kMapThreads;
-  const uint32_t slices = std::min(64u, std::max(2u, 1024u / groups));  // about seven CTAs per SM
-  k_sun_map<<<dim3(groups, slices), kMapThreads, 0, s>>>(m, tris, ntris);
+  const dim3 grid((ntris + kMapThreads - 1) / kMapThreads, sun_map_slices(ntris));
+  k_sun_map<<<grid, kMapThreads, 0, s>>>(m, tris, ntris);
+}
+
+void launch_sun_map_batch(const BakeJobDev* jobs, uint32_t njobs, uint32_t ctas, void* cells, size_t bytes,
+                          cudaStream_t s) {
+  if (!ctas) return;
+  cudaMemsetAsync(cells, 0, bytes, s);
+  k_sun_map_batch<<<ctas, kMapThreads, 0, s>>>(jobs, njobs);
 }
 
 }  // namespace vlbk

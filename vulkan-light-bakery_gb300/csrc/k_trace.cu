@@ -780,6 +780,8 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_trace_batch(const BakeJobD
     const uint32_t R = P * j.S;
     uint32_t r0 = c - j.ray_begin;                // the chunk's first ray in the job
     const uint32_t r1 = min(R, r0 + chunk);       // end of its real rays (the rest is padding)
+    const bool front = j.front && !j.hits_in;
+    int fnext = 0;  // next frontier entry of the group's walks, 0: none left
     for (;;) {
       const unsigned idle = __ballot_sync(kFull, !L.has);
       // a whole idle warp takes the chunk's next rays, in lane order: its rays
@@ -806,6 +808,7 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_trace_batch(const BakeJobD
             }
           }
         }
+        if (front) fnext = lr_front_next(j, L, L.has, 0, stack);
       }
       if (!__any_sync(kFull, L.has)) {
         if (r0 >= r1) break;
@@ -815,6 +818,10 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_trace_batch(const BakeJobD
       lr_park(L, stack);
       if (L.has && L.leaf >= 0) lr_leaf<false>(j, L, w);
       if (__any_sync(kFull, L.has && L.cur != kWalkEnd)) continue;  // the warp shades together, as in k_trace_dyn
+      if (fnext) {  // the group's primary walks go on with the rest of their frontier
+        fnext = lr_front_next(j, L, L.has, fnext, stack);
+        if (fnext || __any_sync(kFull, L.has && L.cur != kWalkEnd)) continue;
+      }
       if (!L.has) continue;
       if (!L.shadow && j.hits_out) j.hits_out[size_t(L.p) * j.S + L.s] = make_int2(L.slot, __float_as_int(L.tb));
       Shaded o;

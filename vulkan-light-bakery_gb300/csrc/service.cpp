@@ -391,7 +391,10 @@ bool vlb_service::launch_next(std::unique_lock<std::mutex>& lk) {
   vlb_bake_params bp = jp[0];
   const vlb_batch_schedule sc{0, 1, 0};
   bool host_out = false;
-  vlb_status st = vlbh::batch_launch(ctx, jobs.data(), ext.data(), uint32_t(nj), &bp, sc, &host_out);
+  // probe frontiers and sun maps (not needed for the results) stay within what the budget leaves
+  const uint64_t held = set_bytes + flight_bytes + bytes - keep_bytes;
+  vlb_status st = vlbh::batch_launch(ctx, jobs.data(), ext.data(), uint32_t(nj), &bp, sc, &host_out,
+                                     budget > held ? budget - held : 0);
   ctx->host_inputs_pending = false;  // pageable inputs were staged before the copies returned
   if (st == VLB_OK) {
     const cudaError_t e1 = cudaMemcpyAsync(bt.h_err, ctx->d_err, vlbk::kErrSlots * sizeof(int), cudaMemcpyDeviceToHost,

@@ -1028,12 +1028,13 @@ static bool grid_mode(const vlb_scene* scene, uint32_t nprobes, uint32_t S, cons
 
 // Entries per probe of a bake's probe frontiers (k_front.cu), 0 for walks from
 // the root.  A frontier costs a warp some twenty dependent loads per probe and
-// its rays share it: at 64 rays a probe that is a wash (64 probes: 94 us with
-// and without), at 256 it saves.  Trees deeper than the lane stack keep the
+// its rays share it: at 64 rays a probe a lone small bake breaks even (64
+// probes: 83 us with and without) and a batch gains (6.1 -> 5.6 ms); fewer
+// share it too little.  Trees deeper than the lane stack keep the
 // root (their walks may overflow the stack, and must say so).  1 GiB of
 // entries at most.
 static uint32_t front_cap(const vlb_scene* scene, uint64_t nprobes, uint32_t S) {
-  if (scene->ntris < 64 || scene->wnodes || scene->depth > uint32_t(vlbk::kLaneStack) || S < 128 || !nprobes) return 0;
+  if (scene->ntris < 64 || scene->wnodes || scene->depth > uint32_t(vlbk::kLaneStack) || S < 64 || !nprobes) return 0;
   const uint64_t cap = std::min<uint64_t>(vlbk::kFrontCap, (1ull << 25) / nprobes);
   return cap < 32 ? 0 : uint32_t(cap);
 }
@@ -1050,6 +1051,10 @@ static float bounds_scale(const vlb_scene* scene) {
 // for 55 us in the tile walk, nothing gained in the fused walk).  256 cells a
 // side: 512 save 6 % more of that trace and cost 25 us more.
 constexpr uint32_t kMapSide = 256;
+constexpr size_t kMapBytes = size_t(kMapSide) * kMapSide * 8;
+// In a batch one launch draws the maps of all jobs, so only the drawing itself
+// counts: about 60 rays a triangle in the box scenes.
+constexpr uint64_t kBatchMapRays = 1ull << 16;
 static bool sun_map_pays(uint64_t rays, uint32_t ntris) { return rays >= std::max(1ull << 19, 24ull * ntris); }
 
 // Plane, extent and margins of a scene's sun map (k_lightmap.cu).
@@ -1154,7 +1159,7 @@ static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const floa
   if (a.lane && !from_root && a.ntris && a.shading == VLB_SHADE_LAMBERT_SUN &&
       sun_map_pays(uint64_t(nprobes) * a.S, scene->ntris)) {
     void* cells;
-    if ((st = scratch(ctx, "sun_map", size_t(kMapSide) * kMapSide * 8, &cells))) return st;
+    if ((st = scratch(ctx, "sun_map", kMapBytes, &cells))) return st;
     sun_map_plan(scene, a.sun, a.bias, kMapSide, static_cast<uint32_t*>(cells), &a.sun_map);
     KScope k(ctx, "sun_map");
     vlbk::launch_sun_map(a.sun_map, scene->tris, scene->ntris, ctx->stream);
@@ -1440,6 +1445,10 @@ struct BatchBufs {
   uint32_t* counter;
   size_t table_bytes, dst_off, p0_off, np_off;
   uint32_t ndev_out;   // jobs whose output is device memory (scattered by a kernel)
+  uint32_t front_total;  // probes with a frontier
+  uint32_t map_ctas;     // CTAs that draw the jobs' sun maps
+  void* maps;
+  size_t map_bytes;
 };
 
 }  // namespace
@@ -1509,6 +1518,14 @@ static vlb_status batch_enqueue(vlb_ctx* ctx, const BatchPlan& pl, const BatchBu
     KScope k(ctx, "probe_order_batch");
     vlbk::launch_probe_order_batch(table, ntable, ctx->stream);
   }
+  if (bb.front_total) {
+    KScope k(ctx, "probe_front_batch");
+    vlbk::launch_probe_front_batch(table, ntable, bb.front_total, ctx->stream);
+  }
+  if (bb.map_ctas) {
+    KScope k(ctx, "sun_map_batch");
+    vlbk::launch_sun_map_batch(table, ntable, bb.map_ctas, bb.maps, bb.map_bytes, ctx->stream);
+  }
   if (pl.fused) {
     KScope k(ctx, "trace_fused_batch");
     vlbk::launch_trace_fused_lane(table, ctx->batch_table[0], ntable, total_rays, pl.K, bb.counter, fs,
@@ -1548,7 +1565,8 @@ static vlb_status batch_enqueue(vlb_ctx* ctx, const BatchPlan& pl, const BatchBu
 // memory); *host_out tells whether there were any.  ext (optional, njobs
 // entries) adds kept-hit outputs and relight inputs per job.
 vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh::JobExt* ext, uint32_t njobs,
-                              const vlb_bake_params* params, const vlb_batch_schedule& sc, bool* host_out_any) {
+                              const vlb_bake_params* params, const vlb_batch_schedule& sc, bool* host_out_any,
+                              uint64_t spare_bytes) {
   *host_out_any = false;
   BatchPlan pl;
   vlb_status st = batch_plan(ctx, jobs, njobs, params, &pl);
@@ -1586,6 +1604,32 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
   bb.sort = static_cast<uint32_t*>(sort); bb.tile = static_cast<uint8_t*>(tile); bb.out = static_cast<float*>(out);
   bb.meta = static_cast<uint8_t*>(meta); bb.counter = static_cast<uint32_t*>(counter);
 
+  // Probe frontiers and sun maps, where they pay and device memory for them is
+  // to be had (without them the walks start at the root and trace every shadow
+  // ray: the same results).
+  uint64_t front_probes = 0;
+  std::vector<uint8_t> fronts(ntable), maps(ntable);
+  for (uint32_t i = 0; i < ntable; ++i) {
+    const BatchJob& b = pl.jobs[i];
+    const vlb_scene* sc = jobs[b.idx].scene;
+    fronts[i] = !(ext && ext[b.idx].hits_in) && front_cap(sc, b.nprobes, b.S) != 0;
+    maps[i] = sc->ntris && b.p->shading == VLB_SHADE_LAMBERT_SUN &&
+              uint64_t(b.nprobes) * b.S >= std::max<uint64_t>(kBatchMapRays, 64ull * sc->ntris);
+    if (fronts[i]) front_probes += b.nprobes;
+    if (maps[i]) bb.map_bytes += kMapBytes;
+  }
+  uint32_t cap = 0;
+  void *front_ent = nullptr, *front_n = nullptr;
+  if (front_probes) {
+    cap = uint32_t(std::min<uint64_t>(vlbk::kFrontCap, std::min<uint64_t>(1ull << 25, spare_bytes / 64) / front_probes));
+    if (cap < 32 || scratch(ctx, "batch_front", front_probes * cap * 32, &front_ent) != VLB_OK ||
+        scratch(ctx, "batch_front_n", front_probes * 4, &front_n) != VLB_OK)
+      cap = 0;
+  }
+  if (bb.map_bytes && (bb.map_bytes > std::min<uint64_t>(256ull << 20, spare_bytes / 4) ||
+                       scratch(ctx, "batch_maps", bb.map_bytes, &bb.maps) != VLB_OK))
+    bb.map_bytes = 0;
+
   // stage host probes, build the job table
   const size_t esz = pl.bf16 && !pl.split ? 2 : 4;
   uint64_t warp_rays = 0;
@@ -1605,7 +1649,7 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
       if ((st = dirset_split_basis(ctx, g.dirs))) return st;
   auto& table = ctx->batch_table;
   table.assign(ntable, vlbk::BakeJobDev{});
-  size_t poff = 0, part_off = 0;
+  size_t poff = 0, part_off = 0, nmaps = 0;
   uint64_t items = 0;
   for (uint32_t t = 0; t < ntable; ++t) {
     const BatchJob& b = pl.jobs[ord[t]];
@@ -1659,6 +1703,21 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
       d.ray_begin = uint32_t(items);
       items += ((uint64_t(b.nprobes) + 31) / 32 * 32 * b.S + chunk - 1) / chunk * chunk;
     }
+    d.front_begin = bb.front_total;
+    if (cap && fronts[ord[t]]) {
+      d.front = static_cast<const float4*>(front_ent) + size_t(bb.front_total) * cap * 2;
+      d.front_n = static_cast<const uint32_t*>(front_n) + bb.front_total;
+      d.front_cap = cap;
+      d.front_scale = bounds_scale(j.scene);
+      bb.front_total += b.nprobes;
+    }
+    d.map_begin = bb.map_ctas;
+    if (bb.map_bytes && maps[ord[t]]) {
+      sun_map_plan(j.scene, d.sun, d.bias, kMapSide,
+                   reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(bb.maps) + nmaps++ * kMapBytes), &d.sun_map);
+      d.map_slices = vlbk::sun_map_slices(d.ntris);
+      bb.map_ctas += vlbk::sun_map_ctas(d.ntris);
+    }
     for (int a = 0; a < 6; ++a) d.bounds[a] = j.scene->bounds[a];
     d.sort_scratch = bb.sort + 4 * b.row0;
     if (ext) { d.hits_out = ext[b.idx].hits_out; d.hits_in = ext[b.idx].hits_in; }
@@ -1688,7 +1747,8 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
                                uint64_t(uintptr_t(tile)), uint64_t(uintptr_t(out)), uint64_t(uintptr_t(meta)),
                                uint64_t(uintptr_t(counter)), uint64_t(ctx->num_sms), pl.fused,
                                uint64_t(uintptr_t(part)), uint64_t(uintptr_t(done)), pl.rows, sc.ctas_per_sm,
-                               sc.node_steps, sc.refill_idle};
+                               sc.node_steps, sc.refill_idle, bb.front_total, bb.map_ctas,
+                               uint64_t(uintptr_t(bb.maps)), bb.map_bytes};
   if (pl.fused && ntable == 1) {  // one job goes to the kernel by value: its fields are part of the shape
     const auto* w = reinterpret_cast<const uint64_t*>(table.data());
     key.insert(key.end(), w, w + sizeof(vlbk::BakeJobDev) / 8);

@@ -204,6 +204,9 @@ struct FrontArgs {
   int* err;
 };
 void launch_probe_front(const FrontArgs& a, cudaStream_t s);
+struct BakeJobDev;
+// The frontiers of all jobs that have one: `total` probes, numbered by front_begin.
+void launch_probe_front_batch(const BakeJobDev* jobs, uint32_t njobs, uint32_t total, cudaStream_t s);
 
 // ---- sun maps (k_lightmap.cu) ------------------------------------------------------
 struct SunMap {
@@ -214,7 +217,13 @@ struct SunMap {
   float margin;
   uint32_t G;
 };
+uint32_t sun_map_slices(uint32_t ntris);
+inline uint32_t sun_map_ctas(uint32_t ntris) { return (ntris + 255) / 256 * sun_map_slices(ntris); }
 void launch_sun_map(const SunMap& m, const float4* tris, uint32_t ntris, cudaStream_t s);
+// The maps of all jobs that have one (`ctas` CTAs numbered by map_begin); their
+// cells, `bytes` from `cells`, are cleared first.
+void launch_sun_map_batch(const BakeJobDev* jobs, uint32_t njobs, uint32_t ctas, void* cells, size_t bytes,
+                          cudaStream_t s);
 
 // ---- trace + shade --------------------------------------------------------------
 struct TraceArgs {
@@ -316,6 +325,9 @@ struct BakeJobDev {
   const float4* front;    // probe frontiers (FrontArgs.ent) or null
   const uint32_t* front_n;
   uint32_t front_cap;
+  float front_scale;      // FrontArgs.scale
+  uint32_t front_begin;   // first warp of this job in the frontier launch
+  uint32_t map_begin, map_slices;  // first CTA of this job in the sun-map launch, CTAs per 256 triangles
   // probes and directions
   const float* probes;    // device nprobes*3
   uint32_t* order;        // device nprobes: packet slot -> probe (written by the batched sort)
@@ -437,7 +449,8 @@ struct JobExt {
   const int2* hits_in = nullptr;
 };
 vlb_status batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const JobExt* ext, uint32_t njobs,
-                        const vlb_bake_params* params, const vlb_batch_schedule& sc, bool* host_out_any);
+                        const vlb_bake_params* params, const vlb_batch_schedule& sc, bool* host_out_any,
+                        uint64_t spare_bytes = ~0ull);
 // Launch-error check, and (sync) stream synchronisation + device error counters.
 vlb_status ctx_finish(vlb_ctx* ctx, bool sync);
 // Collapses the scene's binary traversal tree into the 8-wide quantised tree
