@@ -112,10 +112,18 @@ __device__ __forceinline__ void project_stage(const T* __restrict__ rad, uint32_
 constexpr uint32_t kProjSplitCtas = 304;
 constexpr uint32_t kProjMinSplitSamples = 16 * kProjCols;
 
+//
+// Tiles of at least kProjStream samples stream through the TMA-staged kernel:
+// there the unit is a 256-row tile and a split, three CTAs per SM.
+constexpr size_t kProjStream = size_t(1) << 24;
+constexpr uint32_t kProjStreamUnits = 456;
+
 static uint32_t project_splits(uint32_t rows, uint32_t S, uint32_t* per) {
-  const uint32_t tiles = (rows + kProjRows - 1) / kProjRows;
+  const uint32_t tiles = (rows + kProjRows - 1) / kProjRows, tiles256 = (rows + 255) / 256;
   uint32_t splits = 1;
-  if (tiles && tiles < kProjSplitCtas)
+  if (size_t(rows) * S >= kProjStream && S % 4 == 0 && tiles < kProjSplitCtas)
+    splits = std::max(1u, std::min(kProjStreamUnits / tiles256, S / kProjMinSplitSamples));
+  else if (tiles && tiles < kProjSplitCtas)
     splits = std::max(1u, std::min((kProjSplitCtas + tiles - 1) / tiles, S / kProjMinSplitSamples));
   uint32_t p = (S + splits - 1) / splits;
   p = (p + kProjCols - 1) / kProjCols * kProjCols;  // whole stages
@@ -205,12 +213,18 @@ static void launch_project(const T* rad, uint32_t nprobes, uint32_t S, const flo
 void launch_project_f32(const float* radiance, uint32_t nprobes, uint32_t S, const float* basis16, uint32_t K,
                         float* out, float* partial, cudaStream_t s, int* err, int num_sms, uint32_t hold,
                         uint32_t wait_polls) {
-  // unsplit tiles (enough rows for the whole GPU) go through the TMA-staged kernel
+  // tiles with enough rows for the whole GPU, and split tiles large enough to
+  // stream, go through the TMA-staged kernel (343 probes x 3141 x 1000 samples:
+  // 7.63 ms here, 3.34 there, 57 % of the HBM copy rate)
   uint32_t per = 0;
   const uint32_t rows = nprobes * 3;
-  if (err && num_sms && S && project_splits(rows, S, &per) == 1 &&
-      launch_project_f32_tma(radiance, nprobes, S, basis16, K, out, err, num_sms, s, hold, wait_polls))
+  const uint32_t splits = S ? project_splits(rows, S, &per) : 1;
+  if (err && num_sms && S && (splits == 1 || size_t(rows) * S >= kProjStream) &&
+      launch_project_f32_tma(radiance, nprobes, S, basis16, K, out, partial, splits, splits == 1 ? S : per, err,
+                             num_sms, s, hold, wait_polls)) {
+    if (splits > 1) k_project_reduce<<<(rows * K + 255) / 256, 256, 0, s>>>(partial, splits, rows, K, out);
     return;
+  }
   launch_project<float>(radiance, nprobes, S, basis16, K, out, partial, 0, s);
 }
 
