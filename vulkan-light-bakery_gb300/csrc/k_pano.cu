@@ -1,0 +1,238 @@
+// k_pano.cu -- SH projection of panoramas and equirect env maps
+// (shaders/skybox_sh.comp:23-42, shaders/sh.comp:23-42), row by row.
+//
+// On an equirect image every basis function of l <= 3 is a trigonometric
+// polynomial of degree <= 3 along a row, times a function of the row.  So a row
+// needs only seven sums per channel (five for l <= 2) -- the texels times 1,
+// cos, sin of phi, 2 phi and 3 phi -- instead of sixteen, and no basis per texel:
+//   k_pano_rows     one warp per row segment: the sums, texels in pairs by packed
+//                   FMAs, reduced across the warp; 84 bytes per 1024 texels
+//   k_pano_combine  one CTA per map: the rows' sums into coefficients
+// The reference adds every texel's 48 products into 48 floats with an
+// unsynchronised read-modify-write (skybox_sh.comp:39).  Here the segments and
+// the order of every sum are functions of the image size, so a map's
+// coefficients are the same alone or in a batch.
+//
+// Texel loads need no alignment beyond their own.  One 2048 x 1024 RGBA8 image
+// takes 18.8 us a call, most of it the two launches' latency; with a basis per
+// texel, 2048 partials per value added by one thread and the tables made on the
+// host it took 256 us.
+#include "vlb_device.cuh"
+#include "vlb_internal.h"
+
+namespace vlbk {
+namespace {
+
+constexpr int kPanoWarps = 8;
+constexpr uint32_t kPanoSeg = 1024;   // texels of a row segment
+constexpr int kPanoSums = 24;         // floats per segment: [channel][8], the last of each unused
+constexpr int kPanoThreads = 512;
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(d)
+      : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)),
+        "l"(*reinterpret_cast<uint64_t*>(&c)));
+  return *reinterpret_cast<float2*>(&d);
+}
+
+template <int FMT>
+__device__ __forceinline__ void load_rgb(const void* __restrict__ texels, size_t i, float* c) {
+  if constexpr (FMT == 0) {
+    const float* f = static_cast<const float*>(texels) + 3 * i;
+    c[0] = __ldg(f); c[1] = __ldg(f + 1); c[2] = __ldg(f + 2);
+  } else {
+    const uint32_t q = __ldg(static_cast<const uint32_t*>(texels) + i);  // UNORM bytes, scaled with the row
+    c[0] = float(q & 255u); c[1] = float((q >> 8) & 255u); c[2] = float((q >> 16) & 255u);
+  }
+}
+
+// rows: [map][row][segment][kPanoSums].  LMAX 2 leaves the 3 phi sums out.
+template <int LMAX, int FMT>
+__global__ void __launch_bounds__(kPanoWarps * 32) k_pano_rows(const SkyboxArgs a, float* __restrict__ rows,
+                                                               uint32_t nseg, uint32_t units) {
+  constexpr int M = LMAX == 3 ? 7 : 5;
+  const uint32_t lane = threadIdx.x & 31, u = blockIdx.x * kPanoWarps + (threadIdx.x >> 5);
+  if (u >= units) return;
+  const uint32_t row = u / nseg, seg = u - row * nseg;  // row: over all maps' rows
+  const uint32_t x0 = seg * kPanoSeg, x1 = min(a.w, x0 + kPanoSeg);
+  const size_t at = size_t(row) * a.w;
+  float2 acc[3][M];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int m = 0; m < M; ++m) acc[c][m] = make_float2(0.f, 0.f);
+#pragma unroll 4
+  for (uint32_t x = x0 + lane; x < x1; x += 64) {
+    const bool two = x + 32 < x1;
+    float t0[3], t1[3] = {0.f, 0.f, 0.f};
+    load_rgb<FMT>(a.texels, at + x, t0);
+    if (two) load_rgb<FMT>(a.texels, at + x + 32, t1);
+    const float2 p = __ldg(a.col_tab + x), q = __ldg(a.col_tab + (two ? x + 32 : x));
+    const float2 c1 = make_float2(p.x, q.x), s1 = make_float2(p.y, q.y);
+    const float2 one = make_float2(1.f, 1.f), zero = make_float2(0.f, 0.f), neg = make_float2(-1.f, -1.f);
+    const float2 two_c = fma2(c1, one, c1);
+    const float2 c2 = fma2(two_c, c1, neg), s2 = fma2(two_c, s1, zero);  // cos 2phi = 2 cos^2 - 1, sin 2phi
+    float2 f[7] = {one, c1, s1, c2, s2, zero, zero};
+    if constexpr (M == 7) {
+      f[5] = fma2(two_c, c2, make_float2(-c1.x, -c1.y));  // cos 3phi = 2 cos phi cos 2phi - cos phi
+      f[6] = fma2(two_c, s2, make_float2(-s1.x, -s1.y));
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float2 t = make_float2(t0[c], t1[c]);
+#pragma unroll
+      for (int m = 0; m < M; ++m) acc[c][m] = fma2(t, f[m], acc[c][m]);
+    }
+  }
+  float v[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = i / 8 < 3 && i % 8 < M ? acc[i / 8 < 3 ? i / 8 : 0][i % 8 < M ? i % 8 : 0].x +
+                                                                  acc[i / 8 < 3 ? i / 8 : 0][i % 8 < M ? i % 8 : 0].y
+                                                            : 0.f;
+  const float s = warp_sums<32>(v);
+  if (lane < kPanoSums) rows[size_t(u) * kPanoSums + lane] = s;
+}
+
+// A row's coefficients from its sums f = {1, c1, s1, c2, s2, c3, s3} at (sin
+// theta, cos theta): the products of shaders/sh_common.h:26-116 with the powers
+// of sin phi and cos phi written as multiple angles.  PANO: the basis at dir.xzy
+// (skybox_sh.comp:39).
+template <int LMAX, bool PANO>
+__device__ __forceinline__ void row_coeffs(float s, float c, const float* f, float* o) {
+  const float s2 = s * s, c2 = c * c, sc = s * c, s3 = s2 * s, s2c = s2 * c;
+  o[0] = 0.282095f * f[0];
+  if constexpr (!PANO) {
+    o[1] = -0.488603f * s * f[2];
+    o[2] = 0.488603f * c * f[0];
+    o[3] = -0.488603f * s * f[1];
+    o[4] = 1.092548f * 0.5f * s2 * f[4];
+    o[5] = -1.092548f * sc * f[2];
+    o[6] = 0.315392f * (2.f * c2 - s2) * f[0];
+    o[7] = -1.092548f * sc * f[1];
+    o[8] = 0.546274f * s2 * f[3];
+    if constexpr (LMAX == 3) {
+      o[9] = -0.590044f * s3 * f[6];
+      o[10] = 2.890611f * 0.5f * s2c * f[4];
+      o[11] = -0.457046f * s * (4.f * c2 - s2) * f[2];
+      o[12] = 0.373176f * c * (2.f * c2 - 3.f * s2) * f[0];
+      o[13] = -0.457046f * s * (4.f * c2 - s2) * f[1];
+      o[14] = 1.445306f * s2c * f[3];
+      o[15] = -0.590044f * s3 * f[5];
+    }
+  } else {
+    o[1] = -0.488603f * c * f[0];
+    o[2] = 0.488603f * s * f[2];
+    o[3] = -0.488603f * s * f[1];
+    o[4] = 1.092548f * sc * f[1];
+    o[5] = -1.092548f * sc * f[2];
+    o[6] = 0.315392f * ((0.5f * s2 - c2) * f[0] - 1.5f * s2 * f[3]);
+    o[7] = -1.092548f * 0.5f * s2 * f[4];
+    o[8] = 0.546274f * ((0.5f * s2 - c2) * f[0] + 0.5f * s2 * f[3]);
+    if constexpr (LMAX == 3) {
+      o[9] = -0.590044f * c * ((1.5f * s2 - c2) * f[0] + 1.5f * s2 * f[3]);
+      o[10] = 2.890611f * 0.5f * s2c * f[4];
+      o[11] = -0.457046f * c * ((1.5f * s2 - c2) * f[0] - 2.5f * s2 * f[3]);
+      o[12] = 0.373176f * (s * (0.75f * s2 - 3.f * c2) * f[2] - 1.25f * s3 * f[6]);
+      o[13] = -0.457046f * (s * (0.25f * s2 - c2) * f[1] - 1.25f * s3 * f[5]);
+      o[14] = 1.445306f * (s * (0.25f * s2 - c2) * f[2] + 0.25f * s3 * f[6]);
+      o[15] = -0.590044f * (s * (0.75f * s2 - 3.f * c2) * f[1] + 0.25f * s3 * f[5]);
+    }
+  }
+}
+
+// One CTA per map: a thread takes every kPanoThreads-th row, the warps' sums are
+// added in FP64 in warp order.
+template <int LMAX, bool PANO>
+__global__ void __launch_bounds__(kPanoThreads) k_pano_combine(const SkyboxArgs a, const float* __restrict__ rows,
+                                                               uint32_t nseg, float* __restrict__ out) {
+  constexpr int K = sh_k<LMAX>();
+  __shared__ float s_sum[kPanoThreads / 32][3][16];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, map = blockIdx.x;
+  float acc[3][16];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int k = 0; k < 16; ++k) acc[c][k] = 0.f;
+  for (uint32_t y = tid; y < a.h; y += kPanoThreads) {
+    const float4 rw = __ldg(a.row_tab + y);  // sin theta, cos theta, weight
+    const float w = a.fmt == VLB_TEXEL_RGBA8 ? rw.z * (1.0f / 255.0f) : rw.z;
+    const float4* r = reinterpret_cast<const float4*>(rows) + (size_t(map) * a.h + y) * nseg * (kPanoSums / 4);
+    float f[kPanoSums];
+#pragma unroll
+    for (int i = 0; i < kPanoSums; ++i) f[i] = 0.f;
+    for (uint32_t g = 0; g < nseg; ++g)
+#pragma unroll
+      for (int i = 0; i < kPanoSums / 4; ++i) {
+        const float4 x = __ldg(r + g * (kPanoSums / 4) + i);
+        f[4 * i] += x.x; f[4 * i + 1] += x.y; f[4 * i + 2] += x.z; f[4 * i + 3] += x.w;
+      }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      float o[16];
+      row_coeffs<LMAX, PANO>(rw.x, rw.y, f + 8 * c, o);
+#pragma unroll
+      for (int k = 0; k < K; ++k) acc[c][k] = fmaf(w, o[k], acc[c][k]);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const float s = warp_sums<16>(acc[c]);
+    if (lane < 16) s_sum[warp][c][lane] = s;
+  }
+  __syncthreads();
+  if (tid < 3 * K) {
+    const int k = int(tid) / 3, c = int(tid) - 3 * k;
+    double s = 0.0;
+    for (int w = 0; w < kPanoThreads / 32; ++w) s += double(s_sum[w][c][k]);
+    const int co = a.flags & VLB_SKY_REF_BGRA_SWAP ? 2 - c : c;
+    out[(size_t(map) * K + k) * 3 + co] = float(s);
+  }
+}
+
+template <int LMAX>
+void launch(const SkyboxArgs& a, float* rows, float* out, cudaStream_t s) {
+  const uint32_t nseg = (a.w + kPanoSeg - 1) / kPanoSeg, units = a.count * a.h * nseg;
+  const uint32_t grid = (units + kPanoWarps - 1) / kPanoWarps;
+  if (a.fmt == VLB_TEXEL_RGB32F) k_pano_rows<LMAX, 0><<<grid, kPanoWarps * 32, 0, s>>>(a, rows, nseg, units);
+  else k_pano_rows<LMAX, 1><<<grid, kPanoWarps * 32, 0, s>>>(a, rows, nseg, units);
+  if (a.layout == VLB_SKY_PANORAMA) k_pano_combine<LMAX, true><<<a.count, kPanoThreads, 0, s>>>(a, rows, nseg, out);
+  else k_pano_combine<LMAX, false><<<a.count, kPanoThreads, 0, s>>>(a, rows, nseg, out);
+}
+
+}  // namespace
+
+// Direction tables: per column (cos phi, sin phi), per row (sin theta, cos theta,
+// pixel weight) with the reference's PI (shaders/sh_common.h:1, :14-22;
+// sh.comp:28-33, skybox_sh.comp:28: phi - PI/2).
+__global__ void k_pano_tables(float2* col, float4* row, uint32_t w, uint32_t h, int shift) {
+  const double pi = 3.1415926538;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < w) {
+    double phi = 2.0 * pi * (double(i) + 0.5) / double(w);
+    if (shift) phi -= pi / 2.0;
+    col[i] = make_float2(float(cos(phi)), float(sin(phi)));
+  }
+  if (i < h) {
+    const double th = pi * (double(i) + 0.5) / double(h);
+    const double area = (2.0 * pi / w) * (pi / h);
+    row[i] = make_float4(float(sin(th)), float(cos(th)), float(area * sin(th)), 0.f);
+  }
+}
+
+void launch_pano_tables(float2* col, float4* row, uint32_t w, uint32_t h, bool shift, cudaStream_t s) {
+  const uint32_t n = w > h ? w : h;
+  k_pano_tables<<<(n + 63) / 64, 64, 0, s>>>(col, row, w, h, shift ? 1 : 0);
+}
+
+size_t pano_rows_bytes(uint32_t w, uint32_t h, uint32_t count) {
+  return size_t(count) * h * ((w + kPanoSeg - 1) / kPanoSeg) * kPanoSums * sizeof(float);
+}
+
+void launch_pano_sh(const SkyboxArgs& a, float* rows, float* out, cudaStream_t s) {
+  if (a.lmax == 2) launch<2>(a, rows, out, s);
+  else launch<3>(a, rows, out, s);
+}
+
+}  // namespace vlbk

@@ -66,24 +66,6 @@ cudaError_t scratch_address(int dev, unsigned char** out) {
   return cudaSuccess;
 }
 
-// Panorama direction tables on the device (no host buffers): per column
-// (cos phi, sin phi), per row (sin theta, cos theta, pixel weight) with the
-// reference's PI (shaders/sh_common.h:1, :14-22; sh.comp:32-33).
-__global__ void k_pano_tables(float2* col, float4* row, uint32_t w, uint32_t h, int shift) {
-  const double pi = 3.1415926538;
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < w) {
-    double phi = 2.0 * pi * (double(i) + 0.5) / double(w);
-    if (shift) phi -= pi / 2.0;
-    col[i] = make_float2(float(cos(phi)), float(sin(phi)));
-  }
-  if (i < h) {
-    const double th = pi * (double(i) + 0.5) / double(h);
-    const double area = (2.0 * pi / w) * (pi / h);
-    row[i] = make_float4(float(sin(th)), float(cos(th)), float(area * sin(th)), 0.f);
-  }
-}
-
 bool on_device(const void* p, int dev) {
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
@@ -146,8 +128,7 @@ extern "C" vlb_status vlb_skybox_sh_noalloc(const void* texels, vlb_texel_format
     vlbk::launch_cube_solid_angle(table, w, s);
     a.solid_angle = table;
   } else {
-    const uint32_t n = std::max(w, h);
-    k_pano_tables<<<(n + 255) / 256, 256, 0, s>>>(col, row, w, h, layout == VLB_SKY_PANORAMA);
+    vlbk::launch_pano_tables(col, row, w, h, layout == VLB_SKY_PANORAMA, s);
     a.col_tab = col; a.row_tab = row;
   }
   if (launch_failed()) return VLB_ERR_CUDA;

@@ -447,6 +447,7 @@ void vlb_ctx_destroy(vlb_ctx* ctx) {
   for (auto& kv : ctx->scratch) cudaFree(kv.second.p);
   for (auto& kv : ctx->cube_sa) cudaFree(kv.second);
   for (auto& kv : ctx->cube_pt) cudaFree(kv.second);
+  for (auto& kv : ctx->pano_tab) cudaFree(kv.second);
   if (ctx->d_err) cudaFree(ctx->d_err);
   if (ctx->h_err) cudaFreeHost(ctx->h_err);
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
@@ -809,6 +810,32 @@ static vlb_status cube_sa_table(vlb_ctx* ctx, uint32_t n, const float** out) {
   return VLB_OK;
 }
 
+constexpr size_t kPanoRowBytes = 256u << 20;
+
+// Direction tables of a panorama size: kept by the context like the cubemap
+// tables, all dropped when a 33rd size comes.
+static vlb_status pano_tables_device(vlb_ctx* ctx, uint32_t w, uint32_t h, bool shift, const float2** col,
+                                     const float4** row) {
+  const uint64_t key = (uint64_t(w) << 33) | (uint64_t(h) << 1) | (shift ? 1 : 0);
+  auto it = ctx->pano_tab.find(key);
+  if (it == ctx->pano_tab.end()) {
+    if (ctx->pano_tab.size() >= vlb_ctx::kPanoTables) {
+      VLB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+      for (auto& kv : ctx->pano_tab) cudaFree(kv.second);
+      ctx->pano_tab.clear();
+    }
+    float4* p = nullptr;
+    VLB_CUDA(ctx, cudaMalloc(&p, size_t(h) * 16 + size_t(w) * 8));
+    KScope k(ctx, "pano_tables");
+    vlbk::launch_pano_tables(reinterpret_cast<float2*>(p + h), p, w, h, shift, ctx->stream);
+    it = ctx->pano_tab.emplace(key, p).first;
+    VLB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // a later call may use another stream
+  }
+  *row = it->second;
+  *col = reinterpret_cast<const float2*>(it->second + h);
+  return VLB_OK;
+}
+
 vlb_status vlb_skybox_sh_batched(vlb_ctx* ctx, const void* texels, vlb_texel_format fmt, vlb_sky_layout layout,
                                  uint32_t w, uint32_t h, uint32_t count, uint32_t lmax, uint32_t flags, float* out) {
   if (!ctx) return VLB_ERR_INVALID;
@@ -839,16 +866,27 @@ vlb_status vlb_skybox_sh_batched(vlb_ctx* ctx, const void* texels, vlb_texel_for
     if (!st && w <= 1024) st = cube_pair_table(ctx, w, lmax, &a.pair_table);
     if (st) return st;
   } else {
-    std::vector<float> col, row;
-    pano_tables(w, h, layout == VLB_SKY_PANORAMA, col, row);
-    void *dc, *dr;
-    if ((st = scratch(ctx, "pano_col", col.size() * 4, &dc)) || (st = scratch(ctx, "pano_row", row.size() * 4, &dr)))
-      return st;
-    VLB_CUDA(ctx, cudaMemcpyAsync(dc, col.data(), col.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-    VLB_CUDA(ctx, cudaMemcpyAsync(dr, row.data(), row.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-    VLB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // host vectors go out of scope
-    a.col_tab = static_cast<const float2*>(dc);
-    a.row_tab = static_cast<const float4*>(dr);
+    if ((st = pano_tables_device(ctx, w, h, layout == VLB_SKY_PANORAMA, &a.col_tab, &a.row_tab))) return st;
+    // row by row (k_pano.cu), as many maps at a time as kPanoRowBytes of row
+    // sums hold; images of millions of narrow rows go texel by texel
+    const size_t per_map = vlbk::pano_rows_bytes(w, h, 1);
+    if (per_map <= kPanoRowBytes) {
+      const uint32_t maps = uint32_t(std::min<size_t>(count, kPanoRowBytes / per_map));
+      void* rows;
+      OutBuf ob;
+      if ((st = scratch(ctx, "pano_rows", per_map * maps, &rows)) ||
+          (st = stage_out(ctx, out, size_t(count) * V * 4, "sky_out", &ob)))
+        return st;
+      for (uint32_t m = 0; m < count; m += maps) {
+        vlbk::SkyboxArgs part = a;
+        part.texels = static_cast<const uint8_t*>(dtex) + size_t(m) * T * TB;
+        part.count = std::min(maps, count - m);
+        KScope k(ctx, "pano_sh", 2);
+        vlbk::launch_pano_sh(part, static_cast<float*>(rows), static_cast<float*>(ob.dev) + size_t(m) * V, ctx->stream);
+      }
+      if ((st = copy_out(ctx, ob))) return st;
+      return finish(ctx, ob.host);
+    }
   }
   vlbk::skybox_plan(a, 0);
   const uint32_t spm = a.slabs_per_map;

@@ -107,4 +107,26 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+// Sums N values across the warp, N a power of two up to 32; lane l ends with the
+// sum of v[l % N].  Every step halves the values a lane carries: N - 1
+// shuffles (and log2(32 / N) more), against 5 N of N warp_sums.
+template <int N>
+__device__ __forceinline__ float warp_sums(float (&v)[N]) {
+  const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+  for (int n = N / 2; n >= 1; n /= 2) {
+    const bool up = lane & n;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float send = up ? v[i] : v[i + n];
+      const float keep = up ? v[i + n] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, n);
+    }
+  }
+  float s = v[0];
+#pragma unroll
+  for (int n = N; n < 32; n *= 2) s += __shfl_xor_sync(0xffffffffu, s, n);
+  return s;
+}
+
 }  // namespace vlbk

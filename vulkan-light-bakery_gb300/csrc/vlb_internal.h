@@ -118,6 +118,11 @@ void launch_cube_pair_table(float2* out, uint32_t n, uint32_t lmax, cudaStream_t
 void skybox_plan(SkyboxArgs& a, uint32_t max_slabs);
 // Returns the partials per map it wrote (the slab count for launch_sh_finalize).
 int launch_skybox_sh(const SkyboxArgs& a, bool tma, int num_sms, cudaStream_t s);
+// Panoramas and env maps (k_pano.cu): direction tables (w float2, h float4), and
+// the projection of a.count maps with scratch `rows` of pano_rows_bytes.
+void launch_pano_tables(float2* col, float4* row, uint32_t w, uint32_t h, bool shift, cudaStream_t s);
+size_t pano_rows_bytes(uint32_t w, uint32_t h, uint32_t count);
+void launch_pano_sh(const SkyboxArgs& a, float* rows, float* out, cudaStream_t s);
 // out[m][v] = sum_j partial[m][j][v] in FP64, j in fixed order.
 void launch_sh_finalize(const float* partial, uint32_t nmaps, uint32_t slabs, uint32_t nvals, float* out,
                         cudaStream_t s);
@@ -487,6 +492,10 @@ struct vlb_ctx {
   std::map<std::string, Buf> scratch;
   std::map<uint32_t, float*> cube_sa;  // solid-angle tables by face size
   std::map<uint64_t, float2*> cube_pt;  // texel-pair basis tables by (face size << 8 | lmax)
+  // panorama direction tables by (w, h, shifted): h row entries, then w column
+  // entries; at most kPanoTables sizes are kept
+  static constexpr size_t kPanoTables = 32;
+  std::map<uint64_t, float4*> pano_tab;
   // batched bakes: the shape key of the last batch, its captured graph (made
   // on the second call with that key) and the tuned schedule
   std::vector<uint64_t> batch_key;
