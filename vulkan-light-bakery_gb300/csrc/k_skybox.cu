@@ -28,7 +28,11 @@ constexpr uint32_t kSkySlab = 8192;  // texels per work unit, independent of the
 // k_skybox_cube_group (cubemap batches with the pair table)
 constexpr int kGroupChunk = 256;          // texels per map per stage
 constexpr int kGroupPairs = kGroupChunk / 2;
-constexpr uint32_t kGroupSlab = 4096;     // texels per work unit
+// Texels per work unit.  A lone map has one active warp per unit, so short units
+// spread it (6 x 128^2: 12.8 us a call at 1024, 16.7 at 2048, 19.0 at 4096); 1024
+// maps are 40 units per SM either way, and the units' sums, 31 shuffles per map,
+// cost little.
+constexpr uint32_t kGroupSlab = 1024;
 
 // Exact solid angle of cube-face texel (x, y) of an n x n face, in FP64:
 // corner sum of atan2(u v, sqrt(u^2 + v^2 + 1)), the antiderivative of the
@@ -471,15 +475,25 @@ __global__ void __launch_bounds__(kSkyThreads) k_skybox_cube_group(const SkyboxA
 #pragma unroll
       for (int m = 0; m < MPW; ++m) {
         const uint32_t g = MPW * warp + m;
+        // lane v has value v of the first 32, lane v - 32 the rest
+        float lo[32], hi[16];
 #pragma unroll
-        for (int vv = 0; vv < V; ++vv) {
-          const float s = warp_sum(acc[m][vv].x + acc[m][vv].y);
-          acc[m][vv] = make_float2(0.f, 0.f);
-          if (lane == 0 && g < gv) {
-            const int k = vv / 3, c = vv - 3 * k;
-            const int vo = 3 * k + (swap_rb ? 2 - c : c);  // R/B swap applied to the linear result
-            a.partial[(size_t(m0 + g) * spm + slab) * V + vo] = s;
-          }
+        for (int v = 0; v < 32; ++v) lo[v] = v < V ? acc[m][v < V ? v : 0].x + acc[m][v < V ? v : 0].y : 0.f;
+#pragma unroll
+        for (int v = 0; v < 16; ++v)
+          hi[v] = v + 32 < V ? acc[m][v + 32 < V ? v + 32 : 0].x + acc[m][v + 32 < V ? v + 32 : 0].y : 0.f;
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[m][v] = make_float2(0.f, 0.f);
+        float* to = a.partial + (size_t(m0 + g) * spm + slab) * V;
+        auto put = [&](int v, float s) {
+          const int k = v / 3, c = v - 3 * k;
+          to[3 * k + (swap_rb ? 2 - c : c)] = s;  // R/B swap applied to the linear result
+        };
+        const float s0 = warp_sums<32>(lo);
+        if (g < gv && int(lane) < V) put(int(lane), s0);
+        if constexpr (V > 32) {
+          const float s1 = warp_sums<16>(hi);
+          if (g < gv && int(lane) < V - 32) put(int(lane) + 32, s1);
         }
       }
     }
@@ -559,9 +573,11 @@ int launch_skybox_sh(const SkyboxArgs& a, bool tma, int num_sms, cudaStream_t s)
   return int(a.slabs_per_map) * kSkyPartialsPerSlab;
 }
 
-// One CTA per map: thread (g, v) adds value v of partials g, g + G, ... and
-// the G sums are added in order, all in FP64 (a fixed order for a slab count).
-// One thread per value took 240 us for the 2048 partials of a 2048 x 1024 map.
+// One CTA per map: thread (g, v) adds value v of partials 4g .. 4g + 3 in FP32
+// and every G-th such four in FP64, and the G sums are added in order in FP64
+// (a fixed order for a slab count; FP64 adds run at 1/64 of the FP32 rate, so
+// one per four partials).  One thread per value took 240 us for the 2048
+// partials of a 2048 x 1024 map.
 __global__ void __launch_bounds__(1024) k_sh_finalize(const float* __restrict__ partial, uint32_t slabs,
                                                       uint32_t nvals, float* __restrict__ out) {
   __shared__ double s_sum[1024];
@@ -569,8 +585,12 @@ __global__ void __launch_bounds__(1024) k_sh_finalize(const float* __restrict__ 
   const float* p = partial + size_t(blockIdx.x) * slabs * nvals + v;
   double s = 0.0;
   if (g < G) {
-#pragma unroll 4
-    for (uint32_t j = g; j < slabs; j += G) s += double(__ldg(p + size_t(j) * nvals));
+    for (uint32_t j = 4 * g; j < slabs; j += 4 * G) {
+      float x[4];
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) x[k] = j + k < slabs ? __ldg(p + size_t(j + k) * nvals) : 0.f;
+      s += double((x[0] + x[1]) + (x[2] + x[3]));
+    }
     s_sum[threadIdx.x] = s;
   }
   __syncthreads();
@@ -581,7 +601,7 @@ __global__ void __launch_bounds__(1024) k_sh_finalize(const float* __restrict__ 
 
 void launch_sh_finalize(const float* partial, uint32_t nmaps, uint32_t slabs, uint32_t nvals, float* out,
                         cudaStream_t s) {
-  // up to four partials a thread, whole warps, at most 1024 threads
+  // four partials a thread, whole warps, at most 1024 threads
   const uint32_t want = nvals * ((slabs + 3) / 4);
   const uint32_t threads = want < 1024 ? (want + 31) / 32 * 32 : 1024;
   k_sh_finalize<<<nmaps, threads, 0, s>>>(partial, slabs, nvals, out);
