@@ -436,6 +436,88 @@ int launch_probe_order(const float* probes, uint32_t n, const float bounds[6], u
   return L;
 }
 
+// ---- grouping many points by place ----------------------------------------------------
+// Counting sort of n points by the top 15 bits of their Morton code (32^3 cells
+// of `bounds`): every point takes its place in its cell from the cell's
+// counter, the counters are scanned, the points scattered.  The order inside a
+// cell follows the atomics: only for uses whose results do not depend on it.
+// 1 M points: 40 us (the stable radix sort above: 240 us).
+constexpr uint32_t kPlaceBins = 1u << 15;
+
+struct PlaceBox {
+  float lo[3], s[3];
+};
+
+__device__ __forceinline__ uint32_t place_bin(const float* __restrict__ pts, uint32_t i, const PlaceBox& b) {
+  uint32_t q[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float v = (__ldg(pts + 3 * size_t(i) + a) - b.lo[a]) * b.s[a];
+    q[a] = v > 0.f ? min(__float2uint_rz(v), 31u) : 0u;
+  }
+  return (expand_bits10(q[0]) << 2) | (expand_bits10(q[1]) << 1) | expand_bits10(q[2]);
+}
+
+__global__ void k_place_count(const float* __restrict__ pts, uint32_t n, const PlaceBox b, uint32_t* __restrict__ bins,
+                              uint32_t* __restrict__ rank) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) rank[i] = atomicAdd(bins + place_bin(pts, i, b), 1u);
+}
+
+__global__ void k_place_scatter(const float* __restrict__ pts, uint32_t n, const PlaceBox b,
+                                const uint32_t* __restrict__ bins, const uint32_t* __restrict__ rank,
+                                uint32_t* __restrict__ order) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) order[__ldg(bins + place_bin(pts, i, b)) + rank[i]] = i;
+}
+
+// Exclusive scan of the bins in place, one CTA: a warp scans 1024 bins, 32 at a
+// time, then adds the warps before it.
+__global__ void __launch_bounds__(1024) k_place_scan(uint32_t* __restrict__ bins) {
+  static_assert(kPlaceBins == 32 * 1024, "a bin per thread and step");
+  __shared__ uint32_t s_sum[32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t v[32], run = 0;
+#pragma unroll
+  for (int k = 0; k < 32; ++k) v[k] = bins[warp * 1024 + k * 32 + lane];
+#pragma unroll
+  for (int k = 0; k < 32; ++k) {
+    uint32_t x = v[k];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (int(lane) >= o) x += y;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, x, 31);
+    v[k] = run + x - v[k];
+    run += total;
+  }
+  if (lane == 0) s_sum[warp] = run;
+  __syncthreads();
+  uint32_t base = 0;
+  for (uint32_t k = 0; k < warp; ++k) base += s_sum[k];
+#pragma unroll
+  for (int k = 0; k < 32; ++k) bins[warp * 1024 + k * 32 + lane] = base + v[k];
+}
+
+size_t point_order_scratch_bytes(uint32_t n) { return (size_t(kPlaceBins) + n) * 4; }
+
+int launch_point_order(const float* pts, uint32_t n, const float bounds[6], uint32_t* order, void* scratch,
+                       cudaStream_t st) {
+  PlaceBox b;
+  for (int a = 0; a < 3; ++a) {
+    const float e = bounds[3 + a] - bounds[a];
+    b.lo[a] = bounds[a];
+    b.s[a] = e > 0.f ? 32.0f / e : 0.f;
+  }
+  uint32_t *bins = static_cast<uint32_t*>(scratch), *rank = bins + kPlaceBins;
+  cudaMemsetAsync(bins, 0, kPlaceBins * 4, st);
+  k_place_count<<<(n + 255) / 256, 256, 0, st>>>(pts, n, b, bins, rank);
+  k_place_scan<<<1, 1024, 0, st>>>(bins);
+  k_place_scatter<<<(n + 255) / 256, 256, 0, st>>>(pts, n, b, bins, rank, order);
+  return 3;
+}
+
 // ---- Karras split search ---------------------------------------------------------
 __device__ __forceinline__ int kdelta(const uint32_t* __restrict__ k, int n, int i, int j) {
   if (j < 0 || j >= n) return -1;

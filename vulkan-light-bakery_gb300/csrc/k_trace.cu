@@ -871,11 +871,10 @@ void launch_scatter_rows(const float* src, float* const* dst, const uint32_t* sr
 // ---- probe evaluation: the consumer side of a baked grid -------------------------
 // Restates shaders/main.rchit:124-168 with shaders/sh.rmiss:23-39 (intended
 // math; the reference's grid-origin, probe-index, coefficient-stride and 0/0
-// faults are not reproduced).  One thread per shading point: the cell of
+// faults are not reproduced).  For each shading point: the cell of
 // the grid holding the point, its 8 corner probes (gridVertices order: bit 2
 // x, bit 1 y, bit 0 z), a visibility ray from point + bias * n toward each
-// probe (any hit in (0, |d|), per-lane walk: the rays of a warp share
-// nothing), and the distance-weighted mean of the visible probes' SH
+// probe (any hit in (0, |d|), per-lane walk), and the distance-weighted mean of the visible probes' SH
 // evaluated at the normal.
 __device__ __forceinline__ uint32_t ref_grid_index(const uint32_t* cnt, uint32_t i, uint32_t j, uint32_t k) {
   // breadth-first grid order of LightBaker::probePositionsFromBoudingBox
@@ -883,74 +882,90 @@ __device__ __forceinline__ uint32_t ref_grid_index(const uint32_t* cnt, uint32_t
   return k == 0 ? q : cnt[0] * cnt[1] + q * (cnt[2] - 1) + (k - 1);
 }
 
+//
+// A CTA takes 32 points, warp c their rays toward corner c (one octant, so one
+// copy of the walk), and the corners' terms are added in corner order.  Points
+// come spatially grouped: a warp's rays then run side by side toward one probe.
 template <int LMAX>
-__global__ void __launch_bounds__(128) k_probe_eval(const ProbeEvalArgs a) {
+__global__ void __launch_bounds__(256) k_probe_eval(const ProbeEvalArgs a) {
   constexpr int K = sh_k<LMAX>();
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  float x[3], nv[3];
-  for (int c = 0; c < 3; ++c) {
-    x[c] = a.points[3 * size_t(i) + c];
-    nv[c] = a.normals[3 * size_t(i) + c];
-  }
-  const float rn = rsqrtf(nv[0] * nv[0] + nv[1] * nv[1] + nv[2] * nv[2]);
-  for (float& c : nv) c *= rn;
-  float Y[16];
-  sh_basis<LMAX>(nv[0], nv[1], nv[2], Y);
-  const float o[3] = {fmaf(a.bias, nv[0], x[0]), fmaf(a.bias, nv[1], x[1]), fmaf(a.bias, nv[2], x[2])};
-  int cell[3];
-  for (int c = 0; c < 3; ++c) {
-    const int hi = max(int(a.counts[c]) - 2, 0);
-    cell[c] = hi == 0 ? 0 : min(max(int(floorf(__fdiv_rn(__fsub_rn(x[c], a.org[c]), a.step[c]))), 0), hi);
-  }
-  const float wmax = sqrtf(a.step[0] * a.step[0] + a.step[1] * a.step[1] + a.step[2] * a.step[2]);
-  float sum[3] = {0.f, 0.f, 0.f}, ws = 0.f;
-  uint32_t mask = 0;
-  Work w;
-  for (int c = 0; c < 8; ++c) {
+  __shared__ float s_e[8][4][32];  // per corner: weight (-1: not visible), colour
+  const uint32_t lane = threadIdx.x & 31, c = threadIdx.x >> 5;
+  const uint32_t t = blockIdx.x * 32 + lane;
+  const uint32_t i = t < a.n ? (a.order ? VLB_CLAMP(__ldg(a.order + t), a.n, a.err) : t) : 0xffffffffu;
+  float wc = -1.f, e[3] = {0.f, 0.f, 0.f};
+  if (i != 0xffffffffu) {
+    float x[3], nv[3];
+    for (int k = 0; k < 3; ++k) {
+      x[k] = __ldg(a.points + 3 * size_t(i) + k);
+      nv[k] = __ldg(a.normals + 3 * size_t(i) + k);
+    }
+    const float rn = rsqrtf(nv[0] * nv[0] + nv[1] * nv[1] + nv[2] * nv[2]);
+    for (float& k : nv) k *= rn;
+    const float o[3] = {fmaf(a.bias, nv[0], x[0]), fmaf(a.bias, nv[1], x[1]), fmaf(a.bias, nv[2], x[2])};
+    const float wmax = sqrtf(a.step[0] * a.step[0] + a.step[1] * a.step[1] + a.step[2] * a.step[2]);
     uint32_t ijk[3];
     float d[3];
-    for (int e = 0; e < 3; ++e) {
-      ijk[e] = min(uint32_t(cell[e]) + ((uint32_t(c) >> (2 - e)) & 1u), a.counts[e] - 1);
-      const float p = __fadd_rn(a.org[e], __fmul_rn(a.step[e], float(ijk[e])));
-      d[e] = p - x[e];
+    for (int k = 0; k < 3; ++k) {
+      const int hi = max(int(a.counts[k]) - 2, 0);
+      const int cell =
+          hi == 0 ? 0 : min(max(int(floorf(__fdiv_rn(__fsub_rn(x[k], a.org[k]), a.step[k]))), 0), hi);
+      ijk[k] = min(uint32_t(cell) + ((c >> (2 - k)) & 1u), a.counts[k] - 1);
+      const float p = __fadd_rn(a.org[k], __fmul_rn(a.step[k], float(ijk[k])));
+      d[k] = p - x[k];
     }
-    const float t = sqrtf(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+    const float dist = sqrtf(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
     bool visible = true;
-    if (t > 0.f && a.ntris) {
-      const float it = 1.0f / t;
+    if (dist > 0.f && a.ntris) {
+      const float it = 1.0f / dist;
       const float dx = d[0] * it, dy = d[1] * it, dz = d[2] * it;
       RayCtx ray;
       make_ray(ray, o[0], o[1], o[2], dx, dy, dz);
       bool act = true;
-      float tb = t;
+      float tb = dist;
       int slot = -1, id = -1;
+      Work w;
       traverse<true, false, true>(octant_of(dx, dy, dz), ray, act, a.nodes, a.tris, a.ntris, 0.0f, tb, slot, id,
                                   a.err, w);
       visible = slot < 0;
     }
-    if (!visible) continue;
-    mask |= 1u << c;
-    const float wc = wmax - t;
-    const float* cp = a.coeffs + size_t(ref_grid_index(a.counts, ijk[0], ijk[1], ijk[2])) * K * 3;
+    if (visible) {
+      float Y[16];
+      sh_basis<LMAX>(nv[0], nv[1], nv[2], Y);
+      wc = wmax - dist;
+      const float* cp = a.coeffs + size_t(ref_grid_index(a.counts, ijk[0], ijk[1], ijk[2])) * K * 3;
 #pragma unroll
-    for (int ch = 0; ch < 3; ++ch) {
-      float e = 0.f;
+      for (int ch = 0; ch < 3; ++ch) {
 #pragma unroll
-      for (int k = 0; k < K; ++k) e = fmaf(__ldg(cp + 3 * k + ch), Y[k], e);
-      sum[ch] = fmaf(wc, e, sum[ch]);
+        for (int k = 0; k < K; ++k) e[ch] = fmaf(__ldg(cp + 3 * k + ch), Y[k], e[ch]);
+      }
     }
-    ws += wc;
+    s_e[c][3][lane] = visible ? 1.f : 0.f;
   }
-  for (int ch = 0; ch < 3; ++ch) a.out[3 * size_t(i) + ch] = ws > 0.f ? sum[ch] / ws : 0.f;
-  if (a.vis) a.vis[i] = uint8_t(mask);
+  s_e[c][0][lane] = e[0]; s_e[c][1][lane] = e[1]; s_e[c][2][lane] = e[2];
+  __shared__ float s_w[8][32];
+  s_w[c][lane] = wc;
+  __syncthreads();
+  if (c >= 4 || i == 0xffffffffu) return;
+  // warps 0-2: the channels; warp 3: the mask
+  uint32_t mask = 0;
+  float sum = 0.f, ws = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    if (s_e[k][3][lane] == 0.f) continue;
+    mask |= 1u << k;
+    sum = fmaf(s_w[k][lane], s_e[k][c < 3 ? c : 0][lane], sum);
+    ws += s_w[k][lane];
+  }
+  if (c < 3) a.out[3 * size_t(i) + c] = ws > 0.f ? sum / ws : 0.f;
+  else if (a.vis) a.vis[i] = uint8_t(mask);
 }
 
 void launch_probe_eval(const ProbeEvalArgs& a, uint32_t lmax, cudaStream_t s) {
   if (!a.n) return;
-  const uint32_t g = (a.n + 127) / 128;
-  if (lmax == 3) k_probe_eval<3><<<g, 128, 0, s>>>(a);
-  else k_probe_eval<2><<<g, 128, 0, s>>>(a);
+  const uint32_t g = (a.n + 31) / 32;
+  if (lmax == 3) k_probe_eval<3><<<g, 256, 0, s>>>(a);
+  else k_probe_eval<2><<<g, 256, 0, s>>>(a);
 }
 
 void launch_trace_fused(const TraceArgs& a, int num_sms, cudaStream_t s) {

@@ -1948,6 +1948,10 @@ vlb_status vlb_batch_tune_log(const vlb_ctx* ctx, vlb_tune_trial* out, uint32_t 
 }
 
 // ---- evaluating a baked grid ------------------------------------------------------------------
+// Points from which vlb_probe_eval groups them first: 40 us of kernels against
+// half the walks' time (1 M random points on surfaces: 1540 -> 780 us).
+constexpr uint32_t kEvalSort = 1u << 15;
+
 vlb_status vlb_probe_eval(vlb_ctx* ctx, const vlb_scene* scene, const float* coeffs, uint32_t lmax,
                           const vlb_probe_grid* g, const float* points, const float* normals, uint32_t n,
                           float shadow_bias, float* out_rgb, uint8_t* vis_mask) {
@@ -1987,6 +1991,14 @@ vlb_status vlb_probe_eval(vlb_ctx* ctx, const vlb_scene* scene, const float* coe
   a.out = static_cast<float*>(ob.dev);
   a.vis = static_cast<uint8_t*>(ov.dev);
   a.err = ctx->d_err;
+  // many points: group them by place (results do not depend on their order)
+  void *order, *otmp;
+  if (a.ntris && n >= kEvalSort && scratch(ctx, "eval_order", size_t(n) * 4, &order) == VLB_OK &&
+      scratch(ctx, "eval_order_tmp", vlbk::point_order_scratch_bytes(n), &otmp) == VLB_OK) {
+    KScope k(ctx, "eval_order", 0);
+    k.nkernels = vlbk::launch_point_order(a.points, n, scene->bounds, static_cast<uint32_t*>(order), otmp, ctx->stream);
+    a.order = static_cast<const uint32_t*>(order);
+  }
   {
     KScope k(ctx, "probe_eval");
     vlbk::launch_probe_eval(a, lmax, ctx->stream);

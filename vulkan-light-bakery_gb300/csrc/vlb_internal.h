@@ -196,6 +196,12 @@ size_t probe_order_scratch_bytes(uint32_t n);
 int launch_probe_order(const float* probes, uint32_t n, const float bounds[6], uint32_t* order, void* scratch,
                        uint32_t* zero_word, cudaStream_t s);
 
+// Any order of n points that groups them by place inside `bounds`; returns the
+// kernels launched.
+size_t point_order_scratch_bytes(uint32_t n);
+int launch_point_order(const float* pts, uint32_t n, const float bounds[6], uint32_t* order, void* scratch,
+                       cudaStream_t s);
+
 // ---- probe frontiers (k_front.cu) ------------------------------------------------
 // Entries per probe: 32 bytes each, [lx ly hx hy] [lz hz ref dist^2], the box
 // relative to the probe, nearest first; cnt[probe] of them.
@@ -433,6 +439,7 @@ struct ProbeEvalArgs {
   uint32_t counts[3];
   const float* points;      // n x 3
   const float* normals;     // n x 3 (normalised in the kernel)
+  const uint32_t* order;    // thread -> point, spatially grouped, or null
   uint32_t n;
   float bias;
   float* out;               // n x 3
