@@ -12,10 +12,7 @@
 //   5. Karras split search with ties broken by index (32 + clz(i ^ j));
 //   6. bottom-up refit with one atomic counter per internal node (min/max
 //      unions are order independent);
-//   7. packing into the traversal layout: internal node = 4 float4 holding
-//      both children's boxes (widened by a relative 2^-20 so that the box
-//      tests are conservative) and references; triangle = 3 float4 (v0 | id,
-//      e1, e2) in leaf order.
+//   7. triangles packed in leaf order = 3 float4 (v0 | id, e1, e2).
 #include <algorithm>
 
 #include "vlb_device.cuh"
@@ -82,15 +79,20 @@ __global__ void k_cbounds_partial(const float* __restrict__ cen, uint32_t n, flo
   if (threadIdx.x < 6) part[6 * blockIdx.x + threadIdx.x] = s[threadIdx.x][0];
 }
 
-// params: lo[3], scale[3] with scale = 1024 / (hi - lo) (0 for a flat axis)
+// params: lo[3], scale[3] with scale = 1024 / (hi - lo) (0 for a flat axis);
+// one warp per axis
 __global__ void k_cbounds_final(const float* __restrict__ part, uint32_t nblk, float* __restrict__ params) {
-  if (threadIdx.x >= 3) return;
-  const int a = threadIdx.x;
+  const int a = int(threadIdx.x >> 5);
   float lo = INFINITY, hi = -INFINITY;
-  for (uint32_t b = 0; b < nblk; ++b) {
+  for (uint32_t b = threadIdx.x & 31; b < nblk; b += 32) {
     lo = fminf(lo, part[6 * b + a]);
     hi = fmaxf(hi, part[6 * b + 3 + a]);
   }
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if (threadIdx.x & 31) return;
   const float e = __fsub_rn(hi, lo);
   params[a] = lo;
   params[3 + a] = e > 0.f ? __fdiv_rn(1024.0f, e) : 0.f;
@@ -587,37 +589,6 @@ __global__ void k_refit(const int32_t* __restrict__ parent, const int32_t* __res
   }
 }
 
-// Traversal boxes are the exact boxes widened by (|x| + scene scale) * 2^-20
-// per bound, so that the box tests are conservative: a ray lying in a box's
-// face plane (a zero direction component) or grazing its boundary still
-// enters it, and only the triangle test decides.  The exact boxes stay in
-// `box` (exported and compared with the oracle).
-__device__ __forceinline__ float widen_lo(float x, float scale) {
-  return __fsub_rn(x, __fmul_rn(__fadd_rn(fabsf(x), scale), 0x1p-20f));
-}
-__device__ __forceinline__ float widen_hi(float x, float scale) {
-  return __fadd_rn(x, __fmul_rn(__fadd_rn(fabsf(x), scale), 0x1p-20f));
-}
-
-__global__ void k_pack_nodes(const int32_t* __restrict__ child, const float* __restrict__ box, uint32_t n,
-                             float4* __restrict__ nodes) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i + 1 >= n) return;
-  const int leaf0 = int(n) - 1;
-  const int32_t c0 = child[2 * i], c1 = child[2 * i + 1];
-  const float* r = box;  // root (internal node 0)
-  const float scale = fmaxf(fmaxf(fmaxf(fabsf(r[0]), fabsf(r[1])), fmaxf(fabsf(r[2]), fabsf(r[3]))),
-                            fmaxf(fabsf(r[4]), fabsf(r[5])));
-  const float* p0 = box + 6 * size_t(c0 >= 0 ? c0 : leaf0 + ~c0);
-  const float* p1 = box + 6 * size_t(c1 >= 0 ? c1 : leaf0 + ~c1);
-  float b0[6], b1[6];
-  for (int a = 0; a < 3; ++a) {
-    b0[a] = widen_lo(p0[a], scale); b0[3 + a] = widen_hi(p0[3 + a], scale);
-    b1[a] = widen_lo(p1[a], scale); b1[3 + a] = widen_hi(p1[3 + a], scale);
-  }
-  pack_node(nodes + 4 * size_t(i), b0, b1, c0, c1);
-}
-
 __global__ void k_pack_tris(const uint32_t* __restrict__ order, const float* __restrict__ pos, uint32_t stride,
                             const uint32_t* __restrict__ idx, const float* __restrict__ albedo, uint32_t n,
                             float4* __restrict__ tris, float4* __restrict__ tri_albedo) {
@@ -678,7 +649,7 @@ void launch_lbvh_build(const LbvhBuild& b, cudaStream_t st, int* launches) {
   k_tri_bounds<<<g, 256, 0, st>>>(b.positions, b.stride_floats, b.indices, n, s.tb, s.cen); ++L;
   const uint32_t nred = min(256u, (n + kRedThreads - 1) / kRedThreads);
   k_cbounds_partial<<<nred, kRedThreads, 0, st>>>(s.cen, n, s.part); ++L;
-  k_cbounds_final<<<1, 32, 0, st>>>(s.part, nred, s.params); ++L;
+  k_cbounds_final<<<1, 96, 0, st>>>(s.part, nred, s.params); ++L;
   k_morton<<<g, 256, 0, st>>>(s.cen, n, s.params, s.ka, s.va); ++L;
   uint32_t *kin = s.ka, *kout = s.kb, *vin = s.va, *vout = s.vb;
   L += radix_passes(kin, vin, kout, vout, n, s.hist, 4, st);
@@ -690,7 +661,6 @@ void launch_lbvh_build(const LbvhBuild& b, cudaStream_t st, int* launches) {
     k_karras<<<gi, 256, 0, st>>>(b.codes, int(n), b.child, s.parent); ++L;
     cudaMemsetAsync(s.flags, 0, size_t(n) * 4, st);
     k_refit<<<g, 256, 0, st>>>(s.parent, b.child, n, b.box, s.flags); ++L;
-    k_pack_nodes<<<gi, 256, 0, st>>>(b.child, b.box, n, b.nodes); ++L;
   }
   k_pack_tris<<<g, 256, 0, st>>>(b.order, b.positions, b.stride_floats, b.indices, b.albedo, n, b.tris,
                                  b.tri_albedo); ++L;

@@ -541,6 +541,131 @@ vlb_status vlb_probe_grid_ref_order(const float bounds[6], const uint32_t counts
 }
 
 // ---- scene ----------------------------------------------------------------------------
+// Device workspace of one scene load: the context's scratch up to
+// kSceneScratch bytes (kept for the next load), its own allocation above.
+constexpr size_t kSceneScratch = 256u << 20;
+struct SceneTemp {
+  vlb_ctx* ctx;
+  void* own = nullptr;
+  ~SceneTemp() { cudaFree(own); }
+  vlb_status get(size_t bytes, void** p) {
+    if (bytes <= kSceneScratch) return scratch(ctx, "scene_build", bytes, p);
+    if (cudaMalloc(&own, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return fail(ctx, VLB_ERR_OOM, "scene workspace of %zu bytes", bytes);
+    }
+    *p = own;
+    return VLB_OK;
+  }
+};
+
+// Fills a scene: geometry checks and bounds, LBVH, traversal tree and its node
+// layout, all on the device.  The checks' kernel replaces an index out of range
+// by 0, so the builds run on any input; the verdict is read with the builds'
+// own synchronisation.
+static vlb_status scene_build(vlb_ctx* ctx, vlb_scene* sc, const float* positions, uint32_t sf,
+                              const uint32_t* indices, const float* tri_albedo, uint32_t flags) {
+  const uint32_t n = sc->ntris, nverts = sc->nverts;
+  // persistent arrays, then the workspace, each part on a 256-byte boundary
+  size_t off = 0;
+  auto part = [&off](size_t bytes) { const size_t at = off; off += (bytes + 255) & ~size_t(255); return at; };
+  if (n) {
+    const size_t slots = std::max<size_t>(2 * size_t(n) - 2, 1);
+    const size_t sizes[7] = {size_t(n) * 4, size_t(n) * 4, size_t(2) * (n - 1 + (n == 1)) * 4,
+                             size_t(2 * size_t(n) - 1) * 24, slots * 64, size_t(n) * 48, size_t(n) * 16};
+    size_t at[7];
+    for (int k = 0; k < 7; ++k) { at[k] = part(sizes[k]); sc->bytes += sizes[k]; }
+    if (cudaMalloc(&sc->mem, off) != cudaSuccess) {
+      cudaGetLastError();
+      return fail(ctx, VLB_ERR_OOM, "scene allocation failed (%u triangles)", n);
+    }
+    auto* m = static_cast<uint8_t*>(sc->mem);
+    sc->codes = reinterpret_cast<uint32_t*>(m + at[0]);
+    sc->order = reinterpret_cast<uint32_t*>(m + at[1]);
+    sc->child = reinterpret_cast<int32_t*>(m + at[2]);
+    sc->box = reinterpret_cast<float*>(m + at[3]);
+    sc->nodes = reinterpret_cast<float4*>(m + at[4]);
+    sc->tris = reinterpret_cast<float4*>(m + at[5]);
+    sc->albedo = reinterpret_cast<float4*>(m + at[6]);
+  }
+  off = 0;
+  const bool pos_dev = is_device_ptr(positions), alb_dev = is_device_ptr(tri_albedo);
+  const size_t pos_bytes = size_t(nverts) * sf * 4, idx_bytes = size_t(n) * 12;
+  const size_t o_check = part(sizeof(vlbk::SceneCheck)), o_pos = part(pos_dev ? 0 : pos_bytes), o_idx = part(idx_bytes),
+               o_alb = part(tri_albedo && !alb_dev ? idx_bytes : 0), o_lbvh = part(n ? vlbk::lbvh_scratch_bytes(n) : 0),
+               o_ploc = part(n > 1 ? vlbk::ploc_scratch_bytes(n) : 0), o_pair = part(n ? vlbk::pair_scratch_bytes(n) : 0);
+  SceneTemp temp{ctx};
+  void* base;
+  vlb_status st = temp.get(off, &base);
+  if (st) return st;
+  auto* w = static_cast<uint8_t*>(base);
+  auto* check = reinterpret_cast<vlbk::SceneCheck*>(w + o_check);
+  auto* idx = reinterpret_cast<uint32_t*>(w + o_idx);
+  // device arrays may still be written by the legacy default stream
+  if (pos_dev || alb_dev || is_device_ptr(indices)) VLB_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));
+  const float* pos = positions;
+  if (!pos_dev && pos_bytes) {
+    VLB_CUDA(ctx, cudaMemcpyAsync(w + o_pos, positions, pos_bytes, cudaMemcpyHostToDevice, ctx->stream));
+    pos = reinterpret_cast<const float*>(w + o_pos);
+  }
+  if (n) VLB_CUDA(ctx, cudaMemcpyAsync(idx, indices, idx_bytes, cudaMemcpyDefault, ctx->stream));
+  const float* alb = tri_albedo;
+  if (n && tri_albedo && !alb_dev) {
+    VLB_CUDA(ctx, cudaMemcpyAsync(w + o_alb, tri_albedo, idx_bytes, cudaMemcpyHostToDevice, ctx->stream));
+    alb = reinterpret_cast<const float*>(w + o_alb);
+  }
+  {
+    KScope k(ctx, "scene_check", 3);
+    vlbk::launch_scene_check(pos, sf, nverts, idx, uint64_t(n) * 3, idx, check, ctx->num_sms, ctx->stream);
+  }
+  const int32_t* child = sc->child;
+  const float* ibox = sc->box;
+  int tree = 0;
+  if (n) {
+    vlbk::LbvhBuild b{};
+    b.positions = pos; b.stride_floats = sf; b.nverts = nverts; b.indices = idx; b.albedo = alb; b.ntris = n;
+    b.codes = sc->codes; b.order = sc->order; b.child = sc->child; b.box = sc->box;
+    b.tris = sc->tris; b.tri_albedo = sc->albedo; b.scratch = w + o_lbvh;
+    b.scratch_bytes = vlbk::lbvh_scratch_bytes(n);
+    int launches = 0;
+    KScope k(ctx, "lbvh_build", 0);
+    vlbk::launch_lbvh_build(b, ctx->stream, &launches);
+    k.nkernels = launches;
+  }
+  if (n > 1 && !(flags & VLB_SCENE_TRAVERSAL_LBVH)) {
+    int pl = 0;
+    const int32_t* pc;
+    const float* pb;
+    KScope k(ctx, "ploc_build", 0);
+    tree = vlbk::launch_ploc_build(sc->box + size_t(n - 1) * 6, n, &pc, &pb, w + o_ploc, ctx->stream, &pl);
+    if (tree == 0) { child = pc; ibox = pb; }  // a stalled clustering (1) keeps the LBVH
+    k.nkernels = pl;
+  }
+  if (n > 1 && tree >= 0) {
+    VLB_CUDA(ctx, cudaMemsetAsync(sc->nodes, 0, (2 * size_t(n) - 2) * 64, ctx->stream));  // slots left empty
+    KScope k(ctx, "node_layout", 4);
+    vlbk::launch_pair_siblings(child, ibox, sc->box + size_t(n - 1) * 6, n, sc->nodes, w + o_pair, check, ctx->stream);
+  }
+  vlbk::SceneCheck h;
+  VLB_CUDA(ctx, cudaMemcpyAsync(&h, check, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
+  st = finish(ctx, true);
+  if (st == VLB_ERR_CUDA) return st;
+  if (h.bad_index != 0xffffffffu) {
+    uint32_t v = 0;
+    cudaMemcpy(&v, indices + h.bad_index, 4, cudaMemcpyDefault);
+    return fail(ctx, VLB_ERR_INVALID, "index %u out of range at %u", v, h.bad_index);
+  }
+  if (h.bad_vertex != 0xffffffffu) return fail(ctx, VLB_ERR_INVALID, "vertex %u is not finite", h.bad_vertex);
+  if (tree < 0) return fail(ctx, VLB_ERR_INTERNAL, "traversal tree build failed");
+  if (st) return st;
+  for (int a = 0; a < 3; ++a) {
+    sc->bounds[a] = nverts ? vlbk::from_ordered(h.lo[a]) : 0.f;
+    sc->bounds[3 + a] = nverts ? vlbk::from_ordered(h.hi[a]) : 0.f;
+  }
+  sc->depth = h.depth;
+  return n && (flags & VLB_SCENE_TRAVERSAL_WIDE) ? vlbh::build_wide(ctx, sc) : VLB_OK;
+}
+
 vlb_status vlb_scene_create(vlb_ctx* ctx, const float* positions, uint32_t stride_bytes, uint32_t nverts,
                             const uint32_t* indices, uint32_t ntris, const float* tri_albedo, vlb_scene** out) {
   return vlb_scene_create_ex(ctx, positions, stride_bytes, nverts, indices, ntris, tri_albedo, 0, out);
@@ -556,83 +681,10 @@ vlb_status vlb_scene_create_ex(vlb_ctx* ctx, const float* positions, uint32_t st
   if (ntris && (!positions || !indices || nverts == 0)) return fail(ctx, VLB_ERR_INVALID, "missing geometry");
   if (ntris > (1u << 30)) return fail(ctx, VLB_ERR_INVALID, "too many triangles (%u)", ntris);
   const uint32_t sf = stride_bytes / 4;
-  // Host copies for validation and bounds (scene creation is not on the hot path).
-  std::vector<float> hpos(size_t(nverts) * sf);
-  std::vector<uint32_t> hidx(size_t(ntris) * 3);
-  if (nverts) VLB_CUDA(ctx, cudaMemcpy(hpos.data(), positions, hpos.size() * 4, cudaMemcpyDefault));
-  if (ntris) VLB_CUDA(ctx, cudaMemcpy(hidx.data(), indices, hidx.size() * 4, cudaMemcpyDefault));
-  for (size_t i = 0; i < hidx.size(); ++i)
-    if (hidx[i] >= nverts) return fail(ctx, VLB_ERR_INVALID, "index %u out of range at %zu", hidx[i], i);
-  for (uint32_t v = 0; v < nverts; ++v)
-    for (int a = 0; a < 3; ++a)
-      if (!std::isfinite(hpos[size_t(v) * sf + a])) return fail(ctx, VLB_ERR_INVALID, "vertex %u is not finite", v);
   vlb_scene* sc = new (std::nothrow) vlb_scene();
   if (!sc) return VLB_ERR_OOM;
   sc->ctx = ctx; sc->ntris = ntris; sc->nverts = nverts;
-  for (int a = 0; a < 3; ++a) { sc->bounds[a] = INFINITY; sc->bounds[3 + a] = -INFINITY; }
-  for (uint32_t v = 0; v < nverts; ++v)
-    for (int a = 0; a < 3; ++a) {
-      sc->bounds[a] = std::min(sc->bounds[a], hpos[size_t(v) * sf + a]);
-      sc->bounds[3 + a] = std::max(sc->bounds[3 + a], hpos[size_t(v) * sf + a]);
-    }
-  if (nverts == 0) for (int a = 0; a < 6; ++a) sc->bounds[a] = 0.f;
-  if (ntris == 0) { *out = sc; return VLB_OK; }
-  const uint32_t n = ntris;
-  auto alloc = [&](void** p, size_t bytes) -> bool {
-    if (cudaMalloc(p, std::max<size_t>(bytes, 16)) != cudaSuccess) { cudaGetLastError(); return false; }
-    sc->bytes += bytes;
-    return true;
-  };
-  float* dpos = nullptr; uint32_t* didx = nullptr; float* dalb = nullptr; void* scr = nullptr;
-  bool ok = alloc((void**)&sc->codes, size_t(n) * 4) && alloc((void**)&sc->order, size_t(n) * 4) &&
-            alloc((void**)&sc->child, size_t(2) * (n - 1 + (n == 1)) * 4) &&
-            alloc((void**)&sc->box, size_t(2 * n - 1) * 6 * 4) &&
-            alloc((void**)&sc->nodes, size_t(n - 1 + (n == 1)) * 64) && alloc((void**)&sc->tris, size_t(n) * 48) &&
-            alloc((void**)&sc->albedo, size_t(n) * 16);
-  const size_t scr_bytes = vlbk::lbvh_scratch_bytes(n);
-  ok = ok && cudaMalloc((void**)&dpos, hpos.size() * 4) == cudaSuccess &&
-       cudaMalloc((void**)&didx, hidx.size() * 4) == cudaSuccess &&
-       (!tri_albedo || cudaMalloc((void**)&dalb, size_t(n) * 12) == cudaSuccess) &&
-       cudaMalloc(&scr, scr_bytes) == cudaSuccess;
-  vlb_status st = VLB_OK;
-  if (!ok) {
-    cudaGetLastError();
-    st = fail(ctx, VLB_ERR_OOM, "scene allocation failed (%u triangles)", n);
-  } else {
-    cudaMemcpyAsync(dpos, hpos.data(), hpos.size() * 4, cudaMemcpyHostToDevice, ctx->stream);
-    cudaMemcpyAsync(didx, hidx.data(), hidx.size() * 4, cudaMemcpyHostToDevice, ctx->stream);
-    if (tri_albedo) cudaMemcpyAsync(dalb, tri_albedo, size_t(n) * 12, cudaMemcpyDefault, ctx->stream);
-    vlbk::LbvhBuild b{};
-    b.positions = dpos; b.stride_floats = sf; b.nverts = nverts; b.indices = didx; b.albedo = dalb; b.ntris = n;
-    b.codes = sc->codes; b.order = sc->order; b.child = sc->child; b.box = sc->box; b.nodes = sc->nodes;
-    b.tris = sc->tris; b.tri_albedo = sc->albedo; b.scratch = scr; b.scratch_bytes = scr_bytes;
-    int launches = 0;
-    {
-      KScope k(ctx, "lbvh_build", 0);
-      vlbk::launch_lbvh_build(b, ctx->stream, &launches);
-      k.nkernels = launches;
-    }
-    if (n > 1 && !(flags & VLB_SCENE_TRAVERSAL_LBVH)) {
-      void* pscr = nullptr;
-      if (cudaMalloc(&pscr, vlbk::ploc_scratch_bytes(n)) != cudaSuccess) {
-        cudaGetLastError();
-        st = fail(ctx, VLB_ERR_OOM, "traversal tree scratch allocation failed (%u triangles)", n);
-      } else {
-        int pl = 0;
-        KScope k(ctx, "ploc_build", 0);
-        // a stalled clustering (1) keeps the LBVH already packed into sc->nodes
-        if (vlbk::launch_ploc_build(sc->box + size_t(n - 1) * 6, n, sc->nodes, pscr, ctx->stream, &pl) < 0)
-          st = fail(ctx, VLB_ERR_INTERNAL, "traversal tree build failed");
-        k.nkernels = pl;
-        cudaStreamSynchronize(ctx->stream);
-        cudaFree(pscr);
-      }
-    }
-    if (st == VLB_OK) st = finish(ctx, true);
-    if (st == VLB_OK && (flags & VLB_SCENE_TRAVERSAL_WIDE)) st = vlbh::build_wide(ctx, sc);
-    if (st == VLB_OK) st = vlbh::pair_siblings(ctx, sc);
-  }
-  cudaFree(dpos); cudaFree(didx); if (dalb) cudaFree(dalb); cudaFree(scr);
+  const vlb_status st = nverts || ntris ? scene_build(ctx, sc, positions, sf, indices, tri_albedo, flags) : VLB_OK;
   if (st != VLB_OK) { vlb_scene_destroy(sc); return st; }
   *out = sc;
   return VLB_OK;
@@ -641,8 +693,7 @@ vlb_status vlb_scene_create_ex(vlb_ctx* ctx, const float* positions, uint32_t st
 void vlb_scene_destroy(vlb_scene* s) {
   if (!s) return;
   if (s->ctx) { cudaSetDevice(s->ctx->device); cudaStreamSynchronize(s->ctx->stream); }
-  cudaFree(s->codes); cudaFree(s->order); cudaFree(s->child); cudaFree(s->box);
-  cudaFree(s->nodes); cudaFree(s->wnodes); cudaFree(s->tris); cudaFree(s->albedo);
+  cudaFree(s->mem); cudaFree(s->wnodes);
   delete s;
 }
 

@@ -172,7 +172,6 @@ struct LbvhBuild {
   uint32_t* order;   // n sorted -> original
   int32_t* child;    // 2(n-1)
   float* box;        // (2n-1)*6
-  float4* nodes;     // (n-1)*4
   float4* tris;      // n*3 (sorted order): v0|id, e1, e2
   float4* tri_albedo;  // n (by original index)
   // scratch (device)
@@ -181,13 +180,34 @@ struct LbvhBuild {
 };
 size_t lbvh_scratch_bytes(uint32_t ntris);
 void launch_lbvh_build(const LbvhBuild& b, cudaStream_t s, int* launches);
-// Traversal tree by PLOC clustering over the Morton-sorted leaves
-// (k_ploc.cu): overwrites `nodes` (root 0) and returns 0; returns 1 with
-// `nodes` untouched if clustering stalls (more than 64 + 8 log2 n rounds),
-// -1 on a CUDA error or a round that merges nothing.
+// Traversal tree by PLOC clustering over the Morton-sorted leaves (k_ploc.cu):
+// *child and *ibox (n - 1 inner nodes, root 0) in `scratch`; returns 0, 1 if
+// clustering stalls (more than 64 + 8 log2 n rounds), -1 on a CUDA error or a
+// round that merges nothing.  Synchronises.
 size_t ploc_scratch_bytes(uint32_t ntris);
-int launch_ploc_build(const float* leaf_box, uint32_t n, float4* nodes, void* scratch, cudaStream_t s,
-                      int* launches);
+int launch_ploc_build(const float* leaf_box, uint32_t n, const int32_t** child, const float** ibox, void* scratch,
+                      cudaStream_t s, int* launches);
+
+// ---- scene load (k_scene.cu) ------------------------------------------------------
+struct SceneCheck {
+  uint32_t bad_index;   // position of the first index out of range, or 2^32 - 1
+  uint32_t bad_vertex;  // the first vertex that is not finite, or 2^32 - 1
+  uint32_t lo[3], hi[3];  // vertex bounds as ordered integers
+  uint32_t depth;       // levels of inner nodes of the traversal tree (kLaneStack + 1: deeper)
+};
+inline float from_ordered(uint32_t k) {
+  const uint32_t u = k ^ (k & 0x80000000u ? 0x80000000u : 0xffffffffu);
+  float f;
+  std::memcpy(&f, &u, 4);
+  return f;
+}
+void launch_scene_check(const float* pos, uint32_t stride_floats, uint32_t nverts, const uint32_t* idx, uint64_t nidx,
+                        uint32_t* idx_out, SceneCheck* c, int num_sms, cudaStream_t s);
+// The traversal nodes of a tree (children, inner and leaf boxes) with siblings
+// in one 128-byte line (2n - 2 slots of 64 bytes) and its depth.
+size_t pair_scratch_bytes(uint32_t ntris);
+int launch_pair_siblings(const int32_t* child, const float* ibox, const float* leaf_box, uint32_t ntris, float4* out,
+                         void* scratch, SceneCheck* c, cudaStream_t s);
 // Permutation of the probes by 24-bit Morton code inside `bounds` (min xyz,
 // max xyz), so that each 32-probe packet is spatially compact; also zeroes
 // *zero_word (the trace's work counter; may be null) in stream order.
@@ -471,9 +491,6 @@ vlb_status ctx_finish(vlb_ctx* ctx, bool sync);
 // Collapses the scene's binary traversal tree into the 8-wide quantised tree
 // (sc->wnodes, sc->nwide; wide_bvh.cpp).  Synchronous.
 vlb_status build_wide(vlb_ctx* ctx, vlb_scene* sc);
-// Re-lays the binary traversal tree with siblings in one 128-byte line
-// (2n - 2 node slots); same tree, same results.
-vlb_status pair_siblings(vlb_ctx* ctx, vlb_scene* sc);
 vlb_status ctx_fail(vlb_ctx* ctx, vlb_status s, const char* msg);
 }  // namespace vlbh
 
@@ -525,6 +542,7 @@ struct vlb_scene {
   vlb_ctx* ctx = nullptr;
   uint32_t ntris = 0, nverts = 0;
   float bounds[6] = {0, 0, 0, 0, 0, 0};
+  void* mem = nullptr;       // one allocation behind the arrays below
   uint32_t* codes = nullptr;
   uint32_t* order = nullptr;
   int32_t* child = nullptr;
