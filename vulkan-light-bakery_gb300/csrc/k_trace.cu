@@ -259,9 +259,9 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace_dyn(const TraceArgs 
     if (!exhausted && idle == kFull) {  // a whole idle warp takes its next 32 rays together
       const uint32_t block = a.ray_block;  // set by the launch: the kernel's registers stay free
       uint32_t wb;
-      if (block == 32) {  // one group a block: straight from the counter
+      if (block <= 32) {  // one group a block: straight from the counter
         uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(a.work_counter, 32u);
+        if (lane == 0) base = atomicAdd(a.work_counter, block);
         wb = __shfl_sync(kFull, base, 0);
         if (wb >= R) exhausted = true;
       } else {
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace_dyn(const TraceArgs 
         __syncwarp();
       }
       const uint32_t r = wb + lane;
-      if (r < R) {
+      if (r < R && lane < block) {
         const uint32_t sl = r / a.S, t = r - sl * a.S;
         if (sl < a.nprobes) lr_start(a, L, a.order[sl], __ldg(a.dir_order + t), stack);
       }
@@ -332,12 +332,20 @@ static void launch_dyn(const TraceArgs& a, int num_sms, cudaStream_t s) {
     if (per_sm < 1) per_sm = 1;
   }
   const uint64_t rays = uint64_t((a.nprobes + 31) / 32 * 32) * a.S;
-  const uint64_t ctas = std::max<uint64_t>(
+  uint64_t ctas = std::max<uint64_t>(
       std::min<uint64_t>((rays + kTraceThreads - 1) / kTraceThreads, uint64_t(num_sms) * per_sm), 1);
   // ray blocks: whole 32-ray groups, as many as keep ~64 blocks a warp, at most 16
   TraceArgs b = a;
   const uint64_t groups_per_warp = (rays / 32) / (ctas * kTraceWarps);
   b.ray_block = 32u * uint32_t(std::min<uint64_t>(16, std::max<uint64_t>(1, groups_per_warp / 64)));
+  // Few rays: groups of 16 down to 2 rays while that leaves warps idle, so that a
+  // group's slowest ray holds up fewer others (64 probes x 64 directions: trace
+  // 39 us at 32, 34 at 8, 30 at 2).
+  const uint64_t warps = uint64_t(num_sms) * per_sm * kTraceWarps;
+  while (b.ray_block > 2 && b.ray_block <= 32 && rays / b.ray_block * 2 <= warps) b.ray_block /= 2;
+  if (b.ray_block < 32)
+    ctas = std::max<uint64_t>(
+        std::min<uint64_t>((rays / b.ray_block + kTraceWarps - 1) / kTraceWarps, uint64_t(num_sms) * per_sm), 1);
   kern<<<uint32_t(ctas), kTraceThreads, 0, s>>>(b);
 }
 
