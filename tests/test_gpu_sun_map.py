@@ -1,4 +1,4 @@
-"""Shadow rays answered by the sun map (bakes of at least 2^19 rays) against
+"""Shadow rays answered by the sun map (bakes of many rays) against
 packet walks, which trace every one of them: visibility, radiance and
 coefficients must be the same bits.
 
@@ -46,7 +46,7 @@ def test_mapped_shadows_keep_their_bits(ctx, sun, tmax, bias, precision):
     for name, pos, idx, alb in scenes():
         scene = ctx.scene(pos, idx, alb)
         b = scene.bounds(False)
-        probes = (b[:3] + rng.uniform(-0.1, 1.1, (530, 3)) * np.maximum(b[3:] - b[:3], 0.1)).astype(np.float32)
+        probes = (b[:3] + rng.uniform(-0.1, 1.1, (1300, 3)) * np.maximum(b[3:] - b[:3], 0.1)).astype(np.float32)
         out = []
         for prec, flags in ((vlb.PREC_FP32, vlb.BAKE_TRAVERSAL_PACKET), (precision, vlb.BAKE_TRAVERSAL_LANE)):
             p = vlb.bake_params(ds, 2, prec, sun, flags=flags)

@@ -128,26 +128,43 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_hist(const uint32_t* __restri
   hist[size_t(threadIdx.x) * nblk + blockIdx.x] = h[threadIdx.x];
 }
 
-// Single-CTA exclusive scan of a u32 array in place.
+// Single-CTA exclusive scan of a u32 array in place: tiles of 4096, four
+// consecutive entries a thread, a carry between tiles.
 __global__ void __launch_bounds__(1024) k_scan_exclusive(uint32_t* __restrict__ a, uint32_t total) {
-  __shared__ uint32_t sums[1024];
-  const uint32_t per = (total + 1023) / 1024;
-  const uint32_t b = threadIdx.x * per, e = min(total, b + per);
-  uint32_t s = 0;
-  for (uint32_t i = b; i < e; ++i) s += a[i];
-  sums[threadIdx.x] = s;
-  __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {
-    const uint32_t v = threadIdx.x >= uint32_t(off) ? sums[threadIdx.x - off] : 0u;
+  __shared__ uint32_t s_sum[2][32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t carry = 0;
+  int flip = 0;
+  for (uint32_t t0 = 0; t0 < total; t0 += 4096, flip ^= 1) {
+    const uint32_t i = t0 + threadIdx.x * 4;
+    uint32_t v[4], own = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = i + k < total ? a[i + k] : 0u;
+      own += v[k];
+    }
+    uint32_t x = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (int(lane) >= o) x += y;
+    }
+    if (lane == 31) s_sum[flip][warp] = x;
     __syncthreads();
-    sums[threadIdx.x] += v;
-    __syncthreads();
-  }
-  uint32_t run = sums[threadIdx.x] - s;
-  for (uint32_t i = b; i < e; ++i) {
-    const uint32_t v = a[i];
-    a[i] = run;
-    run += v;
+    const uint32_t w = s_sum[flip][lane];  // every warp scans the 32 warp sums
+    uint32_t ws = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, ws, o);
+      if (int(lane) >= o) ws += y;
+    }
+    uint32_t run = carry + x - own + __shfl_sync(0xffffffffu, ws - w, int(warp));
+    carry += __shfl_sync(0xffffffffu, ws, 31);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i + k < total) a[i + k] = run;
+      run += v[k];
+    }
   }
 }
 
@@ -473,35 +490,6 @@ __global__ void k_place_scatter(const float* __restrict__ pts, uint32_t n, const
   if (i < n) order[__ldg(bins + place_bin(pts, i, b)) + rank[i]] = i;
 }
 
-// Exclusive scan of the bins in place, one CTA: a warp scans 1024 bins, 32 at a
-// time, then adds the warps before it.
-__global__ void __launch_bounds__(1024) k_place_scan(uint32_t* __restrict__ bins) {
-  static_assert(kPlaceBins == 32 * 1024, "a bin per thread and step");
-  __shared__ uint32_t s_sum[32];
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t v[32], run = 0;
-#pragma unroll
-  for (int k = 0; k < 32; ++k) v[k] = bins[warp * 1024 + k * 32 + lane];
-#pragma unroll
-  for (int k = 0; k < 32; ++k) {
-    uint32_t x = v[k];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (int(lane) >= o) x += y;
-    }
-    const uint32_t total = __shfl_sync(0xffffffffu, x, 31);
-    v[k] = run + x - v[k];
-    run += total;
-  }
-  if (lane == 0) s_sum[warp] = run;
-  __syncthreads();
-  uint32_t base = 0;
-  for (uint32_t k = 0; k < warp; ++k) base += s_sum[k];
-#pragma unroll
-  for (int k = 0; k < 32; ++k) bins[warp * 1024 + k * 32 + lane] = base + v[k];
-}
-
 size_t point_order_scratch_bytes(uint32_t n) { return (size_t(kPlaceBins) + n) * 4; }
 
 int launch_point_order(const float* pts, uint32_t n, const float bounds[6], uint32_t* order, void* scratch,
@@ -515,7 +503,7 @@ int launch_point_order(const float* pts, uint32_t n, const float bounds[6], uint
   uint32_t *bins = static_cast<uint32_t*>(scratch), *rank = bins + kPlaceBins;
   cudaMemsetAsync(bins, 0, kPlaceBins * 4, st);
   k_place_count<<<(n + 255) / 256, 256, 0, st>>>(pts, n, b, bins, rank);
-  k_place_scan<<<1, 1024, 0, st>>>(bins);
+  k_scan_exclusive<<<1, 1024, 0, st>>>(bins, kPlaceBins);
   k_place_scatter<<<(n + 255) / 256, 256, 0, st>>>(pts, n, b, bins, rank, order);
   return 3;
 }
@@ -591,19 +579,26 @@ __global__ void k_refit(const int32_t* __restrict__ parent, const int32_t* __res
 
 __global__ void k_pack_tris(const uint32_t* __restrict__ order, const float* __restrict__ pos, uint32_t stride,
                             const uint32_t* __restrict__ idx, const float* __restrict__ albedo, uint32_t n,
-                            float4* __restrict__ tris, float4* __restrict__ tri_albedo) {
+                            float4* __restrict__ tris, float4* __restrict__ tri_albedo, double* __restrict__ area) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t t = order[i];
-  const float* a = pos + size_t(idx[3 * t]) * stride;
-  const float* b = pos + size_t(idx[3 * t + 1]) * stride;
-  const float* c = pos + size_t(idx[3 * t + 2]) * stride;
-  tris[3 * size_t(i) + 0] = make_float4(a[0], a[1], a[2], __int_as_float(int(t)));
-  tris[3 * size_t(i) + 1] = make_float4(__fsub_rn(b[0], a[0]), __fsub_rn(b[1], a[1]), __fsub_rn(b[2], a[2]), 0.f);
-  tris[3 * size_t(i) + 2] = make_float4(__fsub_rn(c[0], a[0]), __fsub_rn(c[1], a[1]), __fsub_rn(c[2], a[2]), 0.f);
-  const float r = albedo ? albedo[3 * size_t(t)] : 1.f, g = albedo ? albedo[3 * size_t(t) + 1] : 1.f,
-              bb = albedo ? albedo[3 * size_t(t) + 2] : 1.f;
-  tri_albedo[t] = make_float4(r, g, bb, 0.f);
+  float twice = 0.f;
+  if (i < n) {
+    const uint32_t t = order[i];
+    const float* a = pos + size_t(idx[3 * t]) * stride;
+    const float* b = pos + size_t(idx[3 * t + 1]) * stride;
+    const float* c = pos + size_t(idx[3 * t + 2]) * stride;
+    tris[3 * size_t(i) + 0] = make_float4(a[0], a[1], a[2], __int_as_float(int(t)));
+    tris[3 * size_t(i) + 1] = make_float4(__fsub_rn(b[0], a[0]), __fsub_rn(b[1], a[1]), __fsub_rn(b[2], a[2]), 0.f);
+    tris[3 * size_t(i) + 2] = make_float4(__fsub_rn(c[0], a[0]), __fsub_rn(c[1], a[1]), __fsub_rn(c[2], a[2]), 0.f);
+    const float r = albedo ? albedo[3 * size_t(t)] : 1.f, g = albedo ? albedo[3 * size_t(t) + 1] : 1.f,
+                bb = albedo ? albedo[3 * size_t(t) + 2] : 1.f;
+    tri_albedo[t] = make_float4(r, g, bb, 0.f);
+    const float4 e1 = tris[3 * size_t(i) + 1], e2 = tris[3 * size_t(i) + 2];
+    const float nx = e1.y * e2.z - e1.z * e2.y, ny = e1.z * e2.x - e1.x * e2.z, nz = e1.x * e2.y - e1.y * e2.x;
+    twice = sqrtf(nx * nx + ny * ny + nz * nz);
+  }
+  for (int o = 16; o > 0; o >>= 1) twice += __shfl_xor_sync(0xffffffffu, twice, o);
+  if ((threadIdx.x & 31) == 0 && twice > 0.f) atomicAdd(area, 0.5 * double(twice));
 }
 
 // ---- orchestration -------------------------------------------------------------------
@@ -663,7 +658,7 @@ void launch_lbvh_build(const LbvhBuild& b, cudaStream_t st, int* launches) {
     k_refit<<<g, 256, 0, st>>>(s.parent, b.child, n, b.box, s.flags); ++L;
   }
   k_pack_tris<<<g, 256, 0, st>>>(b.order, b.positions, b.stride_floats, b.indices, b.albedo, n, b.tris,
-                                 b.tri_albedo); ++L;
+                                 b.tri_albedo, b.area); ++L;
   if (launches) *launches += L;
 }
 

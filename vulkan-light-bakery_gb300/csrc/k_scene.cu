@@ -24,6 +24,7 @@ __global__ void k_check_init(SceneCheck* c) {
   c->bad_index = 0xffffffffu;
   c->bad_vertex = 0xffffffffu;
   c->depth = 0;
+  c->area = 0.0;
   for (int a = 0; a < 3; ++a) { c->lo[a] = 0xffffffffu; c->hi[a] = 0; }
 }
 
@@ -40,14 +41,23 @@ __global__ void __launch_bounds__(256) k_check_vertices(const float* __restrict_
       lo[a] = min(lo[a], k);
       hi[a] = max(hi[a], k);
     }
+  // one atomic per CTA and bound
+  __shared__ uint32_t s_lo[3], s_hi[3];
+  if (threadIdx.x < 3) { s_lo[threadIdx.x] = 0xffffffffu; s_hi[threadIdx.x] = 0; }
+  __syncthreads();
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     lo[a] = __reduce_min_sync(0xffffffffu, lo[a]);
     hi[a] = __reduce_max_sync(0xffffffffu, hi[a]);
     if ((threadIdx.x & 31) == 0) {
-      atomicMin(&c->lo[a], lo[a]);
-      atomicMax(&c->hi[a], hi[a]);
+      atomicMin(&s_lo[a], lo[a]);
+      atomicMax(&s_hi[a], hi[a]);
     }
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    atomicMin(&c->lo[threadIdx.x], s_lo[threadIdx.x]);
+    atomicMax(&c->hi[threadIdx.x], s_hi[threadIdx.x]);
   }
 }
 
@@ -176,7 +186,7 @@ __global__ void k_pair_pack(const int32_t* __restrict__ child, const float* __re
 void launch_scene_check(const float* pos, uint32_t stride_floats, uint32_t nverts, const uint32_t* idx, uint64_t nidx,
                         uint32_t* idx_out, SceneCheck* c, int num_sms, cudaStream_t s) {
   k_check_init<<<1, 1, 0, s>>>(c);
-  const uint32_t cap = uint32_t(num_sms) * 8;
+  const uint32_t cap = uint32_t(num_sms) * 2;
   auto grid = [&](uint64_t n) { return uint32_t(n / 256 + 1 < cap ? n / 256 + 1 : cap); };
   if (nverts) k_check_vertices<<<grid(nverts), 256, 0, s>>>(pos, stride_floats, nverts, c);
   if (nidx) k_check_indices<<<grid(nidx), 256, 0, s>>>(idx, nidx, nverts, idx_out, c);

@@ -625,7 +625,7 @@ static vlb_status scene_build(vlb_ctx* ctx, vlb_scene* sc, const float* position
     vlbk::LbvhBuild b{};
     b.positions = pos; b.stride_floats = sf; b.nverts = nverts; b.indices = idx; b.albedo = alb; b.ntris = n;
     b.codes = sc->codes; b.order = sc->order; b.child = sc->child; b.box = sc->box;
-    b.tris = sc->tris; b.tri_albedo = sc->albedo; b.scratch = w + o_lbvh;
+    b.tris = sc->tris; b.tri_albedo = sc->albedo; b.area = &check->area; b.scratch = w + o_lbvh;
     b.scratch_bytes = vlbk::lbvh_scratch_bytes(n);
     int launches = 0;
     KScope k(ctx, "lbvh_build", 0);
@@ -663,6 +663,7 @@ static vlb_status scene_build(vlb_ctx* ctx, vlb_scene* sc, const float* position
     sc->bounds[3 + a] = nverts ? vlbk::from_ordered(h.hi[a]) : 0.f;
   }
   sc->depth = h.depth;
+  sc->area = h.area;
   return n && (flags & VLB_SCENE_TRAVERSAL_WIDE) ? vlbh::build_wide(ctx, sc) : VLB_OK;
 }
 
@@ -1134,17 +1135,25 @@ static float bounds_scale(const vlb_scene* scene) {
   return m;
 }
 
-// Sun maps (k_lightmap.cu) pay when the rays are many (1 M rays in 778
-// triangles: 15 us for the map, the trace 212 -> 162 us; 4096 rays: 13 us for
-// 6 us) and outnumber the triangles to draw (2.4 M rays, 164 k triangles: 40 us
-// for 55 us in the tile walk, nothing gained in the fused walk).  256 cells a
-// side: 512 save 6 % more of that trace and cost 25 us more.
+// 256 cells a side: 512 save 6 % more of a trace of 1 M rays in 778 triangles and
+// cost 25 us more.
 constexpr uint32_t kMapSide = 256;
 constexpr size_t kMapBytes = size_t(kMapSide) * kMapSide * 8;
-// In a batch one launch draws the maps of all jobs, so only the drawing itself
-// counts: about 60 rays a triangle in the box scenes.
-constexpr uint64_t kBatchMapRays = 1ull << 16;
-static bool sun_map_pays(uint64_t rays, uint32_t ntris) { return rays >= std::max(1ull << 19, 24ull * ntris); }
+
+// Whether a bake's sun map (k_lightmap.cu) saves more than it costs.  It saves
+// some 25 ps a ray (20 in a terrain of 164 k triangles, 45 in 4096 boxes, 50 in
+// 64); it costs 90 ps a triangle and 1 us per layer of triangles over the map's
+// cells (15 us for that terrain, 130 us for the 4096 boxes' 130 layers), and a
+// launch of its own 6 us (a batch draws all its jobs' maps in one).
+static bool sun_map_pays(const vlb_scene* sc, uint64_t rays, double launch_us) {
+  double diag2 = 0.0;
+  for (int a = 0; a < 3; ++a) {
+    const double e = double(sc->bounds[3 + a]) - sc->bounds[a];
+    diag2 += e * e;
+  }
+  const double layers = diag2 > 0.0 ? sc->area / diag2 : 0.0;
+  return sc->ntris && double(rays) * 25e-6 > launch_us + sc->ntris * 90e-6 + layers;
+}
 
 // Plane, extent and margins of a scene's sun map (k_lightmap.cu).
 static void sun_map_plan(const vlb_scene* scene, float3 s, float bias, uint32_t G, uint32_t* cells, vlbk::SunMap* m) {
@@ -1245,8 +1254,8 @@ static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const floa
   a.lane = lane_mode(scene, nprobes, p->flags, p->shading);
   a.shading = p->shading;
   a.light = make_float3(p->light_pos[0], p->light_pos[1], p->light_pos[2]);
-  if (a.lane && !from_root && a.ntris && a.shading == VLB_SHADE_LAMBERT_SUN &&
-      sun_map_pays(uint64_t(nprobes) * a.S, scene->ntris)) {
+  if (a.lane && !from_root && a.shading == VLB_SHADE_LAMBERT_SUN &&
+      sun_map_pays(scene, uint64_t(nprobes) * a.S, 6.0)) {
     void* cells;
     if ((st = scratch(ctx, "sun_map", kMapBytes, &cells))) return st;
     sun_map_plan(scene, a.sun, a.bias, kMapSide, static_cast<uint32_t*>(cells), &a.sun_map);
@@ -1702,8 +1711,7 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
     const BatchJob& b = pl.jobs[i];
     const vlb_scene* sc = jobs[b.idx].scene;
     fronts[i] = !(ext && ext[b.idx].hits_in) && front_cap(sc, b.nprobes, b.S) != 0;
-    maps[i] = sc->ntris && b.p->shading == VLB_SHADE_LAMBERT_SUN &&
-              uint64_t(b.nprobes) * b.S >= std::max<uint64_t>(kBatchMapRays, 64ull * sc->ntris);
+    maps[i] = b.p->shading == VLB_SHADE_LAMBERT_SUN && sun_map_pays(sc, uint64_t(b.nprobes) * b.S, 0.0);
     if (fronts[i]) front_probes += b.nprobes;
     if (maps[i]) bb.map_bytes += kMapBytes;
   }

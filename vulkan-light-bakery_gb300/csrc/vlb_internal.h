@@ -174,6 +174,7 @@ struct LbvhBuild {
   float* box;        // (2n-1)*6
   float4* tris;      // n*3 (sorted order): v0|id, e1, e2
   float4* tri_albedo;  // n (by original index)
+  double* area;        // the triangles' area is added here
   // scratch (device)
   void* scratch;
   size_t scratch_bytes;
@@ -194,6 +195,7 @@ struct SceneCheck {
   uint32_t bad_vertex;  // the first vertex that is not finite, or 2^32 - 1
   uint32_t lo[3], hi[3];  // vertex bounds as ordered integers
   uint32_t depth;       // levels of inner nodes of the traversal tree (kLaneStack + 1: deeper)
+  double area;          // of all triangles (a sum in any order: for launch rules only)
 };
 inline float from_ordered(uint32_t k) {
   const uint32_t u = k ^ (k & 0x80000000u ? 0x80000000u : 0xffffffffu);
@@ -551,6 +553,7 @@ struct vlb_scene {
   float4* wnodes = nullptr;  // 8-wide quantised traversal tree (wide_bvh.cpp), or null
   uint32_t nwide = 0;
   uint32_t depth = 0;        // levels of inner nodes in the binary traversal tree
+  double area = 0.0;         // of all triangles
   float4* tris = nullptr;
   float4* albedo = nullptr;
   uint64_t bytes = 0;
