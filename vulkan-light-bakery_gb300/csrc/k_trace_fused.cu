@@ -35,7 +35,7 @@
 
 namespace vlbk {
 
-constexpr int kSubRays = 32;
+constexpr int kSubRays = int(kFusedSub);
 constexpr int kSubBufs = 2;
 constexpr uint32_t kSubFirst = 1, kSubLast = 2;
 
@@ -104,6 +104,46 @@ __device__ __forceinline__ void retire_head(FusedWarp<3 * K>& fw, const BakeJobD
 #pragma unroll
     for (int h = 0; h < P; ++h) s[h] = fmaf(__ldg(row + k[h]), fw.rad[e][ch[h]][i], s[h]);
   }
+  if (J.sub) {  // a split chunk: the sub-batch's sums, added up by the probe's last item
+    const uint32_t per = J.chunk_rays / kFusedSub;
+    if (VLB_INB(q.p, J.nprobes, J.err) && VLB_INB(q.t0, J.S, J.err)) {
+      float* dst = J.sub + (size_t(q.p) * J.subs + q.c * per + (q.t0 - q.c * J.chunk_rays) / kFusedSub) * V;
+#pragma unroll
+      for (int h = 0; h < P; ++h)
+        if (int(lane) + 32 * h < V) dst[lane + 32 * h] = s[h];
+    }
+    if (q.flags & kSubLast) {
+      __threadfence();
+      __syncwarp();
+      uint32_t ticket = 0;
+      if (lane == 0) ticket = atomicAdd(J.done + q.p, 1u);
+      ticket = __shfl_sync(kFull, ticket, 0);
+      if (ticket == J.items - 1) {
+        __threadfence();
+        const float* src = J.sub + size_t(q.p) * J.subs * V;
+        for (int v = int(lane); v < V; v += 32) {
+          double t = 0.0;
+          float one_chunk = 0.f;
+          for (uint32_t c = 0; c < J.chunks; ++c) {
+            double x = 0.0;
+            const uint32_t e1 = min(J.subs, (c + 1) * per);
+#pragma unroll 4
+            for (uint32_t i = c * per; i < e1; ++i) x += double(__ldcg(src + size_t(i) * V + v));
+            one_chunk = float(x);
+            t += double(one_chunk);
+          }
+          J.out[size_t(q.p) * V + v] = J.chunks == 1 ? one_chunk : float(t);
+        }
+      }
+    }
+    __syncwarp();
+    if (lane == 0) {
+      fw.head = (e + 1) % kSubBufs;
+      fw.n -= 1;
+    }
+    __syncwarp();
+    return;
+  }
 #pragma unroll
   for (int h = 0; h < P; ++h) {
     const int v = int(lane) + 32 * h;
@@ -162,20 +202,22 @@ __device__ __forceinline__ void fill_ring(FW& fw, const BakeJobDev* __restrict__
       const uint32_t j = MULTI ? find_job(jobs, njobs, it) : 0;
       const BakeJobDev& J = job_of<MULTI>(jobs, one, j);
       const uint32_t loc = it - J.item_begin;
-      uint32_t slot, c;
-      if (J.chunk_major) {
+      uint32_t slot, c, part = 0;
+      if (J.chunk_major) {  // never split
         c = loc / J.nprobes;
         slot = loc - c * J.nprobes;
       } else {
-        slot = loc / J.chunks;
-        c = loc - slot * J.chunks;
+        slot = loc / J.items;
+        const uint32_t i = loc - slot * J.items;
+        c = min(i / J.parts, J.chunks - 1);
+        part = i - c * J.parts;
       }
       const uint32_t p = VLB_CLAMP(J.order[VLB_CLAMP(slot, J.nprobes, J.err)], J.nprobes, J.err);
       __syncwarp();
       if (lane == 0) {
         fw.ij = j; fw.ip = p; fw.ic = c;
-        fw.it0 = fw.itn = c * J.chunk_rays;
-        fw.ite = min(J.S, c * J.chunk_rays + J.chunk_rays);
+        fw.it0 = fw.itn = c * J.chunk_rays + part * J.part_rays;
+        fw.ite = min(J.S, min((c + 1) * J.chunk_rays, fw.it0 + J.part_rays));
         fw.have_item = 1;
       }
       __syncwarp();

@@ -1326,6 +1326,11 @@ static vlbk::FusedSched fused_sched(const vlb_batch_schedule& sc) {
   return f;
 }
 
+// Rays of an item of the fused walk's split chunks, 0 for whole chunks.
+static uint32_t fused_part(const vlb_ctx* ctx, uint64_t chunk_items, uint32_t chunk_major) {
+  return chunk_major || chunk_items >= vlbk::kFusedWhole * uint64_t(ctx->num_sms) ? 0u : vlbk::kFusedPart;
+}
+
 // The scene, shading, probe and direction fields of one bake as a job of the
 // fused lane walk (the fused-projection fields are set by the caller).
 static void job_from_trace(const vlbk::TraceArgs& a, vlbk::BakeJobDev* j) {
@@ -1377,16 +1382,22 @@ vlb_status vlb_bake_ex(vlb_ctx* ctx, const vlb_scene* scene, const float* probe_
     j.chunks = (S + j.chunk_rays - 1) / j.chunk_rays;
     j.chunk_major = vlbk::fused_chunk_major(S);
     j.hit_tri = a.hit_tri; j.shadow = a.shadow; j.dbg_radiance = a.dbg_radiance;
-    if (j.chunks > 1) {
-      void *part, *done;
-      if ((st = scratch(ctx, "bake_partial", size_t(nprobes) * j.chunks * V * 4, &part)) ||
+    vlbk::fused_items(&j, fused_part(ctx, uint64_t(nprobes) * j.chunks, j.chunk_major));
+    void *sub, *part, *done;
+    if (j.parts > 1) {
+      const size_t bytes = size_t(nprobes) * j.subs * V * 4;
+      if (bytes > vlbk::kFusedSubBytes || scratch(ctx, "bake_sub", bytes, &sub) != VLB_OK) vlbk::fused_items(&j, 0);
+      else j.sub = static_cast<float*>(sub);
+    }
+    if (j.chunks > 1 || j.sub) {
+      if ((!j.sub && (st = scratch(ctx, "bake_partial", size_t(nprobes) * j.chunks * V * 4, &part))) ||
           (st = scratch(ctx, "bake_chunk_done", size_t(nprobes) * 4, &done)))
         return st;
       VLB_CUDA(ctx, cudaMemsetAsync(done, 0, size_t(nprobes) * 4, ctx->stream));
-      j.partial = static_cast<float*>(part);
+      if (!j.sub) j.partial = static_cast<float*>(part);
       j.done = static_cast<uint32_t*>(done);
     }
-    const uint64_t items = uint64_t(nprobes) * j.chunks;
+    const uint64_t items = uint64_t(nprobes) * j.items;
     if (items >= (1ull << 32) - (1ull << 20)) return fail(ctx, VLB_ERR_INVALID, "too many probes for one bake");
     KScope k(ctx, "trace_fused_lane");
     vlbk::launch_trace_fused_lane(nullptr, j, 1, uint32_t(items), K, a.work_counter,
@@ -1538,6 +1549,7 @@ struct BatchBufs {
   uint8_t* tile;
   float* out;          // rows x V
   float* partial;      // fused: chunk partials
+  float* sub;          // fused, chunks split: sub-batch sums
   uint32_t* done;      // fused: rows chunk tickets
   uint8_t* meta;       // job table + scatter arrays
   uint32_t* counter;
@@ -1723,6 +1735,22 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
         scratch(ctx, "batch_front_n", front_probes * 4, &front_n) != VLB_OK)
       cap = 0;
   }
+  if (pl.fused) {  // few work items: chunks are split
+    uint64_t chunk_items = 0, subs = 0;
+    for (const auto& b : pl.jobs) {
+      vlbk::BakeJobDev t{};
+      t.S = b.S;
+      t.chunk_rays = vlbk::fused_chunk_rays(b.S);
+      t.chunks = (b.S + t.chunk_rays - 1) / t.chunk_rays;
+      vlbk::fused_items(&t, vlbk::kFusedPart);
+      chunk_items += uint64_t(b.nprobes) * t.chunks;
+      subs += uint64_t(b.nprobes) * t.subs;
+    }
+    void* sub;
+    if (fused_part(ctx, chunk_items, 0) && subs * V * 4 <= std::min<uint64_t>(vlbk::kFusedSubBytes, spare_bytes / 4) &&
+        scratch(ctx, "batch_sub", subs * V * 4, &sub) == VLB_OK)
+      bb.sub = static_cast<float*>(sub);
+  }
   if (bb.map_bytes && (bb.map_bytes > std::min<uint64_t>(256ull << 20, spare_bytes / 4) ||
                        scratch(ctx, "batch_maps", bb.map_bytes, &bb.maps) != VLB_OK))
     bb.map_bytes = 0;
@@ -1746,7 +1774,7 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
       if ((st = dirset_split_basis(ctx, g.dirs))) return st;
   auto& table = ctx->batch_table;
   table.assign(ntable, vlbk::BakeJobDev{});
-  size_t poff = 0, part_off = 0, nmaps = 0;
+  size_t poff = 0, part_off = 0, sub_off = 0, nmaps = 0;
   uint64_t items = 0;
   for (uint32_t t = 0; t < ntable; ++t) {
     const BatchJob& b = pl.jobs[ord[t]];
@@ -1785,13 +1813,17 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
       d.chunk_rays = vlbk::fused_chunk_rays(b.S);
       d.chunks = (b.S + d.chunk_rays - 1) / d.chunk_rays;
       d.chunk_major = vlbk::fused_chunk_major(b.S);
-      if (d.chunks > 1) {
+      vlbk::fused_items(&d, bb.sub && !d.chunk_major ? vlbk::kFusedPart : 0);
+      if (d.parts > 1) {
+        d.sub = bb.sub + sub_off;
+        sub_off += size_t(b.nprobes) * d.subs * V;
+      } else if (d.chunks > 1) {
         d.partial = bb.partial + part_off;
         part_off += size_t(b.nprobes) * d.chunks * V;
       }
       d.done = bb.done + b.row0;
       d.item_begin = uint32_t(items);
-      items += uint64_t(b.nprobes) * d.chunks;
+      items += uint64_t(b.nprobes) * d.items;
     } else {
       uint8_t* rad = bb.tile + g.tile_off + (b.row0 - g.row0) * 3 * b.S * esz;
       d.bf16_split = pl.split ? 1 : 0;
@@ -1845,7 +1877,7 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
                                uint64_t(uintptr_t(counter)), uint64_t(ctx->num_sms), pl.fused,
                                uint64_t(uintptr_t(part)), uint64_t(uintptr_t(done)), pl.rows, sc.ctas_per_sm,
                                sc.node_steps, sc.refill_idle, bb.front_total, bb.map_ctas,
-                               uint64_t(uintptr_t(bb.maps)), bb.map_bytes};
+                               uint64_t(uintptr_t(bb.maps)), bb.map_bytes, uint64_t(uintptr_t(bb.sub))};
   if (pl.fused && ntable == 1) {  // one job goes to the kernel by value: its fields are part of the shape
     const auto* w = reinterpret_cast<const uint64_t*>(table.data());
     key.insert(key.end(), w, w + sizeof(vlbk::BakeJobDev) / 8);

@@ -394,6 +394,13 @@ struct BakeJobDev {
   float* partial;         // [nprobes][chunks][K*3] FP32 chunk sums (chunks > 1)
   uint32_t* done;         // [nprobes] chunk tickets, zero before the launch
   uint32_t chunks, chunk_rays;
+  // Small launches split a chunk into `parts` items of part_rays (the last fewer):
+  // an item then leaves its sub-batches' sums in sub [nprobes][subs][K*3] and the
+  // probe's last item adds them in the order an unsplit chunk adds them, so the
+  // split changes no bit.  Unsplit: sub null, parts 1, part_rays = chunk_rays.
+  float* sub;
+  uint32_t subs, parts, part_rays;
+  uint32_t items;         // per probe
   // item order: 0 probe-major (a probe's chunks in a row: the rays in flight
   // share origins), 1 chunk-major (every probe's chunk c in a row: the basis
   // rows of chunk c are read once from HBM while all probes use them; for
@@ -423,6 +430,22 @@ inline uint32_t fused_chunk_rays(uint32_t S) {
 // Chunk-major item order when the direction set's basis (64 B a direction)
 // exceeds 16 MiB.
 inline uint32_t fused_chunk_major(uint32_t S) { return uint64_t(S) * 64 > (16ull << 20) ? 1u : 0u; }
+// Splits job j's chunks (chunks, chunk_rays and S set) into items of part_rays
+// (0: unsplit).
+constexpr uint32_t kFusedSub = 32;  // rays of a sub-batch
+inline void fused_items(BakeJobDev* j, uint32_t part_rays) {
+  const uint32_t D = j->chunk_rays, last = j->S - (j->chunks - 1) * D;
+  j->part_rays = part_rays ? part_rays : D;
+  j->parts = (D + j->part_rays - 1) / j->part_rays;
+  j->items = (j->chunks - 1) * j->parts + (last + j->part_rays - 1) / j->part_rays;
+  j->subs = (j->chunks - 1) * (D / kFusedSub) + (last + kFusedSub - 1) / kFusedSub;
+}
+// Items from which chunks stay whole: with fewer, a warp holds only a few items
+// and waits at the end for those that drew the long ones (4641 probes x 515
+// directions, 13,923 chunks on 4864 warps: 917 -> 755 us).
+constexpr uint32_t kFusedPart = 64;  // 32 and 96 measure the same
+constexpr uint64_t kFusedWhole = 16ull * 32;  // per SM
+constexpr size_t kFusedSubBytes = 256u << 20;
 // Launch knobs of the fused walk (vlb_batch_schedule; results do not depend on them).
 struct FusedSched {
   uint32_t ctas_per_sm = 8;  // register budget: 7, 8 or 9 resident 4-warp CTAs per SM
