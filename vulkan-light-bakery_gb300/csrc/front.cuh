@@ -1,4 +1,4 @@
-// k_front.cu -- probe frontiers: where the rays of one probe enter the
+// front.cuh -- probe frontiers: where the rays of one probe enter the
 // traversal tree.
 //
 // All rays of a probe start at one point, so every one of them enters every
@@ -7,7 +7,7 @@
 // primary ray tests).  This kernel walks those nodes once per probe: one warp
 // expands the tree breadth first from the root wherever the box holds the
 // probe, then, while the list is short, the entries that look largest from
-// the probe, and writes the boxes and references where the expansion stopped
+// the probe, and lists the boxes and references where the expansion stopped
 // (an antichain that covers every triangle), nearest box first.  A lane walk
 // tests its ray against that list -- warp-uniform loads, no divergence -- and
 // starts from the entries it hits instead of from the root (lr_front).
@@ -19,13 +19,13 @@
 //
 // Latency bound: some twenty dependent node loads per warp (16 us for 4096
 // probes; 180 us for 262,144, 0.3 % of that bake).
+#pragma once
+
 #include "vlb_device.cuh"
 #include "vlb_internal.h"
 
 namespace vlbk {
-namespace {
 
-constexpr int kFrontWarps = 4;
 constexpr unsigned kAll = 0xffffffffu;
 
 __device__ __forceinline__ float axis_gap(float lo, float hi, float o) { return fmaxf(fmaxf(lo - o, o - hi), 0.f); }
@@ -60,8 +60,9 @@ constexpr float kFrontLarge = 10.f;
 constexpr int kFrontLook = 32;
 constexpr int kFrontRounds = 8;
 
+constexpr int kFrontOpen = 64;  // nodes of a level expanded; the rest become entries
 struct FrontShared {
-  FrontBox open[2][kFrontCap], done[kFrontCap];
+  FrontBox open[2][kFrontOpen], done[kFrontCap];
 };
 
 // One warp: probe p's frontier.
@@ -95,6 +96,11 @@ __device__ __forceinline__ void front_probe(const FrontArgs& a, uint32_t p, Fron
         front_children(a, ref, ox, oy, oz, c);
 #pragma unroll
         for (int h = 0; h < 2; ++h) go[h] = __float_as_int(c[h].b.z) >= 0 && c[h].b.w == 0.f;
+      }
+      {  // no more than the next level holds
+        const unsigned w0 = __ballot_sync(kAll, expand && go[0]), w1 = __ballot_sync(kAll, expand && go[1]);
+        go[0] = go[0] && n_next + __popc(w0 & below) < kFrontOpen;
+        go[1] = go[1] && n_next + __popc(w0) + __popc(w1 & below) < kFrontOpen;
       }
       const unsigned keep = __ballot_sync(kAll, have && !expand);
       const unsigned g0 = __ballot_sync(kAll, expand && go[0]), g1 = __ballot_sync(kAll, expand && go[1]);
@@ -156,42 +162,6 @@ __device__ __forceinline__ void front_probe(const FrontArgs& a, uint32_t p, Fron
     out[2 * rank + 1] = e.b;
   }
   if (lane == 0) a.cnt[p] = uint32_t(n_done);
-}
-
-__global__ void __launch_bounds__(kFrontWarps * 32) k_probe_front(const FrontArgs a) {
-  __shared__ FrontShared sh[kFrontWarps];
-  const uint32_t warp = threadIdx.x >> 5, p = blockIdx.x * kFrontWarps + warp;
-  if (p < a.nprobes) front_probe(a, p, sh[warp]);
-}
-
-__global__ void __launch_bounds__(kFrontWarps * 32)
-    k_probe_front_batch(const BakeJobDev* __restrict__ jobs, uint32_t njobs, uint32_t total) {
-  __shared__ FrontShared sh[kFrontWarps];
-  const uint32_t warp = threadIdx.x >> 5, w = blockIdx.x * kFrontWarps + warp;
-  if (w >= total) return;
-  uint32_t lo = 0, hi = njobs - 1;  // the last job that begins at or before w
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi + 1) >> 1;
-    if (__ldg(&jobs[mid].front_begin) <= w) lo = mid; else hi = mid - 1;
-  }
-  const BakeJobDev& j = jobs[lo];
-  const uint32_t p = w - j.front_begin;
-  if (!j.front || p >= j.nprobes) return;
-  const FrontArgs a{j.nodes, j.ntris, j.probes, j.nprobes, j.front_scale, j.front_cap, const_cast<float4*>(j.front),
-                    const_cast<uint32_t*>(j.front_n), j.err};
-  front_probe(a, p, sh[warp]);
-}
-
-}  // namespace
-
-void launch_probe_front(const FrontArgs& a, cudaStream_t s) {
-  if (!a.nprobes) return;
-  k_probe_front<<<(a.nprobes + kFrontWarps - 1) / kFrontWarps, kFrontWarps * 32, 0, s>>>(a);
-}
-
-void launch_probe_front_batch(const BakeJobDev* jobs, uint32_t njobs, uint32_t total, cudaStream_t s) {
-  if (!total) return;
-  k_probe_front_batch<<<(total + kFrontWarps - 1) / kFrontWarps, kFrontWarps * 32, 0, s>>>(jobs, njobs, total);
 }
 
 }  // namespace vlbk

@@ -15,6 +15,7 @@
 //   7. triangles packed in leaf order = 3 float4 (v0 | id, e1, e2).
 #include <algorithm>
 
+#include "probe_sort.cuh"
 #include "vlb_device.cuh"
 #include "vlb_internal.h"
 
@@ -28,15 +29,6 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
   uint32_t m;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
   return m;
-}
-
-__device__ __forceinline__ uint32_t expand_bits10(uint32_t v) {
-  v &= 0x3ffu;
-  v = (v | (v << 16)) & 0x030000FFu;
-  v = (v | (v << 8)) & 0x0300F00Fu;
-  v = (v | (v << 4)) & 0x030C30C3u;
-  v = (v | (v << 2)) & 0x09249249u;
-  return v;
 }
 
 __global__ void k_tri_bounds(const float* __restrict__ pos, uint32_t stride, const uint32_t* __restrict__ idx,
@@ -329,72 +321,6 @@ __device__ __forceinline__ void probe_sort_cta(const float* __restrict__ probes,
   }
 }
 
-// Probe order for n <= kCountMax probes in one CTA: a counting sort on the
-// top 12 bits of the 24-bit Morton code (16^3 cells inside the bounds) with
-// shared-memory histogram, scan and atomic cursors -- a handful of barriers
-// instead of the radix sort's dozens.  The order inside a cell follows the
-// atomics; the bake's results never depend on the probe order (each ray's
-// walk and each probe's sums are independent of its packet), only its speed.
-constexpr uint32_t kCountMax = 16384;
-constexpr int kCountBins = 4096;
-
-__device__ __forceinline__ void probe_sort_count(const float* __restrict__ probes, uint32_t n, float lox, float loy,
-                                                 float loz, float sx, float sy, float sz,
-                                                 uint32_t* __restrict__ order) {
-  __shared__ uint32_t bin[kCountBins];
-  __shared__ uint32_t wsum[32];
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  auto cell = [&](uint32_t i) -> uint32_t {
-    auto q = [](float c, float lo, float s) -> uint32_t {
-      const float v = (c - lo) * s;
-      if (!(v > 0.f)) return 0u;
-      return min(__float2uint_rz(v), 255u);
-    };
-    const uint32_t x = q(probes[3 * size_t(i)], lox, sx), y = q(probes[3 * size_t(i) + 1], loy, sy),
-                   z = q(probes[3 * size_t(i) + 2], loz, sz);
-    return ((expand_bits10(x) << 2) | (expand_bits10(y) << 1) | expand_bits10(z)) >> 12;
-  };
-  for (uint32_t b = tid; b < kCountBins; b += 1024) bin[b] = 0;
-  __syncthreads();
-  for (uint32_t i = tid; i < n; i += 1024) atomicAdd(&bin[cell(i)], 1u);
-  __syncthreads();
-  // exclusive scan: 4 bins per thread, warp shuffles, then the 32 warp totals
-  uint32_t v[4], t = 0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) { v[k] = bin[4 * tid + k]; t += v[k]; }
-  uint32_t incl = t;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= uint32_t(o)) incl += y;
-  }
-  if (lane == 31) wsum[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    const uint32_t w = wsum[lane];
-    uint32_t wi = w;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, wi, o);
-      if (lane >= uint32_t(o)) wi += y;
-    }
-    wsum[lane] = wi - w;
-  }
-  __syncthreads();
-  uint32_t run = wsum[warp] + incl - t;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) { bin[4 * tid + k] = run; run += v[k]; }
-  __syncthreads();
-  for (uint32_t i = tid; i < n; i += 1024) order[atomicAdd(&bin[cell(i)], 1u)] = i;
-}
-
-__global__ void __launch_bounds__(1024) k_probe_order_count(const float* __restrict__ probes, uint32_t n, float lox,
-                                                             float loy, float loz, float sx, float sy, float sz,
-                                                             uint32_t* __restrict__ order, uint32_t* zero_word) {
-  if (threadIdx.x == 0 && zero_word) *zero_word = 0;  // the next kernel's work counter
-  probe_sort_count(probes, n, lox, loy, loz, sx, sy, sz, order);
-}
-
 __global__ void __launch_bounds__(1024) k_probe_order_batch(const BakeJobDev* __restrict__ jobs) {
   const BakeJobDev& j = jobs[blockIdx.x];
   const uint32_t n = j.nprobes;
@@ -404,7 +330,8 @@ __global__ void __launch_bounds__(1024) k_probe_order_batch(const BakeJobDev* __
     s[i] = e > 0.f ? 256.0f / e : 0.f;
   }
   if (n <= kCountMax) {
-    probe_sort_count(j.probes, n, j.bounds[0], j.bounds[1], j.bounds[2], s[0], s[1], s[2], j.order);
+    __shared__ ProbeSortShared sh;
+    probe_sort_count<1024>(j.probes, n, j.bounds[0], j.bounds[1], j.bounds[2], s[0], s[1], s[2], j.order, sh);
     return;
   }
   uint32_t* sc = j.sort_scratch;  // 4 arrays of n
@@ -439,11 +366,6 @@ int launch_probe_order(const float* probes, uint32_t n, const float bounds[6], u
   for (int i = 0; i < 3; ++i) {
     const float e = bounds[3 + i] - bounds[i];
     s[i] = e > 0.f ? 256.0f / e : 0.f;
-  }
-  if (n <= kCountMax) {
-    k_probe_order_count<<<1, 1024, 0, st>>>(probes, n, bounds[0], bounds[1], bounds[2], s[0], s[1], s[2], order,
-                                            zero_word);
-    return 1;
   }
   if (zero_word) cudaMemsetAsync(zero_word, 0, 4, st);
   k_probe_codes<<<(n + 255) / 256, 256, 0, st>>>(probes, n, bounds[0], bounds[1], bounds[2], s[0], s[1], s[2], ka,

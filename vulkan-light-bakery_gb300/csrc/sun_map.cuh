@@ -1,8 +1,8 @@
-// k_lightmap.cu -- sun maps: shadow rays answered without a walk.
+// sun_map.cuh -- sun maps: shadow rays answered without a walk.
 //
 // All shadow rays of a bake run toward the sun, so they are parallel: seen
 // along the sun direction a ray is one point of a plane plus its origin's
-// depth.  This kernel rasterises the scene's triangles onto that plane and
+// depth.  A kernel rasterises the scene's triangles onto that plane and
 // keeps two depths (along the direction to the sun) per cell:
 //   cover  the largest depth below which every ray of the cell is occluded:
 //          some triangle covers the whole cell and lies above it everywhere;
@@ -23,13 +23,12 @@
 // before its atomic maximum: in deep scenes most triangles lie below one
 // already drawn.  Latency bound: 15 us for 778 triangles, 40 us for 164 k small
 // ones, 130 us for the 49 k faces of 4096 boxes.
-#include <algorithm>
+#pragma once
 
 #include "vlb_device.cuh"
 #include "vlb_internal.h"
 
 namespace vlbk {
-namespace {
 
 constexpr int kMapThreads = 256;
 // Order-preserving map of a float to an unsigned integer; 0 is below every float.
@@ -154,47 +153,6 @@ __device__ __forceinline__ void map_draw(const SunMap& m, const float4* __restri
     const int at = c - (k ? sh.end[k - 1] : 0), w = T.i1 - T.i0 + 1, r = at / w;
     map_cell(m, T, T.i0 + at - r * w, T.first + r * slices);
   }
-}
-
-__global__ void __launch_bounds__(kMapThreads) k_sun_map(const SunMap m, const float4* __restrict__ tris,
-                                                         uint32_t ntris) {
-  __shared__ MapShared sh;
-  map_draw(m, tris, ntris, blockIdx.x, int(blockIdx.y), int(gridDim.y), sh);
-}
-
-__global__ void __launch_bounds__(kMapThreads) k_sun_map_batch(const BakeJobDev* __restrict__ jobs, uint32_t njobs) {
-  __shared__ MapShared sh;
-  uint32_t lo = 0, hi = njobs - 1;  // the last job that begins at or before this CTA
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi + 1) >> 1;
-    if (__ldg(&jobs[mid].map_begin) <= blockIdx.x) lo = mid; else hi = mid - 1;
-  }
-  const BakeJobDev& j = jobs[lo];
-  const uint32_t c = blockIdx.x - j.map_begin;
-  if (!j.sun_map.cells || c / j.map_slices * kMapThreads >= j.ntris) return;
-  map_draw(j.sun_map, j.tris, j.ntris, c / j.map_slices, int(c % j.map_slices), int(j.map_slices), sh);
-}
-
-}  // namespace
-
-// CTAs per group of triangles: about seven CTAs per SM in all.
-uint32_t sun_map_slices(uint32_t ntris) {
-  const uint32_t groups = (ntris + kMapThreads - 1) / kMapThreads;
-  return std::min(64u, std::max(2u, 1024u / std::max(groups, 1u)));
-}
-
-void launch_sun_map(const SunMap& m, const float4* tris, uint32_t ntris, cudaStream_t s) {
-  if (!ntris) return;
-  cudaMemsetAsync(m.cells, 0, size_t(m.G) * m.G * 8, s);
-  const dim3 grid((ntris + kMapThreads - 1) / kMapThreads, sun_map_slices(ntris));
-  k_sun_map<<<grid, kMapThreads, 0, s>>>(m, tris, ntris);
-}
-
-void launch_sun_map_batch(const BakeJobDev* jobs, uint32_t njobs, uint32_t ctas, void* cells, size_t bytes,
-                          cudaStream_t s) {
-  if (!ctas) return;
-  cudaMemsetAsync(cells, 0, bytes, s);
-  k_sun_map_batch<<<ctas, kMapThreads, 0, s>>>(jobs, njobs);
 }
 
 }  // namespace vlbk

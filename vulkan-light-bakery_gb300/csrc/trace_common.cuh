@@ -534,7 +534,7 @@ __device__ __forceinline__ float ordered_f32(uint32_t k) {
   return __uint_as_float(k ^ (uint32_t(int32_t(~k) >> 31) | 0x80000000u));
 }
 
-// Probe frontiers (k_front.cu).  The lanes `mine` test their primary rays
+// Probe frontiers (front.cuh).  The lanes `mine` test their primary rays
 // against entries [first, first + 32) of their probe's frontier and stack
 // those they hit, nearest on top; returns whether any of them has entries left.
 // The rays share an origin, so relative to it a plane at x is crossed at x / d.

@@ -62,14 +62,22 @@ bool is_device_ptr(const void* p) {
 vlb_status scratch(vlb_ctx* ctx, const char* name, size_t bytes, void** out) {
   auto& b = ctx->scratch[name];
   if (b.bytes < bytes) {
+    const size_t old = b.bytes;
     if (b.p) {
       cudaStreamSynchronize(ctx->stream);
       cudaFree(b.p);
       b.p = nullptr;
       b.bytes = 0;
     }
-    size_t want = std::max<size_t>(bytes, 256);
+    // a buffer that grows grows by half at least: batches of uneven sizes then
+    // reach their largest in a few steps, not in one allocation each
+    size_t want = std::max<size_t>(std::max<size_t>(bytes, 256), old + old / 2);
     cudaError_t e = cudaMalloc(&b.p, want);
+    if (e != cudaSuccess && want > bytes) {
+      cudaGetLastError();
+      want = bytes;
+      e = cudaMalloc(&b.p, want);
+    }
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(ctx, VLB_ERR_OOM, "scratch '%s': cudaMalloc(%zu) failed", name, want);
@@ -1116,7 +1124,7 @@ static bool grid_mode(const vlb_scene* scene, uint32_t nprobes, uint32_t S, cons
          p->shading == VLB_SHADE_LAMBERT_SUN;  // the grids hold the sun's parallel shadow rays
 }
 
-// Entries per probe of a bake's probe frontiers (k_front.cu), 0 for walks from
+// Entries per probe of a bake's probe frontiers (front.cuh), 0 for walks from
 // the root.  A frontier costs a warp some twenty dependent loads per probe and
 // its rays share it: at 64 rays a probe a lone small bake breaks even (64
 // probes: 83 us with and without) and a batch gains (6.1 -> 5.6 ms); fewer
@@ -1140,7 +1148,7 @@ static float bounds_scale(const vlb_scene* scene) {
 constexpr uint32_t kMapSide = 256;
 constexpr size_t kMapBytes = size_t(kMapSide) * kMapSide * 8;
 
-// Whether a bake's sun map (k_lightmap.cu) saves more than it costs.  It saves
+// Whether a bake's sun map (sun_map.cuh) saves more than it costs.  It saves
 // some 25 ps a ray (20 in a terrain of 164 k triangles, 45 in 4096 boxes, 50 in
 // 64); it costs 90 ps a triangle and 1 us per layer of triangles over the map's
 // cells (15 us for that terrain, 130 us for the 4096 boxes' 130 layers), and a
@@ -1155,7 +1163,7 @@ static bool sun_map_pays(const vlb_scene* sc, uint64_t rays, double launch_us) {
   return sc->ntris && double(rays) * 25e-6 > launch_us + sc->ntris * 90e-6 + layers;
 }
 
-// Plane, extent and margins of a scene's sun map (k_lightmap.cu).
+// Plane, extent and margins of a scene's sun map (sun_map.cuh).
 static void sun_map_plan(const vlb_scene* scene, float3 s, float bias, uint32_t G, uint32_t* cells, vlbk::SunMap* m) {
   const double d[3] = {s.x, s.y, s.z};
   int least = 0;
@@ -1228,11 +1236,10 @@ static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const floa
       (st = scratch(ctx, "probe_order_tmp", vlbk::probe_order_scratch_bytes(nprobes), &oscr)) ||
       (st = scratch(ctx, "trace_work", 256, &wc)))
     return st;
-  {
-    float b[6];
-    for (int a = 0; a < 6; ++a) b[a] = scene->bounds[a];
+  const bool order_first = !vlbk::probe_order_in_setup(nprobes);
+  if (order_first) {
     KScope k(ctx, "probe_order", 0);
-    k.nkernels = vlbk::launch_probe_order(static_cast<const float*>(dprobes), nprobes, b,
+    k.nkernels = vlbk::launch_probe_order(static_cast<const float*>(dprobes), nprobes, scene->bounds,
                                           static_cast<uint32_t*>(order), oscr, static_cast<uint32_t*>(wc),
                                           ctx->stream);
   }
@@ -1259,21 +1266,26 @@ static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const floa
     void* cells;
     if ((st = scratch(ctx, "sun_map", kMapBytes, &cells))) return st;
     sun_map_plan(scene, a.sun, a.bias, kMapSide, static_cast<uint32_t*>(cells), &a.sun_map);
-    KScope k(ctx, "sun_map");
-    vlbk::launch_sun_map(a.sun_map, scene->tris, scene->ntris, ctx->stream);
   }
   const bool grid = grid_mode(scene, nprobes, a.S, p);
   const uint32_t cap = a.lane && !grid && !from_root ? front_cap(scene, nprobes, a.S) : 0;
-  void *ent, *cnt;
+  void *ent = nullptr, *cnt = nullptr;
   if (cap && scratch(ctx, "front_ent", size_t(nprobes) * cap * 32, &ent) == VLB_OK &&
       scratch(ctx, "front_cnt", size_t(nprobes) * 4, &cnt) == VLB_OK) {
-    const vlbk::FrontArgs f{scene->nodes, scene->ntris, a.probes, nprobes, bounds_scale(scene), cap,
-                            static_cast<float4*>(ent), static_cast<uint32_t*>(cnt), ctx->d_err};
-    KScope k(ctx, "probe_front");
-    vlbk::launch_probe_front(f, ctx->stream);
-    a.front = f.ent;
-    a.front_n = f.cnt;
+    a.front = static_cast<const float4*>(ent);
+    a.front_n = static_cast<const uint32_t*>(cnt);
     a.front_cap = cap;
+  }
+  if (!order_first || a.front || a.sun_map.cells) {
+    vlbk::SetupArgs su{};
+    su.front = vlbk::FrontArgs{scene->nodes, scene->ntris, a.probes, nprobes, bounds_scale(scene), cap,
+                               a.front ? static_cast<float4*>(ent) : nullptr, static_cast<uint32_t*>(cnt), ctx->d_err};
+    su.map = a.sun_map;
+    su.tris = scene->tris;
+    su.order = order_first ? nullptr : static_cast<uint32_t*>(order);
+    su.zero_word = static_cast<uint32_t*>(wc);
+    KScope k(ctx, "bake_setup");
+    vlbk::launch_bake_setup(su, scene->bounds, ctx->stream);
   }
   if (grid) {
     const uint32_t G = grid_cells_per_side(scene->ntris), T = scene->ntris;
@@ -1298,7 +1310,7 @@ static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const floa
     vlbk::launch_grid_build(a, ctx->stream);
   }
   vlbk::plan_trace(a, ctx->num_sms, p->precision == VLB_PREC_FUSED);
-  a.work_counter = static_cast<uint32_t*>(wc);  // zeroed by the probe-order launch
+  a.work_counter = static_cast<uint32_t*>(wc);  // zeroed with the probe order
   return VLB_OK;
 }
 

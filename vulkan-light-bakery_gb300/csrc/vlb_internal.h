@@ -224,7 +224,7 @@ size_t point_order_scratch_bytes(uint32_t n);
 int launch_point_order(const float* pts, uint32_t n, const float bounds[6], uint32_t* order, void* scratch,
                        cudaStream_t s);
 
-// ---- probe frontiers (k_front.cu) ------------------------------------------------
+// ---- probe frontiers (front.cuh) ------------------------------------------------
 // Entries per probe: 32 bytes each, [lx ly hx hy] [lz hz ref dist^2], the box
 // relative to the probe, nearest first; cnt[probe] of them.
 constexpr int kFrontCap = 128;
@@ -239,12 +239,11 @@ struct FrontArgs {
   uint32_t* cnt;          // [nprobes]
   int* err;
 };
-void launch_probe_front(const FrontArgs& a, cudaStream_t s);
 struct BakeJobDev;
 // The frontiers of all jobs that have one: `total` probes, numbered by front_begin.
 void launch_probe_front_batch(const BakeJobDev* jobs, uint32_t njobs, uint32_t total, cudaStream_t s);
 
-// ---- sun maps (k_lightmap.cu) ------------------------------------------------------
+// ---- sun maps (sun_map.cuh) ------------------------------------------------------
 struct SunMap {
   uint32_t* cells;   // [G][G] (cover, top) as ordered integers, or null: every shadow ray walks
   float3 u, v, s;    // unit: across and along the direction to the sun
@@ -255,11 +254,25 @@ struct SunMap {
 };
 uint32_t sun_map_slices(uint32_t ntris);
 inline uint32_t sun_map_ctas(uint32_t ntris) { return (ntris + 255) / 256 * sun_map_slices(ntris); }
-void launch_sun_map(const SunMap& m, const float4* tris, uint32_t ntris, cudaStream_t s);
 // The maps of all jobs that have one (`ctas` CTAs numbered by map_begin); their
 // cells, `bytes` from `cells`, are cleared first.
 void launch_sun_map_batch(const BakeJobDev* jobs, uint32_t njobs, uint32_t ctas, void* cells, size_t bytes,
                           cudaStream_t s);
+// One bake's probe order (order null: done before, or not wanted here),
+// frontiers (front.ent null: none) and sun map (map.cells null: none) in one
+// launch (k_setup.cu); front.probes, nprobes and ntris are always set.
+struct SetupArgs {
+  FrontArgs front;
+  SunMap map;
+  const float4* tris;
+  uint32_t map_ctas, map_slices;  // set by the launch
+  uint32_t* order;
+  uint32_t* zero_word;
+  float lo[3], s[3];
+};
+void launch_bake_setup(SetupArgs a, const float bounds[6], cudaStream_t s);
+// Whether that launch sorts a bake's probes (else launch_probe_order does).
+uint32_t probe_order_in_setup(uint32_t nprobes);
 
 // ---- trace + shade --------------------------------------------------------------
 struct TraceArgs {
@@ -442,8 +455,9 @@ inline void fused_items(BakeJobDev* j, uint32_t part_rays) {
 }
 // Items from which chunks stay whole: with fewer, a warp holds only a few items
 // and waits at the end for those that drew the long ones (4641 probes x 515
-// directions, 13,923 chunks on 4864 warps: 917 -> 755 us).
-constexpr uint32_t kFusedPart = 64;  // 32 and 96 measure the same
+// directions, 13,923 chunks on 4864 warps: the walk 917 -> 750 us with items of 32
+// rays, 820 us with 64).
+constexpr uint32_t kFusedPart = 32;
 constexpr uint64_t kFusedWhole = 16ull * 32;  // per SM
 constexpr size_t kFusedSubBytes = 256u << 20;
 // Launch knobs of the fused walk (vlb_batch_schedule; results do not depend on them).
