@@ -111,6 +111,9 @@ __device__ __forceinline__ void project_stage(const T* __restrict__ rad, uint32_
 // sequential FP32 sum per row.
 constexpr uint32_t kProjSplitCtas = 304;
 constexpr uint32_t kProjMinSplitSamples = 16 * kProjCols;
+// Longer rows are split down to half of that: a CTA of a few rows waits on its
+// loads stage after stage (6 rows x 149,331 samples: 62 us before, 49 with the sums below in parallel).
+constexpr uint32_t kProjLong = 16384;
 
 //
 // Tiles of at least kProjStream samples stream through the TMA-staged kernel:
@@ -124,7 +127,8 @@ static uint32_t project_splits(uint32_t rows, uint32_t S, uint32_t* per) {
   if (size_t(rows) * S >= kProjStream && S % 4 == 0 && tiles < kProjSplitCtas)
     splits = std::max(1u, std::min(kProjStreamUnits / tiles256, S / kProjMinSplitSamples));
   else if (tiles && tiles < kProjSplitCtas)
-    splits = std::max(1u, std::min((kProjSplitCtas + tiles - 1) / tiles, S / kProjMinSplitSamples));
+    splits = std::max(1u, std::min((kProjSplitCtas + tiles - 1) / tiles,
+                                   S / (S < kProjLong ? kProjMinSplitSamples : kProjMinSplitSamples / 2)));
   uint32_t p = (S + splits - 1) / splits;
   p = (p + kProjCols - 1) / kProjCols * kProjCols;  // whole stages
   *per = p;
@@ -183,16 +187,31 @@ __global__ void __launch_bounds__(kProjRows) k_project(const T* __restrict__ rad
   }
 }
 
-// out (probe, k, channel) = the splits' partials of (row, k) added in FP64 in split order.
-__global__ void k_project_reduce(const float* __restrict__ partial, uint32_t splits, uint32_t rows, uint32_t K,
-                                 float* __restrict__ out) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * K) return;
-  const uint32_t row = i / K, k = i - row * K;
+// out (probe, k, channel) = the splits' partials of (row, k) added in FP64: warp
+// g of a CTA takes 32 outputs' splits g, g + 32, ... and the warps' sums are
+// added in order (a fixed order for a split count).  One thread per output took
+// 30 us for the 145 splits of 6 rows.
+__global__ void __launch_bounds__(1024) k_project_reduce(const float* __restrict__ partial, uint32_t splits,
+                                                         uint32_t rows, uint32_t K, float* __restrict__ out) {
+  __shared__ double s_sum[32][32];
+  const uint32_t lane = threadIdx.x & 31, g = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+  const uint32_t groups = blockDim.x >> 5;
   double sum = 0.0;
-  for (uint32_t y = 0; y < splits; ++y) sum += double(partial[(size_t(y) * rows + row) * K + k]);
-  const uint32_t p = row / 3, c = row - 3 * p;
+  if (i < rows * K)
+#pragma unroll 4
+    for (uint32_t y = g; y < splits; y += groups) sum += double(__ldg(partial + size_t(y) * rows * K + i));
+  s_sum[g][lane] = sum;
+  __syncthreads();
+  if (g || i >= rows * K) return;
+  for (uint32_t w = 1; w < groups; ++w) sum += s_sum[w][lane];
+  const uint32_t row = i / K, k = i - row * K, p = row / 3, c = row - 3 * p;
   out[(size_t(p) * K + k) * 3 + c] = float(sum);
+}
+
+static void launch_reduce(const float* partial, uint32_t splits, uint32_t rows, uint32_t K, float* out,
+                          cudaStream_t s) {
+  const uint32_t groups = std::min(32u, std::max(1u, (splits + 3) / 4));
+  k_project_reduce<<<(rows * K + 31) / 32, groups * 32, 0, s>>>(partial, splits, rows, K, out);
 }
 
 template <typename T>
@@ -207,7 +226,7 @@ static void launch_project(const T* rad, uint32_t nprobes, uint32_t S, const flo
   const dim3 grid(tiles, splits);
   if (K == 9) k_project<T, 9><<<grid, kProjRows, 0, s>>>(rad, rows, S, per, basis16, out, partial, split);
   else k_project<T, 16><<<grid, kProjRows, 0, s>>>(rad, rows, S, per, basis16, out, partial, split);
-  if (splits > 1) k_project_reduce<<<(rows * K + 255) / 256, 256, 0, s>>>(partial, splits, rows, K, out);
+  if (splits > 1) launch_reduce(partial, splits, rows, K, out, s);
 }
 
 void launch_project_f32(const float* radiance, uint32_t nprobes, uint32_t S, const float* basis16, uint32_t K,
@@ -222,7 +241,7 @@ void launch_project_f32(const float* radiance, uint32_t nprobes, uint32_t S, con
   if (err && num_sms && S && (splits == 1 || size_t(rows) * S >= kProjStream) &&
       launch_project_f32_tma(radiance, nprobes, S, basis16, K, out, partial, splits, splits == 1 ? S : per, err,
                              num_sms, s, hold, wait_polls)) {
-    if (splits > 1) k_project_reduce<<<(rows * K + 255) / 256, 256, 0, s>>>(partial, splits, rows, K, out);
+    if (splits > 1) launch_reduce(partial, splits, rows, K, out, s);
     return;
   }
   launch_project<float>(radiance, nprobes, S, basis16, K, out, partial, 0, s);

@@ -201,8 +201,7 @@ static void launch(const TraceArgs& a, int num_sms, cudaStream_t s) {
 // their origin and take neighbouring directions of the trace order (grouped
 // by octant, then by position on the octant's face), so their walks share
 // the nodes around the probe (5 % faster than rays of one direction from
-// Morton-neighbour probes on a 16^3 grid, 19 % on random probes); slots run
-// to the probe count rounded up to 32.  Box tests take the per-lane octant
+// Morton-neighbour probes on a 16^3 grid, 19 % on random probes).  Box tests take the per-lane octant
 // at run time; the tests, the pruning and the tie rule are those of
 // lane_traverse, so each ray's result is unchanged.
 
@@ -233,8 +232,7 @@ template <bool COUNT, bool WIDE, bool REF>
 // (eight CTAs: 130.9 against 125.6 ms); ten CTAs would spill.
 __global__ void __launch_bounds__(kTraceThreads, 9) k_trace_dyn(const TraceArgs a) {
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t P = (a.nprobes + 31) / 32 * 32;
-  const uint32_t R = P * a.S;
+  const uint32_t R = a.nprobes * a.S;
   Work w;
   int stack[kLaneStackFront + 1];
   LaneRay L;
@@ -282,7 +280,7 @@ __global__ void __launch_bounds__(kTraceThreads, 9) k_trace_dyn(const TraceArgs 
       const uint32_t r = wb + lane;
       if (r < R && lane < block) {
         const uint32_t sl = r / a.S, t = r - sl * a.S;
-        if (sl < a.nprobes) lr_start(a, L, a.order[sl], __ldg(a.dir_order + t), stack);
+        lr_start(a, L, a.order[sl], __ldg(a.dir_order + t), stack);
       }
       if constexpr (!WIDE) {
         if (a.front) fnext = lr_front_next(a, L, L.has, 0, stack);
@@ -331,7 +329,7 @@ static void launch_dyn(const TraceArgs& a, int num_sms, cudaStream_t s) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceThreads, 0);
     if (per_sm < 1) per_sm = 1;
   }
-  const uint64_t rays = uint64_t((a.nprobes + 31) / 32 * 32) * a.S;
+  const uint64_t rays = uint64_t(a.nprobes) * a.S;
   uint64_t ctas = std::max<uint64_t>(
       std::min<uint64_t>((rays + kTraceThreads - 1) / kTraceThreads, uint64_t(num_sms) * per_sm), 1);
   // ray blocks: whole 32-ray groups, as many as keep ~64 blocks a warp, at most 16
@@ -754,9 +752,9 @@ __device__ __forceinline__ void batch_emit(const BakeJobDev& j, uint32_t p, uint
   }
 }
 
-// Batched bake.  Job j owns the rays [ray_begin, ray_begin + P*S) of one
-// numbering over all jobs (P: its probe count rounded up to 32; ray r of a job
-// is probe slot r / S, direction position r % S), each job's range rounded up
+// Batched bake.  Job j owns the rays [ray_begin, ray_begin + nprobes*S) of one
+// numbering over all jobs (ray r of a job is probe slot r / S, direction
+// position r % S), each job's range rounded up
 // to whole chunks of 32 * chunk_lanes rays.  A warp takes a chunk from the
 // counter (one atomic), finds its job by binary search over the ranges, and
 // hands the chunk's next 32 rays to its lanes whenever all of them are idle;
@@ -784,8 +782,7 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_trace_batch(const BakeJobD
       if (__ldg(&jobs[mid].ray_begin) <= c) lo = mid; else hi = mid - 1;
     }
     const BakeJobDev& j = jobs[lo];
-    const uint32_t P = (j.nprobes + 31) / 32 * 32;
-    const uint32_t R = P * j.S;
+    const uint32_t R = j.nprobes * j.S;
     uint32_t r0 = c - j.ray_begin;                // the chunk's first ray in the job
     const uint32_t r1 = min(R, r0 + chunk);       // end of its real rays (the rest is padding)
     const bool front = j.front && !j.hits_in;
@@ -800,19 +797,17 @@ __global__ void __launch_bounds__(kTraceThreads, 8) k_trace_batch(const BakeJobD
         r0 = min(r1, r0 + uint32_t(__popc(idle)));
         if (!L.has && r < r1) {
           const uint32_t sl = r / j.S, t = r - sl * j.S;
-          if (sl < j.nprobes) {
-            const uint32_t p = j.order[sl];
-            lr_start(j, L, p, __ldg(j.dir_order + t), stack);
-            if (j.hits_in) {  // relight: the kept primary hit, only the shadow walk remains
-              const int2 h = __ldg(j.hits_in + size_t(p) * j.S + L.s);
-              L.slot = h.x;
-              L.tb = __int_as_float(h.y);
-              L.id = h.x >= 0 ? __float_as_int(__ldg(j.tris + 3 * VLB_CLAMP(h.x, j.ntris, j.err)).w) : -1;
-              Shaded o;
-              if (lr_finish<false, BakeJobDev, REF>(j, L, o, w, stack)) {
-                L.has = false;
-                batch_emit(j, L.p, L.s, o);
-              }
+          const uint32_t p = j.order[sl];
+          lr_start(j, L, p, __ldg(j.dir_order + t), stack);
+          if (j.hits_in) {  // relight: the kept primary hit, only the shadow walk remains
+            const int2 h = __ldg(j.hits_in + size_t(p) * j.S + L.s);
+            L.slot = h.x;
+            L.tb = __int_as_float(h.y);
+            L.id = h.x >= 0 ? __float_as_int(__ldg(j.tris + 3 * VLB_CLAMP(h.x, j.ntris, j.err)).w) : -1;
+            Shaded o;
+            if (lr_finish<false, BakeJobDev, REF>(j, L, o, w, stack)) {
+              L.has = false;
+              batch_emit(j, L.p, L.s, o);
             }
           }
         }

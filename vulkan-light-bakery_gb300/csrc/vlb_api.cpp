@@ -1769,14 +1769,12 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
 
   // stage host probes, build the job table
   const size_t esz = pl.bf16 && !pl.split ? 2 : 4;
-  uint64_t warp_rays = 0;
-  for (const auto& b : pl.jobs) warp_rays += (uint64_t(b.nprobes) + 31) / 32 * b.S;
   // rays per lane per chunk (a warp takes 32 x that many rays at a time):
   // at least ~16 chunks per resident warp, at most 8 rays per lane
   uint32_t dpw = sc.dirs_per_item;
   if (!dpw) {
     uint64_t rays = 0;
-    for (const auto& b : pl.jobs) rays += (uint64_t(b.nprobes) + 31) / 32 * 32 * b.S;
+    for (const auto& b : pl.jobs) rays += uint64_t(b.nprobes) * b.S;
     const uint64_t target = 16ull * 32 * 32 * uint64_t(ctx->num_sms);
     dpw = uint32_t(std::min<uint64_t>(8, std::max<uint64_t>(1, rays / target)));
   }
@@ -1787,7 +1785,7 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
   auto& table = ctx->batch_table;
   table.assign(ntable, vlbk::BakeJobDev{});
   size_t poff = 0, part_off = 0, sub_off = 0, nmaps = 0;
-  uint64_t items = 0;
+  uint64_t items = 0, padded = 0;  // padded: the rays of whole 32-probe packets, the size a batch is limited to
   for (uint32_t t = 0; t < ntable; ++t) {
     const BatchJob& b = pl.jobs[ord[t]];
     const vlb_bake_job& j = jobs[b.idx];
@@ -1842,7 +1840,8 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
       if (pl.bf16) d.radiance_bf16 = reinterpret_cast<uint16_t*>(rad);
       else d.radiance = reinterpret_cast<float*>(rad);
       d.ray_begin = uint32_t(items);
-      items += ((uint64_t(b.nprobes) + 31) / 32 * 32 * b.S + chunk - 1) / chunk * chunk;
+      items += (uint64_t(b.nprobes) * b.S + chunk - 1) / chunk * chunk;
+      padded += (uint64_t(b.nprobes) + 31) / 32 * 32 * b.S;
     }
     d.front_begin = bb.front_total;
     if (cap && fronts[ord[t]]) {
@@ -1863,7 +1862,7 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
     d.sort_scratch = bb.sort + 4 * b.row0;
     if (ext) { d.hits_out = ext[b.idx].hits_out; d.hits_in = ext[b.idx].hits_in; }
   }
-  if (items >= (1ull << 31))
+  if (std::max(items, padded) >= (1ull << 31))
     return fail(ctx, VLB_ERR_INVALID, pl.fused ? "batch has 2^31 work items or more; split it"
                                                : "batch has 2^31 rays or more; split it");
   auto& meta_h = ctx->batch_meta;

@@ -389,8 +389,8 @@ struct BakeJobDev {
   float* radiance;
   uint16_t* radiance_bf16;
   uint32_t bf16_split;    // 1: hi/lo pairs, rows of 2S
-  // rays [ray_begin, ray_begin + P * S) of the batch's numbering (P: nprobes
-  // rounded up to 32), the range rounded up to whole chunks
+  // rays [ray_begin, ray_begin + nprobes * S) of the batch's numbering, the
+  // range rounded up to whole chunks
   uint32_t ray_begin;
   // probe sort: bounds for the Morton codes, 4 scratch arrays of nprobes
   float bounds[6];
