@@ -230,7 +230,7 @@ template <bool COUNT, bool WIDE, bool REF>
 // Nine resident CTAs per SM (at most 56 registers): measured 4 % faster on
 // the 64^3-probe, 1024-direction bake than the unconstrained 60 registers
 // (eight CTAs: 130.9 against 125.6 ms); ten CTAs would spill.
-__global__ void __launch_bounds__(kTraceThreads, 9) k_trace_dyn(const TraceArgs a) {
+__global__ void __launch_bounds__(kTraceThreads, 10) k_trace_dyn(const TraceArgs a) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t R = a.nprobes * a.S;
   Work w;

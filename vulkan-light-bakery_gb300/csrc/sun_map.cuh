@@ -15,6 +15,13 @@
 // (grazing triangles, where that grows, do not cover), and top is raised by
 // the test's depth error, so every ray keeps the answer its walk gives.
 //
+// A point light outside the scene is the same map seen from the light: u and v
+// are divided by the distance along the view axis and the depth is its
+// reciprocal, so triangles stay triangles and depth planes planes.  A shadow ray
+// there runs parallel to the line from the hit to the light, `bias` beside it,
+// and drifts by at most bias (1 / nearest - 1 / farthest) in u and v: cells are
+// widened by that too.
+//
 // Thread k of a CTA sets up one triangle; the CTA's triangles' cells are then
 // numbered through and shared by all its threads (a binary search finds a
 // cell's triangle), so slivers and walls cost what their cells cost.  Several
@@ -51,16 +58,36 @@ __device__ __forceinline__ float dotm(float x, float y, float z, float3 a) {
 
 __device__ __forceinline__ void map_setup(const SunMap& m, const float4 a, const float4 e1, const float4 e2,
                                           MapTri& T) {
-  const float au = dotm(a.x, a.y, a.z, m.u), av = dotm(a.x, a.y, a.z, m.v), ad = dotm(a.x, a.y, a.z, m.s);
-  const float bu = dotm(e1.x, e1.y, e1.z, m.u), bv = dotm(e1.x, e1.y, e1.z, m.v), bd = dotm(e1.x, e1.y, e1.z, m.s);
-  const float cu = dotm(e2.x, e2.y, e2.z, m.u), cv = dotm(e2.x, e2.y, e2.z, m.v), cd = dotm(e2.x, e2.y, e2.z, m.s);
-  const float det = bu * cv - bv * cu;  // twice the projected area, signed
+  float au, av, ad, bu, bv, bd, cu, cv, cd;  // the first vertex, the edges from it
   const float l1 = e1.x * e1.x + e1.y * e1.y + e1.z * e1.z, l2 = e2.x * e2.x + e2.y * e2.y + e2.z * e2.z;
-  // the triangle test's rounding grows with |e1| |e2| / |det|
-  const float grow = sqrtf(l1 * l2) / fabsf(det);
-  const bool steep = !(grow < 256.f);
-  T.slack = steep ? INFINITY : m.margin * (1.f + grow);
-  T.pad = T.slack;
+  float det, facing;  // twice the projected area, signed; |e1 x e2 . direction|
+  if (m.point) {
+    const float x = a.x - m.o.x, y = a.y - m.o.y, z = a.z - m.o.z;
+    auto see = [&](float px, float py, float pz, float& u, float& v, float& d) {
+      d = 1.0f / dotm(px, py, pz, m.s);
+      u = dotm(px, py, pz, m.u) * d;
+      v = dotm(px, py, pz, m.v) * d;
+    };
+    see(x, y, z, au, av, ad);
+    see(x + e1.x, y + e1.y, z + e1.z, bu, bv, bd);
+    see(x + e2.x, y + e2.y, z + e2.z, cu, cv, cd);
+    bu -= au; bv -= av; bd -= ad;
+    cu -= au; cv -= av; cd -= ad;
+    det = bu * cv - bv * cu;
+    const float nx = e1.y * e2.z - e1.z * e2.y, ny = e1.z * e2.x - e1.x * e2.z, nz = e1.x * e2.y - e1.y * e2.x;
+    facing = fabsf(nx * x + ny * y + nz * z) * rsqrtf(x * x + y * y + z * z);
+  } else {
+    au = dotm(a.x, a.y, a.z, m.u); av = dotm(a.x, a.y, a.z, m.v); ad = dotm(a.x, a.y, a.z, m.s);
+    bu = dotm(e1.x, e1.y, e1.z, m.u); bv = dotm(e1.x, e1.y, e1.z, m.v); bd = dotm(e1.x, e1.y, e1.z, m.s);
+    cu = dotm(e2.x, e2.y, e2.z, m.u); cv = dotm(e2.x, e2.y, e2.z, m.v); cd = dotm(e2.x, e2.y, e2.z, m.s);
+    det = bu * cv - bv * cu;
+    facing = fabsf(det);
+  }
+  // the triangle test's rounding grows with |e1| |e2| / |e1 x e2 . direction|
+  const float grow = sqrtf(l1 * l2) / facing;
+  const bool steep = !(grow < 256.f && fabsf(det) > 0.f);
+  T.slack = steep ? INFINITY : m.dmargin * (1.f + grow);
+  T.pad = steep ? INFINITY : m.margin * (1.f + grow);
   T.covers = !steep;
   T.dmax = ad + fmaxf(0.f, fmaxf(bd, cd)) + T.slack;
   const float inv = steep ? 0.f : 1.f / det;

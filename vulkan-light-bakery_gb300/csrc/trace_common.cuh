@@ -627,6 +627,28 @@ __device__ __forceinline__ float ref_srgb(float c) {
 }
 __device__ __forceinline__ float ref_unorm8(float c) { return rintf(fminf(fmaxf(c, 0.f), 1.f) * 255.f) / 255.f; }
 
+// The sun map's answer for a shadow ray from (x, y, z): 0 occluded, 1 lit, 2
+// not known (walk).  A ray occluded at no more than `top` above its origin
+// must meet its occluder before tmax.
+template <bool POINT>
+__device__ __forceinline__ int sun_map_query(const SunMap& m, float x, float y, float z, float tmax) {
+  float d, k = 1.f;
+  if constexpr (POINT) { x -= m.o.x; y -= m.o.y; z -= m.o.z; }
+  d = fmaf(z, m.s.z, fmaf(y, m.s.y, x * m.s.x));
+  if constexpr (POINT) {
+    if (!(d > 0.f)) return 2;
+    d = k = 1.0f / d;
+  }
+  const float fu = (fmaf(z, m.u.z, fmaf(y, m.u.y, x * m.u.x)) * k - m.u0) * m.inv;
+  const float fv = (fmaf(z, m.v.z, fmaf(y, m.v.y, x * m.v.x)) * k - m.v0) * m.inv;
+  const float G = float(m.G);
+  if (!(fu >= 0.f && fu < G && fv >= 0.f && fv < G)) return 2;
+  const uint2 c = __ldg(reinterpret_cast<const uint2*>(m.cells) + (uint32_t(fv) * m.G + uint32_t(fu)));
+  if (ordered_u32(d - m.dmargin) > c.y) return 1;
+  // toward a point light every occluder lies before the light, where the ray ends
+  return ordered_u32(d + m.dmargin) < c.x && (POINT || c.y < ordered_u32(d + 0.99f * tmax)) ? 0 : 2;
+}
+
 // The reference's shading of a primary result (vlb_shading
 // VLB_SHADE_REF_PHONG, shaders/env_map.rchit:51-102): a miss is done; a hit
 // facing the point light starts its shadow walk toward it (returns false;
@@ -660,7 +682,21 @@ __device__ __forceinline__ bool lr_finish_ref_primary(const A& a, LaneRay& L, Sh
   float sp = fmaxf(rx * L.d.x + ry * L.d.y + rz * L.d.z, 0.f);
   sp *= sp; sp *= sp; sp *= sp; sp *= sp;  // ^16
   L.lit = 0.5f * sdn + 0.5f * sp;
-  make_ray(L.ray, px + a.bias * nx, py + a.bias * ny, pz + a.bias * nz, lx, ly, lz);
+  const float hx = px + a.bias * nx, hy = py + a.bias * ny, hz = pz + a.bias * nz;
+  if (a.sun_map.cells) {
+    const int known = sun_map_query<true>(a.sun_map, hx, hy, hz, len);
+    if (known != 2) {
+      o.vis = uint8_t(known);
+      if (known) {
+        const float4 alb = __ldg(a.albedo + VLB_CLAMP(L.id, a.ntris, a.err));
+        o.r = ref_unorm8(ref_srgb(alb.x * L.lit));
+        o.g = ref_unorm8(ref_srgb(alb.y * L.lit));
+        o.b = ref_unorm8(ref_srgb(alb.z * L.lit));
+      }
+      return true;
+    }
+  }
+  make_ray(L.ray, hx, hy, hz, lx, ly, lz);
   L.shadow = true;
   L.cur = walk_root(a.ntris);
   lr_empty(a, L, stack);
@@ -672,20 +708,6 @@ __device__ __forceinline__ bool lr_finish_ref_primary(const A& a, LaneRay& L, Sh
     if (t > 0.0f && t < L.tb) { L.slot = L.oprev; L.cur = kWalkEnd; }
   }
   return false;
-}
-
-// The sun map's answer for a shadow ray from (x, y, z): 0 occluded, 1 lit, 2
-// not known (walk).  A ray occluded at no more than `top` above its origin
-// must meet its occluder before tmax.
-__device__ __forceinline__ int sun_map_query(const SunMap& m, float x, float y, float z, float tmax) {
-  const float fu = (fmaf(z, m.u.z, fmaf(y, m.u.y, x * m.u.x)) - m.u0) * m.inv;
-  const float fv = (fmaf(z, m.v.z, fmaf(y, m.v.y, x * m.v.x)) - m.v0) * m.inv;
-  const float G = float(m.G);
-  if (!(fu >= 0.f && fu < G && fv >= 0.f && fv < G)) return 2;
-  const float d = fmaf(z, m.s.z, fmaf(y, m.s.y, x * m.s.x));
-  const uint2 c = __ldg(reinterpret_cast<const uint2*>(m.cells) + (uint32_t(fv) * m.G + uint32_t(fu)));
-  if (ordered_u32(d - m.margin) > c.y) return 1;
-  return ordered_u32(d + m.margin) < c.x && c.y < ordered_u32(d + 0.99f * tmax) ? 0 : 2;
 }
 
 // After a walk (REF: the reference's shading, vlb_shading
@@ -728,7 +750,7 @@ __device__ __forceinline__ bool lr_finish(const A& a, LaneRay& L, Shaded& o, Wor
                 hz = fmaf(L.tb, L.d.z, L.oz) + a.bias * nz;
     L.lit = a.sun_scale * ndl;
     if (a.sun_map.cells) {
-      const int known = sun_map_query(a.sun_map, hx, hy, hz, a.tmax);
+      const int known = sun_map_query<false>(a.sun_map, hx, hy, hz, a.tmax);
       if (known != 2) {
         o.vis = uint8_t(known);
         if (known) {

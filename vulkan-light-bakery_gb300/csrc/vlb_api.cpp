@@ -1163,9 +1163,23 @@ static bool sun_map_pays(const vlb_scene* sc, uint64_t rays, double launch_us) {
   return sc->ntris && double(rays) * 25e-6 > launch_us + sc->ntris * 90e-6 + layers;
 }
 
-// Plane, extent and margins of a scene's sun map (sun_map.cuh).
-static void sun_map_plan(const vlb_scene* scene, float3 s, float bias, uint32_t G, uint32_t* cells, vlbk::SunMap* m) {
-  const double d[3] = {s.x, s.y, s.z};
+// Plane, extent and margins of a scene's sun map (sun_map.cuh) for a sun toward
+// `sun`, or for the point light at *light; false (m->cells null) for a light that
+// does not stand clear of the scene.
+static bool sun_map_plan(const vlb_scene* scene, float3 sun, const float3* light, float bias, uint32_t* cells,
+                         vlbk::SunMap* m) {
+  const float* bb = scene->bounds;
+  double d[3] = {sun.x, sun.y, sun.z}, o[3] = {0, 0, 0};
+  if (light) {  // the view axis: from the light to the middle of the scene
+    o[0] = light->x; o[1] = light->y; o[2] = light->z;
+    double n = 0.0;
+    for (int a = 0; a < 3; ++a) {
+      d[a] = 0.5 * (double(bb[a]) + bb[3 + a]) - o[a];
+      n += d[a] * d[a];
+    }
+    if (!(n > 0.0)) return false;
+    for (double& x : d) x /= std::sqrt(n);
+  }
   int least = 0;
   for (int a = 1; a < 3; ++a)
     if (std::fabs(d[a]) < std::fabs(d[least])) least = a;
@@ -1175,30 +1189,42 @@ static void sun_map_plan(const vlb_scene* scene, float3 s, float bias, uint32_t 
   const double un = std::sqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
   for (double& x : u) x /= un;
   const double v[3] = {d[1] * u[2] - d[2] * u[1], d[2] * u[0] - d[0] * u[2], d[0] * u[1] - d[1] * u[0]};
-  const double scale = std::max(std::fabs(bias), bounds_scale(scene));
-  double ext = 0.0, mid[2] = {0, 0};
-  for (int c = 0; c < 2; ++c) {
-    const double* ax = c ? v : u;
-    double lo = 0, hi = 0;
-    for (int a = 0; a < 3; ++a) {
-      lo += std::min(ax[a] * scene->bounds[a], ax[a] * scene->bounds[3 + a]);
-      hi += std::max(ax[a] * scene->bounds[a], ax[a] * scene->bounds[3 + a]);
-    }
-    mid[c] = 0.5 * (lo + hi);
-    ext = std::max(ext, hi - lo);
+  auto dot = [](const double* x, const double* y) { return x[0] * y[0] + x[1] * y[1] + x[2] * y[2]; };
+  double lo[2] = {INFINITY, INFINITY}, hi[2] = {-INFINITY, -INFINITY}, near = INFINITY, far = -INFINITY;
+  const double off = std::fabs(double(bias));
+  for (int c = 0; c < 8; ++c) {
+    const double p[3] = {bb[c & 1 ? 3 : 0] - o[0], bb[c & 2 ? 4 : 1] - o[1], bb[c & 4 ? 5 : 2] - o[2]};
+    const double w = dot(p, d);
+    near = std::min(near, w);
+    far = std::max(far, w);
+    if (light && !(w > 0.0)) return false;
+    const double k = light ? 1.0 / w : 1.0, q[2] = {dot(p, u) * k, dot(p, v) * k};
+    for (int a = 0; a < 2; ++a) { lo[a] = std::min(lo[a], q[a]); hi[a] = std::max(hi[a], q[a]); }
   }
-  const double margin = scale * 0x1p-17;
-  ext += 2.0 * (std::fabs(double(bias)) + 4.0 * margin);
+  double scale = std::max(off, double(bounds_scale(scene))), drift = 0.0, k = 1.0;
+  if (light) {
+    for (double x : o) scale = std::max(scale, std::fabs(x));
+    // shadow origins lie up to `off` beside the scene
+    if (!(near - 2.0 * off > 0.05 * (far - near))) return false;
+    k = 1.0 / (near - off);
+    drift = off * (k - 1.0 / (far + off));
+  }
+  const double margin = scale * 0x1p-17 * k + drift;
+  const double ext = std::max(hi[0] - lo[0], hi[1] - lo[1]) + 2.0 * (off * k + 4.0 * margin);
   m->cells = cells;
   m->u = make_float3(float(u[0]), float(u[1]), float(u[2]));
   m->v = make_float3(float(v[0]), float(v[1]), float(v[2]));
-  m->s = s;
-  m->u0 = float(mid[0] - 0.5 * ext);
-  m->v0 = float(mid[1] - 0.5 * ext);
-  m->inv = float(G / ext);
-  m->cell = float(ext / G);
+  m->s = light ? make_float3(float(d[0]), float(d[1]), float(d[2])) : sun;
+  m->o = light ? *light : make_float3(0.f, 0.f, 0.f);
+  m->u0 = float(0.5 * (lo[0] + hi[0]) - 0.5 * ext);
+  m->v0 = float(0.5 * (lo[1] + hi[1]) - 0.5 * ext);
+  m->inv = float(kMapSide / ext);
+  m->cell = float(ext / kMapSide);
   m->margin = float(margin);
-  m->G = G;
+  m->dmargin = float(scale * 0x1p-17 * k * k);
+  m->G = kMapSide;
+  m->point = light ? 1u : 0u;
+  return true;
 }
 
 // Checks the parameters of one bake; *sun_len gets |sun_dir| (FP64).
@@ -1261,11 +1287,11 @@ static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const floa
   a.lane = lane_mode(scene, nprobes, p->flags, p->shading);
   a.shading = p->shading;
   a.light = make_float3(p->light_pos[0], p->light_pos[1], p->light_pos[2]);
-  if (a.lane && !from_root && a.shading == VLB_SHADE_LAMBERT_SUN &&
-      sun_map_pays(scene, uint64_t(nprobes) * a.S, 6.0)) {
+  if (a.lane && !from_root && sun_map_pays(scene, uint64_t(nprobes) * a.S, 6.0)) {
     void* cells;
     if ((st = scratch(ctx, "sun_map", kMapBytes, &cells))) return st;
-    sun_map_plan(scene, a.sun, a.bias, kMapSide, static_cast<uint32_t*>(cells), &a.sun_map);
+    sun_map_plan(scene, a.sun, a.shading == VLB_SHADE_REF_PHONG ? &a.light : nullptr, a.bias,
+                 static_cast<uint32_t*>(cells), &a.sun_map);
   }
   const bool grid = grid_mode(scene, nprobes, a.S, p);
   const uint32_t cap = a.lane && !grid && !from_root ? front_cap(scene, nprobes, a.S) : 0;
@@ -1735,7 +1761,7 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
     const BatchJob& b = pl.jobs[i];
     const vlb_scene* sc = jobs[b.idx].scene;
     fronts[i] = !(ext && ext[b.idx].hits_in) && front_cap(sc, b.nprobes, b.S) != 0;
-    maps[i] = b.p->shading == VLB_SHADE_LAMBERT_SUN && sun_map_pays(sc, uint64_t(b.nprobes) * b.S, 0.0);
+    maps[i] = sun_map_pays(sc, uint64_t(b.nprobes) * b.S, 0.0);
     if (fronts[i]) front_probes += b.nprobes;
     if (maps[i]) bb.map_bytes += kMapBytes;
   }
@@ -1852,9 +1878,9 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
       bb.front_total += b.nprobes;
     }
     d.map_begin = bb.map_ctas;
-    if (bb.map_bytes && maps[ord[t]]) {
-      sun_map_plan(j.scene, d.sun, d.bias, kMapSide,
-                   reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(bb.maps) + nmaps++ * kMapBytes), &d.sun_map);
+    if (bb.map_bytes && maps[ord[t]] &&
+        sun_map_plan(j.scene, d.sun, p->shading == VLB_SHADE_REF_PHONG ? &d.light : nullptr, d.bias,
+                     reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(bb.maps) + nmaps++ * kMapBytes), &d.sun_map)) {
       d.map_slices = vlbk::sun_map_slices(d.ntris);
       bb.map_ctas += vlbk::sun_map_ctas(d.ntris);
     }

@@ -246,11 +246,14 @@ void launch_probe_front_batch(const BakeJobDev* jobs, uint32_t njobs, uint32_t t
 // ---- sun maps (sun_map.cuh) ------------------------------------------------------
 struct SunMap {
   uint32_t* cells;   // [G][G] (cover, top) as ordered integers, or null: every shadow ray walks
-  float3 u, v, s;    // unit: across and along the direction to the sun
+  float3 u, v, s;    // unit: across and along the direction to the sun (from the light)
+  float3 o;          // point light
   float u0, v0;      // origin of cell (0, 0)
   float inv, cell;   // cells per unit, its reciprocal
-  float margin;
+  float margin;      // how far a cell is widened
+  float dmargin;     // rounding of a depth
   uint32_t G;
+  uint32_t point;    // 1: seen from the light at o, depth 1 / (distance along s)
 };
 uint32_t sun_map_slices(uint32_t ntris);
 inline uint32_t sun_map_ctas(uint32_t ntris) { return (ntris + 255) / 256 * sun_map_slices(ntris); }
