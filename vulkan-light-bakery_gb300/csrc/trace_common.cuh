@@ -535,22 +535,23 @@ __device__ __forceinline__ float ordered_f32(uint32_t k) {
 }
 
 // Probe frontiers (front.cuh).  The lanes `mine` test their primary rays
-// against entries [first, first + 32) of their probe's frontier and stack
-// those they hit, nearest on top; returns whether any of them has entries left.
-// The rays share an origin, so relative to it a plane at x is crossed at x / d.
-// First each lane tests one entry against the whole group -- the entry's
-// crossings under the group's range of 1/d per axis (an axis whose directions
-// change sign does not constrain) up to the farthest limit -- then every lane
-// tests its own ray against the entries left, farthest first.  All 32 lanes
-// take part; a group that straddles two probes goes probe by probe.
+// against the next stage of their probe's frontier, the entries from `first` on,
+// and stack those they hit, nearest on top; returns whether any of them has
+// entries left.  The rays share an origin, so relative to it a plane at x is
+// crossed at x / d.  First each lane tests one entry against the whole group --
+// the entry's crossings under the group's range of 1/d per axis (an axis whose
+// directions change sign does not constrain) up to the farthest limit -- then
+// every lane tests its own ray against the entries left, farthest first.  All 32
+// lanes take part; a group that straddles two probes goes probe by probe.
 //
-// A walk takes its frontier 32 entries at a time: entries are sorted by
-// distance, and when the whole group has walked the nearest, the rest are
-// culled by the hits found (262,144 probes x 1024 directions in 4096 boxes,
-// lists of 64: all entries at once 8.1, 32 at a time 6.4, 16 at a time 6.2 ms
-// on an eighth of the probes; 3141 x 1000 directions in 64 boxes 39.6 at 32
-// and 43.6 at 16).
-constexpr int kFrontStage = 32;
+// Stages: entries are sorted by distance, and when the whole group has walked
+// the nearest, the rest are culled by the hits found (32,768 probes x 1024
+// directions in 4096 boxes, lists of 64: all entries at once 8.1, 32 at a time
+// 6.4, 16 at a time 6.2 ms; 3141 x 1000 directions in 64 boxes, lists of 32: 39.6
+// at once, 43.6 in two stages).
+//
+// Lists of at most 32 entries go in one stage, longer ones 16 at a time.
+constexpr int kFrontStage = 16;
 template <class A>
 __device__ __forceinline__ bool lr_front(const A& a, LaneRay& L, bool mine, int first, int* stack) {
   const uint32_t lane = threadIdx.x & 31;
@@ -561,8 +562,9 @@ __device__ __forceinline__ bool lr_front(const A& a, LaneRay& L, bool mine, int 
     const bool now = mine && L.p == q;
     pending &= ~__ballot_sync(kFull, now);
     const int n = int(__ldg(a.front_n + q));
-    if (first >= n) continue;
-    more = more || first + kFrontStage < n;
+    const int end = n <= 32 ? n : min(n, first + kFrontStage);
+    if (first >= n || (first > 0 && n <= 32)) continue;
+    more = more || end < n;
     const float4* f = a.front + (size_t(q) * a.front_cap + first) * 2;
     const float lim = prune_limit(L.tb);
     const float far = __uint_as_float(__reduce_max_sync(kFull, now ? __float_as_uint(lim) : 0u));
@@ -575,7 +577,7 @@ __device__ __forceinline__ bool lr_front(const A& a, LaneRay& L, bool mine, int 
       imax[c] = ordered_f32(__reduce_max_sync(kFull, now ? k : 0u));
     }
     bool in = false;
-    if (first + int(lane) < n) {
+    if (first + int(lane) < end) {
       const float4 x = __ldg(f + 2 * lane), y = __ldg(f + 2 * lane + 1);
       const float lo[3] = {x.x, x.y, y.x}, hi[3] = {x.z, x.w, y.y};
       float tn = 0.f, tf = far;
