@@ -43,7 +43,7 @@ __device__ __forceinline__ void load_rgb(const void* __restrict__ texels, size_t
     const float* f = static_cast<const float*>(texels) + 3 * i;
     c[0] = __ldg(f); c[1] = __ldg(f + 1); c[2] = __ldg(f + 2);
   } else {
-    const uint32_t q = __ldg(static_cast<const uint32_t*>(texels) + i);  // UNORM bytes, scaled with the row
+    const uint32_t q = __ldg(static_cast<const uint32_t*>(texels) + i);  // UNORM bytes, scaled at the end
     c[0] = float(q & 255u); c[1] = float((q >> 8) & 255u); c[2] = float((q >> 16) & 255u);
   }
 }
@@ -96,54 +96,59 @@ __global__ void __launch_bounds__(kPanoWarps * 32) k_pano_rows(const SkyboxArgs 
 }
 
 // A row's coefficients from its sums f = {1, c1, s1, c2, s2, c3, s3} at (sin
-// theta, cos theta): the products of shaders/sh_common.h:26-116 with the powers
-// of sin phi and cos phi written as multiple angles.  PANO: the basis at dir.xzy
-// (skybox_sh.comp:39).
+// theta, cos theta), without the basis' constants: the products of
+// shaders/sh_common.h:26-116 with the powers of sin phi and cos phi written as
+// multiple angles.  PANO: the basis at dir.xzy (skybox_sh.comp:39).
 template <int LMAX, bool PANO>
 __device__ __forceinline__ void row_coeffs(float s, float c, const float* f, float* o) {
   const float s2 = s * s, c2 = c * c, sc = s * c, s3 = s2 * s, s2c = s2 * c;
-  o[0] = 0.282095f * f[0];
+  o[0] = f[0];
   if constexpr (!PANO) {
-    o[1] = -0.488603f * s * f[2];
-    o[2] = 0.488603f * c * f[0];
-    o[3] = -0.488603f * s * f[1];
-    o[4] = 1.092548f * 0.5f * s2 * f[4];
-    o[5] = -1.092548f * sc * f[2];
-    o[6] = 0.315392f * (2.f * c2 - s2) * f[0];
-    o[7] = -1.092548f * sc * f[1];
-    o[8] = 0.546274f * s2 * f[3];
+    o[1] = -s * f[2];
+    o[2] = c * f[0];
+    o[3] = -s * f[1];
+    o[4] = 0.5f * s2 * f[4];
+    o[5] = -sc * f[2];
+    o[6] = (2.f * c2 - s2) * f[0];
+    o[7] = -sc * f[1];
+    o[8] = s2 * f[3];
     if constexpr (LMAX == 3) {
-      o[9] = -0.590044f * s3 * f[6];
-      o[10] = 2.890611f * 0.5f * s2c * f[4];
-      o[11] = -0.457046f * s * (4.f * c2 - s2) * f[2];
-      o[12] = 0.373176f * c * (2.f * c2 - 3.f * s2) * f[0];
-      o[13] = -0.457046f * s * (4.f * c2 - s2) * f[1];
-      o[14] = 1.445306f * s2c * f[3];
-      o[15] = -0.590044f * s3 * f[5];
+      o[9] = -s3 * f[6];
+      o[10] = 0.5f * s2c * f[4];
+      o[11] = -s * (4.f * c2 - s2) * f[2];
+      o[12] = c * (2.f * c2 - 3.f * s2) * f[0];
+      o[13] = -s * (4.f * c2 - s2) * f[1];
+      o[14] = s2c * f[3];
+      o[15] = -s3 * f[5];
     }
   } else {
-    o[1] = -0.488603f * c * f[0];
-    o[2] = 0.488603f * s * f[2];
-    o[3] = -0.488603f * s * f[1];
-    o[4] = 1.092548f * sc * f[1];
-    o[5] = -1.092548f * sc * f[2];
-    o[6] = 0.315392f * ((0.5f * s2 - c2) * f[0] - 1.5f * s2 * f[3]);
-    o[7] = -1.092548f * 0.5f * s2 * f[4];
-    o[8] = 0.546274f * ((0.5f * s2 - c2) * f[0] + 0.5f * s2 * f[3]);
+    o[1] = -c * f[0];
+    o[2] = s * f[2];
+    o[3] = -s * f[1];
+    o[4] = sc * f[1];
+    o[5] = -sc * f[2];
+    o[6] = ((0.5f * s2 - c2) * f[0] - 1.5f * s2 * f[3]);
+    o[7] = -0.5f * s2 * f[4];
+    o[8] = ((0.5f * s2 - c2) * f[0] + 0.5f * s2 * f[3]);
     if constexpr (LMAX == 3) {
-      o[9] = -0.590044f * c * ((1.5f * s2 - c2) * f[0] + 1.5f * s2 * f[3]);
-      o[10] = 2.890611f * 0.5f * s2c * f[4];
-      o[11] = -0.457046f * c * ((1.5f * s2 - c2) * f[0] - 2.5f * s2 * f[3]);
-      o[12] = 0.373176f * (s * (0.75f * s2 - 3.f * c2) * f[2] - 1.25f * s3 * f[6]);
-      o[13] = -0.457046f * (s * (0.25f * s2 - c2) * f[1] - 1.25f * s3 * f[5]);
-      o[14] = 1.445306f * (s * (0.25f * s2 - c2) * f[2] + 0.25f * s3 * f[6]);
-      o[15] = -0.590044f * (s * (0.75f * s2 - 3.f * c2) * f[1] + 0.25f * s3 * f[5]);
+      o[9] = -c * ((1.5f * s2 - c2) * f[0] + 1.5f * s2 * f[3]);
+      o[10] = 0.5f * s2c * f[4];
+      o[11] = -c * ((1.5f * s2 - c2) * f[0] - 2.5f * s2 * f[3]);
+      o[12] = (s * (0.75f * s2 - 3.f * c2) * f[2] - 1.25f * s3 * f[6]);
+      o[13] = -(s * (0.25f * s2 - c2) * f[1] - 1.25f * s3 * f[5]);
+      o[14] = (s * (0.25f * s2 - c2) * f[2] + 0.25f * s3 * f[6]);
+      o[15] = -(s * (0.75f * s2 - 3.f * c2) * f[1] + 0.25f * s3 * f[5]);
     }
   }
 }
 
+// The constants of shaders/sh_common.h:26-116 by coefficient.
+__constant__ double c_sh[16] = {0.282095, 0.488603, 0.488603, 0.488603, 1.092548, 1.092548, 0.315392, 1.092548,
+                                0.546274, 0.590044, 2.890611, 0.457046, 0.373176, 0.457046, 1.445306, 0.590044};
+
 // One CTA per map: a thread takes every kPanoThreads-th row, the warps' sums are
-// added in FP64 in warp order.
+// added in FP64 in warp order; the basis' constants and the 1 / 255 of 8-bit
+// texels multiply the FP64 sum, so neither is rounded to FP32.
 template <int LMAX, bool PANO>
 __global__ void __launch_bounds__(kPanoThreads) k_pano_combine(const SkyboxArgs a, const float* __restrict__ rows,
                                                                uint32_t nseg, float* __restrict__ out) {
@@ -157,7 +162,6 @@ __global__ void __launch_bounds__(kPanoThreads) k_pano_combine(const SkyboxArgs 
     for (int k = 0; k < 16; ++k) acc[c][k] = 0.f;
   for (uint32_t y = tid; y < a.h; y += kPanoThreads) {
     const float4 rw = __ldg(a.row_tab + y);  // sin theta, cos theta, weight
-    const float w = a.fmt == VLB_TEXEL_RGBA8 ? rw.z * (1.0f / 255.0f) : rw.z;
     const float4* r = reinterpret_cast<const float4*>(rows) + (size_t(map) * a.h + y) * nseg * (kPanoSums / 4);
     float f[kPanoSums];
 #pragma unroll
@@ -173,7 +177,7 @@ __global__ void __launch_bounds__(kPanoThreads) k_pano_combine(const SkyboxArgs 
       float o[16];
       row_coeffs<LMAX, PANO>(rw.x, rw.y, f + 8 * c, o);
 #pragma unroll
-      for (int k = 0; k < K; ++k) acc[c][k] = fmaf(w, o[k], acc[c][k]);
+      for (int k = 0; k < K; ++k) acc[c][k] = fmaf(rw.z, o[k], acc[c][k]);
     }
   }
 #pragma unroll
@@ -186,6 +190,7 @@ __global__ void __launch_bounds__(kPanoThreads) k_pano_combine(const SkyboxArgs 
     const int k = int(tid) / 3, c = int(tid) - 3 * k;
     double s = 0.0;
     for (int w = 0; w < kPanoThreads / 32; ++w) s += double(s_sum[w][c][k]);
+    s *= a.fmt == VLB_TEXEL_RGBA8 ? c_sh[k] / 255.0 : c_sh[k];
     const int co = a.flags & VLB_SKY_REF_BGRA_SWAP ? 2 - c : c;
     out[(size_t(map) * K + k) * 3 + co] = float(s);
   }

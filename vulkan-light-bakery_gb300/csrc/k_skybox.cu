@@ -9,9 +9,10 @@
 // 1-D bulk async copies (cp.async.bulk, completion on an mbarrier; one copy
 // per map per stage) from a producer warp.  Cubemaps with faces up to 1024
 // (k_skybox_cube_group) share one weighted-basis row, read from a texel-pair
-// table, among 8-16 maps; panoramas, env maps and larger faces (k_skybox_sh)
-// compute each texel's direction, solid angle and basis once and apply it to
-// G = 1-4 maps with packed FP32x2 FMAs.  Each map's sums are reduced with warp
+// table, among 8-16 maps; larger faces, maps taken without a context and
+// panoramas whose row sums would exceed 256 MiB (k_skybox_sh) compute each texel's
+// direction, solid angle and basis once and apply it to G = 1-4 maps with packed
+// FP32x2 FMAs; other panoramas and env maps go by rows (k_pano.cu).  Each map's sums are reduced with warp
 // shuffles into partials per (map, slab), and a second kernel adds a map's
 // partials in FP64 in a fixed order.  The slab size does not depend on the
 // batch, so a map's result is bit-identical alone or in any batch.
@@ -118,8 +119,7 @@ __device__ __forceinline__ void texel_rgb(const unsigned char* p, uint32_t i, bo
     c[0] = f[0]; c[1] = f[1]; c[2] = f[2];
   } else {
     const uchar4 q = reinterpret_cast<const uchar4*>(p)[i];
-    const float s = 1.0f / 255.0f;
-    c[0] = q.x * s; c[1] = q.y * s; c[2] = q.z * s;
+    c[0] = q.x; c[1] = q.y; c[2] = q.z;  // scaled by k_sh_finalize
   }
   if (swap) { const float t = c[0]; c[0] = c[2]; c[2] = t; }
 }
@@ -576,10 +576,11 @@ int launch_skybox_sh(const SkyboxArgs& a, bool tma, int num_sms, cudaStream_t s)
 // One CTA per map: thread (g, v) adds value v of partials 4g .. 4g + 3 in FP32
 // and every G-th such four in FP64, and the G sums are added in order in FP64
 // (a fixed order for a slab count; FP64 adds run at 1/64 of the FP32 rate, so
-// one per four partials).  One thread per value took 240 us for the 2048
+// one per four partials).  The texels of 8-bit maps are summed as integers 0..255
+// and scaled here, in FP64.  One thread per value took 240 us for the 2048
 // partials of a 2048 x 1024 map.
 __global__ void __launch_bounds__(1024) k_sh_finalize(const float* __restrict__ partial, uint32_t slabs,
-                                                      uint32_t nvals, float* __restrict__ out) {
+                                                      uint32_t nvals, double scale, float* __restrict__ out) {
   __shared__ double s_sum[1024];
   const uint32_t G = blockDim.x / nvals, g = threadIdx.x / nvals, v = threadIdx.x - g * nvals;
   const float* p = partial + size_t(blockIdx.x) * slabs * nvals + v;
@@ -596,15 +597,15 @@ __global__ void __launch_bounds__(1024) k_sh_finalize(const float* __restrict__ 
   __syncthreads();
   if (g != 0) return;
   for (uint32_t k = 1; k < G; ++k) s += s_sum[k * nvals + v];
-  out[size_t(blockIdx.x) * nvals + v] = float(s);
+  out[size_t(blockIdx.x) * nvals + v] = float(s * scale);
 }
 
-void launch_sh_finalize(const float* partial, uint32_t nmaps, uint32_t slabs, uint32_t nvals, float* out,
+void launch_sh_finalize(const float* partial, uint32_t nmaps, uint32_t slabs, uint32_t nvals, int fmt, float* out,
                         cudaStream_t s) {
   // four partials a thread, whole warps, at most 1024 threads
   const uint32_t want = nvals * ((slabs + 3) / 4);
   const uint32_t threads = want < 1024 ? (want + 31) / 32 * 32 : 1024;
-  k_sh_finalize<<<nmaps, threads, 0, s>>>(partial, slabs, nvals, out);
+  k_sh_finalize<<<nmaps, threads, 0, s>>>(partial, slabs, nvals, fmt == VLB_TEXEL_RGBA8 ? 1.0 / 255.0 : 1.0, out);
 }
 
 }  // namespace vlbk

@@ -963,7 +963,8 @@ vlb_status vlb_skybox_sh_batched(vlb_ctx* ctx, const void* texels, vlb_texel_for
   }
   {
     KScope k(ctx, "sh_finalize");
-    vlbk::launch_sh_finalize(a.partial, count, uint32_t(per_map), V, static_cast<float*>(ob.dev), ctx->stream);
+    vlbk::launch_sh_finalize(a.partial, count, uint32_t(per_map), V, fmt,
+                             static_cast<float*>(ob.dev), ctx->stream);
   }
   if ((st = copy_out(ctx, ob))) return st;
   return finish(ctx, ob.host);

@@ -124,7 +124,8 @@ void launch_pano_tables(float2* col, float4* row, uint32_t w, uint32_t h, bool s
 size_t pano_rows_bytes(uint32_t w, uint32_t h, uint32_t count);
 void launch_pano_sh(const SkyboxArgs& a, float* rows, float* out, cudaStream_t s);
 // out[m][v] = sum_j partial[m][j][v] in FP64, j in fixed order.
-void launch_sh_finalize(const float* partial, uint32_t nmaps, uint32_t slabs, uint32_t nvals, float* out,
+// fmt: the maps' texel format (8-bit texels are scaled by 1 / 255 here).
+void launch_sh_finalize(const float* partial, uint32_t nmaps, uint32_t slabs, uint32_t nvals, int fmt, float* out,
                         cudaStream_t s);
 
 // ---- projection of a radiance tile --------------------------------------------
