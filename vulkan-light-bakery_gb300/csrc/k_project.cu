@@ -208,8 +208,8 @@ __global__ void __launch_bounds__(1024) k_project_reduce(const float* __restrict
   out[(size_t(p) * K + k) * 3 + c] = float(sum);
 }
 
-static void launch_reduce(const float* partial, uint32_t splits, uint32_t rows, uint32_t K, float* out,
-                          cudaStream_t s) {
+void launch_project_reduce(const float* partial, uint32_t splits, uint32_t rows, uint32_t K, float* out,
+                           cudaStream_t s) {
   const uint32_t groups = std::min(32u, std::max(1u, (splits + 3) / 4));
   k_project_reduce<<<(rows * K + 31) / 32, groups * 32, 0, s>>>(partial, splits, rows, K, out);
 }
@@ -226,7 +226,7 @@ static void launch_project(const T* rad, uint32_t nprobes, uint32_t S, const flo
   const dim3 grid(tiles, splits);
   if (K == 9) k_project<T, 9><<<grid, kProjRows, 0, s>>>(rad, rows, S, per, basis16, out, partial, split);
   else k_project<T, 16><<<grid, kProjRows, 0, s>>>(rad, rows, S, per, basis16, out, partial, split);
-  if (splits > 1) launch_reduce(partial, splits, rows, K, out, s);
+  if (splits > 1) launch_project_reduce(partial, splits, rows, K, out, s);
 }
 
 void launch_project_f32(const float* radiance, uint32_t nprobes, uint32_t S, const float* basis16, uint32_t K,
@@ -241,7 +241,7 @@ void launch_project_f32(const float* radiance, uint32_t nprobes, uint32_t S, con
   if (err && num_sms && S && (splits == 1 || size_t(rows) * S >= kProjStream) &&
       launch_project_f32_tma(radiance, nprobes, S, basis16, K, out, partial, splits, splits == 1 ? S : per, err,
                              num_sms, s, hold, wait_polls)) {
-    if (splits > 1) launch_reduce(partial, splits, rows, K, out, s);
+    if (splits > 1) launch_project_reduce(partial, splits, rows, K, out, s);
     return;
   }
   launch_project<float>(radiance, nprobes, S, basis16, K, out, partial, 0, s);

@@ -17,6 +17,11 @@
 //               K=16) per stage into one of two TMEM accumulators (2 x 32 cols)
 //   warps 2..5  epilogue: tcgen05.ld of the accumulator rows (warp w reads TMEM
 //               lanes 32*(w%4)..+31), hi+lo combine, store
+// A CTA takes (row tile, split) units: rows of more than kTcSplit values are split
+// along them (343 probes x 3141 x 1000 directions are 9 row tiles), one accumulator
+// a split, added in FP64 by k_project_reduce.  The split length is fixed, so a
+// row's sums do not depend on the rows beside it; it is short, as the accumulator
+// loses up to an ulp per step of 16 values.
 // Every mbarrier wait is bounded; a timeout sets the error counter, stops all
 // roles, waits (bounded) for copies in flight and frees TMEM before exit.
 #include <cuda.h>
@@ -39,6 +44,7 @@ constexpr uint32_t kStageA = kTileM * kTileK * 2;      // 16 KiB
 constexpr uint32_t kStageB = kTileN * kTileK * 2;      // 4 KiB
 constexpr uint32_t kStageBytes = kStageA + kStageB;    // 20 KiB, multiple of 1024
 constexpr uint32_t kTmemCols = 64;                     // two 32-column accumulators
+constexpr uint32_t kTcSplit = 4096;                    // values of a row per unit (8 KiB), a multiple of kTileK
 constexpr size_t kSmemBytes = size_t(kStages) * kStageBytes + 1024;  // + alignment slack
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -118,14 +124,17 @@ struct TcShared {
 
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_project_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, uint32_t rows,
-                 uint32_t S, uint32_t K, float* __restrict__ out, int* err, uint32_t hold, uint32_t polls) {
+                 uint32_t S, uint32_t K, float* __restrict__ out, float* __restrict__ partial, uint32_t splits,
+                 int* err, uint32_t hold, uint32_t polls) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ TcShared sh;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t ntiles = (rows + kTileM - 1) / kTileM;
-  const uint32_t nkb = (S + kTileK - 1) / kTileK;
+  const uint32_t units = ntiles * splits;
+  // K blocks in all and per split
+  const uint32_t nkb = (S + kTileK - 1) / kTileK, per = splits > 1 ? kTcSplit / kTileK : nkb;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) { mbar_init(&sh.full[i], 1); mbar_init(&sh.empty[i], 1); }
@@ -145,8 +154,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   if (warp == 0) {
     if (lane == 0 && !hold) {  // hold (a test hook): no copy is issued, the waits below give up
       uint32_t issued = 0;
-      for (uint32_t tile = blockIdx.x; tile < ntiles && !sh.abort; tile += gridDim.x) {
-        for (uint32_t kb = 0; kb < nkb; ++kb, ++issued) {
+      for (uint32_t u = blockIdx.x; u < units && !sh.abort; u += gridDim.x) {
+        const uint32_t split = u / ntiles, tile = u - split * ntiles, k1 = min(nkb, (split + 1) * per);
+        for (uint32_t kb = split * per; kb < k1; ++kb, ++issued) {
           const uint32_t st = issued % kStages, round = issued / kStages;
           if (!mbar_wait_bounded(&sh.empty[st], (round & 1u) ^ 1u, err, polls)) { sh.abort = 1; break; }
           mbar_arrive_expect_tx(&sh.full[st], kStageBytes);
@@ -163,19 +173,20 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   } else if (warp == 1) {
     if (lane == 0) {
       uint32_t used = 0, it = 0;
-      for (uint32_t tile = blockIdx.x; tile < ntiles && !sh.abort; tile += gridDim.x, ++it) {
+      for (uint32_t u = blockIdx.x; u < units && !sh.abort; u += gridDim.x, ++it) {
+        const uint32_t k0 = u / ntiles * per, k1 = min(nkb, k0 + per);
         const uint32_t acc = it & 1u;
         if (!mbar_wait_bounded(&sh.acc_empty[acc], ((it >> 1) & 1u) ^ 1u, err, polls)) { sh.abort = 1; break; }
         tc_fence_after();
         const uint32_t d = tmem + acc * kTileN;
-        for (uint32_t kb = 0; kb < nkb; ++kb, ++used) {
+        for (uint32_t kb = k0; kb < k1; ++kb, ++used) {
           const uint32_t st = used % kStages;
           if (!mbar_wait_bounded(&sh.full[st], (used / kStages) & 1u, err, polls)) { sh.abort = 1; break; }
           tc_fence_after();
           const uint32_t sa = base + st * kStageBytes, sb = sa + kStageA;
 #pragma unroll
           for (int k = 0; k < kTileK / 16; ++k)
-            mma_bf16(d, smem_desc(sa + 32 * k), smem_desc(sb + 32 * k), kIdesc, (kb | k) != 0);
+            mma_bf16(d, smem_desc(sa + 32 * k), smem_desc(sb + 32 * k), kIdesc, kb != k0 || k != 0);
           mma_commit(&sh.empty[st]);  // the stage is free once these MMAs have read it
         }
         if (sh.abort) break;
@@ -186,7 +197,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     // epilogue warps 2..5: TMEM lanes 32*(warp%4) .. +31
     const uint32_t lane_base = 32u * (warp & 3u);
     uint32_t it = 0;
-    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
+    for (uint32_t u = blockIdx.x; u < units; u += gridDim.x, ++it) {
+      const uint32_t split = u / ntiles, tile = u - split * ntiles;
       const uint32_t acc = it & 1u;
       if (!mbar_wait_bounded(&sh.acc_full[acc], (it >> 1) & 1u, err, polls)) { sh.abort = 1; break; }
       tc_fence_after();
@@ -197,10 +209,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       const uint32_t row = tile * kTileM + lane_base + lane;
       if (row < rows) {
         const uint32_t p = row / 3, c = row - 3 * p;
-        float* o = out + size_t(p) * K * 3 + c;
+        float* o = splits == 1 ? out + size_t(p) * K * 3 + c : partial + (size_t(split) * rows + row) * K;
+        const uint32_t step = splits == 1 ? 3 : 1;
 #pragma unroll
         for (uint32_t k = 0; k < 16; ++k)
-          if (k < K) o[3 * k] = v[k] + v[16 + k];
+          if (k < K) o[step * k] = v[k] + v[16 + k];
       }
       if (sh.abort) break;
     }
@@ -409,8 +422,13 @@ bool project_tc_supported(const void* radiance, uint32_t S) {
   return S > 0 && S % 8 == 0 && (reinterpret_cast<uintptr_t>(radiance) % 16) == 0 && encode_fn() != nullptr;
 }
 
+size_t project_tc_partial_bytes(uint32_t nprobes, uint32_t S, uint32_t K) {
+  const size_t splits = (size_t(S) + kTcSplit - 1) / kTcSplit;
+  return splits > 1 ? splits * nprobes * 3 * K * sizeof(float) : 0;
+}
+
 int launch_project_tc(const uint16_t* radiance, uint32_t nprobes, uint32_t S, const uint16_t* basis_bt,
-                      uint32_t bt_pitch, uint32_t K, float* out, int* err, int num_sms, cudaStream_t s,
+                      uint32_t bt_pitch, uint32_t K, float* out, float* partial, int* err, int num_sms, cudaStream_t s,
                       uint32_t hold, uint32_t wait_polls) {
   const uint32_t rows = nprobes * 3;
   if (rows == 0) return 0;
@@ -420,9 +438,11 @@ int launch_project_tc(const uint16_t* radiance, uint32_t nprobes, uint32_t S, co
   static std::atomic<uint64_t> opted{0};
   smem_opt_in(k_project_tc, int(kSmemBytes), opted);
   const uint32_t ntiles = (rows + kTileM - 1) / kTileM;
-  const uint32_t grid = std::min<uint32_t>(ntiles, uint32_t(num_sms));
-  k_project_tc<<<grid, kTcThreads, kSmemBytes, s>>>(ta, tb, rows, S, K, out, err, hold,
+  const uint32_t splits = partial ? (S + kTcSplit - 1) / kTcSplit : 1;
+  const uint32_t grid = uint32_t(std::min<uint64_t>(uint64_t(ntiles) * splits, uint64_t(num_sms)));
+  k_project_tc<<<grid, kTcThreads, kSmemBytes, s>>>(ta, tb, rows, S, K, out, partial, splits, err, hold,
                                                      wait_polls ? wait_polls : kWaitPolls);
+  if (splits > 1) launch_project_reduce(partial, splits, rows, K, out, s);
   return 1;
 }
 

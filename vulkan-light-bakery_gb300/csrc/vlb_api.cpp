@@ -1058,12 +1058,13 @@ static vlb_status project_bf16(vlb_ctx* ctx, const uint16_t* rad, uint32_t nprob
                                uint32_t K, float* out, bool split, const char* part_name = "project_partial") {
   const uint32_t S = dirs->n;
   if (vlbk::project_tc_supported(rad, split ? 2 * S : S) && (!split || dirs->d_bt2)) {
-    KScope k(ctx, split ? "project_tc_split" : "project_tc");
-    const int r = split ? vlbk::launch_project_tc(rad, nprobes, 2 * S, dirs->d_bt2, dirs->bt2_pitch, K, out,
-                                                  ctx->d_err, ctx->num_sms, ctx->stream, ctx->hold_producer,
-                                                  ctx->wait_polls)
-                        : vlbk::launch_project_tc(rad, nprobes, S, dirs->d_bt, dirs->bt_pitch, K, out, ctx->d_err,
-                                                  ctx->num_sms, ctx->stream, ctx->hold_producer, ctx->wait_polls);
+    void* part = nullptr;  // without it rows stay whole
+    const size_t pb = vlbk::project_tc_partial_bytes(nprobes, split ? 2 * S : S, K);
+    if (pb && scratch(ctx, part_name, pb, &part) != VLB_OK) part = nullptr;
+    KScope k(ctx, split ? "project_tc_split" : "project_tc", part ? 2 : 1);
+    const int r = vlbk::launch_project_tc(rad, nprobes, split ? 2 * S : S, split ? dirs->d_bt2 : dirs->d_bt,
+                                          split ? dirs->bt2_pitch : dirs->bt_pitch, K, out, static_cast<float*>(part),
+                                          ctx->d_err, ctx->num_sms, ctx->stream, ctx->hold_producer, ctx->wait_polls);
     if (r < 0) return fail(ctx, VLB_ERR_CUDA, "tensor map encoding failed for the BF16 projection");
     return VLB_OK;
   }

@@ -135,6 +135,9 @@ size_t project_partial_bytes(uint32_t nprobes, uint32_t S, uint32_t K);
 void launch_project_f32(const float* radiance, uint32_t nprobes, uint32_t S, const float* basis16, uint32_t K,
                         float* out, float* partial, cudaStream_t s, int* err = nullptr, int num_sms = 0,
                         uint32_t hold = 0, uint32_t wait_polls = 0);
+// out = the splits' sums partial [splits][rows][K] added in FP64.
+void launch_project_reduce(const float* partial, uint32_t splits, uint32_t rows, uint32_t K, float* out,
+                           cudaStream_t s);
 // The TMA-staged form of the FP32 projection (per row and split the same sums),
 // `splits` splits of `per` samples (a multiple of 32), their sums in `partial`
 // when there are more than one; returns 0 when the tile does not qualify
@@ -150,9 +153,12 @@ void launch_project_bf16_simt(const uint16_t* radiance, uint32_t nprobes, uint32
 // Needs S % 8 == 0 and a 16-byte aligned tile; returns -1 if the tensor maps
 // cannot be built.
 bool project_tc_supported(const void* radiance, uint32_t S);
+// Device scratch for the splits of long rows (`partial`), 0 for rows taken
+// whole; with a null `partial` every row is taken whole.
+size_t project_tc_partial_bytes(uint32_t nprobes, uint32_t S, uint32_t K);
 // hold / wait_polls: vlb_ctx_test_hook (0, 0 in normal use).
 int launch_project_tc(const uint16_t* radiance, uint32_t nprobes, uint32_t S, const uint16_t* basis_bt,
-                      uint32_t bt_pitch, uint32_t K, float* out, int* err, int num_sms, cudaStream_t s,
+                      uint32_t bt_pitch, uint32_t K, float* out, float* partial, int* err, int num_sms, cudaStream_t s,
                       uint32_t hold = 0, uint32_t wait_polls = 0);
 // out[p][v] <- sum over q <= p of out[q][v] (FP64 running sum, one rounding).
 void launch_probe_prefix(float* out, uint32_t nprobes, uint32_t V, cudaStream_t s);
