@@ -1131,11 +1131,14 @@ static bool grid_mode(const vlb_scene* scene, uint32_t nprobes, uint32_t S, cons
 // its rays share it: at 64 rays a probe a lone small bake breaks even (64
 // probes: 83 us with and without) and a batch gains (6.1 -> 5.6 ms); fewer
 // share it too little.  Trees deeper than the lane stack keep the
-// root (their walks may overflow the stack, and must say so).  1 GiB of
-// entries at most.
+// root (their walks may overflow the stack, and must say so).
+// At most 4 GiB of entries, lists of 32 for 4 M probes (the radiance tile of a
+// bake of that size is a multiple of it).
+constexpr uint64_t kFrontEntries = 1ull << 27;
+
 static uint32_t front_cap(const vlb_scene* scene, uint64_t nprobes, uint32_t S) {
   if (scene->ntris < 64 || scene->wnodes || scene->depth > uint32_t(vlbk::kLaneStack) || S < 64 || !nprobes) return 0;
-  const uint64_t cap = std::min<uint64_t>(vlbk::kFrontCap, (1ull << 25) / nprobes);
+  const uint64_t cap = std::min<uint64_t>(vlbk::kFrontCap, kFrontEntries / nprobes);
   return cap < 32 ? 0 : uint32_t(cap);
 }
 
@@ -1770,7 +1773,7 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
   uint32_t cap = 0;
   void *front_ent = nullptr, *front_n = nullptr;
   if (front_probes) {
-    cap = uint32_t(std::min<uint64_t>(vlbk::kFrontCap, std::min<uint64_t>(1ull << 25, spare_bytes / 64) / front_probes));
+    cap = uint32_t(std::min<uint64_t>(vlbk::kFrontCap, std::min<uint64_t>(kFrontEntries, spare_bytes / 64) / front_probes));
     if (cap < 32 || scratch(ctx, "batch_front", front_probes * cap * 32, &front_ent) != VLB_OK ||
         scratch(ctx, "batch_front_n", front_probes * 4, &front_n) != VLB_OK)
       cap = 0;
