@@ -58,6 +58,34 @@ bool is_device_ptr(const void* p) {
   return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
 }
 
+// Scratch that only makes a call faster (probe frontiers, light maps, split
+// chunks) or that the next call would make again: given back when device memory
+// runs out, unless the call under way uses it (ctx->extras).
+static bool drop_extras(vlb_ctx* ctx) {
+  bool any = false;
+  for (const char* name : {"front_ent", "front_cnt", "sun_map", "bake_sub", "batch_front", "batch_front_n", "batch_maps",
+                           "batch_sub", "scene_build"}) {
+    auto it = ctx->scratch.find(name);
+    if (it == ctx->scratch.end() || !it->second.p) continue;
+    if (!any) cudaStreamSynchronize(ctx->stream);
+    any = true;
+    cudaFree(it->second.p);
+    it->second.p = nullptr;
+    it->second.bytes = 0;
+  }
+  return any;
+}
+
+// Runs a call with its extra scratch and, when memory is short, again without.
+template <class F>
+static vlb_status with_extras(vlb_ctx* ctx, F&& call) {
+  ctx->extras = true;
+  vlb_status st = call(true);
+  ctx->extras = false;
+  if (st == VLB_ERR_OOM && drop_extras(ctx)) st = call(false);
+  return st;
+}
+
 // Grow-only named scratch buffer owned by the context.
 vlb_status scratch(vlb_ctx* ctx, const char* name, size_t bytes, void** out) {
   auto& b = ctx->scratch[name];
@@ -69,17 +97,22 @@ vlb_status scratch(vlb_ctx* ctx, const char* name, size_t bytes, void** out) {
       b.p = nullptr;
       b.bytes = 0;
     }
-    // a buffer that grows grows by half at least: batches of uneven sizes then
-    // reach their largest in a few steps, not in one allocation each
-    size_t want = std::max<size_t>(std::max<size_t>(bytes, 256), old + old / 2);
+    // a buffer that grows grows by half (at most 256 MiB more than asked for): batches
+    // of uneven sizes then reach their largest in a few steps, not in one allocation each
+    size_t want = std::max<size_t>(std::max<size_t>(bytes, 256), std::min<size_t>(old + old / 2, bytes + (256u << 20)));
     cudaError_t e = cudaMalloc(&b.p, want);
     if (e != cudaSuccess && want > bytes) {
       cudaGetLastError();
       want = bytes;
       e = cudaMalloc(&b.p, want);
     }
+    if (e != cudaSuccess && !ctx->extras && drop_extras(ctx)) {
+      cudaGetLastError();
+      e = cudaMalloc(&b.p, want);
+    }
     if (e != cudaSuccess) {
       cudaGetLastError();
+      b.p = nullptr;
       return fail(ctx, VLB_ERR_OOM, "scratch '%s': cudaMalloc(%zu) failed", name, want);
     }
     b.bytes = want;
@@ -1292,13 +1325,12 @@ static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const floa
   a.lane = lane_mode(scene, nprobes, p->flags, p->shading);
   a.shading = p->shading;
   a.light = make_float3(p->light_pos[0], p->light_pos[1], p->light_pos[2]);
-  if (a.lane && !from_root && sun_map_pays(scene, uint64_t(nprobes) * a.S, 6.0)) {
-    void* cells;
-    if ((st = scratch(ctx, "sun_map", kMapBytes, &cells))) return st;
-    sun_map_plan(scene, a.sun, a.shading == VLB_SHADE_REF_PHONG ? &a.light : nullptr, a.bias,
-                 static_cast<uint32_t*>(cells), &a.sun_map);
-  }
   const bool grid = grid_mode(scene, nprobes, a.S, p);
+  void* map_cells;
+  if (a.lane && !grid && !from_root && sun_map_pays(scene, uint64_t(nprobes) * a.S, 6.0) &&
+      scratch(ctx, "sun_map", kMapBytes, &map_cells) == VLB_OK)
+    sun_map_plan(scene, a.sun, a.shading == VLB_SHADE_REF_PHONG ? &a.light : nullptr, a.bias,
+                 static_cast<uint32_t*>(map_cells), &a.sun_map);
   const uint32_t cap = a.lane && !grid && !from_root ? front_cap(scene, nprobes, a.S) : 0;
   void *ent = nullptr, *cnt = nullptr;
   if (cap && scratch(ctx, "front_ent", size_t(nprobes) * cap * 32, &ent) == VLB_OK &&
@@ -1390,14 +1422,10 @@ static void job_from_trace(const vlbk::TraceArgs& a, vlbk::BakeJobDev* j) {
   j->item_begin = 0;
 }
 
-vlb_status vlb_bake_ex(vlb_ctx* ctx, const vlb_scene* scene, const float* probe_xyz, uint32_t nprobes,
-                       const vlb_bake_params* p, float* out, const vlb_bake_debug* dbg) {
-  if (!ctx) return VLB_ERR_INVALID;
-  cudaSetDevice(ctx->device);
-  if (nprobes == 0) return VLB_OK;
-  if (!out) return fail(ctx, VLB_ERR_INVALID, "null output");
+static vlb_status bake_once(vlb_ctx* ctx, const vlb_scene* scene, const float* probe_xyz, uint32_t nprobes,
+                            const vlb_bake_params* p, float* out, const vlb_bake_debug* dbg, bool extras) {
   vlbk::TraceArgs a;
-  vlb_status st = prepare_trace(ctx, scene, probe_xyz, nprobes, p, &a);
+  vlb_status st = prepare_trace(ctx, scene, probe_xyz, nprobes, p, &a, !extras);
   if (st) return st;
   const uint32_t S = a.S, K = a.K, V = 3 * K;
   const uint64_t rays = uint64_t(nprobes) * S;
@@ -1429,7 +1457,7 @@ vlb_status vlb_bake_ex(vlb_ctx* ctx, const vlb_scene* scene, const float* probe_
     void *sub, *part, *done;
     if (j.parts > 1) {
       const size_t bytes = size_t(nprobes) * j.subs * V * 4;
-      if (bytes > vlbk::kFusedSubBytes || scratch(ctx, "bake_sub", bytes, &sub) != VLB_OK) vlbk::fused_items(&j, 0);
+      if (!extras || bytes > vlbk::kFusedSubBytes || scratch(ctx, "bake_sub", bytes, &sub) != VLB_OK) vlbk::fused_items(&j, 0);
       else j.sub = static_cast<float*>(sub);
     }
     if (j.chunks > 1 || j.sub) {
@@ -1502,6 +1530,17 @@ vlb_status vlb_bake_ex(vlb_ctx* ctx, const vlb_scene* scene, const float* probe_
   if ((st = copy_out(ctx, ob)) || (st = copy_out(ctx, oh)) || (st = copy_out(ctx, os)) || (st = copy_out(ctx, orad)))
     return st;
   return finish(ctx, ob.host || oh.host || os.host || orad.host);
+}
+
+vlb_status vlb_bake_ex(vlb_ctx* ctx, const vlb_scene* scene, const float* probe_xyz, uint32_t nprobes,
+                       const vlb_bake_params* p, float* out, const vlb_bake_debug* dbg) {
+  if (!ctx) return VLB_ERR_INVALID;
+  cudaSetDevice(ctx->device);
+  if (nprobes == 0) return VLB_OK;
+  if (!out) return fail(ctx, VLB_ERR_INVALID, "null output");
+  return with_extras(ctx, [&](bool extras) {
+    return bake_once(ctx, scene, probe_xyz, nprobes, p, out, dbg, extras);
+  });
 }
 
 vlb_status vlb_bake(vlb_ctx* ctx, const vlb_scene* scene, const float* probe_xyz, uint32_t nprobes,
@@ -1717,9 +1756,9 @@ static vlb_status batch_enqueue(vlb_ctx* ctx, const BatchPlan& pl, const BatchBu
 // outputs are copied with cudaMemcpyAsync (asynchronous only for pinned
 // memory); *host_out tells whether there were any.  ext (optional, njobs
 // entries) adds kept-hit outputs and relight inputs per job.
-vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh::JobExt* ext, uint32_t njobs,
-                              const vlb_bake_params* params, const vlb_batch_schedule& sc, bool* host_out_any,
-                              uint64_t spare_bytes) {
+static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh::JobExt* ext, uint32_t njobs,
+                             const vlb_bake_params* params, const vlb_batch_schedule& sc, bool* host_out_any,
+                             uint64_t spare_bytes) {
   *host_out_any = false;
   BatchPlan pl;
   vlb_status st = batch_plan(ctx, jobs, njobs, params, &pl);
@@ -1964,6 +2003,14 @@ vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh
                                   ctx->stream));
   }
   return VLB_OK;
+}
+
+vlb_status vlbh::batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh::JobExt* ext, uint32_t njobs,
+                              const vlb_bake_params* params, const vlb_batch_schedule& sc, bool* host_out_any,
+                              uint64_t spare_bytes) {
+  return with_extras(ctx, [&](bool extras) {
+    return batch_once(ctx, jobs, ext, njobs, params, sc, host_out_any, extras ? spare_bytes : 0);
+  });
 }
 
 extern "C" {

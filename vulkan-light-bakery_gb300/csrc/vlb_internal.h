@@ -563,6 +563,7 @@ struct vlb_ctx {
   std::map<std::string, Stat> stats;
   struct Buf { void* p = nullptr; size_t bytes = 0; };
   std::map<std::string, Buf> scratch;
+  bool extras = false;  // the call under way uses the scratch that memory shortage gives back
   std::map<uint32_t, float*> cube_sa;  // solid-angle tables by face size
   std::map<uint64_t, float2*> cube_pt;  // texel-pair basis tables by (face size << 8 | lmax)
   // panorama direction tables by (w, h, shifted): h row entries, then w column
