@@ -57,11 +57,11 @@ METRIC_FULL = "probes/s, Grays/s, p99 bake latency of the default path, <=1e-4 S
 # per launch of the headline workload, ncu's L1 and issue utilisation.
 TRACE_NCU = {
     "trace_tile": {"capture": "profiles/trace_tile_c2.md", "scaled_from": "32^3 probes x 8",
-                   "dram_bytes": 3415800000, "warp_instructions": 126470600000,
-                   "l1tex_throughput_pct": 79.8, "issue_active_pct": 75.4},
+                   "dram_bytes": 5073537000, "warp_instructions": 45352290800,
+                   "l1tex_throughput_pct": 65.1, "issue_active_pct": 74.6},
     "trace_fused_lane": {"capture": "profiles/trace_tile_c2.md", "scaled_from": "32^3 probes x 8",
-                         "dram_bytes": 86500000, "warp_instructions": 125671000000,
-                         "l1tex_throughput_pct": 71.4, "issue_active_pct": 70.3},
+                         "dram_bytes": 847308800, "warp_instructions": 50007091600,
+                         "l1tex_throughput_pct": 61.2, "issue_active_pct": 66.8},
 }
 
 
@@ -296,15 +296,17 @@ def accuracy_vs_fp64(ctx, scene, probes, params, pos, idx, alb, sky, sun, nsampl
 
 
 def trace_roofline(kname, k_avg_ms, stats, clk, sms, hbm_peak, peaks_measured, P, ntri, K, C, tile):
-    """Roofline of the trace kernel.  It is bound by L1 throughput and
-    instruction issue together (the scene's nodes and triangles stay in
-    L1/L2), not by HBM: `bound` is the issue view, the one measured live, with
-    the L1 view beside (the committed ncu capture shows the L1 data stage at
-    80 % and issue at 75 %).  L1: the node and triangle bytes the lanes
-    request (counted by an instrumented bake of the same rays) over the live
-    launch time, against the nominal 128 B/clock/SM.  Issue: the capture's
-    warp instructions per launch over the live launch time, against 4 issue
-    slots/clock/SM.  The HBM view (algorithmic DRAM bytes) is kept beside."""
+    """Roofline of the trace kernel.  It is bound by instruction issue and L1
+    throughput (the scene's nodes and triangles stay in L1/L2), not by HBM:
+    `bound` is the issue view, the one measured live, with the L1 view beside
+    (the committed ncu capture shows issue at 75 % and the L1 data stage at
+    65 %).  Issue: the capture's warp instructions per launch over the live
+    launch time, against 4 issue slots/clock/SM.  L1: the node and triangle
+    bytes of the same rays walked from the root (counted by an instrumented
+    bake; the bake's own walks start at probe frontiers and look most shadow
+    rays up in a map, so they request fewer) over the live launch time, against
+    the nominal 128 B/clock/SM.  The HBM view (algorithmic DRAM bytes) is kept
+    beside."""
     mhz = clk.get("sm_max_mhz") or 2070.0
     secs = k_avg_ms * 1e-3 if k_avg_ms > 0 else None
     l1_bytes = stats["bytes"]
@@ -324,7 +326,7 @@ def trace_roofline(kname, k_avg_ms, stats, clk, sms, hbm_peak, peaks_measured, P
         dram_alg = (P * (12 + 4 + K * 12 + 4) + (P * C * K * 3 * 4 * 2 if C > 1 else 0) + max(ntri - 1, 0) * 64
                     + ntri * (48 + 16) + NDIRS * (16 + 16 + 4 + 64))
     l1 = {"achieved": l1_bytes / secs / 1e9 if secs else None, "peak": l1_peak, "unit": "GB/s",
-          "peak_source": f"nominal L1: {sms} SMs x 128 B/clock x {mhz:.0f} MHz (no measured L1 peak)",
+          "peak_source": f"nominal L1: {sms} SMs x 128 B/clock x {mhz:.0f} MHz (no measured L1 peak); bytes of walks from the root",
           "requested_bytes_per_launch": l1_bytes}
     l1["frac"] = l1["achieved"] / l1_peak if l1["achieved"] else None
     issue = {"achieved": wi / secs if wi and secs else None, "peak": issue_peak, "unit": "warp instructions/s",

@@ -18,7 +18,7 @@
 // bits.
 //
 // Latency bound: some twenty dependent node loads per warp (16 us for 4096
-// probes; 180 us for 262,144, 0.3 % of that bake).
+// probes in 778 triangles; 180 us for 32,768 probes in 49,162, 3 % of that bake).
 #pragma once
 
 #include "vlb_device.cuh"
