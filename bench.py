@@ -616,7 +616,7 @@ def c1_measure(ctx, torch, stream, steps, hbm_peak):
 
 # DRAM bytes per launch of the skybox kernel on this section's 1024-map batch,
 # from the ncu capture summarised in profiles/skybox_c0.md.
-SKYBOX_NCU = {"skybox_cube_group": 1247949000}
+SKYBOX_NCU = {"skybox_cube_group": 1225932800}
 
 
 def skybox_measure(ctx, torch, stream, steps, hbm_peak):

@@ -63,8 +63,7 @@ bool is_device_ptr(const void* p) {
 // runs out, unless the call under way uses it (ctx->extras).
 static bool drop_extras(vlb_ctx* ctx) {
   bool any = false;
-  for (const char* name : {"front_ent", "front_cnt", "sun_map", "bake_sub", "batch_front", "batch_front_n", "batch_maps",
-                           "batch_sub", "scene_build"}) {
+  for (const char* name : {"front", "sun_map", "bake_sub", "batch_front", "batch_maps", "batch_sub", "scene_build"}) {
     auto it = ctx->scratch.find(name);
     if (it == ctx->scratch.end() || !it->second.p) continue;
     if (!any) cudaStreamSynchronize(ctx->stream);
@@ -1332,17 +1331,17 @@ static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const floa
     sun_map_plan(scene, a.sun, a.shading == VLB_SHADE_REF_PHONG ? &a.light : nullptr, a.bias,
                  static_cast<uint32_t*>(map_cells), &a.sun_map);
   const uint32_t cap = a.lane && !grid && !from_root ? front_cap(scene, nprobes, a.S) : 0;
-  void *ent = nullptr, *cnt = nullptr;
-  if (cap && scratch(ctx, "front_ent", size_t(nprobes) * cap * 32, &ent) == VLB_OK &&
-      scratch(ctx, "front_cnt", size_t(nprobes) * 4, &cnt) == VLB_OK) {
+  void* ent = nullptr;  // entries, then counts
+  uint32_t* cnt = nullptr;
+  if (cap && scratch(ctx, "front", size_t(nprobes) * (cap * 32 + 4), &ent) == VLB_OK) {
     a.front = static_cast<const float4*>(ent);
-    a.front_n = static_cast<const uint32_t*>(cnt);
+    a.front_n = cnt = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(ent) + size_t(nprobes) * cap * 32);
     a.front_cap = cap;
   }
   if (!order_first || a.front || a.sun_map.cells) {
     vlbk::SetupArgs su{};
     su.front = vlbk::FrontArgs{scene->nodes, scene->ntris, a.probes, nprobes, bounds_scale(scene), cap,
-                               a.front ? static_cast<float4*>(ent) : nullptr, static_cast<uint32_t*>(cnt), ctx->d_err};
+                               a.front ? static_cast<float4*>(ent) : nullptr, cnt, ctx->d_err};
     su.map = a.sun_map;
     su.tris = scene->tris;
     su.order = order_first ? nullptr : static_cast<uint32_t*>(order);
@@ -1813,9 +1812,8 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
   void *front_ent = nullptr, *front_n = nullptr;
   if (front_probes) {
     cap = uint32_t(std::min<uint64_t>(vlbk::kFrontCap, std::min<uint64_t>(kFrontEntries, spare_bytes / 64) / front_probes));
-    if (cap < 32 || scratch(ctx, "batch_front", front_probes * cap * 32, &front_ent) != VLB_OK ||
-        scratch(ctx, "batch_front_n", front_probes * 4, &front_n) != VLB_OK)
-      cap = 0;
+    if (cap < 32 || scratch(ctx, "batch_front", front_probes * (cap * 32 + 4), &front_ent) != VLB_OK) cap = 0;
+    else front_n = static_cast<uint8_t*>(front_ent) + front_probes * cap * 32;
   }
   if (pl.fused) {  // few work items: chunks are split
     uint64_t chunk_items = 0, subs = 0;
