@@ -34,21 +34,10 @@ struct FrontBox {
   float4 a, b;  // [lx ly hx hy] [lz hz ref dist^2]
 };
 
-// The two children of node `ref` with their squared distances to the probe.
-__device__ __forceinline__ void front_children(const FrontArgs& a, int ref, float ox, float oy, float oz,
-                                               FrontBox* c) {
-  const float4* nd = a.nodes + 4 * size_t(ref);
-  const float4 n0 = __ldg(nd), n1 = __ldg(nd + 1), n2 = __ldg(nd + 2), n3 = __ldg(nd + 3);
-  c[0].a = n0;
-  c[0].b = make_float4(n2.x, n2.y, n3.x, 0.f);
-  c[1].a = n1;
-  c[1].b = make_float4(n2.z, n2.w, n3.y, 0.f);
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const float gx = axis_gap(c[h].a.x, c[h].a.z, ox), gy = axis_gap(c[h].a.y, c[h].a.w, oy),
-                gz = axis_gap(c[h].b.x, c[h].b.y, oz);
-    c[h].b.w = gx * gx + gy * gy + gz * gz;
-  }
+// Child h of node `nd`.
+__device__ __forceinline__ FrontBox front_box(const float4* nd, int h) {
+  const float4 xy = __ldg(nd + h), z = __ldg(nd + 2), r = __ldg(nd + 3);
+  return FrontBox{xy, h ? make_float4(z.z, z.w, r.y, 0.f) : make_float4(z.x, z.y, r.x, 0.f)};
 }
 
 // Entries whose box half area exceeds kFrontLarge times the squared distance
@@ -60,10 +49,63 @@ constexpr float kFrontLarge = 10.f;
 constexpr int kFrontLook = 32;
 constexpr int kFrontRounds = 8;
 
-constexpr int kFrontOpen = 64;  // nodes of a level expanded; the rest become entries
+// Nodes of a level expanded; the rest become entries (16,384 probes in 170,000 boxes,
+// lists of 1024: 16.3 ms with 64, 12.2 with 128, 12.7 with 256; fewer boxes alike).
+constexpr int kFrontOpen = 128;
+
+// A warp's shared memory: two levels of open nodes (the references of the
+// nodes and where they stand), then `cap` entries.  A child is known by its
+// parent's slot and its side; its box is read again when the list is written, so
+// that an entry is 12 bytes here, not 32, and three times the warps fit.
 struct FrontShared {
-  FrontBox open[2][kFrontOpen], done[kFrontCap];
+  int ref[2][kFrontOpen];
+  uint32_t src[2][kFrontOpen];  // 2 * parent + side
 };
+inline __host__ __device__ size_t front_shared_bytes(uint32_t cap) { return sizeof(FrontShared) + size_t(cap) * 12; }
+constexpr uint32_t kFrontWide = 1u << 31;  // in an entry's src: looks large from the probe
+
+struct FrontList {
+  uint32_t* src;
+  int* ref;
+  float* d2;
+  __device__ __forceinline__ void put(int i, uint32_t s, int r, float d) const { src[i] = s; ref[i] = r; d2[i] = d; }
+};
+
+// One warp: sorts the list by distance, then by ref.  Bitonic merges that all
+// ascend (each begins by comparing mirrored entries), so the entries past n, as
+// if at infinity, stay where they are.  Counting, n steps an entry, takes 1.8 ms
+// for 16,384 lists of up to 1024, sorting 0.76 ms; but a sort's steps depend on one
+// another, and lists of 32 lose 4 us by it (64 probes x 64 directions: 74 -> 81 us).
+constexpr int kFrontSort = 256;
+__device__ __forceinline__ void front_sort(const FrontList& l, int n) {
+  const int lane = int(threadIdx.x & 31);
+  int size = 32;
+  while (size < n) size *= 2;
+  auto order = [&](int i, int j) {
+    if (j >= n) return;
+    const float di = l.d2[i], dj = l.d2[j];
+    const int ri = l.ref[i], rj = l.ref[j];
+    if (dj < di || (dj == di && rj < ri)) {
+      const uint32_t si = l.src[i], sj = l.src[j];
+      l.put(i, sj, rj, dj);
+      l.put(j, si, ri, di);
+    }
+  };
+  for (int k = 2; k <= size; k *= 2) {
+    for (int t = lane; t < size / 2; t += 32) {
+      const int in = t & (k / 2 - 1), b = (t - in) * 2;
+      order(b + in, b + k - 1 - in);
+    }
+    __syncwarp();
+    for (int h = k / 4; h >= 1; h /= 2) {
+      for (int t = lane; t < size / 2; t += 32) {
+        const int in = t & (h - 1), b = (t - in) * 2;
+        order(b + in, b + in + h);
+      }
+      __syncwarp();
+    }
+  }
+}
 
 // One warp: probe p's frontier.
 __device__ __forceinline__ void front_probe(const FrontArgs& a, uint32_t p, FrontShared& sh) {
@@ -71,31 +113,46 @@ __device__ __forceinline__ void front_probe(const FrontArgs& a, uint32_t p, Fron
   const int cap = int(a.cap);
   const float ox = a.probes[3 * size_t(p)], oy = a.probes[3 * size_t(p) + 1], oz = a.probes[3 * size_t(p) + 2];
   const unsigned below = (1u << lane) - 1u;
-  FrontBox* done = sh.done;
-  if (lane == 0) {
-    sh.open[0][0].a = make_float4(0.f, 0.f, 0.f, 0.f);
-    sh.open[0][0].b = make_float4(0.f, 0.f, __int_as_float(0), 0.f);
-  }
+  FrontList done;
+  done.src = reinterpret_cast<uint32_t*>(&sh + 1);
+  done.ref = reinterpret_cast<int*>(done.src + cap);
+  done.d2 = reinterpret_cast<float*>(done.ref + cap);
+  // the children of node `ref`: their place (with kFrontWide), reference and squared distance
+  auto children = [&](int ref, uint32_t* src, int* cr, float* d2) {
+    const float4* nd = a.nodes + 4 * size_t(ref);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const FrontBox c = front_box(nd, h);
+      const float gx = axis_gap(c.a.x, c.a.z, ox), gy = axis_gap(c.a.y, c.a.w, oy), gz = axis_gap(c.b.x, c.b.y, oz);
+      const float ex = c.a.z - c.a.x, ey = c.a.w - c.a.y, ez = c.b.y - c.b.x;
+      cr[h] = __float_as_int(c.b.z);
+      d2[h] = gx * gx + gy * gy + gz * gz;
+      src[h] = 2u * uint32_t(ref) + uint32_t(h);
+      if (cr[h] >= 0 && ex * ey + ey * ez + ez * ex > kFrontLarge * d2[h]) src[h] |= kFrontWide;
+    }
+  };
+  if (lane == 0) { sh.ref[0][0] = 0; sh.src[0][0] = 0; }
   __syncwarp();
   int n_open = 1, n_done = 0;
   for (int level = 0; n_open > 0; ++level) {
-    const FrontBox* open = sh.open[level & 1];
-    FrontBox* next = sh.open[(level + 1) & 1];
+    const int cur = level & 1, nxt = cur ^ 1;
     int n_next = 0;
     for (int base = 0; base < n_open; base += 32) {
       const bool have = base + int(lane) < n_open;
-      // entries live now; expanding one adds one
+      // entries live now; expanding one adds one (the root, without a box of its
+      // own, always is: there is room for 32)
       const int room = cap - (n_open - base + n_next + n_done);
-      FrontBox e{};
-      if (have) e = open[base + lane];
-      const int ref = have ? __float_as_int(e.b.z) : 0;
+      const int ref = have ? sh.ref[cur][base + lane] : 0;
+      const uint32_t at = have ? sh.src[cur][base + lane] : 0;
       const bool expand = have && int(lane) < room && VLB_INB(ref, 2 * a.ntris - 2, a.err);
-      FrontBox c[2];
+      uint32_t cs[2];
+      int cr[2];
+      float cd[2];
       bool go[2] = {false, false};  // the child is expanded in turn
       if (expand) {
-        front_children(a, ref, ox, oy, oz, c);
+        children(ref, cs, cr, cd);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) go[h] = __float_as_int(c[h].b.z) >= 0 && c[h].b.w == 0.f;
+        for (int h = 0; h < 2; ++h) go[h] = cr[h] >= 0 && cd[h] == 0.f;
       }
       {  // no more than the next level holds
         const unsigned w0 = __ballot_sync(kAll, expand && go[0]), w1 = __ballot_sync(kAll, expand && go[1]);
@@ -105,13 +162,17 @@ __device__ __forceinline__ void front_probe(const FrontArgs& a, uint32_t p, Fron
       const unsigned keep = __ballot_sync(kAll, have && !expand);
       const unsigned g0 = __ballot_sync(kAll, expand && go[0]), g1 = __ballot_sync(kAll, expand && go[1]);
       const unsigned d0 = __ballot_sync(kAll, expand && !go[0]), d1 = __ballot_sync(kAll, expand && !go[1]);
-      if (have && !expand) done[n_done + __popc(keep & below)] = e;
-      int nd = n_done + __popc(keep);
+      // a node that stays holds the probe
+      if (have && !expand) done.put(n_done + __popc(keep & below), at | kFrontWide, ref, 0.f);
+      const int nd = n_done + __popc(keep);
       if (expand) {
-        if (go[0]) next[n_next + __popc(g0 & below)] = c[0];
-        else done[nd + __popc(d0 & below)] = c[0];
-        if (go[1]) next[n_next + __popc(g0) + __popc(g1 & below)] = c[1];
-        else done[nd + __popc(d0) + __popc(d1 & below)] = c[1];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int g = n_next + (h ? __popc(g0) + __popc(g1 & below) : __popc(g0 & below));
+          const int d = nd + (h ? __popc(d0) + __popc(d1 & below) : __popc(d0 & below));
+          if (go[h]) { sh.ref[nxt][g] = cr[h]; sh.src[nxt][g] = cs[h] & ~kFrontWide; }
+          else done.put(d, cs[h], cr[h], cd[h]);
+        }
       }
       n_done = nd + __popc(d0) + __popc(d1);
       n_next += __popc(g0) + __popc(g1);
@@ -125,20 +186,19 @@ __device__ __forceinline__ void front_probe(const FrontArgs& a, uint32_t p, Fron
     const int n0 = n_done;
     for (int base = 0; base < n0; base += 32) {
       const bool have = base + int(lane) < n0;
-      FrontBox e{};
-      if (have) e = done[base + lane];
-      const float ex = e.a.z - e.a.x, ey = e.a.w - e.a.y, ez = e.b.y - e.b.x;
-      const int ref = __float_as_int(e.b.z);
-      const bool want = have && ref >= 0 && ex * ey + ey * ez + ez * ex > kFrontLarge * e.b.w &&
-                        VLB_INB(ref, 2 * a.ntris - 2, a.err);
+      const uint32_t src = have ? done.src[base + lane] : 0;
+      const int ref = have ? done.ref[base + lane] : 0;
+      const bool want = (src & kFrontWide) && VLB_INB(ref, 2 * a.ntris - 2, a.err);
       const unsigned wm = __ballot_sync(kAll, want);
       const bool expand = want && n_done + __popc(wm & below) < look;
       const unsigned em = __ballot_sync(kAll, expand);
       if (expand) {
-        FrontBox c[2];
-        front_children(a, ref, ox, oy, oz, c);
-        done[base + lane] = c[0];
-        done[n_done + __popc(em & below)] = c[1];
+        uint32_t cs[2];
+        int cr[2];
+        float cd[2];
+        children(ref, cs, cr, cd);
+        done.put(base + int(lane), cs[0], cr[0], cd[0]);
+        done.put(n_done + __popc(em & below), cs[1], cr[1], cd[1]);
       }
       n_done += __popc(em);
       __syncwarp();
@@ -146,13 +206,22 @@ __device__ __forceinline__ void front_probe(const FrontArgs& a, uint32_t p, Fron
     if (n_done == n0) break;
   }
   const float m = (fmaxf(fmaxf(fabsf(ox), fabsf(oy)), fabsf(oz)) + a.scale) * 0x1p-20f;
-  // nearest first (rank by distance, then by position)
+  // nearest first, equal distances by position: short lists by counting the
+  // entries before each, long ones sorted, the position in the references' place
+  const bool sorted = n_done > kFrontSort;
+  if (sorted) {
+    for (int i = int(lane); i < n_done; i += 32) done.ref[i] = i;
+    __syncwarp();
+    front_sort(done, n_done);
+  }
   float4* out = a.ent + size_t(p) * a.cap * 2;
   for (int i = int(lane); i < n_done; i += 32) {
-    FrontBox e = done[i];
-    int rank = 0;
-    for (int j = 0; j < n_done; ++j) {
-      const float dj = done[j].b.w;
+    const uint32_t src = done.src[i] & ~kFrontWide;
+    FrontBox e = front_box(a.nodes + 4 * size_t(src >> 1), int(src & 1u));
+    e.b.w = done.d2[i];
+    int rank = sorted ? i : 0;
+    for (int j = 0; !sorted && j < n_done; ++j) {
+      const float dj = done.d2[j];
       rank += dj < e.b.w || (dj == e.b.w && j < i);
     }
     // relative to the probe, widened by m

@@ -20,7 +20,6 @@ constexpr int kSetupThreads = 256, kSetupWarps = kSetupThreads / 32;
 static_assert(kSetupThreads == kMapThreads, "one CTA draws one slice of a map's triangle group");
 
 union SetupShared {
-  FrontShared front[kSetupWarps];
   MapShared map;
   ProbeSortShared sort;
 };
@@ -43,13 +42,13 @@ __global__ void __launch_bounds__(kSetupThreads) k_bake_setup(const SetupArgs a)
     return;
   }
   const uint32_t warp = threadIdx.x >> 5, p = (cta - a.map_ctas) * kSetupWarps + warp;
-  if (p < a.front.nprobes) front_probe(a.front, p, sh.front[warp]);
+  if (p < a.front.nprobes)
+    front_probe(a.front, p, *reinterpret_cast<FrontShared*>(setup_smem + warp * front_shared_bytes(a.front.cap)));
 }
 
 __global__ void __launch_bounds__(kSetupWarps * 32)
-    k_probe_front_batch(const BakeJobDev* __restrict__ jobs, uint32_t njobs, uint32_t total) {
+    k_probe_front_batch(const BakeJobDev* __restrict__ jobs, uint32_t njobs, uint32_t total, uint32_t cap) {
   extern __shared__ __align__(16) unsigned char setup_smem[];
-  FrontShared* sh = reinterpret_cast<FrontShared*>(setup_smem);
   const uint32_t warp = threadIdx.x >> 5, w = blockIdx.x * kSetupWarps + warp;
   if (w >= total) return;
   uint32_t lo = 0, hi = njobs - 1;  // the last job that begins at or before w
@@ -62,7 +61,7 @@ __global__ void __launch_bounds__(kSetupWarps * 32)
   if (!j.front || p >= j.nprobes) return;
   const FrontArgs a{j.nodes, j.ntris, j.probes, j.nprobes, j.front_scale, j.front_cap, const_cast<float4*>(j.front),
                     const_cast<uint32_t*>(j.front_n), j.err};
-  front_probe(a, p, sh[warp]);
+  front_probe(a, p, *reinterpret_cast<FrontShared*>(setup_smem + warp * front_shared_bytes(cap)));
 }
 
 __global__ void __launch_bounds__(kMapThreads) k_sun_map_batch(const BakeJobDev* __restrict__ jobs, uint32_t njobs) {
@@ -97,20 +96,20 @@ void launch_bake_setup(SetupArgs a, const float bounds[6], cudaStream_t s) {
       (a.order ? 1u : 0u) + a.map_ctas + (a.front.ent ? (a.front.nprobes + kSetupWarps - 1) / kSetupWarps : 0u);
   if (!grid) return;
   // the frontiers' lists take the most; a launch without them keeps its CTAs small
-  const size_t smem = a.front.ent ? sizeof(SetupShared) : std::max(sizeof(MapShared), sizeof(ProbeSortShared));
+  const size_t smem = std::max(sizeof(SetupShared), a.front.ent ? kSetupWarps * front_shared_bytes(a.front.cap) : 0);
   static std::atomic<uint64_t> opted{0};
-  smem_opt_in(k_bake_setup, int(sizeof(SetupShared)), opted);
+  smem_opt_in(k_bake_setup, int(std::max(sizeof(SetupShared), kSetupWarps * front_shared_bytes(kFrontCap))), opted);
   k_bake_setup<<<grid, kSetupThreads, smem, s>>>(a);
 }
 
 uint32_t probe_order_in_setup(uint32_t nprobes) { return nprobes <= kCountMax; }
 
-void launch_probe_front_batch(const BakeJobDev* jobs, uint32_t njobs, uint32_t total, cudaStream_t s) {
+void launch_probe_front_batch(const BakeJobDev* jobs, uint32_t njobs, uint32_t total, uint32_t cap, cudaStream_t s) {
   if (!total) return;
   static std::atomic<uint64_t> opted{0};
-  constexpr size_t smem = kSetupWarps * sizeof(FrontShared);
-  smem_opt_in(k_probe_front_batch, int(smem), opted);
-  k_probe_front_batch<<<(total + kSetupWarps - 1) / kSetupWarps, kSetupThreads, smem, s>>>(jobs, njobs, total);
+  smem_opt_in(k_probe_front_batch, int(kSetupWarps * front_shared_bytes(kFrontCap)), opted);
+  k_probe_front_batch<<<(total + kSetupWarps - 1) / kSetupWarps, kSetupThreads, kSetupWarps * front_shared_bytes(cap),
+                        s>>>(jobs, njobs, total, cap);
 }
 
 // CTAs per group of triangles: about seven CTAs per SM in all.

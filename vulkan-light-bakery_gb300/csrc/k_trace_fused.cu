@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace_fused(const BakeJ
           if (staged) {
             fnext = max(fnext, lr_front_next(J, L, took, 0, stack));
           } else {  // all of it, nearest on top
-            for (int f = kFrontCap - kFrontStage; f > 0; f -= kFrontStage) lr_front(J, L, took, f, stack);
+            for (int f = kFrontWhole - kFrontStage; f > 0; f -= kFrontStage) lr_front(J, L, took, f, stack);
             lr_front(J, L, took, 0, stack);
             if (took) L.cur = stack[--L.sp];
           }

@@ -1168,9 +1168,33 @@ static bool grid_mode(const vlb_scene* scene, uint32_t nprobes, uint32_t S, cons
 // bake of that size is a multiple of it).
 constexpr uint64_t kFrontEntries = 1ull << 27;
 
-static uint32_t front_cap(const vlb_scene* scene, uint64_t nprobes, uint32_t S) {
+// Layers of triangles over a scene: their area over the square of its diagonal (0.7
+// for a terrain, 4 for 64 boxes in a room, 130 for 4096).
+static double scene_layers(const vlb_scene* sc) {
+  double diag2 = 0.0;
+  for (int a = 0; a < 3; ++a) {
+    const double e = double(sc->bounds[3 + a]) - sc->bounds[a];
+    diag2 += e * e;
+  }
+  return diag2 > 0.0 ? sc->area / diag2 : 0.0;
+}
+
+// The longest list: the nodes that hold a probe grow about as the root of the
+// layers, and a list cut short sends the rays into the nodes it left out (1024
+// directions, 64 nodes open a level, lists of 128, 256, 512, 1024: 32,768 probes in 4096 boxes, 130 layers,
+// 6.63, 6.47, 6.48, 6.62 ms; 16,384 probes in 16,384 boxes, 514 layers, 7.33, 5.35,
+// 5.30, 5.33; in 65,536 boxes, 2049 layers, 16.7, 12.3, 8.5, 8.4; in 170,000 boxes
+// 31.4, 24.1, 17.9, 16.3).  whole: the walk does not take the list in stages.
+static uint32_t front_list(const vlb_scene* scene, bool whole) {
+  uint32_t cap = vlbk::kFrontWhole;
+  const double want = 20.0 * std::sqrt(scene_layers(scene));
+  while (!whole && cap < vlbk::kFrontCap && cap < want) cap *= 2;
+  return cap;
+}
+
+static uint32_t front_cap(const vlb_scene* scene, uint64_t nprobes, uint32_t S, bool whole) {
   if (scene->ntris < 64 || scene->wnodes || scene->depth > uint32_t(vlbk::kLaneStack) || S < 64 || !nprobes) return 0;
-  const uint64_t cap = std::min<uint64_t>(vlbk::kFrontCap, kFrontEntries / nprobes);
+  const uint64_t cap = std::min<uint64_t>(front_list(scene, whole), kFrontEntries / nprobes);
   return cap < 32 ? 0 : uint32_t(cap);
 }
 
@@ -1191,13 +1215,7 @@ constexpr size_t kMapBytes = size_t(kMapSide) * kMapSide * 8;
 // cells (15 us for that terrain, 130 us for the 4096 boxes' 130 layers), and a
 // launch of its own 6 us (a batch draws all its jobs' maps in one).
 static bool sun_map_pays(const vlb_scene* sc, uint64_t rays, double launch_us) {
-  double diag2 = 0.0;
-  for (int a = 0; a < 3; ++a) {
-    const double e = double(sc->bounds[3 + a]) - sc->bounds[a];
-    diag2 += e * e;
-  }
-  const double layers = diag2 > 0.0 ? sc->area / diag2 : 0.0;
-  return sc->ntris && double(rays) * 25e-6 > launch_us + sc->ntris * 90e-6 + layers;
+  return sc->ntris && double(rays) * 25e-6 > launch_us + sc->ntris * 90e-6 + scene_layers(sc);
 }
 
 // Plane, extent and margins of a scene's sun map (sun_map.cuh) for a sun toward
@@ -1286,6 +1304,10 @@ static vlb_status check_params(vlb_ctx* ctx, const vlb_scene* scene, const vlb_b
   return VLB_OK;
 }
 
+static uint32_t size_class(uint32_t ntris);
+static vlb_batch_schedule class_sched(const vlb_ctx* ctx, uint32_t cls);
+static vlbk::FusedSched fused_sched(const vlb_batch_schedule& sc);
+
 static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const float* probe_xyz, uint32_t nprobes,
                                 const vlb_bake_params* p, vlbk::TraceArgs* out, bool from_root = false) {
   double sl = 0.0;
@@ -1330,7 +1352,9 @@ static vlb_status prepare_trace(vlb_ctx* ctx, const vlb_scene* scene, const floa
       scratch(ctx, "sun_map", kMapBytes, &map_cells) == VLB_OK)
     sun_map_plan(scene, a.sun, a.shading == VLB_SHADE_REF_PHONG ? &a.light : nullptr, a.bias,
                  static_cast<uint32_t*>(map_cells), &a.sun_map);
-  const uint32_t cap = a.lane && !grid && !from_root ? front_cap(scene, nprobes, a.S) : 0;
+  const bool whole = p->precision == VLB_PREC_FUSED &&
+                     fused_sched(class_sched(ctx, size_class(scene->ntris))).refill_idle < 32;
+  const uint32_t cap = a.lane && !grid && !from_root ? front_cap(scene, nprobes, a.S, whole) : 0;
   void* ent = nullptr;  // entries, then counts
   uint32_t* cnt = nullptr;
   if (cap && scratch(ctx, "front", size_t(nprobes) * (cap * 32 + 4), &ent) == VLB_OK) {
@@ -1637,6 +1661,7 @@ struct BatchBufs {
   size_t table_bytes, dst_off, p0_off, np_off;
   uint32_t ndev_out;   // jobs whose output is device memory (scattered by a kernel)
   uint32_t front_total;  // probes with a frontier
+  uint32_t front_cap;    // their longest list
   uint32_t map_ctas;     // CTAs that draw the jobs' sun maps
   void* maps;
   size_t map_bytes;
@@ -1711,7 +1736,7 @@ static vlb_status batch_enqueue(vlb_ctx* ctx, const BatchPlan& pl, const BatchBu
   }
   if (bb.front_total) {
     KScope k(ctx, "probe_front_batch");
-    vlbk::launch_probe_front_batch(table, ntable, bb.front_total, ctx->stream);
+    vlbk::launch_probe_front_batch(table, ntable, bb.front_total, bb.front_cap, ctx->stream);
   }
   if (bb.map_ctas) {
     KScope k(ctx, "sun_map_batch");
@@ -1799,21 +1824,36 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
   // to be had (without them the walks start at the root and trace every shadow
   // ray: the same results).
   uint64_t front_probes = 0;
-  std::vector<uint8_t> fronts(ntable), maps(ntable);
+  std::vector<uint8_t> maps(ntable);
+  std::vector<uint32_t> caps(ntable, 0);
+  uint64_t entries = 0;
+  const bool whole = pl.fused && fused_sched(sc).refill_idle < 32;
   for (uint32_t i = 0; i < ntable; ++i) {
     const BatchJob& b = pl.jobs[i];
     const vlb_scene* sc = jobs[b.idx].scene;
-    fronts[i] = !(ext && ext[b.idx].hits_in) && front_cap(sc, b.nprobes, b.S) != 0;
+    if (!(ext && ext[b.idx].hits_in)) caps[i] = front_cap(sc, b.nprobes, b.S, whole);
     maps[i] = sun_map_pays(sc, uint64_t(b.nprobes) * b.S, 0.0);
-    if (fronts[i]) front_probes += b.nprobes;
+    if (caps[i]) {
+      front_probes += b.nprobes;
+      entries += uint64_t(b.nprobes) * caps[i];
+    }
     if (maps[i]) bb.map_bytes += kMapBytes;
   }
-  uint32_t cap = 0;
   void *front_ent = nullptr, *front_n = nullptr;
+  uint64_t front_at = 0;
   if (front_probes) {
-    cap = uint32_t(std::min<uint64_t>(vlbk::kFrontCap, std::min<uint64_t>(kFrontEntries, spare_bytes / 64) / front_probes));
-    if (cap < 32 || scratch(ctx, "batch_front", front_probes * (cap * 32 + 4), &front_ent) != VLB_OK) cap = 0;
-    else front_n = static_cast<uint8_t*>(front_ent) + front_probes * cap * 32;
+    const uint64_t most = std::min<uint64_t>(kFrontEntries, spare_bytes / 64);
+    if (entries > most) {  // lists of one length, as long as fits
+      const uint64_t cap = most / front_probes;
+      entries = 0;
+      for (uint32_t i = 0; i < ntable; ++i) {
+        caps[i] = cap < 32 ? 0 : uint32_t(std::min<uint64_t>(caps[i], cap));
+        entries += uint64_t(pl.jobs[i].nprobes) * caps[i];
+      }
+    }
+    if (!entries || scratch(ctx, "batch_front", entries * 32 + front_probes * 4, &front_ent) != VLB_OK)
+      caps.assign(ntable, 0);
+    else front_n = static_cast<uint8_t*>(front_ent) + entries * 32;
   }
   if (pl.fused) {  // few work items: chunks are split
     uint64_t chunk_items = 0, subs = 0;
@@ -1912,10 +1952,12 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
       padded += (uint64_t(b.nprobes) + 31) / 32 * 32 * b.S;
     }
     d.front_begin = bb.front_total;
-    if (cap && fronts[ord[t]]) {
-      d.front = static_cast<const float4*>(front_ent) + size_t(bb.front_total) * cap * 2;
+    if (const uint32_t cap = caps[ord[t]]) {
+      d.front = static_cast<const float4*>(front_ent) + front_at * 2;
       d.front_n = static_cast<const uint32_t*>(front_n) + bb.front_total;
       d.front_cap = cap;
+      front_at += uint64_t(b.nprobes) * cap;
+      bb.front_cap = std::max(bb.front_cap, cap);
       d.front_scale = bounds_scale(j.scene);
       bb.front_total += b.nprobes;
     }
@@ -1955,7 +1997,7 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
                                uint64_t(uintptr_t(tile)), uint64_t(uintptr_t(out)), uint64_t(uintptr_t(meta)),
                                uint64_t(uintptr_t(counter)), uint64_t(ctx->num_sms), pl.fused,
                                uint64_t(uintptr_t(part)), uint64_t(uintptr_t(done)), pl.rows, sc.ctas_per_sm,
-                               sc.node_steps, sc.refill_idle, bb.front_total, bb.map_ctas,
+                               sc.node_steps, sc.refill_idle, bb.front_total, bb.front_cap, bb.map_ctas,
                                uint64_t(uintptr_t(bb.maps)), bb.map_bytes, uint64_t(uintptr_t(bb.sub))};
   if (pl.fused && ntable == 1) {  // one job goes to the kernel by value: its fields are part of the shape
     const auto* w = reinterpret_cast<const uint64_t*>(table.data());

@@ -47,9 +47,10 @@ __device__ __forceinline__ bool inb_checked(long long i, long long n, int* err) 
 // the per-lane stacks of the lane walks (a wide node pushes up to 7 children).
 constexpr int kTraceStack = 64;
 constexpr int kLaneStack = 96;
-// With probe frontiers a walk starts with up to kFrontCap entries on its
+// With probe frontiers a walk starts with up to kFrontWhole entries on its
 // stack; only trees at most kLaneStack deep use them, so it cannot overflow.
-constexpr int kLaneStackFront = kLaneStack + 128;
+constexpr int kFrontWhole = 128;
+constexpr int kLaneStackFront = kLaneStack + kFrontWhole;
 
 // ---- binary traversal node (64 bytes) -------------------------------------------
 // The two children's boxes (lo xyz, hi xyz) grouped by axis, so that one
@@ -233,8 +234,9 @@ int launch_point_order(const float* pts, uint32_t n, const float bounds[6], uint
 
 // ---- probe frontiers (front.cuh) ------------------------------------------------
 // Entries per probe: 32 bytes each, [lx ly hx hy] [lz hz ref dist^2], the box
-// relative to the probe, nearest first; cnt[probe] of them.
-constexpr int kFrontCap = 128;
+// relative to the probe, nearest first; cnt[probe] of them.  Walks that take the
+// list in stages take any length, others at most kFrontWhole.
+constexpr uint32_t kFrontCap = 1024;
 struct FrontArgs {
   const float4* nodes;
   uint32_t ntris;
@@ -248,7 +250,8 @@ struct FrontArgs {
 };
 struct BakeJobDev;
 // The frontiers of all jobs that have one: `total` probes, numbered by front_begin.
-void launch_probe_front_batch(const BakeJobDev* jobs, uint32_t njobs, uint32_t total, cudaStream_t s);
+// cap: the largest of the jobs' front_cap.
+void launch_probe_front_batch(const BakeJobDev* jobs, uint32_t njobs, uint32_t total, uint32_t cap, cudaStream_t s);
 
 // ---- sun maps (sun_map.cuh) ------------------------------------------------------
 struct SunMap {
