@@ -57,11 +57,11 @@ METRIC_FULL = "probes/s, Grays/s, p99 bake latency of the default path, <=1e-4 S
 # per launch of the headline workload, ncu's L1 and issue utilisation.
 TRACE_NCU = {
     "trace_tile": {"capture": "profiles/trace_tile_c2.md", "scaled_from": "32^3 probes x 8",
-                   "dram_bytes": 5073537000, "warp_instructions": 45352290800,
-                   "l1tex_throughput_pct": 65.1, "issue_active_pct": 74.6},
+                   "dram_bytes": 5138901000, "warp_instructions": 44133599200,
+                   "l1tex_throughput_pct": 64.0, "issue_active_pct": 74.8},
     "trace_fused_lane": {"capture": "profiles/trace_tile_c2.md", "scaled_from": "32^3 probes x 8",
-                         "dram_bytes": 847308800, "warp_instructions": 50007091600,
-                         "l1tex_throughput_pct": 61.2, "issue_active_pct": 66.8},
+                         "dram_bytes": 867932200, "warp_instructions": 48756572900,
+                         "l1tex_throughput_pct": 60.3, "issue_active_pct": 67.0},
 }
 
 
@@ -300,7 +300,7 @@ def trace_roofline(kname, k_avg_ms, stats, clk, sms, hbm_peak, peaks_measured, P
     throughput (the scene's nodes and triangles stay in L1/L2), not by HBM:
     `bound` is the issue view, the one measured live, with the L1 view beside
     (the committed ncu capture shows issue at 75 % and the L1 data stage at
-    65 %).  Issue: the capture's warp instructions per launch over the live
+    64 %).  Issue: the capture's warp instructions per launch over the live
     launch time, against 4 issue slots/clock/SM.  L1: the node and triangle
     bytes of the same rays walked from the root (counted by an instrumented
     bake; the bake's own walks start at probe frontiers and look most shadow

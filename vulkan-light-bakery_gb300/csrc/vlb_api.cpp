@@ -1164,9 +1164,9 @@ static bool grid_mode(const vlb_scene* scene, uint32_t nprobes, uint32_t S, cons
 // probes: 83 us with and without) and a batch gains (6.1 -> 5.6 ms); fewer
 // share it too little.  Trees deeper than the lane stack keep the
 // root (their walks may overflow the stack, and must say so).
-// At most 4 GiB of entries, lists of 32 for 4 M probes (the radiance tile of a
+// At most 8 GiB of entries, lists of 32 for 8 M probes (the radiance tile of a
 // bake of that size is a multiple of it).
-constexpr uint64_t kFrontEntries = 1ull << 27;
+constexpr uint64_t kFrontEntries = 1ull << 28;
 
 // Layers of triangles over a scene: their area over the square of its diagonal (0.7
 // for a terrain, 4 for 64 boxes in a room, 130 for 4096).
@@ -1843,11 +1843,11 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
   uint64_t front_at = 0;
   if (front_probes) {
     const uint64_t most = std::min<uint64_t>(kFrontEntries, spare_bytes / 64);
-    if (entries > most) {  // lists of one length, as long as fits
-      const uint64_t cap = most / front_probes;
+    // the longest lists are cut until all fit
+    for (uint32_t cap = vlbk::kFrontCap; entries > most; cap -= cap / 4) {
       entries = 0;
       for (uint32_t i = 0; i < ntable; ++i) {
-        caps[i] = cap < 32 ? 0 : uint32_t(std::min<uint64_t>(caps[i], cap));
+        caps[i] = cap < 32 ? 0 : std::min(caps[i], cap);
         entries += uint64_t(pl.jobs[i].nprobes) * caps[i];
       }
     }
