@@ -1,0 +1,53 @@
+"""Calls made while the context holds probe frontiers of an earlier bake and little
+device memory is free: the frontiers are given back, and the call returns what it
+returns with memory to spare."""
+import contextlib
+
+import numpy as np
+import pytest
+
+import vlb
+
+pytestmark = pytest.mark.gpu
+
+# 65,536 probes: 268 MB of frontiers; 2056 directions make rows of 4112 BF16 values,
+# two splits, whose sums take 25 MB at lmax 3
+PROBES, S = 65536, 2056
+
+
+@contextlib.contextmanager
+def little_memory(torch, left):
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+
+
+def setup(c):
+    pos, idx, alb = vlb.synth_box_scene(3, 64)
+    probes = np.random.default_rng(9).uniform(0, 1, (PROBES, 3)).astype(np.float32)
+    return c.scene(pos, idx, alb), probes, c.fibonacci(S)
+
+
+def params(ds, precision):
+    return vlb.bake_params(ds, lmax=3, precision=precision, sun=vlb.synth_sun(1))
+
+
+def test_split_projection_of_a_bake_keeps_its_bits():
+    torch = pytest.importorskip("torch")
+    got = []
+    for short in (False, True):
+        c = vlb.Context(0)
+        try:
+            scene, probes, ds = setup(c)
+            c.bake(scene, probes, params(ds, vlb.PREC_FP32))  # a tile of the same size, the frontiers
+            c.bake(scene, probes[:64], params(ds, vlb.PREC_MIXED))
+            with little_memory(torch, 12 << 20) if short else contextlib.nullcontext():
+                got.append(c.bake(scene, probes, params(ds, vlb.PREC_MIXED)))
+        finally:
+            c.close()
+    assert np.array_equal(got[0], got[1])

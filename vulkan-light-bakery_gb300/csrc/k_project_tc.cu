@@ -438,7 +438,7 @@ int launch_project_tc(const uint16_t* radiance, uint32_t nprobes, uint32_t S, co
   static std::atomic<uint64_t> opted{0};
   smem_opt_in(k_project_tc, int(kSmemBytes), opted);
   const uint32_t ntiles = (rows + kTileM - 1) / kTileM;
-  const uint32_t splits = partial ? (S + kTcSplit - 1) / kTcSplit : 1;
+  const uint32_t splits = (S + kTcSplit - 1) / kTcSplit;
   const uint32_t grid = uint32_t(std::min<uint64_t>(uint64_t(ntiles) * splits, uint64_t(num_sms)));
   k_project_tc<<<grid, kTcThreads, kSmemBytes, s>>>(ta, tb, rows, S, K, out, partial, splits, err, hold,
                                                      wait_polls ? wait_polls : kWaitPolls);

@@ -1090,10 +1090,14 @@ static vlb_status project_bf16(vlb_ctx* ctx, const uint16_t* rad, uint32_t nprob
                                uint32_t K, float* out, bool split, const char* part_name = "project_partial") {
   const uint32_t S = dirs->n;
   if (vlbk::project_tc_supported(rad, split ? 2 * S : S) && (!split || dirs->d_bt2)) {
-    void* part = nullptr;  // without it rows stay whole
+    // rows whose sums do not fit are not taken whole: that is another sum
+    void* part = nullptr;
     const size_t pb = vlbk::project_tc_partial_bytes(nprobes, split ? 2 * S : S, K);
-    if (pb && scratch(ctx, part_name, pb, &part) != VLB_OK) part = nullptr;
-    KScope k(ctx, split ? "project_tc_split" : "project_tc", part ? 2 : 1);
+    if (pb) {
+      vlb_status st = scratch(ctx, part_name, pb, &part);
+      if (st) return st;
+    }
+    KScope k(ctx, split ? "project_tc_split" : "project_tc", pb ? 2 : 1);
     const int r = vlbk::launch_project_tc(rad, nprobes, split ? 2 * S : S, split ? dirs->d_bt2 : dirs->d_bt,
                                           split ? dirs->bt2_pitch : dirs->bt_pitch, K, out, static_cast<float*>(part),
                                           ctx->d_err, ctx->num_sms, ctx->stream, ctx->hold_producer, ctx->wait_polls);

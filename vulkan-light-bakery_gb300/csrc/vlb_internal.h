@@ -154,8 +154,7 @@ void launch_project_bf16_simt(const uint16_t* radiance, uint32_t nprobes, uint32
 // Needs S % 8 == 0 and a 16-byte aligned tile; returns -1 if the tensor maps
 // cannot be built.
 bool project_tc_supported(const void* radiance, uint32_t S);
-// Device scratch for the splits of long rows (`partial`), 0 for rows taken
-// whole; with a null `partial` every row is taken whole.
+// Device scratch for the splits of long rows (`partial`), 0 for rows taken whole.
 size_t project_tc_partial_bytes(uint32_t nprobes, uint32_t S, uint32_t K);
 // hold / wait_polls: vlb_ctx_test_hook (0, 0 in normal use).
 int launch_project_tc(const uint16_t* radiance, uint32_t nprobes, uint32_t S, const uint16_t* basis_bt,
