@@ -51,3 +51,49 @@ def test_split_projection_of_a_bake_keeps_its_bits():
         finally:
             c.close()
     assert np.array_equal(got[0], got[1])
+
+
+def test_split_projection_of_a_batch_keeps_its_bits():
+    """With memory for the sums or not, and in the calls after it (the second of a shape is captured)."""
+    torch = pytest.importorskip("torch")
+    got = []
+    for short in (False, True):
+        c = vlb.Context(0)
+        try:
+            scene, probes, ds = setup(c)
+            mixed = params(ds, vlb.PREC_MIXED)
+            c.bake_batch([(scene, probes, None)], params(ds, vlb.PREC_FP32))
+            c.bake_batch([(scene, probes[:64], None)], mixed)
+            with little_memory(torch, 12 << 20) if short else contextlib.nullcontext():
+                got.append(c.bake_batch([(scene, probes, None)], mixed)[0])
+            for _ in range(3):
+                got.append(c.bake_batch([(scene, probes, None)], mixed)[0])
+        finally:
+            c.close()
+    for other in got[1:]:
+        assert np.array_equal(got[0], other)
+
+
+def test_batch_that_ran_out_of_memory_runs_later():
+    """The call after a batch that failed for want of its split sums is a first call: nothing
+    of it is captured, and the ones after it are."""
+    torch = pytest.importorskip("torch")
+    c = vlb.Context(0)
+    try:
+        # few triangles and many jobs: no frontiers and no light maps that could be given back
+        scene = c.scene(*vlb.synth_box_scene(3, 2))
+        probes = np.random.default_rng(9).uniform(0, 1, (PROBES, 3)).astype(np.float32)
+        jobs = [(scene, part, None) for part in np.array_split(probes, 600)]
+        ds = c.fibonacci(S)
+        mixed = params(ds, vlb.PREC_MIXED)
+        c.bake_batch(jobs, params(ds, vlb.PREC_FP32))
+        c.bake_batch([(scene, probes[:64], None)], mixed)
+        with little_memory(torch, 12 << 20):
+            with pytest.raises(vlb.VlbError) as e:
+                c.bake_batch(jobs, mixed)
+            assert e.value.status == vlb.ERR_OOM
+        got = [np.concatenate(c.bake_batch(jobs, mixed)) for _ in range(3)]
+        assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+        assert np.array_equal(got[0], c.bake(scene, probes, mixed))
+    finally:
+        c.close()

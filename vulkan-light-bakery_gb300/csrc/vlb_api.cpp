@@ -1079,38 +1079,36 @@ static vlb_status dirset_split_basis(vlb_ctx* ctx, const vlb_dirset* d) {
   return VLB_OK;
 }
 
+static bool tc_tile(const void* rad, const vlb_dirset* dirs, bool split) {
+  return vlbk::project_tc_supported(rad, split ? 2 * dirs->n : dirs->n) && (!split || dirs->d_bt2);
+}
+
+// Bytes for the split sums of a tile's projection, 0 for rows taken whole.
+static size_t project_part_bytes(const void* rad, uint32_t nprobes, const vlb_dirset* dirs, uint32_t K, bool bf16,
+                                 bool split) {
+  return bf16 && tc_tile(rad, dirs, split)
+             ? vlbk::project_tc_partial_bytes(nprobes, split ? 2 * dirs->n : dirs->n, K)
+             : vlbk::project_partial_bytes(nprobes, dirs->n, K);
+}
+
 // BF16 tile projection: the tcgen05 kernel when the tile meets its alignment
 // (columns a multiple of 8, 16-byte aligned), else the CUDA-core kernel.
 // split: the tile holds hi/lo pairs ([rows][2S]); the tensor-core form then
 // runs K = 2S against the split basis, so out = hi*bhi + lo*bhi + hi*blo.
-// `part_name`: the scratch for split partials (the batch path, whose launches
-// a CUDA graph may replay, keeps its own).  Split tiles need
-// dirset_split_basis first.
+// Split tiles need dirset_split_basis first.  part: project_part_bytes of scratch
+// (rows whose sums do not fit are not taken whole: that is another sum).
 static vlb_status project_bf16(vlb_ctx* ctx, const uint16_t* rad, uint32_t nprobes, const vlb_dirset* dirs,
-                               uint32_t K, float* out, bool split, const char* part_name = "project_partial") {
+                               uint32_t K, float* out, bool split, void* part) {
   const uint32_t S = dirs->n;
-  if (vlbk::project_tc_supported(rad, split ? 2 * S : S) && (!split || dirs->d_bt2)) {
-    // rows whose sums do not fit are not taken whole: that is another sum
-    void* part = nullptr;
-    const size_t pb = vlbk::project_tc_partial_bytes(nprobes, split ? 2 * S : S, K);
-    if (pb) {
-      vlb_status st = scratch(ctx, part_name, pb, &part);
-      if (st) return st;
-    }
-    KScope k(ctx, split ? "project_tc_split" : "project_tc", pb ? 2 : 1);
+  if (tc_tile(rad, dirs, split)) {
+    KScope k(ctx, split ? "project_tc_split" : "project_tc", part ? 2 : 1);
     const int r = vlbk::launch_project_tc(rad, nprobes, split ? 2 * S : S, split ? dirs->d_bt2 : dirs->d_bt,
                                           split ? dirs->bt2_pitch : dirs->bt_pitch, K, out, static_cast<float*>(part),
                                           ctx->d_err, ctx->num_sms, ctx->stream, ctx->hold_producer, ctx->wait_polls);
     if (r < 0) return fail(ctx, VLB_ERR_CUDA, "tensor map encoding failed for the BF16 projection");
     return VLB_OK;
   }
-  void* part = nullptr;
-  const size_t pb = vlbk::project_partial_bytes(nprobes, S, K);
-  if (pb) {
-    vlb_status st = scratch(ctx, part_name, pb, &part);
-    if (st) return st;
-  }
-  KScope k(ctx, "project_bf16", pb ? 2 : 1);
+  KScope k(ctx, "project_bf16", part ? 2 : 1);
   vlbk::launch_project_bf16_simt(rad, nprobes, S, dirs->d_basis16, K, out, static_cast<float*>(part), split ? 1 : 0,
                                  ctx->stream);
   return VLB_OK;
@@ -1118,17 +1116,23 @@ static vlb_status project_bf16(vlb_ctx* ctx, const uint16_t* rad, uint32_t nprob
 
 // FP32 tile projection (k_project; few-row tiles split along the samples).
 static vlb_status project_f32(vlb_ctx* ctx, const float* rad, uint32_t nprobes, const vlb_dirset* dirs, uint32_t K,
-                              float* out, const char* part_name = "project_partial") {
-  void* part = nullptr;
-  const size_t pb = vlbk::project_partial_bytes(nprobes, dirs->n, K);
-  if (pb) {
-    vlb_status st = scratch(ctx, part_name, pb, &part);
-    if (st) return st;
-  }
-  KScope k(ctx, "project_f32", pb ? 2 : 1);
+                              float* out, void* part) {
+  KScope k(ctx, "project_f32", part ? 2 : 1);
   vlbk::launch_project_f32(rad, nprobes, dirs->n, dirs->d_basis16, K, out, static_cast<float*>(part), ctx->stream,
                            ctx->d_err, ctx->num_sms, ctx->hold_producer, ctx->wait_polls);
   return VLB_OK;
+}
+
+// The projection of a tile (bf16; split: hi/lo pairs; else FP32) with its scratch.
+static vlb_status project_tile(vlb_ctx* ctx, const void* rad, uint32_t nprobes, const vlb_dirset* dirs, uint32_t K,
+                               float* out, bool bf16, bool split) {
+  void* part = nullptr;
+  if (const size_t pb = project_part_bytes(rad, nprobes, dirs, K, bf16, split)) {
+    const vlb_status st = scratch(ctx, "project_partial", pb, &part);
+    if (st) return st;
+  }
+  return bf16 ? project_bf16(ctx, static_cast<const uint16_t*>(rad), nprobes, dirs, K, out, split, part)
+              : project_f32(ctx, static_cast<const float*>(rad), nprobes, dirs, K, out, part);
 }
 
 // Common part of a bake launch: validated parameters -> trace arguments,
@@ -1543,12 +1547,7 @@ static vlb_status bake_once(vlb_ctx* ctx, const vlb_scene* scene, const float* p
       KScope k(ctx, "trace_tile");
       vlbk::launch_trace_tile(a, ctx->num_sms, ctx->stream);
     }
-    if (bf16) {
-      if ((st = project_bf16(ctx, a.radiance_bf16, nprobes, p->dirs, K, static_cast<float*>(ob.dev), split)))
-        return st;
-    } else if ((st = project_f32(ctx, a.radiance, nprobes, p->dirs, K, static_cast<float*>(ob.dev)))) {
-      return st;
-    }
+    if ((st = project_tile(ctx, tile, nprobes, p->dirs, K, static_cast<float*>(ob.dev), bf16, split))) return st;
   }
   if (p->flags & VLB_BAKE_REF_ACCUMULATE) {
     KScope k(ctx, "probe_prefix");
@@ -1657,6 +1656,7 @@ struct BatchBufs {
   uint32_t* sort;      // 4 x rows
   uint8_t* tile;
   float* out;          // rows x V
+  void* project;       // split sums of the projections, one group after another
   float* partial;      // fused: chunk partials
   float* sub;          // fused, chunks split: sub-batch sums
   uint32_t* done;      // fused: rows chunk tickets
@@ -1759,15 +1759,12 @@ static vlb_status batch_enqueue(vlb_ctx* ctx, const BatchPlan& pl, const BatchBu
     if (pl.fused) break;  // the fused walk wrote the projected rows
     float* out = bb.out + g.row0 * V;
     const uint32_t n = uint32_t(g.rows);
-    if (pl.bf16) {
-      vlb_status st = project_bf16(ctx, reinterpret_cast<const uint16_t*>(bb.tile + g.tile_off), n, g.dirs, pl.K, out,
-                                   pl.split, "batch_project_partial");
-      if (st) return st;
-    } else {
-      vlb_status st = project_f32(ctx, reinterpret_cast<const float*>(bb.tile + g.tile_off), n, g.dirs, pl.K, out,
-                                  "batch_project_partial");
-      if (st) return st;
-    }
+    const uint8_t* rad = bb.tile + g.tile_off;
+    void* part = project_part_bytes(rad, n, g.dirs, pl.K, pl.bf16, pl.split) ? bb.project : nullptr;
+    const vlb_status st =
+        pl.bf16 ? project_bf16(ctx, reinterpret_cast<const uint16_t*>(rad), n, g.dirs, pl.K, out, pl.split, part)
+                : project_f32(ctx, reinterpret_cast<const float*>(rad), n, g.dirs, pl.K, out, part);
+    if (st) return st;
   }
   if (bb.ndev_out) {
     KScope k(ctx, "scatter_rows");
@@ -1894,6 +1891,12 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
   if (pl.split)  // the split basis is built before anything is enqueued (or captured)
     for (const auto& g : pl.groups)
       if ((st = dirset_split_basis(ctx, g.dirs))) return st;
+  size_t project_bytes = 0;
+  for (const auto& g : pl.groups)
+    if (!pl.fused)
+      project_bytes = std::max(project_bytes, project_part_bytes(bb.tile + g.tile_off, uint32_t(g.rows), g.dirs, K,
+                                                                 pl.bf16, pl.split));
+  if (project_bytes && (st = scratch(ctx, "batch_project_partial", project_bytes, &bb.project))) return st;
   auto& table = ctx->batch_table;
   table.assign(ntable, vlbk::BakeJobDev{});
   size_t poff = 0, part_off = 0, sub_off = 0, nmaps = 0;
@@ -2002,7 +2005,8 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
                                uint64_t(uintptr_t(counter)), uint64_t(ctx->num_sms), pl.fused,
                                uint64_t(uintptr_t(part)), uint64_t(uintptr_t(done)), pl.rows, sc.ctas_per_sm,
                                sc.node_steps, sc.refill_idle, bb.front_total, bb.front_cap, bb.map_ctas,
-                               uint64_t(uintptr_t(bb.maps)), bb.map_bytes, uint64_t(uintptr_t(bb.sub))};
+                               uint64_t(uintptr_t(bb.maps)), bb.map_bytes, uint64_t(uintptr_t(bb.sub)),
+                               uint64_t(uintptr_t(bb.project))};
   if (pl.fused && ntable == 1) {  // one job goes to the kernel by value: its fields are part of the shape
     const auto* w = reinterpret_cast<const uint64_t*>(table.data());
     key.insert(key.end(), w, w + sizeof(vlbk::BakeJobDev) / 8);
@@ -2318,13 +2322,8 @@ vlb_status vlb_project(vlb_ctx* ctx, const void* radiance, vlb_dtype dtype, uint
   if ((st = stage_in(ctx, radiance, size_t(nprobes) * 3 * S * eb, "proj_in", &drad))) return st;
   OutBuf ob;
   if ((st = stage_out(ctx, out, size_t(nprobes) * K * 12, "proj_out", &ob))) return st;
-  if (dtype == VLB_DTYPE_F32) {
-    if ((st = project_f32(ctx, static_cast<const float*>(drad), nprobes, dirs, K, static_cast<float*>(ob.dev))))
-      return st;
-  } else if ((st = project_bf16(ctx, static_cast<const uint16_t*>(drad), nprobes, dirs, K,
-                                static_cast<float*>(ob.dev), split))) {
+  if ((st = project_tile(ctx, drad, nprobes, dirs, K, static_cast<float*>(ob.dev), dtype != VLB_DTYPE_F32, split)))
     return st;
-  }
   if ((st = copy_out(ctx, ob))) return st;
   return finish(ctx, ob.host);
 }
