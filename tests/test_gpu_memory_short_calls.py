@@ -97,3 +97,31 @@ def test_batch_that_ran_out_of_memory_runs_later():
         assert np.array_equal(got[0], c.bake(scene, probes, mixed))
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("what", ["scene", "directions", "sky", "cubemap tables"])
+def test_objects_are_made(what):
+    torch = pytest.importorskip("torch")
+    c = vlb.Context(0)
+    try:
+        scene, probes, ds = setup(c)
+        few = c.fibonacci(64)
+        big = vlb.synth_box_scene(5, 6000)
+        cube = vlb.synth_cubemap(4, 512)
+        texels = torch.from_numpy(vlb.synth_cubemap(6, 256)).cuda()
+        out = torch.zeros((16, 3), device="cuda")
+        c.bake(scene, probes, params(few, vlb.PREC_FP32))
+        c.skybox_sh(vlb.synth_cubemap(6, 64), vlb.SKY_CUBEMAP, 64, 64, 3)  # the kernels are loaded
+        with little_memory(torch, 6 << 20):
+            if what == "scene":
+                assert c.scene(*big).device_bytes > 8 << 20
+            elif what == "directions":
+                c.fibonacci(1 << 19)
+            elif what == "sky":
+                c.sky(cube, 512)
+            else:
+                c.skybox_sh(texels, vlb.SKY_CUBEMAP, 256, 256, 3, out=out)
+                c.synchronize()
+                assert torch.isfinite(out).all() and out[0, 0] != 0
+    finally:
+        c.close()

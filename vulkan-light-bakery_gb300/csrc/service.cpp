@@ -331,9 +331,17 @@ bool vlb_service::launch_next(std::unique_lock<std::mutex>& lk) {
         const size_t S = r->params.dirs->n;
         if (x.off == 0) {
           const size_t rays = size_t(r->n) * S;
-          if (cudaMallocAsync(reinterpret_cast<void**>(&s->d_hits), rays * 8, ctx->stream) != cudaSuccess ||
-              cudaMallocAsync(reinterpret_cast<void**>(&s->d_probes), size_t(r->n) * 12, ctx->stream) !=
-                  cudaSuccess ||
+          // memory the batches' extra scratch holds is given to the kept hits
+          auto alloc = [&](void** p, size_t b) {
+            cudaError_t e = cudaMallocAsync(p, b, ctx->stream);
+            if (e == cudaErrorMemoryAllocation) {
+              cudaGetLastError();
+              if (vlbh::give_back_extras(ctx)) e = cudaMallocAsync(p, b, ctx->stream);
+            }
+            return e;
+          };
+          if (alloc(reinterpret_cast<void**>(&s->d_hits), rays * 8) != cudaSuccess ||
+              alloc(reinterpret_cast<void**>(&s->d_probes), size_t(r->n) * 12) != cudaSuccess ||
               cudaMemcpyAsync(s->d_probes, r->probes.data(), size_t(r->n) * 12, cudaMemcpyHostToDevice,
                               ctx->stream) != cudaSuccess) {
             cudaGetLastError();

@@ -85,6 +85,24 @@ static vlb_status with_extras(vlb_ctx* ctx, F&& call) {
   return st;
 }
 
+// cudaMalloc; when memory is short, once more without the extra scratch.
+cudaError_t device_alloc(vlb_ctx* ctx, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && !ctx->extras) {
+    cudaGetLastError();
+    if (drop_extras(ctx)) e = cudaMalloc(p, bytes);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+  }
+  return e;
+}
+template <class T>
+cudaError_t device_alloc(vlb_ctx* ctx, T** p, size_t bytes) {
+  return device_alloc(ctx, reinterpret_cast<void**>(p), bytes);
+}
+
 // Grow-only named scratch buffer owned by the context.
 vlb_status scratch(vlb_ctx* ctx, const char* name, size_t bytes, void** out) {
   auto& b = ctx->scratch[name];
@@ -105,15 +123,11 @@ vlb_status scratch(vlb_ctx* ctx, const char* name, size_t bytes, void** out) {
       want = bytes;
       e = cudaMalloc(&b.p, want);
     }
-    if (e != cudaSuccess && !ctx->extras && drop_extras(ctx)) {
-      cudaGetLastError();
-      e = cudaMalloc(&b.p, want);
-    }
     if (e != cudaSuccess) {
       cudaGetLastError();
-      b.p = nullptr;
-      return fail(ctx, VLB_ERR_OOM, "scratch '%s': cudaMalloc(%zu) failed", name, want);
+      e = device_alloc(ctx, &b.p, want);
     }
+    if (e != cudaSuccess) return fail(ctx, VLB_ERR_OOM, "scratch '%s': cudaMalloc(%zu) failed", name, want);
     b.bytes = want;
   }
   *out = b.p;
@@ -295,9 +309,9 @@ vlb_status dirset_finish(vlb_ctx* ctx, vlb_dirset* d, const std::vector<double>&
       }
     }
   });
-  VLB_CUDA(ctx, cudaMalloc(&d->d_dirs, size_t(n) * sizeof(float4)));
-  VLB_CUDA(ctx, cudaMalloc(&d->d_dinv, size_t(n) * sizeof(float4)));
-  VLB_CUDA(ctx, cudaMalloc(&d->d_basis16, size_t(n) * 16 * sizeof(float)));
+  VLB_CUDA(ctx, device_alloc(ctx, &d->d_dirs, size_t(n) * sizeof(float4)));
+  VLB_CUDA(ctx, device_alloc(ctx, &d->d_dinv, size_t(n) * sizeof(float4)));
+  VLB_CUDA(ctx, device_alloc(ctx, &d->d_basis16, size_t(n) * 16 * sizeof(float)));
   VLB_CUDA(ctx, cudaMemcpy(d->d_dirs, d4.data(), d4.size() * 4, cudaMemcpyHostToDevice));
   VLB_CUDA(ctx, cudaMemcpy(d->d_dinv, i4.data(), i4.size() * 4, cudaMemcpyHostToDevice));
   VLB_CUDA(ctx, cudaMemcpy(d->d_basis16, d->h_basis32.data(), d->h_basis32.size() * 4, cudaMemcpyHostToDevice));
@@ -340,7 +354,7 @@ vlb_status dirset_finish(vlb_ctx* ctx, vlb_dirset* d, const std::vector<double>&
     for (uint32_t s = 0; s < n; ++s) tmp[cnt[(keys[order[s]] >> shift) & 4095u]++] = order[s];
     order.swap(tmp);
   }
-  VLB_CUDA(ctx, cudaMalloc(&d->d_order, size_t(n) * 4));
+  VLB_CUDA(ctx, device_alloc(ctx, &d->d_order, size_t(n) * 4));
   VLB_CUDA(ctx, cudaMemcpy(d->d_order, order.data(), size_t(n) * 4, cudaMemcpyHostToDevice));
   // BF16 basis for the tensor-core projection, transposed [32][pitch]: row k
   // the BF16 rounding of w_s Y_k, row 16 + k the BF16 rounding of the rest
@@ -355,7 +369,7 @@ vlb_status dirset_finish(vlb_ctx* ctx, vlb_dirset* d, const std::vector<double>&
         bt[size_t(16 + k) * d->bt_pitch + s] = bf16_rne(float(b - double(bf16_to_float(hi))));
       }
   });
-  VLB_CUDA(ctx, cudaMalloc(&d->d_bt, bt.size() * 2));
+  VLB_CUDA(ctx, device_alloc(ctx, &d->d_bt, bt.size() * 2));
   VLB_CUDA(ctx, cudaMemcpy(d->d_bt, bt.data(), bt.size() * 2, cudaMemcpyHostToDevice));
   return VLB_OK;
 }
@@ -590,10 +604,8 @@ struct SceneTemp {
   ~SceneTemp() { cudaFree(own); }
   vlb_status get(size_t bytes, void** p) {
     if (bytes <= kSceneScratch) return scratch(ctx, "scene_build", bytes, p);
-    if (cudaMalloc(&own, bytes) != cudaSuccess) {
-      cudaGetLastError();
+    if (device_alloc(ctx, &own, bytes) != cudaSuccess)
       return fail(ctx, VLB_ERR_OOM, "scene workspace of %zu bytes", bytes);
-    }
     *p = own;
     return VLB_OK;
   }
@@ -615,10 +627,8 @@ static vlb_status scene_build(vlb_ctx* ctx, vlb_scene* sc, const float* position
                              size_t(2 * size_t(n) - 1) * 24, slots * 64, size_t(n) * 48, size_t(n) * 16};
     size_t at[7];
     for (int k = 0; k < 7; ++k) { at[k] = part(sizes[k]); sc->bytes += sizes[k]; }
-    if (cudaMalloc(&sc->mem, off) != cudaSuccess) {
-      cudaGetLastError();
+    if (device_alloc(ctx, &sc->mem, off) != cudaSuccess)
       return fail(ctx, VLB_ERR_OOM, "scene allocation failed (%u triangles)", n);
-    }
     auto* m = static_cast<uint8_t*>(sc->mem);
     sc->codes = reinterpret_cast<uint32_t*>(m + at[0]);
     sc->order = reinterpret_cast<uint32_t*>(m + at[1]);
@@ -878,7 +888,7 @@ static vlb_status cube_pair_table(vlb_ctx* ctx, uint32_t n, uint32_t lmax, const
   auto it = ctx->cube_pt.find(key);
   if (it != ctx->cube_pt.end()) { *out = it->second; return VLB_OK; }
   float2* p = nullptr;
-  VLB_CUDA(ctx, cudaMalloc(&p, vlbk::cube_pair_table_bytes(n, lmax)));
+  VLB_CUDA(ctx, device_alloc(ctx, &p, vlbk::cube_pair_table_bytes(n, lmax)));
   {
     KScope k(ctx, "cube_pair_table");
     vlbk::launch_cube_pair_table(p, n, lmax, ctx->stream);
@@ -892,7 +902,7 @@ static vlb_status cube_sa_table(vlb_ctx* ctx, uint32_t n, const float** out) {
   auto it = ctx->cube_sa.find(n);
   if (it != ctx->cube_sa.end()) { *out = it->second; return VLB_OK; }
   float* p = nullptr;
-  VLB_CUDA(ctx, cudaMalloc(&p, size_t(n) * n * 4));
+  VLB_CUDA(ctx, device_alloc(ctx, &p, size_t(n) * n * 4));
   {
     KScope k(ctx, "cube_solid_angle");
     vlbk::launch_cube_solid_angle(p, n, ctx->stream);
@@ -917,7 +927,7 @@ static vlb_status pano_tables_device(vlb_ctx* ctx, uint32_t w, uint32_t h, bool 
       ctx->pano_tab.clear();
     }
     float4* p = nullptr;
-    VLB_CUDA(ctx, cudaMalloc(&p, size_t(h) * 16 + size_t(w) * 8));
+    VLB_CUDA(ctx, device_alloc(ctx, &p, size_t(h) * 16 + size_t(w) * 8));
     KScope k(ctx, "pano_tables");
     vlbk::launch_pano_tables(reinterpret_cast<float2*>(p + h), p, w, h, shift, ctx->stream);
     it = ctx->pano_tab.emplace(key, p).first;
@@ -1015,8 +1025,7 @@ vlb_status vlb_sky_create(vlb_ctx* ctx, const float* cubemap_rgb, uint32_t n, vl
   if (!s) return VLB_ERR_OOM;
   s->ctx = ctx; s->n = n;
   const size_t bytes = size_t(6) * n * n * 12;
-  if (cudaMalloc(&s->d_texels, bytes) != cudaSuccess) {
-    cudaGetLastError();
+  if (device_alloc(ctx, &s->d_texels, bytes) != cudaSuccess) {
     delete s;
     return fail(ctx, VLB_ERR_OOM, "sky allocation");
   }
@@ -1071,7 +1080,7 @@ static vlb_status dirset_split_basis(vlb_ctx* ctx, const vlb_dirset* d) {
       }
   });
   uint16_t* dev = nullptr;
-  VLB_CUDA(ctx, cudaMalloc(&dev, bt.size() * 2));
+  VLB_CUDA(ctx, device_alloc(ctx, &dev, bt.size() * 2));
   const cudaError_t e = cudaMemcpy(dev, bt.data(), bt.size() * 2, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) { cudaFree(dev); return cuda_fail(ctx, e, "split basis upload"); }
   d->bt2_pitch = pitch;
@@ -2072,6 +2081,10 @@ static vlb_status batch_run(vlb_ctx* ctx, const vlb_bake_job* jobs, uint32_t njo
 }
 
 }  // extern "C"
+
+cudaError_t vlbh::device_alloc(vlb_ctx* ctx, void** p, size_t bytes) { return ::device_alloc(ctx, p, bytes); }
+
+bool vlbh::give_back_extras(vlb_ctx* ctx) { return drop_extras(ctx); }
 
 vlb_status vlbh::ctx_finish(vlb_ctx* ctx, bool sync) { return finish(ctx, sync); }
 

@@ -537,6 +537,10 @@ struct JobExt {
 vlb_status batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const JobExt* ext, uint32_t njobs,
                         const vlb_bake_params* params, const vlb_batch_schedule& sc, bool* host_out_any,
                         uint64_t spare_bytes = ~0ull);
+// cudaMalloc that gives the context's extra scratch back when memory is short.
+cudaError_t device_alloc(vlb_ctx* ctx, void** p, size_t bytes);
+// Gives the extra scratch back (waits for the work that uses it); whether there was any.
+bool give_back_extras(vlb_ctx* ctx);
 // Launch-error check, and (sync) stream synchronisation + device error counters.
 vlb_status ctx_finish(vlb_ctx* ctx, bool sync);
 // Collapses the scene's binary traversal tree into the 8-wide quantised tree

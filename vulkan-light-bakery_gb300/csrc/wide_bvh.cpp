@@ -145,8 +145,7 @@ vlb_status vlbh::build_wide(vlb_ctx* ctx, vlb_scene* sc) {
     for (const float4& v : f) wide.push_back(v);
   }
   float4* dev = nullptr;
-  if (cudaMalloc(&dev, wide.size() * sizeof(float4)) != cudaSuccess) {
-    cudaGetLastError();
+  if (device_alloc(ctx, reinterpret_cast<void**>(&dev), wide.size() * sizeof(float4)) != cudaSuccess) {
     return ctx_fail(ctx, VLB_ERR_OOM, "wide tree allocation failed");
   }
   if (cudaMemcpy(dev, wide.data(), wide.size() * sizeof(float4), cudaMemcpyHostToDevice) != cudaSuccess) {
