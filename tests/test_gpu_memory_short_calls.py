@@ -125,3 +125,32 @@ def test_objects_are_made(what):
                 assert torch.isfinite(out).all() and out[0, 0] != 0
     finally:
         c.close()
+
+
+def test_service_keeps_frontiers_within_its_budget():
+    """Frontiers of a large batch do not stay beside kept hits that use the budget up."""
+    torch = pytest.importorskip("torch")
+    c = vlb.Context(0)
+    try:
+        pos, idx, alb = vlb.synth_box_scene(3, 64)
+        scene, ds = c.scene(pos, idx, alb), c.fibonacci(64)
+        n, m, budget = 1 << 18, 1 << 15, 1 << 30
+        probes = np.random.default_rng(9).uniform(0, 1, (n, 3)).astype(np.float32)
+        p = vlb.bake_params(ds, 2, vlb.PREC_FP32, vlb.synth_sun(1))
+        want = c.bake(scene, probes, p)
+        c.bake_batch([(scene, probes[:64], None)], p)  # the kernels are loaded
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info()[0]
+        svc = vlb.Service(c, budget_bytes=budget, lmax=2, precision=vlb.PREC_FP32, slice_probes=0xFFFFFFFF)
+        assert np.array_equal(svc.wait(svc.submit(scene, probes, p))[0], want)  # its lists are cut to fit
+        # the radiance tile, outputs and order of the large batch stay: 904 bytes a probe
+        must = n * (64 * 12 + 12 + 4 + 16 + 108)
+        keep = m * 64 * 8 + m * 12  # a kept set
+        for k in range((budget - m * 1024) // keep):
+            svc.wait(svc.submit(scene, probes[:m], p, keep_hits=True))
+        assert svc.stats()["evictions"] == 0
+        used = free - torch.cuda.mem_get_info()[0]
+        svc.close()
+        assert used < budget + must + (96 << 20)  # the rest: allocation granularity, the stream-ordered pool
+    finally:
+        c.close()

@@ -32,7 +32,9 @@
 //
 // Budget accounting: device bytes of the batches in flight (radiance tile or
 // fused chunk partials, outputs, probe and sort scratch) plus the resident
-// kept sets.
+// kept sets.  Probe frontiers, light maps and split sums, which no result needs,
+// take of the rest: each launch says how much that is, and what earlier batches
+// left beyond it is freed first.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -289,6 +291,8 @@ bool vlb_service::launch_next(std::unique_lock<std::mutex>& lk) {
     else ++qi;
   }
   if (take.empty()) return false;
+  const uint64_t held = set_bytes + flight_bytes + bytes, spare = budget > held ? budget - held : 0;
+  vlbh::trim_batch_extras(ctx, spare);
 
   // jobs (the lock stays held: the worker is the only user of ctx and of the
   // sets' device state; submitters only append to the queue)
@@ -399,10 +403,7 @@ bool vlb_service::launch_next(std::unique_lock<std::mutex>& lk) {
   vlb_bake_params bp = jp[0];
   const vlb_batch_schedule sc{0, 1, 0};
   bool host_out = false;
-  // probe frontiers and sun maps (not needed for the results) stay within what the budget leaves
-  const uint64_t held = set_bytes + flight_bytes + bytes - keep_bytes;
-  vlb_status st = vlbh::batch_launch(ctx, jobs.data(), ext.data(), uint32_t(nj), &bp, sc, &host_out,
-                                     budget > held ? budget - held : 0);
+  vlb_status st = vlbh::batch_launch(ctx, jobs.data(), ext.data(), uint32_t(nj), &bp, sc, &host_out, spare);
   ctx->host_inputs_pending = false;  // pageable inputs were staged before the copies returned
   if (st == VLB_OK) {
     const cudaError_t e1 = cudaMemcpyAsync(bt.h_err, ctx->d_err, vlbk::kErrSlots * sizeof(int), cudaMemcpyDeviceToHost,

@@ -103,8 +103,9 @@ cudaError_t device_alloc(vlb_ctx* ctx, T** p, size_t bytes) {
   return device_alloc(ctx, reinterpret_cast<void**>(p), bytes);
 }
 
-// Grow-only named scratch buffer owned by the context.
-vlb_status scratch(vlb_ctx* ctx, const char* name, size_t bytes, void** out) {
+// Grow-only named scratch buffer owned by the context; it grows to no more than
+// `most` bytes unless more are asked for.
+vlb_status scratch(vlb_ctx* ctx, const char* name, size_t bytes, void** out, size_t most = ~size_t(0)) {
   auto& b = ctx->scratch[name];
   if (b.bytes < bytes) {
     const size_t old = b.bytes;
@@ -116,7 +117,8 @@ vlb_status scratch(vlb_ctx* ctx, const char* name, size_t bytes, void** out) {
     }
     // a buffer that grows grows by half (at most 256 MiB more than asked for): batches
     // of uneven sizes then reach their largest in a few steps, not in one allocation each
-    size_t want = std::max<size_t>(std::max<size_t>(bytes, 256), std::min<size_t>(old + old / 2, bytes + (256u << 20)));
+    size_t want = std::max<size_t>(
+        std::max<size_t>(bytes, 256), std::min<size_t>(std::min<size_t>(old + old / 2, bytes + (256u << 20)), most));
     cudaError_t e = cudaMalloc(&b.p, want);
     if (e != cudaSuccess && want > bytes) {
       cudaGetLastError();
@@ -1786,6 +1788,28 @@ static vlb_status batch_enqueue(vlb_ctx* ctx, const BatchPlan& pl, const BatchBu
 
 }  // extern "C"
 
+// What a batch's extra scratch may take of the bytes it is given: half for the
+// frontiers, a quarter each, at most 256 MiB, for the light maps and the split sums.
+struct ExtraShares {
+  uint64_t front, maps, sub;
+  explicit ExtraShares(uint64_t spare)
+      : front(spare / 2), maps(std::min<uint64_t>(256ull << 20, spare / 4)),
+        sub(std::min<uint64_t>(vlbk::kFusedSubBytes, spare / 4)) {}
+};
+
+void vlbh::trim_batch_extras(vlb_ctx* ctx, uint64_t spare_bytes) {
+  const ExtraShares share(spare_bytes);
+  const std::pair<const char*, uint64_t> limits[] = {
+      {"batch_front", share.front}, {"batch_maps", share.maps}, {"batch_sub", share.sub}};
+  for (const auto& l : limits) {
+    auto it = ctx->scratch.find(l.first);
+    if (it == ctx->scratch.end() || it->second.bytes <= l.second) continue;
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(it->second.p);
+    it->second = {};
+  }
+}
+
 // Enqueues a batch on ctx->stream and returns without waiting.  Host
 // outputs are copied with cudaMemcpyAsync (asynchronous only for pinned
 // memory); *host_out tells whether there were any.  ext (optional, njobs
@@ -1851,8 +1875,10 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
   }
   void *front_ent = nullptr, *front_n = nullptr;
   uint64_t front_at = 0;
+  const ExtraShares share(spare_bytes);
   if (front_probes) {
-    const uint64_t most = std::min<uint64_t>(kFrontEntries, spare_bytes / 64);
+    const uint64_t most =
+        std::min<uint64_t>(kFrontEntries, (share.front - std::min(share.front, front_probes * 4)) / 32);
     // the longest lists are cut until all fit
     for (uint32_t cap = vlbk::kFrontCap; entries > most; cap -= cap / 4) {
       entries = 0;
@@ -1861,7 +1887,7 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
         entries += uint64_t(pl.jobs[i].nprobes) * caps[i];
       }
     }
-    if (!entries || scratch(ctx, "batch_front", entries * 32 + front_probes * 4, &front_ent) != VLB_OK)
+    if (!entries || scratch(ctx, "batch_front", entries * 32 + front_probes * 4, &front_ent, share.front) != VLB_OK)
       caps.assign(ntable, 0);
     else front_n = static_cast<uint8_t*>(front_ent) + entries * 32;
   }
@@ -1877,12 +1903,12 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
       subs += uint64_t(b.nprobes) * t.subs;
     }
     void* sub;
-    if (fused_part(ctx, chunk_items, 0) && subs * V * 4 <= std::min<uint64_t>(vlbk::kFusedSubBytes, spare_bytes / 4) &&
-        scratch(ctx, "batch_sub", subs * V * 4, &sub) == VLB_OK)
+    if (fused_part(ctx, chunk_items, 0) && subs * V * 4 <= share.sub &&
+        scratch(ctx, "batch_sub", subs * V * 4, &sub, share.sub) == VLB_OK)
       bb.sub = static_cast<float*>(sub);
   }
-  if (bb.map_bytes && (bb.map_bytes > std::min<uint64_t>(256ull << 20, spare_bytes / 4) ||
-                       scratch(ctx, "batch_maps", bb.map_bytes, &bb.maps) != VLB_OK))
+  if (bb.map_bytes && (bb.map_bytes > share.maps ||
+                       scratch(ctx, "batch_maps", bb.map_bytes, &bb.maps, share.maps) != VLB_OK))
     bb.map_bytes = 0;
 
   // stage host probes, build the job table

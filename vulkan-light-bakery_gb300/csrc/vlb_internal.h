@@ -541,6 +541,8 @@ vlb_status batch_launch(vlb_ctx* ctx, const vlb_bake_job* jobs, const JobExt* ex
 cudaError_t device_alloc(vlb_ctx* ctx, void** p, size_t bytes);
 // Gives the extra scratch back (waits for the work that uses it); whether there was any.
 bool give_back_extras(vlb_ctx* ctx);
+// Gives back what batches on ctx hold of it beyond their shares of spare_bytes.
+void trim_batch_extras(vlb_ctx* ctx, uint64_t spare_bytes);
 // Launch-error check, and (sync) stream synchronisation + device error counters.
 vlb_status ctx_finish(vlb_ctx* ctx, bool sync);
 // Collapses the scene's binary traversal tree into the 8-wide quantised tree
