@@ -573,11 +573,18 @@ int launch_skybox_sh(const SkyboxArgs& a, bool tma, int num_sms, cudaStream_t s)
   return int(a.slabs_per_map) * kSkyPartialsPerSlab;
 }
 
-// One CTA per map: thread (g, v) adds value v of partials 4g .. 4g + 3 in FP32
-// and every G-th such four in FP64, and the G sums are added in order in FP64
-// (a fixed order for a slab count; FP64 adds run at 1/64 of the FP32 rate, so
-// one per four partials).  The texels of 8-bit maps are summed as integers 0..255
-// and scaled here, in FP64.  One thread per value took 240 us for the 2048
+// The rounding error of s = a + b (Knuth's two-sum; exact for finite s).
+__device__ __forceinline__ float sum_error(float a, float b, float s) {
+  const float t = __fsub_rn(s, a);
+  return __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
+}
+
+// One CTA per map: thread (g, v) adds value v of partials 4g .. 4g + 3, then of
+// every G-th such four, and the G sums are added in order (a fixed order for a
+// slab count).  FP64 adds run at 1/64 of the FP32 rate, so a four is added in FP32
+// with the rounding errors kept beside the sum, and takes one FP64 add; a four whose
+// FP32 sum is not finite takes four.  The texels of 8-bit maps are summed as integers
+// 0..255 and scaled here, in FP64.  One thread per value took 240 us for the 2048
 // partials of a 2048 x 1024 map.
 __global__ void __launch_bounds__(1024) k_sh_finalize(const float* __restrict__ partial, uint32_t slabs,
                                                       uint32_t nvals, double scale, float* __restrict__ out) {
@@ -586,12 +593,20 @@ __global__ void __launch_bounds__(1024) k_sh_finalize(const float* __restrict__ 
   const float* p = partial + size_t(blockIdx.x) * slabs * nvals + v;
   double s = 0.0;
   if (g < G) {
+    float lost = 0.f;
     for (uint32_t j = 4 * g; j < slabs; j += 4 * G) {
       float x[4];
 #pragma unroll
       for (uint32_t k = 0; k < 4; ++k) x[k] = j + k < slabs ? __ldg(p + size_t(j + k) * nvals) : 0.f;
-      s += double((x[0] + x[1]) + (x[2] + x[3]));
+      const float a = __fadd_rn(x[0], x[1]), b = __fadd_rn(x[2], x[3]), t = __fadd_rn(a, b);
+      if (isfinite(t)) {
+        s += double(t);
+        lost += sum_error(x[0], x[1], a) + sum_error(x[2], x[3], b) + sum_error(a, b, t);
+      } else {
+        for (int k = 0; k < 4; ++k) s += double(x[k]);
+      }
     }
+    s += double(lost);
     s_sum[threadIdx.x] = s;
   }
   __syncthreads();
