@@ -13,6 +13,12 @@
 // the order of every sum are functions of the image size, so a map's
 // coefficients are the same alone or in a batch.
 //
+// Sums of FP32 texels are scaled by a power of two (PanoScale) so that no sum of
+// finite ones overflows, although a row is added up before its weight is applied.  A sum
+// over a row segment that holds infinities or NaNs says little about the products
+// with the basis, so such a segment leaves the signs of those products instead
+// (kPanoCode): every coefficient is what adding the products one by one gives.
+//
 // Texel loads need no alignment beyond their own.  One 2048 x 1024 RGBA8 image
 // takes 18.8 us a call, most of it the two launches' latency; with a basis per
 // texel, 2048 partials per value added by one thread and the tables made on the
@@ -25,8 +31,25 @@ namespace {
 
 constexpr int kPanoWarps = 8;
 constexpr uint32_t kPanoSeg = 1024;   // texels of a row segment
-constexpr int kPanoSums = 24;         // floats per segment: [channel][8], the last of each unused
+constexpr int kPanoSums = 24;         // floats per segment: [channel][8], seven sums and a code
+// The code, an integer: 0, or for a channel with texels that are not finite bit k:
+// coefficient k gets +inf from one of them, bit 16 + k: -inf (both: NaN).
+constexpr int kPanoCode = 7;
 constexpr int kPanoThreads = 512;
+
+// A segment's sums are multiplied by `down`, coefficients by `up`, its reciprocal: a
+// sum times the largest factor of row_coeffs (5) and the row's weight stays finite.
+struct PanoScale {
+  float down = 1.f;
+  double up = 1.0;
+  PanoScale(const SkyboxArgs& a) {
+    if (a.fmt != VLB_TEXEL_RGB32F) return;
+    double most = 16.0 * (a.w < kPanoSeg ? a.w : kPanoSeg);
+    const double weight = 2.0 * 3.1415926538 / a.w * (3.1415926538 / a.h);
+    if (weight > 1.0) most *= weight;
+    while (up < most) { up *= 2.0; down *= 0.5f; }
+  }
+};
 
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   uint64_t d;
@@ -48,10 +71,33 @@ __device__ __forceinline__ void load_rgb(const void* __restrict__ texels, size_t
   }
 }
 
+// The code of channel c of a segment with texels that are not finite (one warp):
+// their products with the weighted basis, as the texel-by-texel kernel forms them.
+template <int LMAX>
+__device__ __noinline__ uint32_t pano_code(const float* __restrict__ row_texels, const float2* __restrict__ col_tab,
+                                           const float4 rw, bool pano, uint32_t x0, uint32_t x1, int c) {
+  uint32_t code = 0;
+  for (uint32_t x = x0 + (threadIdx.x & 31); x < x1; x += 32) {
+    const float t = __ldg(row_texels + 3 * size_t(x) + c);
+    if (isfinite(t)) continue;
+    const float2 cs = __ldg(col_tab + x);
+    const float dx = rw.x * cs.x, dy = rw.x * cs.y, dz = rw.y;
+    float Y[16];
+    sh_basis<LMAX>(dx, pano ? dz : dy, pano ? dy : dz, Y);
+#pragma unroll
+    for (int k = 0; k < sh_k<LMAX>(); ++k) {
+      const float p = t * (Y[k] * rw.z);
+      if (!(p < 0.f)) code |= 1u << k;
+      if (!(p > 0.f)) code |= 0x10000u << k;
+    }
+  }
+  return __reduce_or_sync(0xffffffffu, code);
+}
+
 // rows: [map][row][segment][kPanoSums].  LMAX 2 leaves the 3 phi sums out.
 template <int LMAX, int FMT>
 __global__ void __launch_bounds__(kPanoWarps * 32) k_pano_rows(const SkyboxArgs a, float* __restrict__ rows,
-                                                               uint32_t nseg, uint32_t units) {
+                                                               uint32_t nseg, uint32_t units, float down) {
   constexpr int M = LMAX == 3 ? 7 : 5;
   const uint32_t lane = threadIdx.x & 31, u = blockIdx.x * kPanoWarps + (threadIdx.x >> 5);
   if (u >= units) return;
@@ -71,13 +117,16 @@ __global__ void __launch_bounds__(kPanoWarps * 32) k_pano_rows(const SkyboxArgs 
     if (two) load_rgb<FMT>(a.texels, at + x + 32, t1);
     const float2 p = __ldg(a.col_tab + x), q = __ldg(a.col_tab + (two ? x + 32 : x));
     const float2 c1 = make_float2(p.x, q.x), s1 = make_float2(p.y, q.y);
-    const float2 one = make_float2(1.f, 1.f), zero = make_float2(0.f, 0.f), neg = make_float2(-1.f, -1.f);
+    const float2 one = make_float2(1.f, 1.f), zero = make_float2(0.f, 0.f);
     const float2 two_c = fma2(c1, one, c1);
-    const float2 c2 = fma2(two_c, c1, neg), s2 = fma2(two_c, s1, zero);  // cos 2phi = 2 cos^2 - 1, sin 2phi
-    float2 f[7] = {one, c1, s1, c2, s2, zero, zero};
+    // times `down`, a power of two: the texels' scale, exact here as on them
+    const float d = FMT == 0 ? down : 1.f;
+    const float2 f0 = make_float2(d, d), f1 = FMT == 0 ? fma2(c1, f0, zero) : c1, f2 = FMT == 0 ? fma2(s1, f0, zero) : s1;
+    const float2 c2 = fma2(two_c, f1, make_float2(-d, -d)), s2 = fma2(two_c, f2, zero);  // cos 2phi = 2 cos^2 - 1, sin 2phi
+    float2 f[7] = {f0, f1, f2, c2, s2, zero, zero};
     if constexpr (M == 7) {
-      f[5] = fma2(two_c, c2, make_float2(-c1.x, -c1.y));  // cos 3phi = 2 cos phi cos 2phi - cos phi
-      f[6] = fma2(two_c, s2, make_float2(-s1.x, -s1.y));
+      f[5] = fma2(two_c, c2, make_float2(-f1.x, -f1.y));  // cos 3phi = 2 cos phi cos 2phi - cos phi
+      f[6] = fma2(two_c, s2, make_float2(-f2.x, -f2.y));
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -91,7 +140,16 @@ __global__ void __launch_bounds__(kPanoWarps * 32) k_pano_rows(const SkyboxArgs 
   for (int i = 0; i < 32; ++i) v[i] = i / 8 < 3 && i % 8 < M ? acc[i / 8 < 3 ? i / 8 : 0][i % 8 < M ? i % 8 : 0].x +
                                                                   acc[i / 8 < 3 ? i / 8 : 0][i % 8 < M ? i % 8 : 0].y
                                                             : 0.f;
-  const float s = warp_sums<32>(v);
+  float s = warp_sums<32>(v);
+  if constexpr (FMT == 0) {
+    const unsigned bad = __ballot_sync(0xffffffffu, lane < kPanoSums && !isfinite(s));
+    for (int c = 0; bad && c < 3; ++c) {
+      if (!(bad >> (8 * c) & 0xffu)) continue;
+      const uint32_t code = pano_code<LMAX>(static_cast<const float*>(a.texels) + 3 * at, a.col_tab,
+                                            __ldg(a.row_tab + row % a.h), a.layout == VLB_SKY_PANORAMA, x0, x1, c);
+      if (lane == uint32_t(8 * c + kPanoCode)) s = __uint_as_float(code);
+    }
+  }
   if (lane < kPanoSums) rows[size_t(u) * kPanoSums + lane] = s;
 }
 
@@ -151,9 +209,12 @@ __constant__ double c_sh[16] = {0.282095, 0.488603, 0.488603, 0.488603, 1.092548
 // texels multiply the FP64 sum, so neither is rounded to FP32.
 template <int LMAX, bool PANO>
 __global__ void __launch_bounds__(kPanoThreads) k_pano_combine(const SkyboxArgs a, const float* __restrict__ rows,
-                                                               uint32_t nseg, float* __restrict__ out) {
+                                                               uint32_t nseg, double up, float* __restrict__ out) {
   constexpr int K = sh_k<LMAX>();
   __shared__ float s_sum[kPanoThreads / 32][3][16];
+  __shared__ uint32_t s_code[3];
+  if (threadIdx.x < 3) s_code[threadIdx.x] = 0;
+  __syncthreads();
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, map = blockIdx.x;
   float acc[3][16];
 #pragma unroll
@@ -168,9 +229,13 @@ __global__ void __launch_bounds__(kPanoThreads) k_pano_combine(const SkyboxArgs 
     for (int i = 0; i < kPanoSums; ++i) f[i] = 0.f;
     for (uint32_t g = 0; g < nseg; ++g)
 #pragma unroll
-      for (int i = 0; i < kPanoSums / 4; ++i) {
-        const float4 x = __ldg(r + g * (kPanoSums / 4) + i);
-        f[4 * i] += x.x; f[4 * i + 1] += x.y; f[4 * i + 2] += x.z; f[4 * i + 3] += x.w;
+      for (int c = 0; c < 3; ++c) {
+        const float4 x = __ldg(r + g * (kPanoSums / 4) + 2 * c), y = __ldg(r + g * (kPanoSums / 4) + 2 * c + 1);
+        const bool sums = __float_as_uint(y.w) == 0;
+        if (!sums) atomicOr(&s_code[c], __float_as_uint(y.w));
+        const float v[7] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z};
+#pragma unroll
+        for (int i = 0; i < 7; ++i) f[8 * c + i] += sums ? v[i] : 0.f;
       }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -190,7 +255,9 @@ __global__ void __launch_bounds__(kPanoThreads) k_pano_combine(const SkyboxArgs 
     const int k = int(tid) / 3, c = int(tid) - 3 * k;
     double s = 0.0;
     for (int w = 0; w < kPanoThreads / 32; ++w) s += double(s_sum[w][c][k]);
-    s *= a.fmt == VLB_TEXEL_RGBA8 ? c_sh[k] / 255.0 : c_sh[k];
+    s *= a.fmt == VLB_TEXEL_RGBA8 ? c_sh[k] / 255.0 : c_sh[k] * up;
+    if (s_code[c] >> k & 1u) s += INFINITY;
+    if (s_code[c] >> (16 + k) & 1u) s -= INFINITY;
     const int co = a.flags & VLB_SKY_REF_BGRA_SWAP ? 2 - c : c;
     out[(size_t(map) * K + k) * 3 + co] = float(s);
   }
@@ -200,10 +267,15 @@ template <int LMAX>
 void launch(const SkyboxArgs& a, float* rows, float* out, cudaStream_t s) {
   const uint32_t nseg = (a.w + kPanoSeg - 1) / kPanoSeg, units = a.count * a.h * nseg;
   const uint32_t grid = (units + kPanoWarps - 1) / kPanoWarps;
-  if (a.fmt == VLB_TEXEL_RGB32F) k_pano_rows<LMAX, 0><<<grid, kPanoWarps * 32, 0, s>>>(a, rows, nseg, units);
-  else k_pano_rows<LMAX, 1><<<grid, kPanoWarps * 32, 0, s>>>(a, rows, nseg, units);
-  if (a.layout == VLB_SKY_PANORAMA) k_pano_combine<LMAX, true><<<a.count, kPanoThreads, 0, s>>>(a, rows, nseg, out);
-  else k_pano_combine<LMAX, false><<<a.count, kPanoThreads, 0, s>>>(a, rows, nseg, out);
+  const PanoScale scale(a);
+  if (a.fmt == VLB_TEXEL_RGB32F)
+    k_pano_rows<LMAX, 0><<<grid, kPanoWarps * 32, 0, s>>>(a, rows, nseg, units, scale.down);
+  else
+    k_pano_rows<LMAX, 1><<<grid, kPanoWarps * 32, 0, s>>>(a, rows, nseg, units, scale.down);
+  if (a.layout == VLB_SKY_PANORAMA)
+    k_pano_combine<LMAX, true><<<a.count, kPanoThreads, 0, s>>>(a, rows, nseg, scale.up, out);
+  else
+    k_pano_combine<LMAX, false><<<a.count, kPanoThreads, 0, s>>>(a, rows, nseg, scale.up, out);
 }
 
 }  // namespace
