@@ -1,11 +1,13 @@
 """Panoramas with texels that are not finite, or beyond the FP32 range once a row of them
-is added up: as the texel-by-texel projection (vlb_skybox_sh_noalloc) has them."""
+is added up: as the texel-by-texel projection (vlb_skybox_sh_noalloc) has them; and
+rows whose sums cancel."""
 import numpy as np
 import pytest
 
 import vlb
 
 pytestmark = pytest.mark.gpu
+PI = 3.1415926538  # shaders/sh_common.h:1
 
 
 def texel_by_texel(torch, image, layout, w, h, lmax):
@@ -56,3 +58,20 @@ def test_texels_whose_row_overflows(ctx, w, h, layout):
     got, ref = ctx.skybox_sh(image, layout, w, h, 3), texel_by_texel(torch, image, layout, w, h, 3)
     assert np.all(np.isfinite(ref)) and np.linalg.norm(got.astype(np.float64) - ref) <= 1e-5 * np.linalg.norm(
         ref.astype(np.float64))
+
+
+@pytest.mark.parametrize("layout", [vlb.SKY_PANORAMA, vlb.SKY_ENVMAP])
+@pytest.mark.parametrize("w,h", [(64, 33), (2048, 1024), (1500, 700), (8192, 4096)])
+def test_rows_that_cancel(ctx, w, h, layout):
+    """Rows of one whole number each: their sums are exact, so the first coefficient is,
+    up to one rounding, an FP64 sum over the rows with the row weights in FP32."""
+    rng = np.random.default_rng(w)
+    c = rng.integers(-1000, 1001, h).astype(np.float64)
+    c = np.where(np.arange(h) < h // 2, c, -c[::-1])
+    th = PI * (np.arange(h) + 0.5) / h
+    weight = np.float32((2.0 * PI / w) * (PI / h) * np.sin(th)).astype(np.float64)
+    terms = 0.282095 * weight * (c * w)
+    image = np.broadcast_to(np.float32(c)[:, None, None], (h, w, 3)).copy()
+    got = ctx.skybox_sh(image, layout, w, h, 3)[0]
+    ref = terms.sum()
+    assert np.all(np.abs(got - ref) <= 2.0**-23 * abs(ref) + 2.0**-45 * np.abs(terms).sum())

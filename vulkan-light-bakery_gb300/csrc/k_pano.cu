@@ -7,7 +7,7 @@
 // cos, sin of phi, 2 phi and 3 phi -- instead of sixteen, and no basis per texel:
 //   k_pano_rows     one warp per row segment: the sums, texels in pairs by packed
 //                   FMAs, reduced across the warp; 84 bytes per 1024 texels
-//   k_pano_combine  one CTA per map: the rows' sums into coefficients
+//   k_pano_combine  one cluster per map: the rows' sums into coefficients
 // The reference adds every texel's 48 products into 48 floats with an
 // unsynchronised read-modify-write (skybox_sh.comp:39).  Here the segments and
 // the order of every sum are functions of the image size, so a map's
@@ -20,9 +20,11 @@
 // (kPanoCode): every coefficient is what adding the products one by one gives.
 //
 // Texel loads need no alignment beyond their own.  One 2048 x 1024 RGBA8 image
-// takes 18.8 us a call, most of it the two launches' latency; with a basis per
+// takes 16.8 us a call, most of it the two launches' latency; with a basis per
 // texel, 2048 partials per value added by one thread and the tables made on the
 // host it took 256 us.
+#include <cooperative_groups.h>
+
 #include "vlb_device.cuh"
 #include "vlb_internal.h"
 
@@ -35,7 +37,7 @@ constexpr int kPanoSums = 24;         // floats per segment: [channel][8], seven
 // The code, an integer: 0, or for a channel with texels that are not finite bit k:
 // coefficient k gets +inf from one of them, bit 16 + k: -inf (both: NaN).
 constexpr int kPanoCode = 7;
-constexpr int kPanoThreads = 512;
+constexpr int kPanoThreads = 128;
 
 // A segment's sums are multiplied by `down`, coefficients by `up`, its reciprocal: a
 // sum times the largest factor of row_coeffs (5) and the row's weight stays finite.
@@ -204,63 +206,113 @@ __device__ __forceinline__ void row_coeffs(float s, float c, const float* f, flo
 __constant__ double c_sh[16] = {0.282095, 0.488603, 0.488603, 0.488603, 1.092548, 1.092548, 0.315392, 1.092548,
                                 0.546274, 0.590044, 2.890611, 0.457046, 0.373176, 0.457046, 1.445306, 0.590044};
 
-// One CTA per map: a thread takes every kPanoThreads-th row, the warps' sums are
-// added in FP64 in warp order; the basis' constants and the 1 / 255 of 8-bit
-// texels multiply the FP64 sum, so neither is rounded to FP32.
+// warp_sums of 16 values v + e, e what rounding took from v: lane l < 16 ends with the
+// sum of v[l] and e[l].
+__device__ __forceinline__ double warp_sums_kept(float (&v)[16], float (&e)[16]) {
+  const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+  for (int n = 16; n >= 1; n /= 2) {  // first the lane 16 away, all values; then half of the values less a step
+    const bool up = n < 16 && (lane & n);
+    const int m = n < 16 ? n : 16;
+#pragma unroll
+    for (int i = 0; i < m; ++i) {
+      const int j = n < 16 ? i + n : i;
+      const float sv = up ? v[i] : v[j], se = up ? e[i] : e[j], kv = up ? v[j] : v[i], ke = up ? e[j] : e[i];
+      const float ov = __shfl_xor_sync(0xffffffffu, sv, n), oe = __shfl_xor_sync(0xffffffffu, se, n);
+      v[i] = __fadd_rn(kv, ov);
+      e[i] = __fadd_rn(__fadd_rn(ke, oe), sum_error(kv, ov, v[i]));
+    }
+  }
+  return double(v[0]) + double(e[0]);
+}
+
+// One cluster per map: a thread takes every n-th row segment, n its threads.  Segments
+// are added as the texel-by-texel kernel's partials are, in more than FP32: threads and
+// lanes keep, beside their FP32 sums, what rounding took from the products with the
+// row's weight and from the sums; warps and CTAs are added in FP64, in order.  (FP64
+// adds across the lanes, at 1/64 of the FP32 rate: 256 maps of 256 x 128 at lmax 3 136
+// against 41 us a call.)  The basis' constants and the 1 / 255 of 8-bit texels multiply
+// the FP64 sum, so neither is rounded to FP32.  A cluster has the CTAs that its segments
+// keep busy (pano_ctas): one CTA per map, with FP32 sums, took 18.9 us for 2048 x 1024
+// and 207 us for 8192 x 4096, now 16.8 and 142 us.
 template <int LMAX, bool PANO>
-__global__ void __launch_bounds__(kPanoThreads) k_pano_combine(const SkyboxArgs a, const float* __restrict__ rows,
-                                                               uint32_t nseg, double up, float* __restrict__ out) {
+__global__ void __launch_bounds__(kPanoThreads)
+    k_pano_combine(const SkyboxArgs a, const float* __restrict__ rows, uint32_t nseg, double up,
+                   float* __restrict__ out) {
   constexpr int K = sh_k<LMAX>();
-  __shared__ float s_sum[kPanoThreads / 32][3][16];
+  __shared__ double s_warp[kPanoThreads / 32][48], s_sum[48];
   __shared__ uint32_t s_code[3];
-  if (threadIdx.x < 3) s_code[threadIdx.x] = 0;
+  namespace cg = cooperative_groups;
+  const auto cluster = cg::this_cluster();
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t ctas = cluster.num_blocks(), map = blockIdx.x / ctas, rank = blockIdx.x % ctas, units = a.h * nseg;
+  if (tid < 3) s_code[tid] = 0;
   __syncthreads();
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, map = blockIdx.x;
-  float acc[3][16];
+  float sum[3][K], lost[3][K];
 #pragma unroll
   for (int c = 0; c < 3; ++c)
 #pragma unroll
-    for (int k = 0; k < 16; ++k) acc[c][k] = 0.f;
-  for (uint32_t y = tid; y < a.h; y += kPanoThreads) {
-    const float4 rw = __ldg(a.row_tab + y);  // sin theta, cos theta, weight
-    const float4* r = reinterpret_cast<const float4*>(rows) + (size_t(map) * a.h + y) * nseg * (kPanoSums / 4);
-    float f[kPanoSums];
-#pragma unroll
-    for (int i = 0; i < kPanoSums; ++i) f[i] = 0.f;
-    for (uint32_t g = 0; g < nseg; ++g)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const float4 x = __ldg(r + g * (kPanoSums / 4) + 2 * c), y = __ldg(r + g * (kPanoSums / 4) + 2 * c + 1);
-        const bool sums = __float_as_uint(y.w) == 0;
-        if (!sums) atomicOr(&s_code[c], __float_as_uint(y.w));
-        const float v[7] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z};
-#pragma unroll
-        for (int i = 0; i < 7; ++i) f[8 * c + i] += sums ? v[i] : 0.f;
-      }
+    for (int k = 0; k < K; ++k) sum[c][k] = lost[c][k] = 0.f;
+  for (uint32_t u = rank * kPanoThreads + tid; u < units; u += ctas * kPanoThreads) {
+    const float4 rw = __ldg(a.row_tab + u / nseg);  // sin theta, cos theta, weight
+    const float4* r = reinterpret_cast<const float4*>(rows) + (size_t(map) * units + u) * (kPanoSums / 4);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      float o[16];
-      row_coeffs<LMAX, PANO>(rw.x, rw.y, f + 8 * c, o);
+      const float4 x = __ldg(r + 2 * c), y = __ldg(r + 2 * c + 1);
+      const bool sums = __float_as_uint(y.w) == 0;
+      if (!sums) atomicOr(&s_code[c], __float_as_uint(y.w));
+      float f[7] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z}, o[16];
 #pragma unroll
-      for (int k = 0; k < K; ++k) acc[c][k] = fmaf(rw.z, o[k], acc[c][k]);
+      for (int i = 0; i < 7; ++i) f[i] = sums ? f[i] : 0.f;
+      row_coeffs<LMAX, PANO>(rw.x, rw.y, f, o);
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const float p = __fmul_rn(rw.z, o[k]), t = __fadd_rn(sum[c][k], p);
+        lost[c][k] += __fadd_rn(sum_error(sum[c][k], p, t), __fmaf_rn(rw.z, o[k], -p));
+        sum[c][k] = t;
+      }
     }
   }
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const float s = warp_sums<16>(acc[c]);
-    if (lane < 16) s_sum[warp][c][lane] = s;
+    float v[16], e[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      v[k] = k < K ? sum[c][k < K ? k : 0] : 0.f;
+      e[k] = k < K ? lost[c][k < K ? k : 0] : 0.f;
+    }
+    const double s = warp_sums_kept(v, e);
+    if (lane < 16) s_warp[warp][3 * lane + c] = s;
   }
   __syncthreads();
   if (tid < 3 * K) {
+    double s = 0.0;
+    for (int w = 0; w < kPanoThreads / 32; ++w) s += s_warp[w][tid];
+    s_sum[tid] = s;
+  }
+  cluster.sync();
+  if (rank == 0 && tid < 3 * K) {
     const int k = int(tid) / 3, c = int(tid) - 3 * k;
     double s = 0.0;
-    for (int w = 0; w < kPanoThreads / 32; ++w) s += double(s_sum[w][c][k]);
+    uint32_t code = 0;
+    for (uint32_t q = 0; q < ctas; ++q) {
+      s += *cluster.map_shared_rank(&s_sum[tid], q);
+      code |= *cluster.map_shared_rank(&s_code[c], q);
+    }
     s *= a.fmt == VLB_TEXEL_RGBA8 ? c_sh[k] / 255.0 : c_sh[k] * up;
-    if (s_code[c] >> k & 1u) s += INFINITY;
-    if (s_code[c] >> (16 + k) & 1u) s -= INFINITY;
+    if (code >> k & 1u) s += INFINITY;
+    if (code >> (16 + k) & 1u) s -= INFINITY;
     const int co = a.flags & VLB_SKY_REF_BGRA_SWAP ? 2 - c : c;
     out[(size_t(map) * K + k) * 3 + co] = float(s);
   }
+  cluster.sync();  // no CTA leaves while its sums are read
+}
+
+// CTAs of a map's cluster: two row segments a thread keep a CTA busy.
+uint32_t pano_ctas(uint32_t units) {
+  uint32_t n = 1;
+  while (n < 8 && n * kPanoThreads * 2 <= units) n *= 2;
+  return n;
 }
 
 template <int LMAX>
@@ -272,10 +324,18 @@ void launch(const SkyboxArgs& a, float* rows, float* out, cudaStream_t s) {
     k_pano_rows<LMAX, 0><<<grid, kPanoWarps * 32, 0, s>>>(a, rows, nseg, units, scale.down);
   else
     k_pano_rows<LMAX, 1><<<grid, kPanoWarps * 32, 0, s>>>(a, rows, nseg, units, scale.down);
-  if (a.layout == VLB_SKY_PANORAMA)
-    k_pano_combine<LMAX, true><<<a.count, kPanoThreads, 0, s>>>(a, rows, nseg, scale.up, out);
-  else
-    k_pano_combine<LMAX, false><<<a.count, kPanoThreads, 0, s>>>(a, rows, nseg, scale.up, out);
+  cudaLaunchAttribute cluster{};
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = pano_ctas(a.h * nseg);
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(a.count * cluster.val.clusterDim.x);
+  cfg.blockDim = dim3(kPanoThreads);
+  cfg.stream = s;
+  cfg.attrs = &cluster;
+  cfg.numAttrs = 1;
+  if (a.layout == VLB_SKY_PANORAMA) cudaLaunchKernelEx(&cfg, k_pano_combine<LMAX, true>, a, rows, nseg, scale.up, out);
+  else cudaLaunchKernelEx(&cfg, k_pano_combine<LMAX, false>, a, rows, nseg, scale.up, out);
 }
 
 }  // namespace

@@ -573,12 +573,6 @@ int launch_skybox_sh(const SkyboxArgs& a, bool tma, int num_sms, cudaStream_t s)
   return int(a.slabs_per_map) * kSkyPartialsPerSlab;
 }
 
-// The rounding error of s = a + b (Knuth's two-sum; exact for finite s).
-__device__ __forceinline__ float sum_error(float a, float b, float s) {
-  const float t = __fsub_rn(s, a);
-  return __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
-}
-
 // One CTA per map: thread (g, v) adds value v of partials 4g .. 4g + 3, then of
 // every G-th such four, and the G sums are added in order (a fixed order for a
 // slab count).  FP64 adds run at 1/64 of the FP32 rate, so a four is added in FP32

@@ -107,6 +107,12 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+// The rounding error of s = a + b (Knuth's two-sum; exact for finite s).
+__device__ __forceinline__ float sum_error(float a, float b, float s) {
+  const float t = __fsub_rn(s, a);
+  return __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
+}
+
 // Sums N values across the warp, N a power of two up to 32; lane l ends with the
 // sum of v[l % N].  Every step halves the values a lane carries: N - 1
 // shuffles (and log2(32 / N) more), against 5 N of N warp_sums.
