@@ -1283,7 +1283,7 @@ static bool sun_map_plan(const vlb_scene* scene, float3 sun, const float3* light
     k = 1.0 / (near - off);
     drift = off * (k - 1.0 / (far + off));
   }
-  const double margin = scale * 0x1p-17 * k + drift;
+  const double round = scale * 0x1p-17 * k, margin = round + drift;
   const double ext = std::max(hi[0] - lo[0], hi[1] - lo[1]) + 2.0 * (off * k + 4.0 * margin);
   m->cells = cells;
   m->u = make_float3(float(u[0]), float(u[1]), float(u[2]));
@@ -1295,6 +1295,7 @@ static bool sun_map_plan(const vlb_scene* scene, float3 sun, const float3* light
   m->inv = float(kMapSide / ext);
   m->cell = float(ext / kMapSide);
   m->margin = float(margin);
+  m->round = float(round);
   m->dmargin = float(scale * 0x1p-17 * k * k);
   m->G = kMapSide;
   m->point = light ? 1u : 0u;

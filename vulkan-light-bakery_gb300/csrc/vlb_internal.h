@@ -259,7 +259,8 @@ struct SunMap {
   float3 o;          // point light
   float u0, v0;      // origin of cell (0, 0)
   float inv, cell;   // cells per unit, its reciprocal
-  float margin;      // how far a cell is widened
+  float margin;      // how far a cell is widened: round, and a point light's drift
+  float round;       // rounding of a position
   float dmargin;     // rounding of a depth
   uint32_t G;
   uint32_t point;    // 1: seen from the light at o, depth 1 / (distance along s)
