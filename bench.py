@@ -18,7 +18,8 @@ probe sample, directly and with the device's per-ray decisions replayed.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 
-Prints one JSON line.  Under torchrun each rank bakes its own replica of the
+Prints one JSON line of at most 8000 characters on stdout (a longer one was cut by
+its reader), and all that was measured as another on stderr.  Under torchrun each rank bakes its own replica of the
 workload (probes are independent: weak scaling, no data-path collective); the
 max step time over ranks is reported.  `--impl reference` times the FP64 CPU
 restatement (the reference's own bake needs Vulkan ray tracing) on a probe
@@ -347,6 +348,38 @@ def trace_roofline(kname, k_avg_ms, stats, clk, sms, hbm_peak, peaks_measured, P
             "node_tests_per_ray": stats["node_tests_per_ray"], "node_fetches_per_ray": stats["node_fetches_per_ray"]}
 
 
+LINE_LIMIT = 8000
+# the keys that are printed as they are; the others are sections
+LINE_KEYS = ("metric", "metric_full", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better",
+             "scaling", "vs_baseline", "dtype", "data", "config", "timing", "grays_per_s", "grays_incl_shadow_per_s",
+             "latency_ms", "e2e", "gpu_launches", "roofline", "kernels_ms", "cpu_baseline", "clocks")
+SECTION_LESS = ("workload", "note", "peak_source", "l2", "trials", "schedule", "checked", "kernels_ms", "requests",
+                "batches", "relights", "relights_rebaked", "evictions", "wall_s", "max_ms", "bytes_peak")
+SECTION_SHORT = {"roofline": ("kernel", "bound", "frac"), "rel_err_vs_fp64": ("max", "mean"),
+                 "autotune": ("gain_vs_default",)}
+
+
+def printed_line(line):
+    """`line` in at most LINE_LIMIT characters: its sections without the texts, tables and
+    counts of SECTION_LESS, numbers to five digits; the longest are left out, by name,
+    if that is still too long."""
+    def brief(x, keys=None):
+        if isinstance(x, dict):
+            return {k: brief(v, SECTION_SHORT.get(k)) for k, v in x.items()
+                    if k not in SECTION_LESS and (keys is None or k in keys)}
+        if isinstance(x, list):
+            return [brief(v) for v in x]
+        return float(f"{x:.5g}") if isinstance(x, float) else x
+
+    out = {k: line[k] for k in line if k in LINE_KEYS}
+    sections = {k: brief(v) for k, v in line.items() if k not in LINE_KEYS}
+    left_out = []
+    while len(json.dumps({**out, **sections, "left_out": left_out})) > LINE_LIMIT and sections:
+        left_out.append(max(sections, key=lambda k: len(json.dumps(sections[k]))))
+        del sections[left_out[-1]]
+    return {**out, **sections, **({"left_out": left_out} if left_out else {})}
+
+
 def main():
     args = parse()
     rank = int(os.environ.get("RANK", "0"))
@@ -542,7 +575,8 @@ def main():
             / b3["mixed_bf16_hilo_tcgen05"]["ms_per_batch"],
             "c4_served_mixed_vs_sequential_fp32_bakes": s4["served_mixed_vs_plain_fp32"],
             "target": 5.0}
-    print(json.dumps(line), flush=True)
+    print(json.dumps(line), file=sys.stderr, flush=True)
+    print(json.dumps(printed_line(line)), flush=True)
     if dist is not None:
         dist.destroy_process_group()
     return 0
