@@ -299,19 +299,16 @@ def accuracy_vs_fp64(ctx, scene, probes, params, pos, idx, alb, sky, sun, nsampl
 def trace_roofline(kname, k_avg_ms, stats, clk, sms, hbm_peak, peaks_measured, P, ntri, K, C, tile):
     """Roofline of the trace kernel.  It is bound by instruction issue and L1
     throughput (the scene's nodes and triangles stay in L1/L2), not by HBM:
-    `bound` is the issue view, the one measured live, with the L1 view beside
-    (the committed ncu capture shows issue at 75 % and the L1 data stage at
-    64 %).  Issue: the capture's warp instructions per launch over the live
-    launch time, against 4 issue slots/clock/SM.  L1: the node and triangle
-    bytes of the same rays walked from the root (counted by an instrumented
-    bake; the bake's own walks start at probe frontiers and look most shadow
-    rays up in a map, so they request fewer) over the live launch time, against
-    the nominal 128 B/clock/SM.  The HBM view (algorithmic DRAM bytes) is kept
-    beside."""
+    `bound` is the issue view, the one measured live (the committed ncu capture
+    shows issue at 75 % and the L1 data stage at 64 %).  Issue: the capture's warp
+    instructions per launch over the live launch time, against 4 issue
+    slots/clock/SM.  `l1` is the capture's utilisation; the bytes beside it are those
+    of the same rays walked from the root (counted by an instrumented bake), which
+    the timed walks, started at probe frontiers and spared most shadow rays, do not
+    request: they give no rate.  The HBM view (algorithmic DRAM bytes) is kept
+    beside, and stands in for a kernel without a capture."""
     mhz = clk.get("sm_max_mhz") or 2070.0
     secs = k_avg_ms * 1e-3 if k_avg_ms > 0 else None
-    l1_bytes = stats["bytes"]
-    l1_peak = sms * 128 * mhz * 1e6 / 1e9
     issue_peak = sms * 4 * mhz * 1e6
     ncu = TRACE_NCU.get(kname, {"capture": None, "dram_bytes": None, "warp_instructions": None,
                                 "l1tex_throughput_pct": None, "issue_active_pct": None})
@@ -326,10 +323,8 @@ def trace_roofline(kname, k_avg_ms, stats, clk, sms, hbm_peak, peaks_measured, P
         # partials written and read once, the scene, the direction and basis tables
         dram_alg = (P * (12 + 4 + K * 12 + 4) + (P * C * K * 3 * 4 * 2 if C > 1 else 0) + max(ntri - 1, 0) * 64
                     + ntri * (48 + 16) + NDIRS * (16 + 16 + 4 + 64))
-    l1 = {"achieved": l1_bytes / secs / 1e9 if secs else None, "peak": l1_peak, "unit": "GB/s",
-          "peak_source": f"nominal L1: {sms} SMs x 128 B/clock x {mhz:.0f} MHz (no measured L1 peak); bytes of walks from the root",
-          "requested_bytes_per_launch": l1_bytes}
-    l1["frac"] = l1["achieved"] / l1_peak if l1["achieved"] else None
+    l1 = {"l1tex_throughput_pct": ncu["l1tex_throughput_pct"], "requested_bytes_per_launch": stats["bytes"],
+          "bytes_of": "walks from the root"}
     issue = {"achieved": wi / secs if wi and secs else None, "peak": issue_peak, "unit": "warp instructions/s",
              "warp_instructions_per_launch": wi, "peak_source": f"{sms} SMs x 4 issue slots x {mhz:.0f} MHz"}
     issue["frac"] = issue["achieved"] / issue_peak if issue["achieved"] else None
@@ -337,11 +332,7 @@ def trace_roofline(kname, k_avg_ms, stats, clk, sms, hbm_peak, peaks_measured, P
            "algorithmic_bytes_per_launch": dram_alg,
            "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured)" if peaks_measured else "fallback 6.8 TB/s"}
     hbm["frac"] = hbm["achieved"] / hbm_peak if hbm["achieved"] else None
-    # The issue view is the one measured live (the capture's instructions over
-    # this run's launch time); the L1 data stage (ncu's wavefront throughput,
-    # which the requested bytes understate) is the co-limit and stays beside.
-    main = issue if wi else l1
-    bound = "issue" if main is issue else "l1"
+    main, bound = (issue, "issue") if wi else (hbm, "hbm")
     return {"kernel": kname, "bound": bound, "achieved": main["achieved"], "peak": main["peak"], "unit": main["unit"],
             "frac": main["frac"], "traffic": ncu["dram_bytes"], "avg_launch_ms": k_avg_ms,
             "peak_source": main["peak_source"], "l1": l1, "issue": issue, "hbm": hbm, "ncu": ncu,

@@ -1,5 +1,5 @@
 """The line bench.py prints: short enough for its reader whatever was measured, with
-the contract's keys as they are."""
+the contract's keys as they are, and no rate of work that the timed kernel does not do."""
 import json
 import sys
 from pathlib import Path
@@ -21,3 +21,11 @@ def test_line_is_short_and_keeps_its_keys():
     assert line["section_1"] == {"fused": {"ms": 1.2346}, "runs": [{"p50_ms": 0.12346, "p99_ms": 2.0}]}
     assert line["left_out"] == ["section_400"] and "section_60" in line
     assert bench.printed_line(core) == core
+
+
+def test_roofline_gives_no_rate_of_walks_from_the_root():
+    stats = {"bytes": 1.5e12, "node_tests_per_ray": 58.0, "node_fetches_per_ray": 58.0}
+    for kname, bound in (("trace_tile", "issue"), ("a kernel without a capture", "hbm")):
+        r = bench.trace_roofline(kname, 47.0, stats, {"sm_max_mhz": 2070.0}, 152, 6788.6, True, 262144, 49162, 9, 4, True)
+        assert r["bound"] == bound and 0 < r["frac"] < 1.2
+        assert not {"achieved", "frac", "peak"} & set(r["l1"])
