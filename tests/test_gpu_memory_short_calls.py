@@ -13,6 +13,8 @@ pytestmark = pytest.mark.gpu
 # 65,536 probes: 268 MB of frontiers; 2056 directions make rows of 4112 BF16 values,
 # two splits, whose sums take 25 MB at lmax 3
 PROBES, S = 65536, 2056
+# a bake that holds all a bake of those takes but split sums: its rows are whole
+WARM_PROBES, WARM_S = 66200, 2040
 
 
 @contextlib.contextmanager
@@ -29,8 +31,8 @@ def little_memory(torch, left):
 
 def setup(c):
     pos, idx, alb = vlb.synth_box_scene(3, 64)
-    probes = np.random.default_rng(9).uniform(0, 1, (PROBES, 3)).astype(np.float32)
-    return c.scene(pos, idx, alb), probes, c.fibonacci(S)
+    probes = np.random.default_rng(9).uniform(0, 1, (WARM_PROBES, 3)).astype(np.float32)
+    return c.scene(pos, idx, alb), probes[:PROBES], c.fibonacci(S), (probes, c.fibonacci(WARM_S))
 
 
 def params(ds, precision):
@@ -43,8 +45,8 @@ def test_split_projection_of_a_bake_keeps_its_bits():
     for short in (False, True):
         c = vlb.Context(0)
         try:
-            scene, probes, ds = setup(c)
-            c.bake(scene, probes, params(ds, vlb.PREC_FP32))  # a tile of the same size, the frontiers
+            scene, probes, ds, warm = setup(c)
+            c.bake(scene, warm[0], params(warm[1], vlb.PREC_FP32))
             c.bake(scene, probes[:64], params(ds, vlb.PREC_MIXED))
             with little_memory(torch, 12 << 20) if short else contextlib.nullcontext():
                 got.append(c.bake(scene, probes, params(ds, vlb.PREC_MIXED)))
@@ -60,9 +62,9 @@ def test_split_projection_of_a_batch_keeps_its_bits():
     for short in (False, True):
         c = vlb.Context(0)
         try:
-            scene, probes, ds = setup(c)
+            scene, probes, ds, warm = setup(c)
             mixed = params(ds, vlb.PREC_MIXED)
-            c.bake_batch([(scene, probes, None)], params(ds, vlb.PREC_FP32))
+            c.bake_batch([(scene, warm[0], None)], params(warm[1], vlb.PREC_FP32))
             c.bake_batch([(scene, probes[:64], None)], mixed)
             with little_memory(torch, 12 << 20) if short else contextlib.nullcontext():
                 got.append(c.bake_batch([(scene, probes, None)], mixed)[0])
@@ -82,11 +84,13 @@ def test_batch_that_ran_out_of_memory_runs_later():
     try:
         # few triangles and many jobs: no frontiers and no light maps that could be given back
         scene = c.scene(*vlb.synth_box_scene(3, 2))
-        probes = np.random.default_rng(9).uniform(0, 1, (PROBES, 3)).astype(np.float32)
+        warm = np.random.default_rng(9).uniform(0, 1, (WARM_PROBES, 3)).astype(np.float32)
+        probes = warm[:PROBES]
         jobs = [(scene, part, None) for part in np.array_split(probes, 600)]
         ds = c.fibonacci(S)
         mixed = params(ds, vlb.PREC_MIXED)
-        c.bake_batch(jobs, params(ds, vlb.PREC_FP32))
+        c.bake_batch([(scene, part, None) for part in np.array_split(warm, 600)],
+                     params(c.fibonacci(WARM_S), vlb.PREC_FP32))
         c.bake_batch([(scene, probes[:64], None)], mixed)
         with little_memory(torch, 12 << 20):
             with pytest.raises(vlb.VlbError) as e:
@@ -104,7 +108,7 @@ def test_objects_are_made(what):
     torch = pytest.importorskip("torch")
     c = vlb.Context(0)
     try:
-        scene, probes, ds = setup(c)
+        scene, probes, ds, _ = setup(c)
         few = c.fibonacci(64)
         big = vlb.synth_box_scene(5, 6000)
         cube = vlb.synth_cubemap(4, 512)

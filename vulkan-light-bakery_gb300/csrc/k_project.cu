@@ -10,8 +10,8 @@
 // thread's copies are all in flight at once; rows padded to 65 words so the
 // per-thread column walk is bank-conflict free), and the matching 64 x 16
 // basis block is read as warp-wide broadcasts.  Each row's sum runs in FP32
-// over its samples in a fixed order, so the result does not depend on the
-// launch shape or on other probes in the tile.
+// over its samples (or over splits of a fixed length of them) in a fixed order, so
+// the result does not depend on the launch shape or on other probes in the tile.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -102,42 +102,36 @@ __device__ __forceinline__ void project_stage(const T* __restrict__ rad, uint32_
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// Launch grid: row tiles x sample splits.  A tile of few rows and many
-// samples (the reference's 343 probes x 3.14 M samples: 9 row tiles) is split
-// along the samples so that about kProjSplitCtas CTAs run; each split sums its
-// range in FP32 in order and k_project_reduce adds the splits in FP64 in
-// split order.  The split count depends on the tile's shape only, so results
-// stay deterministic; tiles with enough rows (C1, C2) run unsplit, one
-// sequential FP32 sum per row.
-constexpr uint32_t kProjSplitCtas = 304;
+// Launch grid: row tiles x sample splits.  Rows of 2048 samples and more are split:
+// each split sums its range in FP32 in order and k_project_reduce adds the splits in
+// FP64.  A split's length is a function of the row's length alone, so a probe has the
+// same bits beside any number of others, in a bake, a batch or a slice.  It is
+// short enough for one probe to fill the GPU (the reference's 3.14 M samples: 456
+// splits; 149,331: 292), and long enough that the sums of a tile of many rows cost
+// little beside the tile (at 512 samples 3 % of its bytes each way at K = 16).  Calls,
+// with split counts by the tile's shape and by the row's length: 1 probe x 149,331
+// samples 46.8 and 43.8 us, 343 x 149,332 184 and 179, 2000 x 149,332 788 and 818,
+// 20,000 x 8192 614 and 415, x 2048 161 and 147.
+constexpr uint32_t kProjSplitCtas = 456;      // three CTAs per SM
 constexpr uint32_t kProjMinSplitSamples = 16 * kProjCols;
-// Longer rows are split down to half of that: a CTA of a few rows waits on its
-// loads stage after stage (6 rows x 149,331 samples: 62 us before, 49 with the sums below in parallel).
-constexpr uint32_t kProjLong = 16384;
-
-//
-// Tiles of at least kProjStream samples stream through the TMA-staged kernel:
-// there the unit is a 256-row tile and a split, three CTAs per SM.
+constexpr uint32_t kProjLong = 16384;         // from here down to half of that
+// Split tiles of at least kProjStream samples stream through the TMA-staged kernel
+// (there the unit is a 256-row tile and a split).
 constexpr size_t kProjStream = size_t(1) << 24;
-constexpr uint32_t kProjStreamUnits = 456;
 
-static uint32_t project_splits(uint32_t rows, uint32_t S, uint32_t* per) {
-  const uint32_t tiles = (rows + kProjRows - 1) / kProjRows, tiles256 = (rows + 255) / 256;
-  uint32_t splits = 1;
-  if (size_t(rows) * S >= kProjStream && S % 4 == 0 && tiles < kProjSplitCtas)
-    splits = std::max(1u, std::min(kProjStreamUnits / tiles256, S / kProjMinSplitSamples));
-  else if (tiles && tiles < kProjSplitCtas)
-    splits = std::max(1u, std::min((kProjSplitCtas + tiles - 1) / tiles,
-                                   S / (S < kProjLong ? kProjMinSplitSamples : kProjMinSplitSamples / 2)));
-  uint32_t p = (S + splits - 1) / splits;
-  p = (p + kProjCols - 1) / kProjCols * kProjCols;  // whole stages
+static uint32_t project_splits(uint32_t S, uint32_t* per) {
+  uint32_t p = S;
+  if (S >= 2 * kProjMinSplitSamples) {
+    p = std::max(S < kProjLong ? kProjMinSplitSamples : kProjMinSplitSamples / 2, (S + kProjSplitCtas - 1) / kProjSplitCtas);
+    p = (p + kProjCols - 1) / kProjCols * kProjCols;  // whole stages
+  }
   *per = p;
   return p ? (S + p - 1) / p : 1;
 }
 
 size_t project_partial_bytes(uint32_t nprobes, uint32_t S, uint32_t K) {
   uint32_t per;
-  const uint32_t splits = project_splits(nprobes * 3, S, &per);
+  const uint32_t splits = project_splits(S, &per);
   return splits > 1 ? size_t(splits) * nprobes * 3 * K * sizeof(float) : 0;
 }
 
@@ -188,30 +182,36 @@ __global__ void __launch_bounds__(kProjRows) k_project(const T* __restrict__ rad
 }
 
 // out (probe, k, channel) = the splits' partials of (row, k) added in FP64: warp
-// g of a CTA takes 32 outputs' splits g, g + 32, ... and the warps' sums are
-// added in order (a fixed order for a split count).  One thread per output took
-// 30 us for the 145 splits of 6 rows.
+// g of a CTA's `groups` takes 32 outputs' splits g, g + groups, ... and the warps'
+// sums are added in order (a fixed order for a split count).  One thread per output
+// took 30 us for the 145 splits of 6 rows.  A CTA has at least eight warps, with few
+// splits of several 32 outputs (20,000 probes x 2048 samples, two splits: 180 us a call
+// with one warp a CTA and 4-byte stores of the sums, 147 so).
 __global__ void __launch_bounds__(1024) k_project_reduce(const float* __restrict__ partial, uint32_t splits,
-                                                         uint32_t rows, uint32_t K, float* __restrict__ out) {
+                                                         uint32_t groups, uint32_t rows, uint32_t K,
+                                                         float* __restrict__ out) {
   __shared__ double s_sum[32][32];
-  const uint32_t lane = threadIdx.x & 31, g = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
-  const uint32_t groups = blockDim.x >> 5;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = warp % groups;
+  const uint32_t i = (blockIdx.x * (blockDim.x / 32 / groups) + warp / groups) * 32 + lane;
   double sum = 0.0;
   if (i < rows * K)
 #pragma unroll 4
     for (uint32_t y = g; y < splits; y += groups) sum += double(__ldg(partial + size_t(y) * rows * K + i));
-  s_sum[g][lane] = sum;
-  __syncthreads();
+  if (groups > 1) {
+    s_sum[warp][lane] = sum;
+    __syncthreads();
+    for (uint32_t w = 1; g == 0 && w < groups; ++w) sum += s_sum[warp + w][lane];
+  }
   if (g || i >= rows * K) return;
-  for (uint32_t w = 1; w < groups; ++w) sum += s_sum[w][lane];
   const uint32_t row = i / K, k = i - row * K, p = row / 3, c = row - 3 * p;
   out[(size_t(p) * K + k) * 3 + c] = float(sum);
 }
 
 void launch_project_reduce(const float* partial, uint32_t splits, uint32_t rows, uint32_t K, float* out,
                            cudaStream_t s) {
-  const uint32_t groups = std::min(32u, std::max(1u, (splits + 3) / 4));
-  k_project_reduce<<<(rows * K + 31) / 32, groups * 32, 0, s>>>(partial, splits, rows, K, out);
+  const uint32_t groups = std::min(32u, std::max(1u, (splits + 3) / 4)), sets = std::max(1u, 8 / groups);
+  const uint32_t warps = (rows * K + 31) / 32;
+  k_project_reduce<<<(warps + sets - 1) / sets, groups * sets * 32, 0, s>>>(partial, splits, groups, rows, K, out);
 }
 
 template <typename T>
@@ -221,8 +221,7 @@ static void launch_project(const T* rad, uint32_t nprobes, uint32_t S, const flo
   const uint32_t tiles = (rows + kProjRows - 1) / kProjRows;
   if (tiles == 0) return;
   uint32_t per = 0;
-  const uint32_t splits = S ? project_splits(rows, S, &per) : 1;
-  if (!S) per = 0;
+  const uint32_t splits = project_splits(S, &per);
   const dim3 grid(tiles, splits);
   if (K == 9) k_project<T, 9><<<grid, kProjRows, 0, s>>>(rad, rows, S, per, basis16, out, partial, split);
   else k_project<T, 16><<<grid, kProjRows, 0, s>>>(rad, rows, S, per, basis16, out, partial, split);
@@ -237,10 +236,10 @@ void launch_project_f32(const float* radiance, uint32_t nprobes, uint32_t S, con
   // 7.63 ms here, 3.34 there, 57 % of the HBM copy rate)
   uint32_t per = 0;
   const uint32_t rows = nprobes * 3;
-  const uint32_t splits = S ? project_splits(rows, S, &per) : 1;
+  const uint32_t splits = project_splits(S, &per);
   if (err && num_sms && S && (splits == 1 || size_t(rows) * S >= kProjStream) &&
-      launch_project_f32_tma(radiance, nprobes, S, basis16, K, out, partial, splits, splits == 1 ? S : per, err,
-                             num_sms, s, hold, wait_polls)) {
+      launch_project_f32_tma(radiance, nprobes, S, basis16, K, out, partial, splits, per, err, num_sms, s, hold,
+                             wait_polls)) {
     if (splits > 1) launch_project_reduce(partial, splits, rows, K, out, s);
     return;
   }

@@ -393,11 +393,19 @@ __global__ void __launch_bounds__(kF32Threads) k_project_f32_tma(const __grid_co
       const uint32_t in = tid + 128 * h, row = tile * tile_rows + in;
       if (in < tile_rows && row < rows) {
         const uint32_t p = row / 3, ch = row - 3 * p;
+        float* part = partial + (size_t(split) * rows + row) * K;
+        if (K % 4 == 0 && splits > 1) {
+#pragma unroll
+          for (int k = 0; k < K / 4; ++k)
+            reinterpret_cast<float4*>(part)[k] =
+                make_float4(acc[h][2 * k].x, acc[h][2 * k].y, acc[h][2 * k + 1].x, acc[h][2 * k + 1].y);
+          continue;
+        }
 #pragma unroll
         for (int k = 0; k < K; ++k) {
           const float v = k & 1 ? acc[h][k / 2].y : acc[h][k / 2].x;
           if (splits == 1) out[(size_t(p) * K + k) * 3 + ch] = v;
-          else partial[(size_t(split) * rows + row) * K + k] = v;
+          else part[k] = v;
         }
       }
     }
@@ -474,7 +482,7 @@ int launch_project_f32_tma(const float* radiance, uint32_t nprobes, uint32_t S, 
       (reinterpret_cast<uintptr_t>(basis16) % 16) ||
       (splits == 1 && (rows + kF32Rows - 1) / kF32Rows < uint32_t(num_sms)))
     return 0;
-  // a split tile has few row tiles: even ones, so that none is nearly empty
+  // split tiles may have few row tiles: even ones, so that none is nearly empty
   const uint32_t ntiles = (rows + kF32Rows - 1) / kF32Rows;
   const uint32_t tile_rows = splits == 1 ? kF32Rows : ((rows + ntiles - 1) / ntiles + 7) / 8 * 8;
   CUtensorMap tm;
