@@ -14,7 +14,7 @@
 // direction, solid angle and basis once and apply it to G = 1-4 maps with packed
 // FP32x2 FMAs; other panoramas and env maps go by rows (k_pano.cu).  Each map's sums are reduced with warp
 // shuffles into partials per (map, slab), and a second kernel adds a map's
-// partials in FP64 in a fixed order.  The slab size does not depend on the
+// partials to FP64 accuracy in a fixed order.  The slab size does not depend on the
 // batch, so a map's result is bit-identical alone or in any batch.
 #include "vlb_device.cuh"
 #include "vlb_internal.h"
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(kSkyThreads) k_skybox_sh(const SkyboxArgs a) {
 // as one float2, so each packed FP32x2 FMA adds both texels' products.  The
 // producer warp streams, per stage, the table chunk and the group's texel
 // chunks (1-D bulk copies into an NST-stage ring).  One partial per (map,
-// slab), added in FP64 by k_sh_finalize: a map's result does not depend on
+// slab), added by k_sh_finalize: a map's result does not depend on
 // the batch or on the map's place in it.
 
 // The pair table: [chunk][k][p] float2 for chunks of kGroupChunk texels;

@@ -191,12 +191,13 @@ static void launch(const TraceArgs& a, int num_sms, cudaStream_t s) {
 
 // ---- lane mode with per-lane ray fetch (tile output) ---------------------------------
 // Persistent warps; every lane runs its own ray through a small state machine
-// -- primary walk, shading, shadow walk, output -- and takes a new ray as
-// soon as it is done (a turn walks nodes until the warp's lanes have each
-// found a leaf, then tests those leaves: lr_node / lr_leaf).  Idle lanes refill
-// together from a global ray counter (one atomic per refill, when half the
-// warp or all of it is idle), so a warp no longer waits for its slowest ray
-// and primary and shadow walks of different rays overlap.  Ray r is
+// -- primary walk, shading, shadow walk, output (a turn walks nodes until the
+// warp's lanes have each found a leaf, then tests those leaves: lr_node /
+// lr_leaf).  The warp shades when all its walks have ended, and takes its next
+// rays from a global counter when all its lanes are done: rays that start
+// together share the nodes around their origin, which gains more than a warp
+// loses by waiting for its slowest walk (refill at 8 to 28 idle lanes: only a
+// scene of few layers gains).  Ray r is
 // (probe slot r / S, direction position r % S): rays fetched together share
 // their origin and take neighbouring directions of the trace order (grouped
 // by octant, then by position on the octant's face), so their walks share

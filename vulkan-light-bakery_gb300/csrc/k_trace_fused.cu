@@ -11,13 +11,12 @@
 // Sub-batches.  A warp cuts its items into sub-batches of up to kSubRays rays
 // and keeps up to kSubBufs in flight in a shared-memory ring (the RGB of each
 // ray).  Idle lanes take the oldest sub-batch's unissued rays first, then the
-// next one's, so lanes that finish early run ahead into the
-// next sub-batch (or the next item) while others finish their walks: a warp
-// waits for a slow ray only when kSubBufs sub-batches are behind it.  Each lane
-// runs the per-lane state machine of the lane walk (primary walk, shading,
-// shadow walk) and writes its ray's RGB into the ring when done.  As in the
-// tile lane walk, a warp does this bookkeeping only when enough of its lanes
-// are idle; the turns in between are pure traversal.
+// next one's.  Each lane runs the per-lane state machine of the lane walk (primary
+// walk, shading, shadow walk) and writes its ray's RGB into the ring when done.  A
+// warp does this bookkeeping only when refill_idle of its lanes are idle; the turns
+// in between are pure traversal.  At 32, the default, it shades and refills as one,
+// as the tile lane walk does; below, lanes that finish early run ahead into the next
+// sub-batch (or the next item) while others finish their walks.
 //
 // Projection.  When the oldest sub-batch is complete the warp projects it:
 // output v = 3k + ch (lane v, and lane v - 32 for v >= 32) sums

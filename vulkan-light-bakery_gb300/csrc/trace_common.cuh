@@ -44,6 +44,7 @@ __device__ __forceinline__ float safe_inv(float d) {
   return 1.0f / (fabsf(d) > 1e-30f ? d : copysignf(1e-30f, d));
 }
 
+// make_ray with the reciprocals of d precomputed (host_safe_inv: the same bits).
 __device__ __forceinline__ void make_ray_inv(RayCtx& r, float ox, float oy, float oz, float dx, float dy, float dz,
                                              float ix, float iy, float iz) {
   r.ox = ox; r.oy = oy; r.oz = oz; r.dx = dx; r.dy = dy; r.dz = dz;
@@ -69,7 +70,6 @@ __device__ __forceinline__ float2 fma_pair(float ax, float ay, float2 b, float2 
   return d;
 }
 
-// make_ray with the reciprocals of d precomputed (host_safe_inv: the same bits).
 // Slab test for a ray in octant OCT (bit a set: 1/d_a < 0).  The octant is
 // the same for every lane of a packet (one direction per packet), so the
 // entry and exit planes of each axis are chosen at compile time and no
@@ -474,8 +474,10 @@ struct LaneRay {
 // best distance (or ends an occluded shadow walk at once): the closest hit is
 // the minimum over all triangles with the same tie rule whatever order they
 // are tested in, and an occluded shadow ray is occluded by any occluder, so
-// every ray's result is unchanged.  A slot is tested only if it is a slot of
-// the current scene (a lane of a batch may change scenes between rays).
+// every ray's result is unchanged (but for what the FP32 test finds outside the
+// box of a triangle seen edge on, which a walk does not test there).  A slot is
+// tested only if it is a slot of the current scene (a lane of a batch may change
+// scenes between rays).
 template <class A>
 __device__ __forceinline__ float lr_try(const A& a, const LaneRay& L, int ts, int* id) {
   ts = VLB_CLAMP(ts, a.ntris, a.err);

@@ -1203,7 +1203,11 @@ static double scene_layers(const vlb_scene* sc) {
 // directions, 64 nodes open a level, lists of 128, 256, 512, 1024: 32,768 probes in 4096 boxes, 130 layers,
 // 6.63, 6.47, 6.48, 6.62 ms; 16,384 probes in 16,384 boxes, 514 layers, 7.33, 5.35,
 // 5.30, 5.33; in 65,536 boxes, 2049 layers, 16.7, 12.3, 8.5, 8.4; in 170,000 boxes
-// 31.4, 24.1, 17.9, 16.3).  whole: the walk does not take the list in stages.
+// 31.4, 24.1, 17.9, 16.3).  Fewer directions share a list's cost among fewer rays, but
+// gain by it too: 16,384 probes x 64 directions in the first three scenes 665, 939,
+// 1604 us by this rule, 656, 952, 1782 with lists of 128 (1066, 1784, 3101 from the
+// root); the best lists there are shorter by half (512 in the third scene: 1396).
+// whole: the walk does not take the list in stages.
 static uint32_t front_list(const vlb_scene* scene, bool whole) {
   uint32_t cap = vlbk::kFrontWhole;
   const double want = 20.0 * std::sqrt(scene_layers(scene));
