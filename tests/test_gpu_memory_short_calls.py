@@ -158,3 +158,20 @@ def test_service_keeps_frontiers_within_its_budget():
         assert used < budget + must + (96 << 20)  # the rest: allocation granularity, the stream-ordered pool
     finally:
         c.close()
+
+
+def test_service_gives_its_frontiers_back():
+    """A batch whose radiance tile fits only without the frontiers of the batch before it."""
+    torch = pytest.importorskip("torch")
+    c = vlb.Context(0)
+    try:
+        scene, probes, _, _ = setup(c)
+        first, second = (vlb.bake_params(c.fibonacci(s), 2, vlb.PREC_FP32, vlb.synth_sun(1)) for s in (64, 128))
+        want = c.bake(scene, probes, second)
+        svc = vlb.Service(c, lmax=2, precision=vlb.PREC_FP32, slice_probes=0xFFFFFFFF)
+        svc.wait(svc.submit(scene, probes, first))
+        with little_memory(torch, 24 << 20):  # the tile grows from 50 to 101 MB
+            assert np.array_equal(svc.wait(svc.submit(scene, probes, second))[0], want)
+        svc.close()
+    finally:
+        c.close()

@@ -58,20 +58,33 @@ bool is_device_ptr(const void* p) {
   return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
 }
 
+// Frees a scratch buffer behind the work that uses it.
+static void free_buf(vlb_ctx* ctx, vlb_ctx::Buf& b) {
+  if (b.pooled) {
+    cudaFreeAsync(b.p, ctx->stream);
+  } else if (b.p) {
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(b.p);
+  }
+  b = {};
+}
+
 // Scratch that only makes a call faster (probe frontiers, light maps, split
 // chunks) or that the next call would make again: given back when device memory
 // runs out, unless the call under way uses it (ctx->extras).
 static bool drop_extras(vlb_ctx* ctx) {
-  bool any = false;
+  bool any = false, pooled = false;
   for (const char* name : {"front", "sun_map", "bake_sub", "batch_front", "batch_maps", "batch_sub", "scene_build"}) {
     auto it = ctx->scratch.find(name);
     if (it == ctx->scratch.end() || !it->second.p) continue;
-    if (!any) cudaStreamSynchronize(ctx->stream);
     any = true;
-    cudaFree(it->second.p);
-    it->second.p = nullptr;
-    it->second.bytes = 0;
+    pooled = pooled || it->second.pooled;
+    free_buf(ctx, it->second);
   }
+  cudaMemPool_t pool;
+  if (pooled && cudaStreamSynchronize(ctx->stream) == cudaSuccess &&
+      cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess)
+    cudaMemPoolTrimTo(pool, 0);
   return any;
 }
 
@@ -104,22 +117,21 @@ cudaError_t device_alloc(vlb_ctx* ctx, T** p, size_t bytes) {
 }
 
 // Grow-only named scratch buffer owned by the context; it grows to no more than
-// `most` bytes unless more are asked for.
-vlb_status scratch(vlb_ctx* ctx, const char* name, size_t bytes, void** out, size_t most = ~size_t(0)) {
+// `most` bytes unless more are asked for.  pooled: from the stream-ordered pool, so
+// that growing and giving back wait for nothing (all users on ctx->stream, none of
+// them a captured graph).
+vlb_status scratch(vlb_ctx* ctx, const char* name, size_t bytes, void** out, size_t most = ~size_t(0),
+                   bool pooled = false) {
   auto& b = ctx->scratch[name];
   if (b.bytes < bytes) {
     const size_t old = b.bytes;
-    if (b.p) {
-      cudaStreamSynchronize(ctx->stream);
-      cudaFree(b.p);
-      b.p = nullptr;
-      b.bytes = 0;
-    }
+    free_buf(ctx, b);
     // a buffer that grows grows by half (at most 256 MiB more than asked for): batches
     // of uneven sizes then reach their largest in a few steps, not in one allocation each
     size_t want = std::max<size_t>(
         std::max<size_t>(bytes, 256), std::min<size_t>(std::min<size_t>(old + old / 2, bytes + (256u << 20)), most));
-    cudaError_t e = cudaMalloc(&b.p, want);
+    cudaError_t e = pooled ? cudaMallocAsync(&b.p, want, ctx->stream) : cudaMalloc(&b.p, want);
+    b.pooled = pooled && e == cudaSuccess;
     if (e != cudaSuccess && want > bytes) {
       cudaGetLastError();
       want = bytes;
@@ -1808,10 +1820,7 @@ void vlbh::trim_batch_extras(vlb_ctx* ctx, uint64_t spare_bytes) {
       {"batch_front", share.front}, {"batch_maps", share.maps}, {"batch_sub", share.sub}};
   for (const auto& l : limits) {
     auto it = ctx->scratch.find(l.first);
-    if (it == ctx->scratch.end() || it->second.bytes <= l.second) continue;
-    cudaStreamSynchronize(ctx->stream);
-    cudaFree(it->second.p);
-    it->second = {};
+    if (it != ctx->scratch.end() && it->second.bytes > l.second) free_buf(ctx, it->second);
   }
 }
 
@@ -1881,6 +1890,8 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
   void *front_ent = nullptr, *front_n = nullptr;
   uint64_t front_at = 0;
   const ExtraShares share(spare_bytes);
+  // a service frees and allocates these as its budget fills, between batches in flight
+  const bool pooled = ctx->parent && !sc.graph;
   if (front_probes) {
     const uint64_t most =
         std::min<uint64_t>(kFrontEntries, (share.front - std::min(share.front, front_probes * 4)) / 32);
@@ -1892,7 +1903,7 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
         entries += uint64_t(pl.jobs[i].nprobes) * caps[i];
       }
     }
-    if (!entries || scratch(ctx, "batch_front", entries * 32 + front_probes * 4, &front_ent, share.front) != VLB_OK)
+    if (!entries || scratch(ctx, "batch_front", entries * 32 + front_probes * 4, &front_ent, share.front, pooled) != VLB_OK)
       caps.assign(ntable, 0);
     else front_n = static_cast<uint8_t*>(front_ent) + entries * 32;
   }
@@ -1909,11 +1920,11 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
     }
     void* sub;
     if (fused_part(ctx, chunk_items, 0) && subs * V * 4 <= share.sub &&
-        scratch(ctx, "batch_sub", subs * V * 4, &sub, share.sub) == VLB_OK)
+        scratch(ctx, "batch_sub", subs * V * 4, &sub, share.sub, pooled) == VLB_OK)
       bb.sub = static_cast<float*>(sub);
   }
   if (bb.map_bytes && (bb.map_bytes > share.maps ||
-                       scratch(ctx, "batch_maps", bb.map_bytes, &bb.maps, share.maps) != VLB_OK))
+                       scratch(ctx, "batch_maps", bb.map_bytes, &bb.maps, share.maps, pooled) != VLB_OK))
     bb.map_bytes = 0;
 
   // stage host probes, build the job table

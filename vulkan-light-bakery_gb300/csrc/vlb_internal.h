@@ -571,7 +571,7 @@ struct vlb_ctx {
   std::vector<cudaEvent_t> event_pool;
   struct Stat { uint32_t launches = 0; double ms = 0; };
   std::map<std::string, Stat> stats;
-  struct Buf { void* p = nullptr; size_t bytes = 0; };
+  struct Buf { void* p = nullptr; size_t bytes = 0; bool pooled = false; };
   std::map<std::string, Buf> scratch;
   bool extras = false;  // the call under way uses the scratch that memory shortage gives back
   std::map<uint32_t, float*> cube_sa;  // solid-angle tables by face size
