@@ -573,13 +573,14 @@ int launch_skybox_sh(const SkyboxArgs& a, bool tma, int num_sms, cudaStream_t s)
   return int(a.slabs_per_map) * kSkyPartialsPerSlab;
 }
 
-// One CTA per map: thread (g, v) adds value v of partials 4g .. 4g + 3, then of
-// every G-th such four, and the G sums are added in order (a fixed order for a
-// slab count).  FP64 adds run at 1/64 of the FP32 rate, so a four is added in FP32
-// with the rounding errors kept beside the sum, and takes one FP64 add; a four whose
-// FP32 sum is not finite takes four.  The texels of 8-bit maps are summed as integers
-// 0..255 and scaled here, in FP64.  One thread per value took 240 us for the 2048
-// partials of a 2048 x 1024 map.
+// One CTA per map: thread (g, v) adds value v of partials 16 g .. 16 g + 15, then of
+// every G-th such sixteen, and the G sums are added in order (a fixed order for a slab
+// count).  FP64 adds and conversions run at 1/64 of the FP32 rate, so a thread adds in
+// FP32, keeps beside the sum what rounding takes, and makes one FP64 number of both
+// (1024 maps of 96 partials 216 us a call, 223 with one per four partials); if the sum is not finite, it adds again in FP64.
+// The texels of 8-bit maps are summed as integers 0..255 and scaled here, in FP64.  One
+// thread per value took 240 us for the 2048 partials of a 2048 x 1024 map.
+constexpr uint32_t kFinalizePer = 16;
 __global__ void __launch_bounds__(1024) k_sh_finalize(const float* __restrict__ partial, uint32_t slabs,
                                                       uint32_t nvals, double scale, float* __restrict__ out) {
   __shared__ double s_sum[1024];
@@ -587,20 +588,26 @@ __global__ void __launch_bounds__(1024) k_sh_finalize(const float* __restrict__ 
   const float* p = partial + size_t(blockIdx.x) * slabs * nvals + v;
   double s = 0.0;
   if (g < G) {
-    float lost = 0.f;
-    for (uint32_t j = 4 * g; j < slabs; j += 4 * G) {
-      float x[4];
+    float sum = 0.f, lost = 0.f;
+    for (uint32_t j = kFinalizePer * g; j < slabs; j += kFinalizePer * G) {
+      float x[kFinalizePer];
 #pragma unroll
-      for (uint32_t k = 0; k < 4; ++k) x[k] = j + k < slabs ? __ldg(p + size_t(j + k) * nvals) : 0.f;
-      const float a = __fadd_rn(x[0], x[1]), b = __fadd_rn(x[2], x[3]), t = __fadd_rn(a, b);
-      if (isfinite(t)) {
-        s += double(t);
-        lost += sum_error(x[0], x[1], a) + sum_error(x[2], x[3], b) + sum_error(a, b, t);
-      } else {
-        for (int k = 0; k < 4; ++k) s += double(x[k]);
+      for (uint32_t k = 0; k < kFinalizePer; ++k) x[k] = j + k < slabs ? __ldg(p + size_t(j + k) * nvals) : 0.f;
+#pragma unroll
+      for (uint32_t k = 0; k < kFinalizePer; k += 4) {
+        const float a = __fadd_rn(x[k], x[k + 1]), b = __fadd_rn(x[k + 2], x[k + 3]), t = __fadd_rn(a, b);
+        const float next = __fadd_rn(sum, t);
+        lost += (sum_error(x[k], x[k + 1], a) + sum_error(x[k + 2], x[k + 3], b)) +
+                (sum_error(a, b, t) + sum_error(sum, t, next));
+        sum = next;
       }
     }
-    s += double(lost);
+    s = double(sum) + double(lost);
+    if (!isfinite(sum)) {
+      s = 0.0;
+      for (uint32_t j = kFinalizePer * g; j < slabs; j += kFinalizePer * G)
+        for (uint32_t k = j; k < min(slabs, j + kFinalizePer); ++k) s += double(__ldg(p + size_t(k) * nvals));
+    }
     s_sum[threadIdx.x] = s;
   }
   __syncthreads();
@@ -611,8 +618,8 @@ __global__ void __launch_bounds__(1024) k_sh_finalize(const float* __restrict__ 
 
 void launch_sh_finalize(const float* partial, uint32_t nmaps, uint32_t slabs, uint32_t nvals, int fmt, float* out,
                         cudaStream_t s) {
-  // four partials a thread, whole warps, at most 1024 threads
-  const uint32_t want = nvals * ((slabs + 3) / 4);
+  // kFinalizePer partials a thread, whole warps, at most 1024 threads
+  const uint32_t want = nvals * ((slabs + kFinalizePer - 1) / kFinalizePer);
   const uint32_t threads = want < 1024 ? (want + 31) / 32 * 32 : 1024;
   k_sh_finalize<<<nmaps, threads, 0, s>>>(partial, slabs, nvals, fmt == VLB_TEXEL_RGBA8 ? 1.0 / 255.0 : 1.0, out);
 }

@@ -124,8 +124,7 @@ int launch_skybox_sh(const SkyboxArgs& a, bool tma, int num_sms, cudaStream_t s)
 void launch_pano_tables(float2* col, float4* row, uint32_t w, uint32_t h, bool shift, cudaStream_t s);
 size_t pano_rows_bytes(uint32_t w, uint32_t h, uint32_t count);
 void launch_pano_sh(const SkyboxArgs& a, float* rows, float* out, cudaStream_t s);
-// out[m][v] = sum_j partial[m][j][v], j in fixed order: fours in FP32 with their
-// rounding errors kept, the rest in FP64.
+// out[m][v] = sum_j partial[m][j][v], j in fixed order, to FP64 accuracy.
 // fmt: the maps' texel format (8-bit texels are scaled by 1 / 255 here).
 void launch_sh_finalize(const float* partial, uint32_t nmaps, uint32_t slabs, uint32_t nvals, int fmt, float* out,
                         cudaStream_t s);
