@@ -1890,8 +1890,14 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
   void *front_ent = nullptr, *front_n = nullptr;
   uint64_t front_at = 0;
   const ExtraShares share(spare_bytes);
-  // a service frees and allocates these as its budget fills, between batches in flight
-  const bool pooled = ctx->parent && !sc.graph;
+  // A service frees and allocates these between batches in flight: while they grow,
+  // and as its budget fills.  From the pool that waits for nothing, but the pool
+  // takes longer to grow by hundreds of MB (80 requests, scenes of up to 2 M
+  // triangles: 1222 a second, 1239 with cudaMalloc), so large ones far from their
+  // share do not come from it.
+  auto pooled = [&](uint64_t bytes, uint64_t most) {
+    return ctx->parent && !sc.graph && (bytes <= (64u << 20) || bytes > most / 4);
+  };
   if (front_probes) {
     const uint64_t most =
         std::min<uint64_t>(kFrontEntries, (share.front - std::min(share.front, front_probes * 4)) / 32);
@@ -1903,7 +1909,9 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
         entries += uint64_t(pl.jobs[i].nprobes) * caps[i];
       }
     }
-    if (!entries || scratch(ctx, "batch_front", entries * 32 + front_probes * 4, &front_ent, share.front, pooled) != VLB_OK)
+    const uint64_t bytes = entries * 32 + front_probes * 4;
+    if (!entries ||
+        scratch(ctx, "batch_front", bytes, &front_ent, share.front, pooled(bytes, share.front)) != VLB_OK)
       caps.assign(ntable, 0);
     else front_n = static_cast<uint8_t*>(front_ent) + entries * 32;
   }
@@ -1920,11 +1928,11 @@ static vlb_status batch_once(vlb_ctx* ctx, const vlb_bake_job* jobs, const vlbh:
     }
     void* sub;
     if (fused_part(ctx, chunk_items, 0) && subs * V * 4 <= share.sub &&
-        scratch(ctx, "batch_sub", subs * V * 4, &sub, share.sub, pooled) == VLB_OK)
+        scratch(ctx, "batch_sub", subs * V * 4, &sub, share.sub, pooled(subs * V * 4, share.sub)) == VLB_OK)
       bb.sub = static_cast<float*>(sub);
   }
-  if (bb.map_bytes && (bb.map_bytes > share.maps ||
-                       scratch(ctx, "batch_maps", bb.map_bytes, &bb.maps, share.maps, pooled) != VLB_OK))
+  if (bb.map_bytes && (bb.map_bytes > share.maps || scratch(ctx, "batch_maps", bb.map_bytes, &bb.maps, share.maps,
+                                                            pooled(bb.map_bytes, share.maps)) != VLB_OK))
     bb.map_bytes = 0;
 
   // stage host probes, build the job table
